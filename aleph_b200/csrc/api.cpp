@@ -1498,7 +1498,7 @@ int aleph_b200_sample_cumulative_noalloc(aleph_b200_handle* h, aleph_b200_state*
   if (!h || !st || (shots && (!variates || !out))) return ALEPH_B200_INVALID_ARGUMENT;
   const size_t sb = sample_scratch_bytes(st->n, ALEPH_B200_SAMPLE_CUMULATIVE, shots);
   const size_t vb = (size_t)shots * 8;
-  const size_t need = al(sb) + 2 * al(vb) + 256;
+  const size_t need = al(sb - sample_chunk_fn_bytes(st->n)) + 2 * al(vb) + 256;
   if (need > kFixedSampleScratchBytes)
     return set_error(h, ALEPH_B200_INVALID_ARGUMENT,
                      "fixed sampling buffer holds %zu bytes; n=%u with %u shots needs %zu (n <= 30 fits up to 65536 shots)",

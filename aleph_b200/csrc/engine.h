@@ -299,6 +299,10 @@ cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t 
 // __device__ array of this many bytes; its address is looked up with
 // cudaGetSymbolAddress, with the target device current.
 constexpr size_t kFixedSampleScratchBytes = (size_t)8 << 20;
+// ... plus room for the chunk functions of the exact resolution, which do not
+// count against that limit: 20 bytes per 2048 amplitudes at n = 28.
+constexpr size_t kFixedChunkFnBytes = (((size_t)1 << kExactCumulativeMaxN) / 2048) * 20 + 4096;
+size_t sample_chunk_fn_bytes(uint32_t n);
 cudaError_t fixed_sample_scratch_address(void** out);
 
 // Split-BF16 hi/lo operand images of a 128x128 real matrix (kernels_block.cu), 64 KiB.

@@ -5,18 +5,22 @@
 //   probabilities p_i = re*re + im*im rounded exactly like the CPU (no FMA),
 //   Vose's table built by AliasTable::build (crates/aleph-sv/src/sampling.rs:104-167)
 //   with the same LIFO stack discipline and the same floating-point operation
-//   order, so the table is bit-identical; the table build's sequential chain
-//   runs on one thread (it is inherently sequential), the O(N) partition and
-//   all draws run in parallel. Draw: index = (word >> 32) & (N-1),
-//   u = (u32)word * 2^-32, u < prob[i] ? i : alias[i] (sampling.rs:179-197).
+//   order, so the table is bit-identical. The build's chain of dependent
+//   additions is evaluated in parallel chunks, exactly (see ALIAS below).
+//   Draw: index = (word >> 32) & (N-1), u = (u32)word * 2^-32,
+//   u < prob[i] ? i : alias[i] (sampling.rs:179-197).
 // CUMULATIVE (the reference's shots <= 1 path, sampling.rs:59-91): the
 //   inverse CDF of the sequential left-to-right prefix sum with strict
 //   `target < cumulative`, zero bins skipped, last positive bin as fallback.
-//   Shots are resolved in parallel on a two-level prefix (tree block sums +
-//   a sequential scan inside the block); a shot whose target lies within the
+//   Shots are resolved by a warp each on a two-level prefix (tree block sums,
+//   then the block added in order); a shot whose target lies within the
 //   rounding bound of a bin boundary is re-resolved against the exact
 //   sequential running sum (for n <= 28), so the outcome equals the
-//   sequential CPU result.
+//   sequential CPU result. The running sum, too, is evaluated in parallel.
+//
+// Measured on B200: alias table and 1024 shots at n = 22 FP64 0.78 ms (234 ms
+// with the chain on one lane); 4096 cumulative shots at n = 26 FP32 1.0 ms (458
+// ms with the sum on one lane).
 
 #include <cmath>
 
@@ -35,26 +39,135 @@ __device__ __forceinline__ double prob_exact(const V2<Real>* amps, uint64_t i) {
 }
 
 // ------------------------------------------------------------------ ALIAS ----
+// Vose's loop (AliasTable::build) is one chain of dependent FP64 steps. With
+// LIFO stacks the element pushed in one step is popped in the next, so the
+// chain has a single state V, the value of the element in hand, and a fixed
+// operand order per stack: smalls a_0, a_1, ... and larges b_0, b_1, ... from
+// the stack tops. V starts as b_0; a step is
+//     V >= 1: pop a_i,  alias[a_i] = current large,          V = fl(V + a_i) - 1
+//     V <  1: pop b_j+1, alias[b_j] = b_j+1, threshold V,    V = fl(V + b_j+1) - 1
+// One lane needs about 57 ns a step (two dependent FP64 adds, a compare and
+// selects): 234 ms for a scrambled n = 22 state. The table must match it bit
+// for bit, and it is built in parallel as follows.
+//
+// * Order. In exact arithmetic V = 1 + E_j - D_i with D_i = sum of the deficits
+//   1 - a of the smalls popped before a_i and E_j = sum of the surpluses b - 1 up
+//   to b_j, so the pops are the merge of the two sorted sequences D and E (small
+//   first on ties). D and E are prefix sums in 64.64 fixed point; the merge is
+//   cut into chunks of about CH steps by binary search (merge path).
+// * Rounding. fl(V + v) - 1 depends on V only through its binade and its low
+//   bits: with S = fl(V + v) in [2^b, 2^(b+1)), moving V by a multiple D of
+//   2^(b+1) units (unit = 2^-52) moves S by exactly D (ties to even included),
+//   as long as S stays in the binade. S >= 2 is also the decision V' >= 1. So a
+//   chunk is run once for each of 32 residues of its start value, one per lane,
+//   around the value that the prefix sums predict; the true start (which differs
+//   by the accumulated rounding, some 1e3 units) has one of these residues, and
+//   the chunk's true end is that lane's end plus the difference, provided the
+//   difference is smaller than the least distance of any S to a binade
+//   boundary (the chunk's margin). Chunks start where V is large (its grid is
+//   coarse there), so that 32 residues cover the binades of the whole chunk.
+// * Composition. 64 chunks compose to one of the same form; one warp then steps
+//   from group to group, checking each condition, and runs what fails one (about
+//   one chunk in 1e8 for a scrambled state, chunks in which V jumps by more than
+//   five binades, and the chain's end) step by step.
+// * A last kernel replays every chunk from its true start and writes the table.
+using u128 = unsigned __int128;
+
 struct AliasScratch {
   double* prob;       // N: scaled probabilities, then the table thresholds
   uint32_t* alias;    // N
-  uint32_t* small;    // N: indices with scaled < 1, ascending
-  uint32_t* large;    // N: indices with scaled >= 1, ascending
-  uint32_t* bcount;   // 2 * nb: per-block small / large counts, then exclusive offsets
-  uint32_t* totals;   // 2: small / large counts
-  double* normsum;    // 2 * nb partial [sum p, non-finite]
+  double* val;        // N: scaled values in pop order, the m smalls, then the k larges
+  uint32_t* idx;      // N: their basis states
+  u128* pre;          // N: D_i of small i (deficits before it), E_j of large j (surpluses up to it)
+  // per partition block: smalls, deficits, surpluses (then what pops before the block), norm partials
+  uint32_t* bcount;
+  u128* bdef;
+  u128* bsur;
+  double* normsum;    // 2 per block: [sum p, non-finite]
+  uint32_t* totals;   // smalls m, larges k, smalls popped, index of the last current large
+  // chunks of the merged order (nc + 1 cuts)
+  uint32_t *ci, *cj;  // smalls popped and current large at the cut
+  double *cbase, *cunit;  // lane r starts at base + r * unit
+  long long* cmargin;     // least distance to a binade boundary, units of 2^-52 (<= 0: not usable)
+  int* cmax;              // exponent of the largest S
+  double* cend;           // 32 per chunk: end values
+  double* cstart;         // true start value
+  uint8_t* cflag;         // 1: replay from cstart (0: its steps were run one by one)
+  // groups of CGROUP chunks, the same form
+  long long* gmargin;
+  double* gend;
+  double* gstart;
+  uint8_t* gflag;
 };
 
 constexpr uint32_t PART_B = 1024;  // elements per partition block
+constexpr uint32_t CH = 256;       // merged steps per chunk: a cut lies within the next 32 steps
+constexpr uint32_t CH_MAX = CH + 31;
+constexpr uint32_t CGROUP = 64;    // chunks per group
+constexpr double kUnits = 4503599627370496.0;  // 2^52
 
+// Chunks of a chain over n elements: the last two chunks' worth of steps stay
+// with the step-by-step walk, which ends where a stack runs empty.
+static inline uint32_t alias_chunks(uint64_t len) { return len > 4 * CH ? (uint32_t)((len - 1 - 2 * CH) / CH) : 0u; }
+
+__device__ __forceinline__ u128 fx_deficit(double a) {  // 1 - a for a in [0, 1), 64 fraction bits
+  return ((u128)1 << 64) - (u128)__double2ull_rd(a * 18446744073709551616.0);
+}
+__device__ __forceinline__ u128 fx_surplus(double b) {  // b - 1 for b >= 1
+  const double x = b - 1.0, f = floor(x);
+  return ((u128)__double2ull_rd(f) << 64) + (u128)__double2ull_rd((x - f) * 18446744073709551616.0);
+}
+__device__ __forceinline__ u128 shfl_up_u128(u128 v, int o) {
+  const unsigned long long lo = __shfl_up_sync(0xffffffffu, (unsigned long long)v, o);
+  const unsigned long long hi = __shfl_up_sync(0xffffffffu, (unsigned long long)(v >> 64), o);
+  return ((u128)hi << 64) | lo;
+}
+// Inclusive prefix over a block of 1024 threads (warp_tot: 32 slots of shared memory).
+template <typename T, typename Up>
+__device__ __forceinline__ T block_scan_1024(T v, T* warp_tot, Up&& up) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const T x = up(v, o);
+    if (lane >= o) v += x;
+  }
+  if (lane == 31) warp_tot[w] = v;
+  __syncthreads();
+  if (w == 0) {
+    T t = warp_tot[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const T x = up(t, o);
+      if (lane >= o) t += x;
+    }
+    warp_tot[lane] = t;
+  }
+  __syncthreads();
+  if (w) v += warp_tot[w - 1];
+  return v;
+}
+__device__ __forceinline__ u128 block_scan_u128(u128 v, u128* tot) {
+  return block_scan_1024<u128>(v, tot, [](u128 x, int o) { return shfl_up_u128(x, o); });
+}
+__device__ __forceinline__ uint32_t block_scan_u32(uint32_t v, uint32_t* tot) {
+  return block_scan_1024<uint32_t>(v, tot, [](uint32_t x, int o) { return __shfl_up_sync(0xffffffffu, x, o); });
+}
+
+// Thread t of block b takes element b * PART_B + (PART_B - 1 - t): ascending
+// threads are the pop order (stacks are filled in ascending index order).
+__device__ __forceinline__ uint64_t part_element() { return (uint64_t)blockIdx.x * PART_B + (PART_B - 1 - threadIdx.x); }
+
+// Scaled values, per-block small counts, deficit / surplus sums and norm partials.
 template <typename Real>
-__global__ void alias_scale_kernel(const V2<Real>* __restrict__ amps, uint64_t len, AliasScratch s) {
-  // one block per PART_B elements: scaled values + per-block small/large counts + norm partials
-  __shared__ uint32_t cs[32], cl[32];
+__global__ void __launch_bounds__(PART_B) alias_scale_kernel(const V2<Real>* __restrict__ amps, uint64_t len,
+                                                             AliasScratch s) {
+  __shared__ uint32_t cs[32];
+  __shared__ u128 sd[32], se[32];
   __shared__ double ns[32], nb[32];
   const double nf = (double)len;
-  const uint64_t i = (uint64_t)blockIdx.x * PART_B + threadIdx.x;
-  uint32_t small = 0, large = 0;
+  const uint64_t i = part_element();
+  bool small = false;
+  u128 d = 0, e = 0;
   double psum = 0.0, bad = 0.0;
   if (i < len) {
     const double p = prob_exact<Real>(amps, i);
@@ -62,241 +175,527 @@ __global__ void alias_scale_kernel(const V2<Real>* __restrict__ amps, uint64_t l
     else psum = p;
     const double sc = __dmul_rn(nf, p);
     s.prob[i] = sc;
-    if (sc < 1.0) small = 1;
-    else large = 1;
+    small = sc < 1.0;
+    if (small) d = fx_deficit(sc);
+    else e = fx_surplus(sc);
   }
-  const unsigned bs = __ballot_sync(0xffffffffu, small), bl = __ballot_sync(0xffffffffu, large);
+  const unsigned bs = __ballot_sync(0xffffffffu, small);
   for (int o = 16; o; o >>= 1) {
     psum += __shfl_down_sync(0xffffffffu, psum, o);
     bad += __shfl_down_sync(0xffffffffu, bad, o);
+    d += ((u128)__shfl_down_sync(0xffffffffu, (unsigned long long)(d >> 64), o) << 64) +
+         (u128)__shfl_down_sync(0xffffffffu, (unsigned long long)d, o);
+    e += ((u128)__shfl_down_sync(0xffffffffu, (unsigned long long)(e >> 64), o) << 64) +
+         (u128)__shfl_down_sync(0xffffffffu, (unsigned long long)e, o);
   }
   const int w = threadIdx.x >> 5;
   if ((threadIdx.x & 31) == 0) {
     cs[w] = __popc(bs);
-    cl[w] = __popc(bl);
     ns[w] = psum;
     nb[w] = bad;
+    sd[w] = d;
+    se[w] = e;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t a = 0, b = 0;
+    uint32_t a = 0;
     double x = 0.0, y = 0.0;
-    for (int k = 0; k < (int)(PART_B / 32); ++k) {
+    u128 dd = 0, ee = 0;
+    for (int k = (int)(PART_B / 32) - 1; k >= 0; --k) {  // ascending element order
       a += cs[k];
-      b += cl[k];
       x += ns[k];
       y += nb[k];
+      dd += sd[k];
+      ee += se[k];
     }
-    s.bcount[2 * blockIdx.x] = a;
-    s.bcount[2 * blockIdx.x + 1] = b;
+    s.bcount[blockIdx.x] = a;
+    s.bdef[blockIdx.x] = dd;
+    s.bsur[blockIdx.x] = ee;
     s.normsum[2 * blockIdx.x] = x;
     s.normsum[2 * blockIdx.x + 1] = y;
   }
 }
 
-// Exclusive scan of the per-block counts (one thread; nb <= 2^18 blocks).
-__global__ void alias_offsets_kernel(AliasScratch s, uint32_t nblocks, double* norm_out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  uint32_t a = 0, b = 0;
+// What pops before each block (blocks pop from the last to the first): counts
+// of smalls, deficits and surpluses; the totals and the norm. One CTA; a
+// thread takes a contiguous range of blocks. (One thread for all of them was
+// 0.7 ms at n = 22.)
+__global__ void __launch_bounds__(1024) alias_offsets_kernel(AliasScratch s, uint64_t len, uint32_t nblocks,
+                                                             double* norm_out) {
+  __shared__ u128 tot[32];
+  __shared__ uint32_t tot32[32];
+  __shared__ double red[2][32];
+  const uint32_t per = (nblocks + 1023) / 1024;
+  const uint32_t q0 = min(nblocks, threadIdx.x * per), q1 = min(nblocks, q0 + per);
+  uint32_t c = 0;
+  u128 d = 0, e = 0;
   double x = 0.0, y = 0.0;
-  for (uint32_t k = 0; k < nblocks; ++k) {
-    const uint32_t ca = s.bcount[2 * k], cb = s.bcount[2 * k + 1];
-    s.bcount[2 * k] = a;
-    s.bcount[2 * k + 1] = b;
-    a += ca;
-    b += cb;
-    x += s.normsum[2 * k];
-    y += s.normsum[2 * k + 1];
+  for (uint32_t q = q0; q < q1; ++q) {
+    const uint32_t b = nblocks - 1 - q;
+    c += s.bcount[b];
+    d += s.bdef[b];
+    e += s.bsur[b];
+    x += s.normsum[2 * b];
+    y += s.normsum[2 * b + 1];
   }
-  s.totals[0] = a;
-  s.totals[1] = b;
-  norm_out[0] = x;
-  norm_out[1] = y;
-}
-
-__global__ void alias_partition_kernel(uint64_t len, AliasScratch s) {
-  __shared__ uint32_t ws[32], wl[32];
-  const uint64_t i = (uint64_t)blockIdx.x * PART_B + threadIdx.x;
-  bool is_small = false, valid = i < len;
-  if (valid) is_small = s.prob[i] < 1.0;
-  const unsigned bs = __ballot_sync(0xffffffffu, valid && is_small);
-  const unsigned bl = __ballot_sync(0xffffffffu, valid && !is_small);
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) {
-    ws[w] = __popc(bs);
-    wl[w] = __popc(bl);
+  const uint32_t ci = block_scan_u32(c, tot32);
+  const u128 di = block_scan_u128(d, tot);
+  __syncthreads();  // tot is reused
+  const u128 ei = block_scan_u128(e, tot);
+  uint32_t rc = ci - c;
+  u128 rd = di - d, re = ei - e;
+  for (uint32_t q = q0; q < q1; ++q) {
+    const uint32_t b = nblocks - 1 - q;
+    const uint32_t cb = s.bcount[b];
+    const u128 db = s.bdef[b], eb = s.bsur[b];
+    s.bcount[b] = rc;
+    s.bdef[b] = rd;
+    s.bsur[b] = re;
+    rc += cb;
+    rd += db;
+    re += eb;
+  }
+  for (int o = 16; o; o >>= 1) {
+    x += __shfl_down_sync(0xffffffffu, x, o);
+    y += __shfl_down_sync(0xffffffffu, y, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = x;
+    red[1][threadIdx.x >> 5] = y;
+  }
+  if (threadIdx.x == 1023) {
+    s.totals[0] = ci;
+    s.totals[1] = (uint32_t)(len - ci);
+    s.totals[2] = 0;
+    s.totals[3] = 0;
   }
   __syncthreads();
-  uint32_t os = s.bcount[2 * blockIdx.x], ol = s.bcount[2 * blockIdx.x + 1];
-  for (int k = 0; k < w; ++k) {
-    os += ws[k];
-    ol += wl[k];
-  }
-  const unsigned below = (1u << lane) - 1u;
-  if (valid) {
-    if (is_small) s.small[os + __popc(bs & below)] = (uint32_t)i;
-    else s.large[ol + __popc(bl & below)] = (uint32_t)i;
+  if (threadIdx.x == 0) {
+    double a = 0.0, b = 0.0;
+    for (int w = 0; w < 32; ++w) {
+      a += red[0][w];
+      b += red[1][w];
+    }
+    norm_out[0] = a;
+    norm_out[1] = b;
   }
 }
 
-// The Vose loop of AliasTable::build, one warp.
-//
-// With LIFO stacks, the element pushed in one step is popped in the next: a
-// large whose residual stays >= 1 is the next large, one that drops below 1
-// is the next small. So that element lives in lane 0's registers, and the
-// stacks themselves are only ever popped: their entries below the top, and
-// the scaled values of those entries, are read-only until popped. The warp
-// therefore streams them into shared-memory buffers ahead of the chain
-// (descending stack order), and lane 0 runs the dependent chain out of
-// shared memory with the reference's operation order,
-//   alias[s] = l, threshold[s] = value(s), value(l) = (value(l) + value(s)) - 1.
-// status[0] is set on failure (never expected: the rounds are bounded).
-// Lane 0's step is the add / subtract / compare and selects, without
-// data-dependent branches: the next entry of each buffer sits in registers one
-// step ahead (the buffers carry one spare slot so that this read never leaves
-// them), and each step's outputs (alias[s] = l, threshold[s]) go to a
-// shared-memory record ring that the whole warp scatters to global memory
-// when it fills or a buffer runs dry.
-constexpr int CHAIN_CH = 1024;
-constexpr int REC_CAP = 1024;
-__global__ void __launch_bounds__(32) alias_chain_kernel(uint64_t len, AliasScratch s, int32_t* status) {
-  __shared__ uint32_t sbi[CHAIN_CH + 1], lbi[CHAIN_CH + 1];
-  __shared__ double sbv[CHAIN_CH + 1], lbv[CHAIN_CH + 1];
-  __shared__ uint32_t rec_s[REC_CAP], rec_l[REC_CAP];
-  __shared__ double rec_v[REC_CAP];
-  const int lane = threadIdx.x;
-  if (len == 1) {
-    if (lane == 0) {
-      s.prob[0] = 1.0;
-      s.alias[0] = 0;
-    }
-    return;
+// Values, basis states and prefix sums in pop order.
+__global__ void __launch_bounds__(PART_B) alias_partition_kernel(uint64_t len, AliasScratch s, const int32_t* status) {
+  __shared__ u128 tot[32];
+  __shared__ uint32_t tot32[32];
+  if (status[0] != 0) return;  // not a normalised state: uniform over the grid
+  const uint64_t i = part_element();
+  const bool valid = i < len;
+  const double sc = valid ? s.prob[i] : 0.0;
+  const bool small = valid && sc < 1.0;
+  const u128 d = small ? fx_deficit(sc) : 0, e = valid && !small ? fx_surplus(sc) : 0;
+  const uint32_t rank = block_scan_u32(small ? 1u : 0u, tot32);  // smalls up to this element, in pop order
+  const u128 di = block_scan_u128(d, tot);
+  __syncthreads();
+  const u128 ei = block_scan_u128(e, tot);
+  if (!valid) return;
+  // elements of this block that pop before this one: threadIdx.x less the padding of the last block
+  const uint64_t top = ((uint64_t)blockIdx.x + 1) * PART_B;
+  const uint32_t pad = top > len ? (uint32_t)(top - len) : 0u;
+  const uint32_t m = s.totals[0], sb = s.bcount[blockIdx.x];
+  const uint64_t popped = len > top ? len - top : 0;  // elements of later blocks
+  uint64_t at;
+  if (small) at = sb + rank - 1;
+  else at = m + (popped - sb) + (threadIdx.x - pad - rank);
+  s.val[at] = sc;
+  s.idx[at] = (uint32_t)i;
+  s.pre[at] = small ? s.bdef[blockIdx.x] + di - d : s.bsur[blockIdx.x] + ei;
+}
+
+// Smalls among the first t pops of the merged order; lo..hi brackets the answer.
+__device__ __forceinline__ uint32_t merge_smalls(const AliasScratch& s, uint32_t m, uint32_t t, uint32_t lo, uint32_t hi) {
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    // small mid against large t - mid, whose key is E of the large before it
+    if (s.pre[mid] <= s.pre[(uint64_t)m + (t - 1 - mid)]) lo = mid + 1;
+    else hi = mid;
   }
-  int64_t ts = (int64_t)s.totals[0];  // small entries not yet buffered: small[0..ts)
-  int64_t tl = (int64_t)s.totals[1];  // large entries not yet buffered: large[0..tl)
-  int ns = 0, ps = 0, nl = 0, pl = 0;  // buffer fill / consumed counts (uniform over the warp)
-  bool hs = false, hl = false;         // lane 0: current small / large held in registers
-  uint32_t si = 0, li = 0;
-  double sv = 0.0, lv = 0.0;
-  uint64_t guard = 0;
-  int fail = 0;
-  while (true) {
-    if (ps == ns && ts > 0) {  // refill the small buffer from the stack top
-      const int m = ts < CHAIN_CH ? (int)ts : CHAIN_CH;
-      for (int k = lane; k < m; k += 32) {
-        const uint32_t id = s.small[ts - 1 - k];
-        sbi[k] = id;
-        sbv[k] = s.prob[id];
+  return lo;
+}
+
+// The exponent of x >= 2^-1022 (unbiased).
+__device__ __forceinline__ int exponent_of(double x) {
+  return (int)((__double_as_longlong(x) >> 52) & 0x7ff) - 1023;
+}
+__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+
+// Cut c lies within 32 steps from c * CH, where the predicted V is largest.
+// One warp per cut, a lane per candidate.
+__global__ void __launch_bounds__(128) alias_cuts_kernel(AliasScratch s, uint32_t nc, const int32_t* status) {
+  const uint32_t c = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  const uint32_t m = s.totals[0], k = s.totals[1];
+  if (c > nc || status[0] != 0 || m == 0 || k == 0) return;
+  const uint32_t t0 = c * CH, nl = k - 1;
+  uint32_t i0 = 0;
+  if (lane == 0) i0 = merge_smalls(s, m, t0, t0 > nl ? t0 - nl : 0u, min(t0, m));
+  i0 = __shfl_sync(0xffffffffu, i0, 0);
+  const uint32_t t = c == 0 ? 0u : t0 + lane;
+  const uint32_t i = merge_smalls(s, m, t, max(i0, t > nl ? t - nl : 0u), min(min(t, m), i0 + (t - t0)));
+  const uint32_t j = t - i;
+  // V = 1 + E_j - D_i (D of one small past the last: the running total; such cuts are never used)
+  const __int128 x = (__int128)s.pre[(uint64_t)m + j] - (__int128)(i < m ? s.pre[i] : s.pre[m - 1]);
+  double V = 1.0 + ((double)(long long)(x >> 64) + (double)(unsigned long long)x * 0x1p-64);
+  if (!(V > 0.0)) V = 0.0;
+  double best = V;
+  for (int o = 16; o; o >>= 1) best = fmax(best, __shfl_xor_sync(0xffffffffu, best, o));
+  const unsigned who = __ballot_sync(0xffffffffu, V == best);
+  if (lane != __ffs(who) - 1) return;
+  int g = exponent_of(V + 1.0);  // V is a multiple of ulp(V + 1) after a step
+  if (c == 0) {
+    V = s.val[m];  // the first large itself
+    g = exponent_of(V);
+  }
+  const double unit = pow2(g - 52);
+  s.ci[c] = i;
+  s.cj[c] = j;
+  s.cbase[c] = floor(V / (32.0 * unit)) * (32.0 * unit);
+  s.cunit[c] = unit;
+  s.cflag[c] = 0;
+}
+
+// A chunk's operands in shared memory: its smalls, and the larges after its first one.
+struct ChunkOps {
+  double a[CH_MAX + 1], b[CH_MAX + 1];
+};
+__device__ __forceinline__ void stage_chunk(const AliasScratch& s, uint32_t m, uint32_t i0, uint32_t j0, uint32_t ns,
+                                            uint32_t nl, ChunkOps& o) {
+  const int lane = threadIdx.x & 31;
+  for (uint32_t x = lane; x < ns; x += 32) o.a[x] = s.val[i0 + x];
+  for (uint32_t x = lane; x < nl; x += 32) o.b[x] = s.val[(uint64_t)m + j0 + 1 + x];
+  __syncwarp();
+}
+
+// One warp per chunk, one start residue per lane.
+__global__ void __launch_bounds__(128) alias_spec_kernel(AliasScratch s, uint32_t nc, const int32_t* status) {
+  __shared__ ChunkOps ops[4];
+  const uint32_t c = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  const uint32_t m = s.totals[0], k = s.totals[1];
+  if (c >= nc || status[0] != 0 || m == 0 || k == 0) return;
+  ChunkOps& o = ops[threadIdx.x >> 5];
+  const uint32_t i0 = s.ci[c], j0 = s.cj[c];
+  const uint32_t ns = s.ci[c + 1] - i0, nl = s.cj[c + 1] - j0, len = ns + nl;  // len <= CH_MAX
+  stage_chunk(s, m, i0, j0, ns, nl, o);
+  const double unit = s.cunit[c];
+  double V = s.cbase[c] + (double)lane * unit;
+  const long long one = 1ll << 52;
+  long long margin = (long long)fmin(fabs(V - 1.0) * kUnits, 0x1p60);
+  int smax = 0;
+  uint32_t is = 0, il = 0;
+  double va = o.a[0], vb = o.b[0];
+  for (uint32_t t = 0; t < len; ++t) {
+    const bool small = V >= 1.0;
+    const double S = __dadd_rn(V, small ? va : vb);
+    is += small ? 1u : 0u;
+    il += small ? 0u : 1u;
+    va = o.a[is];  // is, il <= len <= CH_MAX: inside the arrays whatever this lane decided
+    vb = o.b[il];
+    const long long bits = __double_as_longlong(S);
+    const long long mant = bits & (one - 1);
+    const int hi = (int)(bits >> 32);
+    // distance to the binade's ends, at least this many units of 2^-52 (S >= 1 always)
+    long long d = one - mant;
+    if (hi >= 0x40000000) d = min(d, mant);
+    margin = min(margin, d);
+    smax = max(smax, hi);
+    V = __dsub_rn(S, 1.0);
+  }
+  const bool ok = is == ns && il == nl;  // this lane popped what the prefix sums predicted
+  for (int x = 16; x; x >>= 1) {
+    margin = min(margin, __shfl_xor_sync(0xffffffffu, margin, x));
+    smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, x));
+  }
+  const int g = (smax >> 20) - 1023;
+  const bool all = __all_sync(0xffffffffu, ok);
+  s.cend[(size_t)c * 32 + lane] = V;
+  if (lane == 0) {
+    // 32 residues of `unit` fix every rounding up to binade exponent_of(unit) + 52 + 4
+    s.cmargin[c] = all && g <= exponent_of(unit) + 56 ? margin : 0;
+    s.cmax[c] = g;
+  }
+}
+
+// Where the true value V enters a chunk: the lane with its residue and the
+// distance to that lane's start. False when the chunk does not cover V.
+struct Entry {
+  int lane;
+  double shift;
+};
+// A group's chunks are entered within 2^28 units of their lanes, and so is the
+// group itself, so that no chunk of a walked group is further than 2^30 off.
+constexpr long long kMoved = 1ll << 28;
+__device__ __forceinline__ bool enter_chunk(double V, double base, double unit, long long margin, long long max_moved,
+                                            Entry* e, long long* left) {
+  const double q = (V - base) / unit;  // exact: a power of two, and V close to base on its grid
+  if (!(fabs(q) < 0x1p30)) return false;
+  const long long qi = (long long)q;
+  if ((double)qi != q) return false;  // not on this chunk's grid
+  const int r = (int)(qi & 31);
+  const long long D = qi - r;
+  const int g = exponent_of(unit) + 52;
+  if (g < 0 || g > 30) return false;
+  const long long moved = (D < 0 ? -D : D) << g;  // units of 2^-52
+  *left = margin - moved;
+  if (*left <= 0 || moved > max_moved) return false;
+  e->lane = r;
+  e->shift = (double)D * unit;
+  return true;
+}
+
+// One warp per group: lane r follows its chunk-0 start through the group's chunks.
+__global__ void __launch_bounds__(128) alias_compose_kernel(AliasScratch s, uint32_t nc, uint32_t ng,
+                                                            const int32_t* status) {
+  const uint32_t q = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (q >= ng || status[0] != 0 || s.totals[0] == 0 || s.totals[1] == 0) return;
+  const uint32_t c0 = q * CGROUP, c1 = min(nc, c0 + CGROUP);
+  const double unit0 = s.cunit[c0];
+  double V = s.cbase[c0] + (double)lane * unit0;
+  long long margin = 1ll << 60;
+  int g = 0;
+  bool ok = true;
+#pragma unroll 4
+  for (uint32_t c = c0; c < c1; ++c) {
+    const double end = s.cend[(size_t)c * 32 + lane], base = s.cbase[c], unit = s.cunit[c];
+    const long long cm = s.cmargin[c];
+    g = max(g, s.cmax[c]);
+    Entry e{0, 0.0};
+    long long left = 0;
+    if (!enter_chunk(V, base, unit, cm, kMoved, &e, &left)) ok = false;
+    // a start that is D off takes the lane of another residue when D is no
+    // multiple of this chunk's 32 units: up to 31 units further off
+    margin = min(margin, left - (long long)(32.0 * unit * kUnits));
+    V = __shfl_sync(0xffffffffu, end, e.lane) + e.shift;
+  }
+  for (int x = 16; x; x >>= 1) margin = min(margin, __shfl_xor_sync(0xffffffffu, margin, x));
+  const bool all = __all_sync(0xffffffffu, ok);
+  s.gend[(size_t)q * 32 + lane] = V;
+  if (lane == 0) {
+    s.gmargin[q] = all && g <= exponent_of(unit0) + 56 ? margin : 0;
+    s.gflag[q] = 0;
+  }
+}
+
+// The chain one step at a time (lane 0 out of shared memory; the warp stages
+// operands and scatters the records): at most `steps` steps from (V, i, j).
+// Returns false when the chain has ended: the stack it needs is empty.
+constexpr uint32_t RAW = 512;
+struct RawShared {
+  double a[RAW + 1], b[RAW + 1], v[RAW];
+  uint32_t rec[RAW];  // pop: bit 31 set for a large, local index below
+  uint32_t cur[RAW];  // local index of the current large
+};
+__device__ bool raw_steps(const AliasScratch& s, uint32_t m, uint32_t k, RawShared& sh, double& V, uint32_t& i,
+                          uint32_t& j, uint64_t steps) {
+  const int lane = threadIdx.x & 31;
+  for (;;) {
+    if (V >= 1.0 ? i >= m : j + 1 >= k) return false;
+    if (steps == 0) return true;
+    const uint32_t ns = min(RAW, m - i), nl = min(RAW, k - 1 - j);
+    for (uint32_t x = lane; x < ns; x += 32) sh.a[x] = s.val[i + x];
+    for (uint32_t x = lane; x < nl; x += 32) sh.b[x] = s.val[(uint64_t)m + j + 1 + x];
+    __syncwarp();
+    uint32_t is = 0, il = 0, n = 0;
+    if (lane == 0) {
+      const uint32_t lim = steps < RAW ? (uint32_t)steps : RAW;
+      double va = sh.a[0], vb = sh.b[0];
+      while (n < lim) {
+        const bool t = V >= 1.0;
+        if (t ? is >= ns : il >= nl) break;
+        sh.rec[n] = t ? is : (0x80000000u | il);
+        sh.cur[n] = il;
+        sh.v[n] = V;
+        ++n;
+        V = __dsub_rn(__dadd_rn(V, t ? va : vb), 1.0);
+        is += t ? 1u : 0u;
+        il += t ? 0u : 1u;
+        va = sh.a[is];
+        vb = sh.b[il];
       }
-      ts -= m;
-      ns = m;
-      ps = 0;
     }
-    if (pl == nl && tl > 0) {
-      const int m = tl < CHAIN_CH ? (int)tl : CHAIN_CH;
-      for (int k = lane; k < m; k += 32) {
-        const uint32_t id = s.large[tl - 1 - k];
-        lbi[k] = id;
-        lbv[k] = s.prob[id];
+    n = __shfl_sync(0xffffffffu, n, 0);
+    is = __shfl_sync(0xffffffffu, is, 0);
+    il = __shfl_sync(0xffffffffu, il, 0);
+    V = __shfl_sync(0xffffffffu, V, 0);
+    __syncwarp();
+    for (uint32_t x = lane; x < n; x += 32) {
+      const uint32_t r = sh.rec[x], l = s.idx[(uint64_t)m + j + sh.cur[x]];
+      if (r >> 31) {  // the current large fell below 1: it gets the next large
+        s.alias[l] = s.idx[(uint64_t)m + j + sh.cur[x] + 1];
+        s.prob[l] = sh.v[x];
+      } else {
+        s.alias[s.idx[i + r]] = l;
       }
-      tl -= m;
-      nl = m;
-      pl = 0;
     }
     __syncwarp();
-    int done = 0, nrec = 0;
-    if (lane == 0) {
-      if (++guard > 4 * (len / 256) + 64) fail = 1;  // rounds: refills plus ring flushes
-      if (!hs && ps < ns) {
-        si = sbi[ps];
-        sv = sbv[ps];
-        ++ps;
-        hs = true;
+    i += is;
+    j += il;
+    steps -= n;
+  }
+}
+
+// One warp walks the groups with the true value, and what they do not cover
+// chunk by chunk or step by step; then the chain's end.
+constexpr uint32_t WALK = 16;  // records staged at a time
+__global__ void __launch_bounds__(32) alias_walk_kernel(AliasScratch s, uint32_t nc, uint32_t ng, const int32_t* status) {
+  __shared__ RawShared raw;
+  __shared__ double send[WALK][32], sbase[WALK], sunit[WALK];
+  __shared__ long long smargin[WALK];
+  __shared__ uint32_t si[WALK + 1], sj[WALK + 1];
+  const int lane = threadIdx.x;
+  const uint32_t m = s.totals[0], k = s.totals[1];
+  if (status[0] != 0 || m == 0 || k == 0) return;
+  double V = s.val[m];
+  uint32_t i = 0, j = 0;
+  bool more = true;
+  // records [r0, r1) of chunks (per = 1) or groups (per = CGROUP): staged in shared memory
+  auto stage = [&](uint32_t r0, uint32_t n, uint32_t per, const long long* margin, const double* end) {
+    __syncwarp();
+    for (uint32_t x = lane; x <= n; x += 32) {
+      const uint32_t c = min(nc, (r0 + x) * per);
+      si[x] = s.ci[c];
+      sj[x] = s.cj[c];
+      if (x < n) {
+        sbase[x] = s.cbase[c];
+        sunit[x] = s.cunit[c];
+        smargin[x] = margin[r0 + x];
       }
-      if (!hl && pl < nl) {
-        li = lbi[pl];
-        lv = lbv[pl];
-        ++pl;
-        hl = true;
+    }
+    for (uint32_t x = 0; x < n; ++x) send[x][lane] = end[(size_t)(r0 + x) * 32 + lane];
+    __syncwarp();
+  };
+  uint32_t w0 = 0, wn = 0;  // staged groups
+  for (uint32_t g = 0; g < ng && more; ++g) {
+    if (g >= w0 + wn) {
+      w0 = g;
+      wn = min(WALK, ng - g);
+      stage(w0, wn, CGROUP, s.gmargin, s.gend);
+    }
+    const uint32_t x = g - w0;
+    Entry e;
+    long long left;
+    if (i == si[x] && j == sj[x] && enter_chunk(V, sbase[x], sunit[x], smargin[x], kMoved, &e, &left)) {
+      if (lane == 0) {
+        s.gstart[g] = V;
+        s.gflag[g] = 1;
       }
-      if (hs && hl && !fail) {
-        // next entries of each buffer (meaningful while ps < ns / pl < nl)
-        uint32_t nsi = sbi[ps], nli = lbi[pl];
-        double nsv = sbv[ps], nlv = lbv[pl];
-        while (true) {
-          rec_s[nrec] = si;
-          rec_l[nrec] = li;
-          rec_v[nrec] = sv;  // threshold = value of the small
-          ++nrec;
-          const double r = __dsub_rn(__dadd_rn(lv, sv), 1.0);
-          const bool t = r < 1.0;  // the large becomes the next small
-          if (t ? pl >= nl : ps >= ns) {  // its successor is not buffered yet
-            if (t) {
-              si = li;
-              sv = r;
-              hl = false;
-            } else {
-              lv = r;
-              hs = false;
-            }
-            break;
+      V = send[x][e.lane] + e.shift;
+      i = si[x + 1];
+      j = sj[x + 1];
+      continue;
+    }
+    const uint32_t c1 = min(nc, (g + 1) * CGROUP);
+    for (uint32_t c0 = g * CGROUP; c0 < c1 && more; c0 += WALK) {
+      const uint32_t n = min(WALK, c1 - c0);
+      stage(c0, n, 1, s.cmargin, s.cend);
+      for (uint32_t y = 0; y < n && more; ++y) {
+        if (i == si[y] && j == sj[y] && enter_chunk(V, sbase[y], sunit[y], smargin[y], 1ll << 60, &e, &left)) {
+          if (lane == 0) {
+            s.cstart[c0 + y] = V;
+            s.cflag[c0 + y] = 1;
           }
-          const uint32_t si2 = t ? li : nsi, li2 = t ? nli : li;
-          const double sv2 = t ? r : nsv, lv2 = t ? nlv : r;
-          si = si2;
-          li = li2;
-          sv = sv2;
-          lv = lv2;
-          ps += t ? 0 : 1;
-          pl += t ? 1 : 0;
-          nsi = sbi[ps];
-          nsv = sbv[ps];
-          nli = lbi[pl];
-          nlv = lbv[pl];
-          if (nrec == REC_CAP) break;  // the warp flushes the ring first
+          V = send[y][e.lane] + e.shift;
+          i = si[y + 1];
+          j = sj[y + 1];
+        } else {
+          const uint64_t to = (uint64_t)si[y + 1] + sj[y + 1], at = (uint64_t)i + j;
+          if (to > at) more = raw_steps(s, m, k, raw, V, i, j, to - at);
         }
       }
-      done = fail || (!hs && ps == ns && ts == 0) || (!hl && pl == nl && tl == 0);
     }
-    ps = __shfl_sync(0xffffffffu, ps, 0);
-    pl = __shfl_sync(0xffffffffu, pl, 0);
-    done = __shfl_sync(0xffffffffu, done, 0);
-    nrec = __shfl_sync(0xffffffffu, nrec, 0);
-    __syncwarp();
-    for (int k = lane; k < nrec; k += 32) {  // scatter the step records
-      s.alias[rec_s[k]] = rec_l[k];
-      s.prob[rec_s[k]] = rec_v[k];
-    }
-    __syncwarp();
-    if (done) break;
+    wn = 0;  // the chunk records took the place of the group records
   }
+  while (more) more = raw_steps(s, m, k, raw, V, i, j, ~0ull);
   if (lane == 0) {
-    if (fail) {
-      status[0] = ALEPH_B200_DEVICE_FAILURE;
-      return;
-    }
-    // Leftovers, drained below as self-aliases with threshold 1: the stack
-    // entries never popped (still in memory below the buffered ones) plus the
-    // element held in registers, pushed back on its stack.
-    int64_t rs = ts + (ns - ps), rl = tl + (nl - pl);
-    if (hs) s.small[rs++] = si;
-    if (hl) s.large[rl++] = li;
-    s.totals[0] = (uint32_t)rs;
-    s.totals[1] = (uint32_t)rl;
+    s.totals[2] = i;
+    s.totals[3] = j;
   }
 }
 
-__global__ void alias_drain_kernel(AliasScratch s) {
-  const uint32_t ts = s.totals[0], tl = s.totals[1];
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < ts + tl; k += gridDim.x * blockDim.x) {
-    const uint32_t i = k < ts ? s.small[k] : s.large[k - ts];
+// One warp per walked group: the true start of each of its chunks.
+__global__ void __launch_bounds__(128) alias_expand_kernel(AliasScratch s, uint32_t nc, uint32_t ng,
+                                                           int32_t* status) {
+  const uint32_t q = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (q >= ng || status[0] != 0 || s.totals[0] == 0 || s.totals[1] == 0 || !s.gflag[q]) return;
+  const uint32_t c0 = q * CGROUP, c1 = min(nc, c0 + CGROUP);
+  double V = s.gstart[q];
+#pragma unroll 4
+  for (uint32_t c = c0; c < c1; ++c) {
+    const double end = s.cend[(size_t)c * 32 + lane];
+    Entry e{0, 0.0};
+    long long left;
+    const bool in = enter_chunk(V, s.cbase[c], s.cunit[c], s.cmargin[c], 1ll << 60, &e, &left);
+    if (lane == 0) {
+      if (!in) status[0] = ALEPH_B200_DEVICE_FAILURE;  // never: the group's margin covers its chunks
+      s.cstart[c] = V;
+      s.cflag[c] = 1;
+    }
+    V = __shfl_sync(0xffffffffu, end, e.lane) + e.shift;
+  }
+}
+
+// One warp per chunk: replay from the true start, then write its table entries.
+__global__ void __launch_bounds__(128) alias_emit_kernel(AliasScratch s, uint32_t nc, const int32_t* status) {
+  __shared__ ChunkOps ops[4];
+  __shared__ uint16_t cur[4][CH_MAX + 1];
+  const uint32_t c = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  const uint32_t m = s.totals[0], k = s.totals[1];
+  if (c >= nc || status[0] != 0 || m == 0 || k == 0 || !s.cflag[c]) return;
+  ChunkOps& o = ops[threadIdx.x >> 5];
+  uint16_t* cl = cur[threadIdx.x >> 5];  // per small: local index of its large
+  const uint32_t i0 = s.ci[c], j0 = s.cj[c];
+  const uint32_t ns = s.ci[c + 1] - i0, nl = s.cj[c + 1] - j0, len = ns + nl;
+  stage_chunk(s, m, i0, j0, ns, nl, o);
+  if (lane == 0) {
+    double V = s.cstart[c];
+    uint32_t is = 0, il = 0;
+    double va = o.a[0], vb = o.b[0];
+    for (uint32_t t = 0; t < len; ++t) {
+      const bool small = V >= 1.0;
+      const double v = small ? va : vb;
+      if (small) cl[is] = (uint16_t)il;
+      else o.b[il] = V;  // the threshold of large il takes the place of its successor's value, already read
+      is += small ? 1u : 0u;
+      il += small ? 0u : 1u;
+      va = o.a[is];
+      vb = o.b[il];
+      V = __dsub_rn(__dadd_rn(V, v), 1.0);
+    }
+  }
+  __syncwarp();
+  for (uint32_t x = lane; x < ns; x += 32) s.alias[s.idx[i0 + x]] = s.idx[(uint64_t)m + j0 + cl[x]];
+  for (uint32_t x = lane; x < nl; x += 32) {
+    const uint32_t l = s.idx[(uint64_t)m + j0 + x];
+    s.alias[l] = s.idx[(uint64_t)m + j0 + x + 1];
+    s.prob[l] = o.b[x];
+  }
+}
+
+// What was never popped keeps itself with threshold 1, and so does the large in hand.
+__global__ void alias_drain_kernel(AliasScratch s, const int32_t* status) {
+  if (status[0] != 0) return;
+  const uint32_t m = s.totals[0], k = s.totals[1], i0 = s.totals[2], j0 = s.totals[3];
+  const uint64_t n = (uint64_t)(m - i0) + (k - j0);
+  for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t i = s.idx[x < m - i0 ? i0 + x : (uint64_t)m + j0 + (x - (m - i0))];
     s.prob[i] = 1.0;
     s.alias[i] = i;
   }
 }
 
 __global__ void alias_draw_kernel(AliasScratch s, uint64_t mask, const uint64_t* __restrict__ words, uint32_t shots,
-                                  uint64_t* __restrict__ out) {
+                                  uint64_t* __restrict__ out, const int32_t* status) {
+  if (status[0] != 0) return;
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < shots; k += gridDim.x * blockDim.x) {
     const uint64_t bits = words[k];
     const uint64_t i = (bits >> 32) & mask;
@@ -314,6 +713,39 @@ __global__ void check_norm_kernel(const double* norm2, double tol, int32_t* stat
 }
 
 // ------------------------------------------------------------- CUMULATIVE ----
+// A run of S <- fl(S + p) with S in one binade [2^e, 2^(e+1)) adds to S, in
+// units of 2^(e-52), the integer nearest to p; only an exact tie depends on S,
+// through its parity. So a run of additions is a function of the start's
+// parity, two integers, and runs compose: the reference's left-to-right sum is
+// evaluated in parallel, bit for bit, binade by binade. (One lane adding in
+// order took 6.8 ns an element, 459 ms at n = 26.)
+struct SeqFn {
+  long long o0, o1;  // units added to an even / odd start
+};
+__device__ __forceinline__ SeqFn seq_then(const SeqFn& a, const SeqFn& b) {
+  SeqFn r;
+  r.o0 = a.o0 + ((a.o0 & 1) ? b.o1 : b.o0);
+  r.o1 = a.o1 + ((a.o1 & 1) ? b.o0 : b.o1);
+  return r;
+}
+constexpr long long kSeqOver = 1ll << 53;  // at least this many units leave the binade
+// One addition of p >= 0; scale = 2^(52-e). *tie is set when the rounding depends on the parity.
+__device__ __forceinline__ SeqFn seq_fn(double p, double scale, bool* tie) {
+  const double x = p * scale;  // exact: a power of two, and the result is normal or zero (e >= -500)
+  if (!(x < 0x1p53)) return SeqFn{kSeqOver, kSeqOver};
+  const double f = floor(x), d = x - f;
+  const long long fi = (long long)f;
+  if (d != 0.5) {
+    const long long r = d > 0.5 ? fi + 1 : fi;
+    return SeqFn{r, r};
+  }
+  *tie = true;
+  return SeqFn{fi + (fi & 1), fi + ((fi + 1) & 1)};
+}
+// S + off units of 2^(e-52), for a sum inside the binade (exact).
+__device__ __forceinline__ double seq_add(double S, long long off, double unit) { return S + (double)off * unit; }
+constexpr double kSeqMin = 0x1p-500;  // smaller sums (zero among them) are added one by one
+
 struct CumScratch {
   double* bsum;      // nb + 1: block sums, then exclusive block prefix (bsum[nb] = total)
   double* norm;      // 2: [total, non-finite count]
@@ -321,7 +753,10 @@ struct CumScratch {
   uint32_t* amb;     // shots: ambiguous shot ids
   double* ck;        // exact mode: sequential sum at the end of every SEQ_CH chunk
   double* seq;       // exact mode: [sequential total, last positive index (bits)]
+  SeqFn* fn;         // exact mode: the chunk as a function of the start's parity
+  int* fe;           // exact mode: its binade (kNoBinade: crosses one; kAnyBinade: adds nothing)
 };
+constexpr int kNoBinade = -100000, kAnyBinade = 100000;
 
 template <typename Real>
 __global__ void cum_blocks_kernel(const V2<Real>* __restrict__ amps, uint64_t len, CumScratch c) {
@@ -385,43 +820,102 @@ __global__ void __launch_bounds__(PREFIX_T) cum_prefix_kernel(CumScratch c, uint
   }
 }
 
+// One warp adds amplitudes [b, e) to S in order and stops at the first index i
+// with target < S_i: *before = S_i-1, *at = S_i; *last_pos is the last positive
+// bin seen. Returns -1 when there is none. Every S is the sequential sum.
 template <typename Real>
-__global__ void cum_draw_kernel(const V2<Real>* __restrict__ amps, uint64_t len, uint32_t nb, CumScratch c,
-                                const double* __restrict__ uniforms, uint32_t shots, uint64_t* __restrict__ out,
-                                int32_t* status) {
+__device__ int64_t seq_search(const V2<Real>* __restrict__ amps, uint64_t b, uint64_t e, double S, double target,
+                              double* before, double* at, int64_t* last_pos) {
+  const int lane = threadIdx.x & 31;
+  for (uint64_t r0 = b; r0 < e; r0 += 32) {
+    const double p = r0 + lane < e ? prob_exact<Real>(amps, r0 + lane) : 0.0;
+    const unsigned pos = __ballot_sync(0xffffffffu, p > 0.0);
+    if (pos == 0) continue;
+    double mine;
+    bool in_binade = false;
+    if (S >= kSeqMin) {
+      const int ex = (int)((__double_as_longlong(S) >> 52) & 0x7ff) - 1023;
+      const double unit = __longlong_as_double((long long)(ex - 52 + 1023) << 52);
+      const double scale = __longlong_as_double((long long)(52 - ex + 1023) << 52);
+      bool tie = false;
+      SeqFn f = seq_fn(p, scale, &tie);
+      long long off;
+      if (__any_sync(0xffffffffu, tie)) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          SeqFn g;
+          g.o0 = __shfl_up_sync(0xffffffffu, f.o0, o);
+          g.o1 = __shfl_up_sync(0xffffffffu, f.o1, o);
+          if (lane >= o) f = seq_then(g, f);
+        }
+        off = (__double_as_longlong(S) & 1) ? f.o1 : f.o0;
+      } else {
+        off = f.o0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const long long g = __shfl_up_sync(0xffffffffu, off, o);
+          if (lane >= o) off += g;
+        }
+      }
+      const long long mant = (__double_as_longlong(S) & ((1ll << 52) - 1)) | (1ll << 52);
+      in_binade = __all_sync(0xffffffffu, mant + off < kSeqOver);  // offsets ascend: at most 32 * 2^53
+      mine = seq_add(S, off, unit);
+    }
+    if (!in_binade) {  // a binade boundary in these 32 (or a sum near zero): one by one
+      double run = S;
+      mine = S;
+#pragma unroll
+      for (int q = 0; q < 32; ++q) {
+        run = __dadd_rn(run, __shfl_sync(0xffffffffu, p, q));
+        if (lane == q) mine = run;
+      }
+    }
+    const unsigned hit = __ballot_sync(0xffffffffu, p > 0.0 && target < mine);
+    double prev = __shfl_up_sync(0xffffffffu, mine, 1);
+    if (lane == 0) prev = S;
+    if (hit) {
+      const int w = __ffs(hit) - 1;
+      *before = __shfl_sync(0xffffffffu, prev, w);
+      *at = __shfl_sync(0xffffffffu, mine, w);
+      return (int64_t)(r0 + w);
+    }
+    *last_pos = (int64_t)(r0 + (31 - __clz(pos)));
+    S = __shfl_sync(0xffffffffu, mine, 31);
+  }
+  return -1;
+}
+
+// One warp per shot: the block by binary search over the prefix, the bin by
+// adding the block in order.
+template <typename Real>
+__global__ void __launch_bounds__(128) cum_draw_kernel(const V2<Real>* __restrict__ amps, uint64_t len, uint32_t nb,
+                                                       CumScratch c, const double* __restrict__ uniforms,
+                                                       uint32_t shots, uint64_t* __restrict__ out) {
+  const uint32_t k = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (k >= shots) return;
   const double total = c.bsum[nb];
   // Bound on |sequential - two-level| for prefixes and for u * total.
   const double E = 8.0 * ((double)len + 64.0) * 1.1102230246251565e-16 * total;
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < shots; k += gridDim.x * blockDim.x) {
-    const double target = uniforms[k] * total;
-    // last block whose exclusive prefix <= target
-    uint32_t lo = 0, hi = nb;  // invariant: prefix[lo] <= target (prefix[0] = 0)
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (c.bsum[mid] <= target) lo = mid;
-      else hi = mid;
-    }
-    double cum = c.bsum[lo];
-    double margin = fabs(target - cum);
-    int64_t found = -1, last_pos = -1;
-    for (uint64_t i = (uint64_t)lo * CUM_BLOCK; i < len; ++i) {
-      const double p = prob_exact<Real>(amps, i);
-      if (p > 0.0) {
-        last_pos = (int64_t)i;
-        cum += p;
-        margin = fmin(margin, fabs(cum - target));
-        if (target < cum) {
-          found = (int64_t)i;
-          break;
-        }
-      }
-    }
-    if (found < 0) {
-      // ran off the end: the last positive bin at or after the start block,
-      // or, if none, any earlier positive bin (resolved exactly below)
-      found = last_pos;
-      margin = 0.0;
-    }
+  const double target = uniforms[k] * total;
+  // last block whose exclusive prefix <= target
+  uint32_t lo = 0, hi = nb;  // invariant: prefix[lo] <= target (prefix[0] = 0)
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (c.bsum[mid] <= target) lo = mid;
+    else hi = mid;
+  }
+  double before = 0.0, at = 0.0;
+  int64_t last_pos = -1;
+  int64_t found = seq_search<Real>(amps, (uint64_t)lo * CUM_BLOCK, len, c.bsum[lo], target, &before, &at, &last_pos);
+  // the sums ascend, so the boundary next to the target is the nearest one
+  double margin = fmin(fabs(target - before), fabs(at - target));
+  if (found < 0) {
+    // ran off the end: the last positive bin at or after the start block,
+    // or, if none, any earlier positive bin (resolved exactly below)
+    found = last_pos;
+    margin = 0.0;
+  }
+  if ((threadIdx.x & 31) == 0) {
     out[k] = (uint64_t)(found < 0 ? 0 : found);
     if (margin <= E) {
       const uint32_t slot = atomicAdd(c.namb, 1u);
@@ -430,106 +924,382 @@ __global__ void cum_draw_kernel(const V2<Real>* __restrict__ amps, uint64_t len,
   }
 }
 
-// Exact resolution of the ambiguous shots, in two kernels.
+// Exact resolution of the ambiguous shots, in three kernels.
 //
-// cum_seq_kernel: the reference's sequential left-to-right sum
-// (validate_norm's total and cumulative_index's running sum are the same
-// sequence S_i = fl(S_{i-1} + p_i)), done once by one thread while the rest
-// of the CTA stages the next chunk of probabilities in shared memory. It
-// records S at the end of every SEQ_CH-element chunk (exact checkpoints),
-// the total and the last positive index.
+// cum_fn_kernel: every SEQ_CH-element chunk as a function of its start's parity
+// (SeqFn), in the binade that the approximate prefix predicts, and the last
+// positive index.
+// cum_walk_kernel: the reference's sequential left-to-right sum (validate_norm's
+// total and cumulative_index's running sum are the same sequence
+// S_i = fl(S_{i-1} + p_i)) through the chunks: exact checkpoints at the end of
+// every chunk and the total. One CTA: 1024 segments of chunks compose, one
+// lane steps through the segments, and the chunks that cross a binade (some
+// log2(chunks) of them) are scanned by the whole CTA.
 // cum_exact_kernel: per ambiguous shot, the first chunk whose checkpoint
-// exceeds the target, rescanned sequentially from the previous checkpoint,
+// exceeds the target, added again in order from the previous checkpoint,
 // so every outcome equals the sequential CPU scan's.
 constexpr uint32_t SEQ_CH = 2048;
-constexpr uint32_t SEQ_T = 512;
+static_assert(SEQ_CH == CUM_BLOCK, "the chunks' binades come from the block prefix");
 
 template <typename Real>
-__global__ void __launch_bounds__(SEQ_T) cum_seq_kernel(const V2<Real>* __restrict__ amps, uint64_t len, CumScratch c) {
-  __shared__ double buf[2][SEQ_CH];
-  if (*c.namb == 0) return;  // uniform over the CTA: no ambiguous shot, nothing to resolve
-  const uint64_t nch = (len + SEQ_CH - 1) / SEQ_CH;
-  auto stage = [&](uint64_t ch, int slot) {
-    const uint64_t b0 = ch * SEQ_CH;
-    for (uint32_t j = threadIdx.x; j < SEQ_CH; j += SEQ_T)
-      buf[slot][j] = b0 + j < len ? prob_exact<Real>(amps, b0 + j) : 0.0;
-  };
-  stage(0, 0);
+__global__ void __launch_bounds__(256) cum_fn_kernel(const V2<Real>* __restrict__ amps, uint64_t len, CumScratch c) {
+  __shared__ long long red[8];
+  __shared__ SeqFn fr[8];
+  __shared__ uint32_t lastp;
+  if (*c.namb == 0) return;  // uniform: no ambiguous shot, nothing to resolve
+  const uint32_t ch = blockIdx.x, tid = threadIdx.x;
+  const uint64_t b0 = (uint64_t)ch * SEQ_CH;
+  const double s0 = c.bsum[ch], s1 = c.bsum[ch + 1];
+  const int e = (int)((__double_as_longlong(s0) >> 52) & 0x7ff) - 1023;
+  const bool one = s0 >= kSeqMin && (int)((__double_as_longlong(s1) >> 52) & 0x7ff) - 1023 == e;
+  const double scale = one ? __longlong_as_double((long long)(52 - e + 1023) << 52) : 1.0;
+  if (tid == 0) lastp = 0;
   __syncthreads();
-  double S = 0.0;
-  int64_t last_pos = -1;
-  for (uint64_t ch = 0; ch < nch; ++ch) {
-    if (threadIdx.x == 0) {
-      const double* b = buf[ch & 1];
-      const uint64_t left = len - ch * SEQ_CH;
-      const uint32_t m = left < SEQ_CH ? (uint32_t)left : SEQ_CH;
-#pragma unroll 16
-      for (uint32_t j = 0; j < m; ++j) {
-        const double p = b[j];
-        S += p;
-        if (p > 0.0) last_pos = (int64_t)(ch * SEQ_CH + j);
+  double p[SEQ_CH / 256];
+#pragma unroll
+  for (int r = 0; r < (int)(SEQ_CH / 256); ++r) {
+    const uint64_t i = b0 + r * 256 + tid;
+    p[r] = i < len ? prob_exact<Real>(amps, i) : 0.0;
+  }
+  long long sum = 0;
+  bool tie = false;
+  uint32_t last = 0;  // 1 + last positive element of the chunk
+#pragma unroll
+  for (int r = 0; r < (int)(SEQ_CH / 256); ++r) {
+    if (p[r] > 0.0) last = r * 256 + tid + 1;
+    sum += seq_fn(p[r], scale, &tie).o0;
+  }
+  last = __reduce_max_sync(0xffffffffu, last);
+  if ((tid & 31) == 0 && last) atomicMax(&lastp, last);
+  const bool ties = __syncthreads_or(tie ? 1 : 0) != 0;
+  if (lastp == 0) {
+    if (tid == 0) c.fe[ch] = kAnyBinade;
+    return;
+  }
+  if (tid == 0) atomicMax((unsigned long long*)&c.seq[1], (unsigned long long)(b0 + lastp));  // 1 + index
+  if (!one) {
+    if (tid == 0) c.fe[ch] = kNoBinade;
+    return;
+  }
+  if (!ties) {
+    for (int o = 16; o; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+    if ((tid & 31) == 0) red[tid >> 5] = sum;
+    __syncthreads();
+    if (tid == 0) {
+      long long t = 0;
+      for (int w = 0; w < 8; ++w) t += red[w];
+      c.fn[ch] = SeqFn{t, t};
+      c.fe[ch] = e;
+    }
+    return;
+  }
+  // ties: the order matters, so each thread composes 8 consecutive elements
+  SeqFn f{0, 0};
+  for (int r = 0; r < (int)(SEQ_CH / 256); ++r) {
+    const uint64_t i = b0 + (uint64_t)tid * (SEQ_CH / 256) + r;
+    bool t = false;
+    f = seq_then(f, seq_fn(i < len ? prob_exact<Real>(amps, i) : 0.0, scale, &t));
+  }
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    SeqFn g;
+    g.o0 = __shfl_down_sync(0xffffffffu, f.o0, o);
+    g.o1 = __shfl_down_sync(0xffffffffu, f.o1, o);
+    f = seq_then(f, g);  // lane 0's is the warp's, in order
+  }
+  if ((tid & 31) == 0) fr[tid >> 5] = f;
+  __syncthreads();
+  if (tid == 0) {
+    SeqFn t = fr[0];
+    for (int w = 1; w < 8; ++w) t = seq_then(t, fr[w]);
+    c.fn[ch] = t;
+    c.fe[ch] = e;
+  }
+}
+
+// Applies a chunk's (or segment's) function to *S; false when S is not in its
+// binade at both ends.
+__device__ __forceinline__ bool seq_step(double* S, int e, const SeqFn& f) {
+  if (e == kAnyBinade) return true;
+  const long long bits = __double_as_longlong(*S);
+  if (e == kNoBinade || (int)((bits >> 52) & 0x7ff) - 1023 != e) return false;
+  const long long off = (bits & 1) ? f.o1 : f.o0;
+  const long long mant = (bits & ((1ll << 52) - 1)) | (1ll << 52);
+  if (mant + off >= kSeqOver) return false;
+  *S = seq_add(*S, off, __longlong_as_double((long long)(e - 52 + 1023) << 52));
+  return true;
+}
+
+constexpr uint32_t WALK_T = 1024;
+template <typename Real>
+__global__ void __launch_bounds__(WALK_T) cum_walk_kernel(const V2<Real>* __restrict__ amps, uint64_t len,
+                                                          uint32_t nch, CumScratch c) {
+  __shared__ SeqFn sfn[WALK_T];
+  __shared__ int se[WALK_T];
+  __shared__ double sstart[WALK_T];
+  __shared__ bool swalked[WALK_T];
+  __shared__ SeqFn wtot[32];
+  __shared__ double S_sh;
+  __shared__ uint32_t seg_sh, ch_sh, first_sh;
+  if (*c.namb == 0) return;
+  const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const uint32_t per = (nch + WALK_T - 1) / WALK_T;
+  const uint32_t c0 = min(nch, t * per), c1 = min(nch, c0 + per);
+  {
+    SeqFn f{0, 0};
+    int e = kAnyBinade;
+    for (uint32_t k = c0; k < c1; ++k) {
+      const int ek = c.fe[k];
+      if (ek == kAnyBinade) continue;
+      if (e == kAnyBinade) {
+        e = ek;
+        f = c.fn[k];
+      } else if (ek == e) {
+        f = seq_then(f, c.fn[k]);
+      } else {
+        e = kNoBinade;
       }
-      c.ck[ch] = S;
-    } else if (ch + 1 < nch) {
-      // threads 1.. stage the next chunk (thread 0's share falls to the others)
-      const uint64_t b0 = (ch + 1) * SEQ_CH;
-      for (uint32_t j = threadIdx.x - 1; j < SEQ_CH; j += SEQ_T - 1)
-        buf[(ch + 1) & 1][j] = b0 + j < len ? prob_exact<Real>(amps, b0 + j) : 0.0;
+      if (e == kNoBinade) break;
+    }
+    sfn[t] = f;
+    se[t] = e;
+    swalked[t] = false;
+  }
+  if (t == 0) {
+    S_sh = 0.0;
+    seg_sh = 0;
+  }
+  __syncthreads();
+  const uint32_t nseg = per ? (nch + per - 1) / per : 0;
+  for (;;) {
+    if (t == 0) {  // as many whole segments as hold
+      double S = S_sh;
+      uint32_t g = seg_sh;
+      for (; g < nseg; ++g) {
+        const double at = S;
+        if (!seq_step(&S, se[g], sfn[g])) break;
+        sstart[g] = at;
+        swalked[g] = true;
+      }
+      S_sh = S;
+      seg_sh = g;
+      ch_sh = g * per;
     }
     __syncthreads();
+    const uint32_t g = seg_sh;
+    if (g >= nseg) break;
+    const uint32_t end = min(nch, (g + 1) * per);
+    for (;;) {  // its chunks one by one
+      __syncthreads();
+      if (t == 0) {
+        double S = S_sh;
+        uint32_t k = ch_sh;
+        for (; k < end; ++k) {
+          const int ek = c.fe[k];
+          if (!seq_step(&S, ek, ek == kNoBinade || ek == kAnyBinade ? SeqFn{0, 0} : c.fn[k])) break;
+          c.ck[k] = S;
+        }
+        S_sh = S;
+        ch_sh = k;
+      }
+      __syncthreads();
+      const uint32_t k = ch_sh;
+      if (k >= end) break;
+      // a chunk that crosses a binade: two elements a thread, scanned once per binade
+      const uint64_t b0 = (uint64_t)k * SEQ_CH + 2 * t;
+      const double p0 = b0 < len ? prob_exact<Real>(amps, b0) : 0.0;
+      const double p1 = b0 + 1 < len ? prob_exact<Real>(amps, b0 + 1) : 0.0;
+      uint32_t pos = 0;  // elements before pos are in S
+      while (pos < SEQ_CH) {
+        const double S = S_sh;
+        const bool a0 = 2 * t >= pos, a1 = 2 * t + 1 >= pos;
+        double before = S;  // the sum before the element where the scan stops
+        uint32_t stop = SEQ_CH;
+        if (t == 0) first_sh = SEQ_CH;
+        __syncthreads();
+        if (S < kSeqMin) {  // near zero: the next positive element by itself
+          if (a0 && p0 > 0.0) stop = 2 * t;
+          else if (a1 && p1 > 0.0) stop = 2 * t + 1;
+        } else {
+          const long long bits = __double_as_longlong(S);
+          const int ex = (int)((bits >> 52) & 0x7ff) - 1023;
+          const double scale = __longlong_as_double((long long)(52 - ex + 1023) << 52);
+          const double unit = __longlong_as_double((long long)(ex - 52 + 1023) << 52);
+          bool tie = false;
+          const SeqFn f0 = a0 ? seq_fn(p0, scale, &tie) : SeqFn{0, 0}, f1 = a1 ? seq_fn(p1, scale, &tie) : SeqFn{0, 0};
+          SeqFn f = seq_then(f0, f1);
+          SeqFn inc = f;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            SeqFn x;
+            x.o0 = __shfl_up_sync(0xffffffffu, inc.o0, o);
+            x.o1 = __shfl_up_sync(0xffffffffu, inc.o1, o);
+            if (lane >= (uint32_t)o) inc = seq_then(x, inc);
+          }
+          if (lane == 31) wtot[w] = inc;
+          SeqFn ex_lane;  // exclusive within the warp
+          ex_lane.o0 = __shfl_up_sync(0xffffffffu, inc.o0, 1);
+          ex_lane.o1 = __shfl_up_sync(0xffffffffu, inc.o1, 1);
+          if (lane == 0) ex_lane = SeqFn{0, 0};
+          __syncthreads();
+          SeqFn pre{0, 0};
+          for (uint32_t x = 0; x < w; ++x) pre = seq_then(pre, wtot[x]);
+          pre = seq_then(pre, ex_lane);
+          const bool odd = bits & 1;
+          const long long mant = (bits & ((1ll << 52) - 1)) | (1ll << 52);
+          // sums of up to 2048 marked elements stay below 2^64
+          const long long m0 = mant + (odd ? pre.o1 : pre.o0);
+          const long long g0 = (m0 & 1) ? f0.o1 : f0.o0;
+          const long long m1 = m0 + g0;
+          const long long g1 = (m1 & 1) ? f1.o1 : f1.o0;
+          if (a0 && m1 >= kSeqOver) {
+            stop = 2 * t;
+            before = seq_add(S, m0 - mant, unit);
+          } else if (a1 && m1 + g1 >= kSeqOver) {
+            stop = 2 * t + 1;
+            before = seq_add(S, m1 - mant, unit);
+          }
+          if (stop < SEQ_CH) atomicMin(&first_sh, stop);
+          __syncthreads();
+          if (first_sh == SEQ_CH) {  // the rest stays in the binade
+            if (t == WALK_T - 1) S_sh = seq_add(S, m1 + g1 - mant, unit);
+            __syncthreads();
+            break;
+          }
+          if (stop == first_sh) S_sh = __dadd_rn(before, (stop & 1) ? p1 : p0);
+          pos = first_sh + 1;
+          __syncthreads();
+          continue;
+        }
+        if (stop < SEQ_CH) atomicMin(&first_sh, stop);
+        __syncthreads();
+        if (first_sh == SEQ_CH) break;
+        if (stop == first_sh) S_sh = __dadd_rn(S, (stop & 1) ? p1 : p0);
+        pos = first_sh + 1;
+        __syncthreads();
+      }
+      __syncthreads();
+      if (t == 0) {
+        c.ck[k] = S_sh;
+        ch_sh = k + 1;
+      }
+      __syncthreads();
+    }
+    if (t == 0) seg_sh = g + 1;
+    __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    c.seq[0] = S;
-    c.seq[1] = __longlong_as_double(last_pos);
+  if (t < nseg && swalked[t]) {  // the checkpoints inside the walked segments
+    double S = sstart[t];
+    for (uint32_t k = c0; k < c1; ++k) {
+      const int ek = c.fe[k];
+      if (ek != kAnyBinade) seq_step(&S, ek, c.fn[k]);
+      c.ck[k] = S;
+    }
+  }
+  if (t == 0) c.seq[0] = S_sh;
+}
+
+// One warp per ambiguous shot.
+template <typename Real>
+__global__ void __launch_bounds__(128) cum_exact_kernel(const V2<Real>* __restrict__ amps, uint64_t len, CumScratch c,
+                                                        const double* __restrict__ uniforms,
+                                                        uint64_t* __restrict__ out, int32_t* status) {
+  const uint32_t na = *c.namb;
+  const uint32_t a = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (a >= na) return;
+  const uint64_t nch = (len + SEQ_CH - 1) / SEQ_CH;
+  const double total = c.seq[0];
+  const int64_t last_pos = __double_as_longlong(c.seq[1]) - 1;  // -1: none
+  const uint32_t k = c.amb[a];
+  const double target = uniforms[k] * total;
+  // first chunk whose inclusive checkpoint exceeds the target
+  uint64_t lo = 0, hi = nch;
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi) >> 1;
+    if (target < c.ck[mid]) hi = mid;
+    else lo = mid + 1;
+  }
+  int64_t found = last_pos;  // target >= total: the last positive bin
+  if (lo < nch) {
+    const uint64_t e = (lo + 1) * SEQ_CH < len ? (lo + 1) * SEQ_CH : len;
+    double before, at;
+    int64_t seen = -1;
+    found = seq_search<Real>(amps, lo * SEQ_CH, e, lo ? c.ck[lo - 1] : 0.0, target, &before, &at, &seen);
+    if (found < 0) return;  // never: the checkpoint exceeds the target
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (found < 0) status[0] = ALEPH_B200_INVALID_STATE;
+    else out[k] = (uint64_t)found;
   }
 }
 
-template <typename Real>
-__global__ void cum_exact_kernel(const V2<Real>* __restrict__ amps, uint64_t len, CumScratch c,
-                                 const double* __restrict__ uniforms, uint64_t* __restrict__ out, int32_t* status) {
-  const uint32_t na = *c.namb;
-  const uint64_t nch = (len + SEQ_CH - 1) / SEQ_CH;
-  const double total = c.seq[0];
-  const int64_t last_pos = __double_as_longlong(c.seq[1]);
-  for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < na; a += gridDim.x * blockDim.x) {
-    const uint32_t k = c.amb[a];
-    const double target = uniforms[k] * total;
-    // first chunk whose inclusive checkpoint exceeds the target
-    uint64_t lo = 0, hi = nch;
-    while (lo < hi) {
-      const uint64_t mid = (lo + hi) >> 1;
-      if (target < c.ck[mid]) hi = mid;
-      else lo = mid + 1;
-    }
-    if (lo == nch) {  // target >= total: the last positive bin
-      if (last_pos < 0) status[0] = ALEPH_B200_INVALID_STATE;
-      else out[k] = (uint64_t)last_pos;
-      continue;
-    }
-    double S = lo ? c.ck[lo - 1] : 0.0;
-    const uint64_t e = (lo + 1) * SEQ_CH < len ? (lo + 1) * SEQ_CH : len;
-    for (uint64_t i = lo * SEQ_CH; i < e; ++i) {
-      const double p = prob_exact<Real>(amps, i);
-      if (p > 0.0) {
-        S += p;
-        if (target < S) {
-          out[k] = i;
-          break;
-        }
-      }
-    }
-  }
+// The chunk functions of the exact resolution (SeqFn and binade per chunk).
+size_t sample_chunk_fn_bytes(uint32_t n) {
+  const uint64_t len = 1ull << n;
+  const uint64_t nch = n <= EXACT_MAX_N ? (len + SEQ_CH - 1) / SEQ_CH : 0;
+  return nch * (sizeof(SeqFn) + 4) + 32;
 }
+
+namespace {
+// Lays fields out one after the other, 16-byte aligned; with a null base it only counts bytes.
+struct Carver {
+  char* base;
+  size_t off = 0;
+  template <typename T>
+  T* take(uint64_t count) {
+    off = (off + 15) & ~(size_t)15;
+    T* p = base ? (T*)(base + off) : nullptr;
+    off += count * sizeof(T);
+    return p;
+  }
+};
+
+// The alias table's scratch (40 bytes per amplitude and 1.3 more for the
+// chunks); *norm2 receives the norm's two words.
+AliasScratch alias_scratch(Carver& c, uint32_t n, double** norm2) {
+  const uint64_t len = 1ull << n;
+  const uint64_t nb = (len + PART_B - 1) / PART_B;
+  const uint64_t nc = alias_chunks(len), ng = (nc + CGROUP - 1) / CGROUP;
+  AliasScratch s;
+  s.prob = c.take<double>(len);
+  s.alias = c.take<uint32_t>(len);
+  s.val = c.take<double>(len);
+  s.idx = c.take<uint32_t>(len);
+  s.pre = c.take<u128>(len);
+  s.bcount = c.take<uint32_t>(nb);
+  s.bdef = c.take<u128>(nb);
+  s.bsur = c.take<u128>(nb);
+  s.normsum = c.take<double>(2 * nb);
+  s.totals = c.take<uint32_t>(4);
+  *norm2 = c.take<double>(2);
+  s.ci = c.take<uint32_t>(nc + 1);
+  s.cj = c.take<uint32_t>(nc + 1);
+  s.cbase = c.take<double>(nc + 1);
+  s.cunit = c.take<double>(nc + 1);
+  s.cmargin = c.take<long long>(nc);
+  s.cmax = c.take<int>(nc);
+  s.cend = c.take<double>(nc * 32);
+  s.cstart = c.take<double>(nc);
+  s.cflag = c.take<uint8_t>(nc + 1);
+  s.gmargin = c.take<long long>(ng);
+  s.gend = c.take<double>(ng * 32);
+  s.gstart = c.take<double>(ng);
+  s.gflag = c.take<uint8_t>(ng);
+  return s;
+}
+}  // namespace
 
 size_t sample_scratch_bytes(uint32_t n, int mode, uint32_t shots) {
   const uint64_t len = 1ull << n;
   if (mode == ALEPH_B200_SAMPLE_ALIAS) {
-    const uint64_t nb = (len + PART_B - 1) / PART_B;
-    return len * (8 + 4 + 4 + 4) + nb * (8 + 16) + 256;
+    Carver c{nullptr};
+    double* norm2;
+    alias_scratch(c, n, &norm2);
+    return c.off + 256;
   }
   const uint64_t nb = (len + CUM_BLOCK - 1) / CUM_BLOCK;
   const uint64_t nch = n <= EXACT_MAX_N ? (len + SEQ_CH - 1) / SEQ_CH : 0;  // exact-mode checkpoints
-  return (nb + 1) * 8 + 64 + 256 + (size_t)shots * 4 + 16 + nch * 8 + 32;
+  return (nb + 1) * 8 + 64 + 256 + (size_t)shots * 4 + 16 + nch * 8 + 32 + sample_chunk_fn_bytes(n);
 }
 
 static inline char* align_up(char* p, size_t a) {
@@ -541,65 +1311,69 @@ cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t 
                           cudaStream_t st) {
   const uint64_t len = 1ull << n;
   const bool f64 = precision == ALEPH_B200_F64;
-  char* p = (char*)scratch;
   if (mode == ALEPH_B200_SAMPLE_ALIAS) {
     const uint32_t nb = (uint32_t)((len + PART_B - 1) / PART_B);
-    AliasScratch s;
-    s.prob = (double*)p; p += len * 8;
-    s.normsum = (double*)p; p += (size_t)nb * 16;
-    s.alias = (uint32_t*)p; p += len * 4;
-    s.small = (uint32_t*)p; p += len * 4;
-    s.large = (uint32_t*)p; p += len * 4;
-    s.bcount = (uint32_t*)p; p += (size_t)nb * 8;
-    p = align_up(p, 16);
-    s.totals = (uint32_t*)p; p += 16;
-    double* norm2 = (double*)p; p += 16;
-    if ((size_t)(p - (char*)scratch) > scratch_bytes) return cudaErrorInvalidValue;
+    const uint32_t nc = alias_chunks(len), ng = (nc + CGROUP - 1) / CGROUP;
+    Carver c{(char*)scratch};
+    double* norm2;
+    const AliasScratch s = alias_scratch(c, n, &norm2);
+    if (c.off > scratch_bytes) return cudaErrorInvalidValue;
     if (f64) alias_scale_kernel<double><<<nb, PART_B, 0, st>>>((const double2*)amps, len, s);
     else alias_scale_kernel<float><<<nb, PART_B, 0, st>>>((const float2*)amps, len, s);
-    alias_offsets_kernel<<<1, 32, 0, st>>>(s, nb, norm2);
+    alias_offsets_kernel<<<1, 1024, 0, st>>>(s, len, nb, norm2);
     check_norm_kernel<<<1, 32, 0, st>>>(norm2, norm_tolerance(len, precision), status);
-    alias_partition_kernel<<<nb, PART_B, 0, st>>>(len, s);
-    alias_chain_kernel<<<1, 32, 0, st>>>(len, s, status);
-    alias_drain_kernel<<<(unsigned)sm_count * 4, 256, 0, st>>>(s);
+    alias_partition_kernel<<<nb, PART_B, 0, st>>>(len, s, status);
+    if (nc) {
+      alias_cuts_kernel<<<nc / 4 + 1, 128, 0, st>>>(s, nc, status);
+      alias_spec_kernel<<<(nc + 3) / 4, 128, 0, st>>>(s, nc, status);
+      alias_compose_kernel<<<(ng + 3) / 4, 128, 0, st>>>(s, nc, ng, status);
+    }
+    alias_walk_kernel<<<1, 32, 0, st>>>(s, nc, ng, status);
+    if (nc) {
+      alias_expand_kernel<<<(ng + 3) / 4, 128, 0, st>>>(s, nc, ng, status);
+      alias_emit_kernel<<<(nc + 3) / 4, 128, 0, st>>>(s, nc, status);
+    }
+    alias_drain_kernel<<<(unsigned)sm_count * 4, 256, 0, st>>>(s, status);
     if (shots)
-      alias_draw_kernel<<<(shots + 255) / 256, 256, 0, st>>>(s, len - 1, (const uint64_t*)variates, shots, out);
+      alias_draw_kernel<<<(shots + 255) / 256, 256, 0, st>>>(s, len - 1, (const uint64_t*)variates, shots, out, status);
     return cudaGetLastError();
   }
+  char* p = (char*)scratch;
   const uint32_t nb = (uint32_t)((len + CUM_BLOCK - 1) / CUM_BLOCK);
   CumScratch c;
   c.bsum = (double*)p; p += ((size_t)nb + 1) * 8;
   p = align_up(p, 16);
   c.norm = (double*)p; p += 16;
   c.namb = (uint32_t*)p; p += 16;
-  c.amb = (uint32_t*)align_up(p, 16);
-  p = (char*)(c.amb + shots);
-  const uint64_t nch = n <= EXACT_MAX_N ? (len + SEQ_CH - 1) / SEQ_CH : 0;
-  c.seq = (double*)align_up(p, 16); p = (char*)(c.seq + 2);
-  c.ck = (double*)p; p += nch * 8;
+  c.seq = (double*)p; p += 16;
+  c.amb = (uint32_t*)p;
+  p = align_up((char*)(c.amb + shots), 16);
+  const uint32_t nch = n <= EXACT_MAX_N ? (uint32_t)((len + SEQ_CH - 1) / SEQ_CH) : 0u;
+  c.ck = (double*)p; p += (size_t)nch * 8;
+  c.fn = (SeqFn*)align_up(p, 16); p = (char*)(c.fn + nch);
+  c.fe = (int*)p; p += (size_t)nch * 4;
   if ((size_t)(p - (char*)scratch) > scratch_bytes) return cudaErrorInvalidValue;
-  cudaMemsetAsync(c.norm, 0, 32, st);
+  cudaMemsetAsync(c.norm, 0, 48, st);  // norm, namb, seq
   if (f64) cum_blocks_kernel<double><<<nb, 256, 0, st>>>((const double2*)amps, len, c);
   else cum_blocks_kernel<float><<<nb, 256, 0, st>>>((const float2*)amps, len, c);
   cum_prefix_kernel<<<1, PREFIX_T, 0, st>>>(c, nb);
   check_norm_kernel<<<1, 32, 0, st>>>(c.norm, norm_tolerance(len, precision), status);
   if (shots) {
-    if (f64)
-      cum_draw_kernel<double><<<(shots + 127) / 128, 128, 0, st>>>((const double2*)amps, len, nb, c,
-                                                                   (const double*)variates, shots, out, status);
-    else
-      cum_draw_kernel<float><<<(shots + 127) / 128, 128, 0, st>>>((const float2*)amps, len, nb, c,
-                                                                  (const double*)variates, shots, out, status);
+    const unsigned wb = (shots + 3) / 4;  // a warp per shot
+    const double* u = (const double*)variates;
+    if (f64) cum_draw_kernel<double><<<wb, 128, 0, st>>>((const double2*)amps, len, nb, c, u, shots, out);
+    else cum_draw_kernel<float><<<wb, 128, 0, st>>>((const float2*)amps, len, nb, c, u, shots, out);
     // status[2]: the shots inside the guard band (re-resolved below when n <= EXACT_MAX_N)
     cudaMemcpyAsync(status + 2, c.namb, 4, cudaMemcpyDeviceToDevice, st);
     if (n <= EXACT_MAX_N) {
-      const unsigned eb = (shots + 127) / 128;
       if (f64) {
-        cum_seq_kernel<double><<<1, SEQ_T, 0, st>>>((const double2*)amps, len, c);
-        cum_exact_kernel<double><<<eb, 128, 0, st>>>((const double2*)amps, len, c, (const double*)variates, out, status);
+        cum_fn_kernel<double><<<nch, 256, 0, st>>>((const double2*)amps, len, c);
+        cum_walk_kernel<double><<<1, WALK_T, 0, st>>>((const double2*)amps, len, nch, c);
+        cum_exact_kernel<double><<<wb, 128, 0, st>>>((const double2*)amps, len, c, u, out, status);
       } else {
-        cum_seq_kernel<float><<<1, SEQ_T, 0, st>>>((const float2*)amps, len, c);
-        cum_exact_kernel<float><<<eb, 128, 0, st>>>((const float2*)amps, len, c, (const double*)variates, out, status);
+        cum_fn_kernel<float><<<nch, 256, 0, st>>>((const float2*)amps, len, c);
+        cum_walk_kernel<float><<<1, WALK_T, 0, st>>>((const float2*)amps, len, nch, c);
+        cum_exact_kernel<float><<<wb, 128, 0, st>>>((const float2*)amps, len, c, u, out, status);
       }
     }
   }
@@ -610,7 +1384,7 @@ cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t 
 // Reserved when this module is loaded on a device, so the entry point that
 // uses it never allocates. One copy per device; calls that overlap on one
 // device share it.
-static __device__ __align__(256) unsigned char g_fixed_sample_scratch[kFixedSampleScratchBytes];
+static __device__ __align__(256) unsigned char g_fixed_sample_scratch[kFixedSampleScratchBytes + kFixedChunkFnBytes];
 
 cudaError_t fixed_sample_scratch_address(void** out) {
   return cudaGetSymbolAddress(out, g_fixed_sample_scratch);
