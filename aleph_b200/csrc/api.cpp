@@ -1382,6 +1382,21 @@ int aleph_b200_measure(aleph_b200_handle* h, aleph_b200_state* st, uint32_t qubi
   return ALEPH_B200_OK;
 }
 
+// validate_norm on the device's two sums (sum |a|^2, non-finite count).
+static int check_norm(aleph_b200_handle* h, aleph_b200_state* st, const double* res) {
+  aleph_b200_error_info e{};
+  e.status = ALEPH_B200_INVALID_STATE;
+  if (res[1] > 0.0) {
+    std::snprintf(e.kind, sizeof(e.kind), "non-finite amplitude norm2");
+    return report(h, e);
+  }
+  if (!std::isfinite(res[0]) || std::fabs(res[0] - 1.0) > norm_tolerance(1ull << st->n, st->precision)) {
+    std::snprintf(e.kind, sizeof(e.kind), "state norm2 deviates from 1");
+    return report(h, e);
+  }
+  return 0;
+}
+
 static int check_norm_host(aleph_b200_handle* h, aleph_b200_state* st, double* norm_out) {
   const uint32_t nb = reduce_blocks(st->n, h->sm_count);
   if (int r = ensure(h, h->reduce, (size_t)nb * 3 * 8 + 256)) return r;
@@ -1393,19 +1408,7 @@ static int check_norm_host(aleph_b200_handle* h, aleph_b200_state* st, double* n
   CK(copy_async(h, res, out2, 16, cudaMemcpyDeviceToHost, h->stream), "norm readback");
   CK(cudaStreamSynchronize(h->stream), "stream synchronize");
   if (norm_out) *norm_out = res[0];
-  if (res[1] > 0.0) {
-    aleph_b200_error_info e{};
-    e.status = ALEPH_B200_INVALID_STATE;
-    std::snprintf(e.kind, sizeof(e.kind), "non-finite amplitude norm2");
-    return report(h, e);
-  }
-  if (!std::isfinite(res[0]) || std::fabs(res[0] - 1.0) > norm_tolerance(1ull << st->n, st->precision)) {
-    aleph_b200_error_info e{};
-    e.status = ALEPH_B200_INVALID_STATE;
-    std::snprintf(e.kind, sizeof(e.kind), "state norm2 deviates from 1");
-    return report(h, e);
-  }
-  return 0;
+  return check_norm(h, st, res);
 }
 
 // status[2] of a CUMULATIVE sampling call: its shots inside the guard band
@@ -1713,11 +1716,11 @@ int aleph_b200_probabilities(aleph_b200_handle* h, aleph_b200_state* st, const u
                              double* out) {
   if (!h || !st || !out || (k && !qubits)) return ALEPH_B200_INVALID_ARGUMENT;
   if (int r = bind(h)) return r;
-  // validate_state first (measure.rs:245)
-  if (int r = check_norm_host(h, st, nullptr)) return r;
+  // validate_state first (measure.rs:245): the qubit errors come after it
   for (uint32_t t = 0; t < k; ++t) {
     aleph_b200_error_info e{};
     if (qubits[t] >= st->n) {
+      if (int r = check_norm_host(h, st, nullptr)) return r;
       e.status = ALEPH_B200_QUBIT_OUT_OF_RANGE;
       e.qubit = qubits[t];
       e.num_qubits = st->n;
@@ -1725,32 +1728,38 @@ int aleph_b200_probabilities(aleph_b200_handle* h, aleph_b200_state* st, const u
     }
     for (uint32_t j = 0; j < t; ++j)
       if (qubits[j] == qubits[t]) {
+        if (int r = check_norm_host(h, st, nullptr)) return r;
         e.status = ALEPH_B200_DUPLICATE_QUBIT;
         e.qubit = qubits[t];
         return report(h, e);
       }
   }
   if (k == 0) {
+    if (int r = check_norm_host(h, st, nullptr)) return r;
     out[0] = 1.0;
     return ALEPH_B200_OK;
   }
-  const uint32_t nb = reduce_blocks(st->n, h->sm_count);
   const size_t dim = (size_t)1 << k;
-  const size_t part_bytes = k <= 10 ? (size_t)nb * (dim + 2) * 8 : (size_t)nb * 3 * 8;
-  if (int r = ensure(h, h->reduce, part_bytes + 256)) return r;
+  if (int r = ensure(h, h->reduce, probabilities_scratch_bytes(st->n, qubits, k, h->sm_count) + 256)) return r;
   if (int r = ensure(h, h->sample, dim * 8 + 256)) return r;
-  uint32_t* dq = nullptr;
-  CK(cudaMalloc(&dq, 64 * 4), "qubit list");
-  cudaError_t e = copy_async(h, dq, qubits, k * 4, cudaMemcpyHostToDevice, h->stream);
-  double* dout = (double*)h->sample.ptr;
-  double* dnorm = dout + dim;
-  if (e == cudaSuccess)
-    e = launch_probabilities(st->amps, st->precision, st->n, dq, k, (double*)h->reduce.ptr, nb, dout, dnorm, h->stream);
-  if (e == cudaSuccess) e = copy_async(h, out, dout, dim * 8, cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  cudaFree(dq);
-  if (e != cudaSuccess) return cuda_fail(h, e, "probabilities");
-  h->stats.kernel_launches += 2;
+  double* dnorm = (double*)h->sample.ptr;  // the norm's two sums, then the marginal
+  double* dout = dnorm + 2;
+  CK(launch_probabilities(st->amps, st->precision, st->n, qubits, k, (double*)h->reduce.ptr, dout, dnorm, h->sm_count,
+                          h->stream),
+     "probabilities");
+  h->stats.kernel_launches += 3;
+  // a small marginal comes back with the norm in one copy
+  const size_t head = dim <= 4096 ? dim + 2 : 2;
+  std::vector<double> host(head);
+  CK(copy_async(h, host.data(), dnorm, head * 8, cudaMemcpyDeviceToHost, h->stream), "probabilities readback");
+  CK(cudaStreamSynchronize(h->stream), "stream synchronize");
+  if (int r = check_norm(h, st, host.data())) return r;
+  if (head > 2) {
+    std::memcpy(out, host.data() + 2, dim * 8);
+    return ALEPH_B200_OK;
+  }
+  CK(copy_async(h, out, dout, dim * 8, cudaMemcpyDeviceToHost, h->stream), "probabilities readback");
+  CK(cudaStreamSynchronize(h->stream), "stream synchronize");
   return ALEPH_B200_OK;
 }
 

@@ -262,8 +262,11 @@ struct PauliGroup {
 // out: [sum |a|^2, non-finite count, Re <P_0>, ..., Re <P_15>] (2 + MAX_TERMS doubles)
 cudaError_t launch_pauli_group(const void* amps, int precision, uint32_t n, const PauliGroup& g, double* partials,
                                uint32_t nblocks, double* out, cudaStream_t s);
-cudaError_t launch_probabilities(const void* amps, int precision, uint32_t n, const uint32_t* qubits_dev, uint32_t k,
-                                 double* partials, uint32_t nblocks, double* out, double* norm_out, cudaStream_t s);
+// Marginal of the qubits (host list, at most 64) with the norm's two sums; scratch of
+// probabilities_scratch_bytes bytes, out 2^k doubles.
+size_t probabilities_scratch_bytes(uint32_t n, const uint32_t* qubits, uint32_t k, int sm_count);
+cudaError_t launch_probabilities(const void* amps, int precision, uint32_t n, const uint32_t* qubits, uint32_t k,
+                                 double* scratch, double* out, double* norm_out, int sm_count, cudaStream_t s);
 uint32_t reduce_blocks(uint32_t n, int sm_count);
 
 // learned planner cost model (kernels_mlp.cu): F -> H -> H -> H -> 1 MLP

@@ -45,14 +45,31 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* out)
   }
 }
 
-// partials[b*NV + k] -> out[k], summed in block order by one thread.
+// Sum over the blocks of one of NV partials: every lane of a warp adds a
+// strided share (four loads in flight), then a shuffle tree; the order is fixed.
+// (One thread adding 1184 partials in order took 65 us, as long as a sweep
+// over 2^25 complex64 amplitudes; a warp takes 4 us.)
 template <int NV>
-__global__ void finish_kernel(const double* __restrict__ partials, uint32_t nblocks, double* __restrict__ out) {
-  if (threadIdx.x < NV) {
-    double s = 0.0;
-    for (uint32_t b = 0; b < nblocks; ++b) s += partials[(size_t)b * NV + threadIdx.x];
-    out[threadIdx.x] = s;
+__device__ __forceinline__ double sum_partials(const double* __restrict__ partials, uint32_t nblocks, int k) {
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  uint32_t b = threadIdx.x & 31;
+  for (; b + 96 < nblocks; b += 128) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s[u] += partials[(size_t)(b + 32 * u) * NV + k];
   }
+  for (; b < nblocks; b += 32) s[0] += partials[(size_t)b * NV + k];
+  double x = (s[0] + s[1]) + (s[2] + s[3]);
+  for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+// partials[b*NV + k] -> out[k], one warp per k.
+template <int NV>
+__global__ void __launch_bounds__(32 * NV) finish_kernel(const double* __restrict__ partials, uint32_t nblocks,
+                                                         double* __restrict__ out) {
+  const int k = threadIdx.x >> 5;
+  const double s = sum_partials<NV>(partials, nblocks, k);
+  if ((threadIdx.x & 31) == 0) out[k] = s;
 }
 
 template <typename Real>
@@ -94,7 +111,7 @@ cudaError_t launch_norm(const void* amps, int precision, uint32_t n, double* par
   const uint64_t len = 1ull << n;
   if (precision == ALEPH_B200_F64) norm_kernel<double><<<nblocks, RB, 0, s>>>((const double2*)amps, len, partials);
   else norm_kernel<float><<<nblocks, RB, 0, s>>>((const float2*)amps, len, partials);
-  finish_kernel<2><<<1, 32, 0, s>>>(partials, nblocks, out2);
+  finish_kernel<2><<<1, 64, 0, s>>>(partials, nblocks, out2);
   return cudaGetLastError();
 }
 
@@ -124,9 +141,15 @@ __global__ void __launch_bounds__(RB) branch_kernel(const V2<Real>* __restrict__
 
 // status[0]: error code (0 ok), status[1]: uniforms consumed, status[2]: failing qubit;
 // dec[0] = outcome (0/1), dec[1] = 1/norm scale; dval[0] = reported probability.
-__global__ void measure_decide_kernel(const double* __restrict__ sums, uint32_t qubit, uint64_t len,
-                                      const double* __restrict__ uniforms, uint32_t n_uniforms, int32_t* status,
-                                      double* dec, uint8_t* outcome_slot, double tol) {
+// One warp per sum of the block partials, then one thread decides.
+__global__ void __launch_bounds__(96) measure_decide_kernel(const double* __restrict__ partials, uint32_t nblocks,
+                                                            uint32_t qubit, const double* __restrict__ uniforms,
+                                                            uint32_t n_uniforms, int32_t* status, double* dec,
+                                                            uint8_t* outcome_slot, double tol) {
+  __shared__ double sums[3];
+  const double part = sum_partials<3>(partials, nblocks, threadIdx.x >> 5);
+  if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = part;
+  __syncthreads();
   if (threadIdx.x != 0) return;
   dec[0] = -1.0;  // "skip collapse" unless a decision is made below
   if (status[0] != 0) return;  // an earlier instruction failed: do nothing further
@@ -168,23 +191,39 @@ __global__ void measure_decide_kernel(const double* __restrict__ sums, uint32_t 
   if (outcome_slot) *outcome_slot = outcome ? 1 : 0;
 }
 
+// The kept half is read, divided and written; the other half is only written.
+// A thread takes pairs (bit 0, bit 1) of the measured qubit, four per step, so
+// that four loads are in flight and the discarded amplitudes are never loaded.
 template <typename Real>
-__global__ void collapse_kernel(V2<Real>* __restrict__ amps, uint64_t len, uint64_t qb, const double* __restrict__ dec) {
+__global__ void __launch_bounds__(256) collapse_kernel(V2<Real>* __restrict__ amps, uint64_t pairs, uint32_t qubit,
+                                                       const double* __restrict__ dec) {
   const double o = dec[0];
   if (o < 0.0) return;
-  const bool outcome = o > 0.5;
+  const uint64_t qb = 1ull << qubit, keep = o > 0.5 ? qb : 0, drop = qb ^ keep;
   const double norm = dec[1];
   const double d = norm * norm;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (uint64_t)gridDim.x * blockDim.x) {
-    const bool bit = (i & qb) != 0;
-    V2<Real> a = ld_amp<Real>(amps + i);
-    if (bit == outcome) {
-      // num-complex division by Complex::new(norm, 0.0), as the reference's `*a /= ...`
-      a = mk<Real>((Real)(((double)a.x * norm) / d), (Real)(((double)a.y * norm) / d));
-    } else {
-      a = mk<Real>(0, 0);
+  // num-complex division by Complex::new(norm, 0.0), as the reference's `*a /= ...`
+  auto scaled = [&](V2<Real> a) { return mk<Real>((Real)(((double)a.x * norm) / d), (Real)(((double)a.y * norm) / d)); };
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (; p + 3 * stride < pairs; p += 4 * stride) {
+    V2<Real> a[4];
+    uint64_t at[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      at[k] = insert_zero(p + k * stride, qubit);
+      a[k] = ld_amp<Real>(amps + (at[k] | keep));
     }
-    st_amp<Real>(amps + i, a);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      st_amp<Real>(amps + (at[k] | keep), scaled(a[k]));
+      st_amp<Real>(amps + (at[k] | drop), mk<Real>(0, 0));
+    }
+  }
+  for (; p < pairs; p += stride) {
+    const uint64_t i = insert_zero(p, qubit);
+    st_amp<Real>(amps + (i | keep), scaled(ld_amp<Real>(amps + (i | keep))));
+    st_amp<Real>(amps + (i | drop), mk<Real>(0, 0));
   }
 }
 
@@ -193,233 +232,310 @@ cudaError_t launch_measure_pass(void* amps, int precision, uint32_t n, uint32_t 
                                 uint8_t* outcome_slot, cudaStream_t s) {
   const uint64_t len = 1ull << n;
   const uint64_t qb = 1ull << qubit;
-  double* sums = partials + 3 * (size_t)nblocks;
-  double* dec = sums + 4;
+  double* dec = partials + 3 * (size_t)nblocks;
   if (precision == ALEPH_B200_F64) branch_kernel<double><<<nblocks, RB, 0, s>>>((const double2*)amps, len, qb, partials);
   else branch_kernel<float><<<nblocks, RB, 0, s>>>((const float2*)amps, len, qb, partials);
-  finish_kernel<3><<<1, 32, 0, s>>>(partials, nblocks, sums);
-  measure_decide_kernel<<<1, 32, 0, s>>>(sums, qubit, len, uniforms, n_uniforms, status, dec, outcome_slot,
+  measure_decide_kernel<<<1, 96, 0, s>>>(partials, nblocks, qubit, uniforms, n_uniforms, status, dec, outcome_slot,
                                          norm_tolerance(len, precision));
-  const uint64_t b = (len + 255) / 256;
+  const uint64_t pairs = len / 2, b = (pairs + 255) / 256;
   const unsigned blocks = (unsigned)(b > 148ull * 32 ? 148ull * 32 : b);
-  if (precision == ALEPH_B200_F64) collapse_kernel<double><<<blocks, 256, 0, s>>>((double2*)amps, len, qb, dec);
-  else collapse_kernel<float><<<blocks, 256, 0, s>>>((float2*)amps, len, qb, dec);
-  return cudaGetLastError();
-}
-
-// ---- Pauli expectation: [sum |a|^2, non-finite count, Re <psi|P|psi>] ----------
-// P = (x) Paulis with X/Y positions `xmask` (flip), Z/Y positions `zmask`
-// (sign), ny = number of Y factors. (P psi)_i = i^ny (-1)^{popc(zmask & j)} psi_j
-// with j = i ^ xmask: Y = i X Z, X flips, Z signs the pre-image bit.
-template <typename Real>
-__global__ void __launch_bounds__(RB) expect_kernel(const V2<Real>* __restrict__ amps, uint64_t len, uint64_t xmask,
-                                                    uint64_t zmask, uint32_t ny, double* __restrict__ partials) {
-  double v[3] = {0.0, 0.0, 0.0};
-  for (uint64_t i = (uint64_t)blockIdx.x * RB + threadIdx.x; i < len; i += (uint64_t)gridDim.x * RB) {
-    const V2<Real> a = ld_amp<Real>(amps + i);
-    const double p = abs2<Real>(a);
-    if (!isfinite(p)) {
-      v[1] += 1.0;
-      continue;
-    }
-    v[0] += p;
-    const uint64_t j = i ^ xmask;
-    const V2<Real> b = (xmask == 0) ? a : ld_amp<Real>(amps + j);
-    // conj(a) * b
-    double re = (double)a.x * b.x + (double)a.y * b.y;
-    double im = (double)a.x * b.y - (double)a.y * b.x;
-    if (__popcll(zmask & j) & 1) {
-      re = -re;
-      im = -im;
-    }
-    // multiply by i^ny and keep the real part
-    switch (ny & 3) {
-      case 0: v[2] += re; break;
-      case 1: v[2] += -im; break;
-      case 2: v[2] += -re; break;
-      default: v[2] += im; break;
-    }
-  }
-  block_reduce_store<3>(v, partials + 3 * blockIdx.x);
-}
-
-cudaError_t launch_expectation(const void* amps, int precision, uint32_t n, uint64_t xmask, uint64_t zmask,
-                               uint32_t ny, double* partials, uint32_t nblocks, double* out3, cudaStream_t s) {
-  const uint64_t len = 1ull << n;
-  if (precision == ALEPH_B200_F64)
-    expect_kernel<double><<<nblocks, RB, 0, s>>>((const double2*)amps, len, xmask, zmask, ny, partials);
-  else
-    expect_kernel<float><<<nblocks, RB, 0, s>>>((const float2*)amps, len, xmask, zmask, ny, partials);
-  finish_kernel<3><<<1, 32, 0, s>>>(partials, nblocks, out3);
+  if (precision == ALEPH_B200_F64) collapse_kernel<double><<<blocks, 256, 0, s>>>((double2*)amps, pairs, qubit, dec);
+  else collapse_kernel<float><<<blocks, 256, 0, s>>>((float2*)amps, pairs, qubit, dec);
   return cudaGetLastError();
 }
 
 // ---- Pauli sum: up to 16 terms that share one X/Y (flip) mask, one sweep ----------
-// For every term: Re <psi|P|psi> with P as in expect_kernel. (P psi)_i differs
-// between the terms of a group only in the sign (-1)^{popc(zmask & j)} and the
-// factor i^ny, so conj(a_i) a_j is formed once per amplitude and shared.
-// partials per block: [sum |a|^2, non-finite count, term 0 .. 15].
-template <typename Real, bool DIAG>
-__global__ void __launch_bounds__(RB) pauli_group_kernel(const V2<Real>* __restrict__ amps, uint64_t len,
-                                                         const PauliGroup g, double* __restrict__ partials) {
-  double v[2 + PauliGroup::MAX_TERMS];
+// P = (x) Paulis with X/Y positions `xmask` (flip), Z/Y positions `zmask`
+// (sign), ny = number of Y factors. (P psi)_i = i^ny (-1)^{popc(zmask & j)} psi_j
+// with j = i ^ xmask: Y = i X Z, X flips, Z signs the pre-image bit. The terms of
+// a group differ only in the sign and in i^ny, so conj(a_i) a_j is formed once
+// per pair and shared. i and j contribute the same real part (P is Hermitian:
+// the two products are conjugate to each other), so with a flip a thread takes
+// the pair once, at the member with the mask's highest bit clear: every
+// amplitude is read once and the products are formed once. (One thread per
+// member read everything twice: 93 us a group at n = 23 FP64 against 28 us
+// now, with the terms unrolled to the group's size and not to 16.)
+// partials per block: [sum |a|^2, non-finite count, term 0 .. NT-1].
+template <typename Real, bool DIAG, int NT>
+__global__ void __launch_bounds__(RB) pauli_group_kernel(const V2<Real>* __restrict__ amps, uint64_t count,
+                                                         const PauliGroup g, uint32_t pivot,
+                                                         double* __restrict__ partials) {
+  constexpr int NV = 2 + NT, U = 4;
+  double v[NV];
 #pragma unroll
-  for (int k = 0; k < 2 + PauliGroup::MAX_TERMS; ++k) v[k] = 0.0;
+  for (int k = 0; k < NV; ++k) v[k] = 0.0;
   const uint64_t stride = (uint64_t)gridDim.x * RB;
-  uint64_t i0 = (uint64_t)blockIdx.x * RB + threadIdx.x;
-  if constexpr (DIAG) {  // no X/Y factor: Re conj(a) a = |a|^2 and ny = 0
-    auto add = [&](uint64_t i, double p) {
-      if (!isfinite(p)) {
-        v[1] += 1.0;
-        return;
-      }
-      v[0] += p;
-#pragma unroll
-      for (int k = 0; k < PauliGroup::MAX_TERMS; ++k)
-        if (k < (int)g.count) v[2 + k] += (__popcll(g.zmask[k] & i) & 1) ? -p : p;
-    };
-    for (; i0 + 3 * stride < len; i0 += 4 * stride) {  // four loads in flight per step (see norm_kernel)
-      V2<Real> a[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) a[k] = ld_amp<Real>(amps + i0 + k * stride);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) add(i0 + k * stride, abs2<Real>(a[k]));
-    }
-  }
-  for (uint64_t i = i0; i < len; i += stride) {
-    const V2<Real> a = ld_amp<Real>(amps + i);
-    const double p = abs2<Real>(a);
-    if (!isfinite(p)) {
+  auto add = [&](uint64_t i, V2<Real> a, V2<Real> b) {
+    const double p = abs2<Real>(a), q = DIAG ? 0.0 : abs2<Real>(b);
+    if (!isfinite(p) || !isfinite(q)) {
       v[1] += 1.0;
-      continue;
+      return;
     }
-    v[0] += p;
-    if constexpr (DIAG) {
+    v[0] += p + q;
+    if constexpr (DIAG) {  // no X/Y factor: Re conj(a) a = |a|^2 and ny = 0
 #pragma unroll
-      for (int k = 0; k < PauliGroup::MAX_TERMS; ++k)
+      for (int k = 0; k < NT; ++k)
         if (k < (int)g.count) v[2 + k] += (__popcll(g.zmask[k] & i) & 1) ? -p : p;
     } else {
       const uint64_t j = i ^ g.xmask;
-      const V2<Real> b = ld_amp<Real>(amps + j);
       const double re = (double)a.x * b.x + (double)a.y * b.y;  // conj(a) * b
       const double im = (double)a.x * b.y - (double)a.y * b.x;
 #pragma unroll
-      for (int k = 0; k < PauliGroup::MAX_TERMS; ++k)
+      for (int k = 0; k < NT; ++k)
         if (k < (int)g.count) {
           // i^ny: ny & 3 = 0, 1, 2, 3 keeps re, -im, -re, im
-          const uint32_t q = g.ny[k] & 3;
-          double t = (q & 1) ? im : re;
-          if ((q == 1 || q == 2) != (bool)(__popcll(g.zmask[k] & j) & 1)) t = -t;
+          const uint32_t y = g.ny[k] & 3;
+          double t = (y & 1) ? im : re;
+          if ((y == 1 || y == 2) != (bool)(__popcll(g.zmask[k] & j) & 1)) t = -t;
           v[2 + k] += t;
         }
     }
+  };
+  auto index = [&](uint64_t p) { return DIAG ? p : insert_zero(p, pivot); };
+  uint64_t p0 = (uint64_t)blockIdx.x * RB + threadIdx.x;
+  for (; p0 + (U - 1) * stride < count; p0 += U * stride) {  // loads in flight (see norm_kernel)
+    V2<Real> a[U], b[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const uint64_t i = index(p0 + k * stride);
+      a[k] = ld_amp<Real>(amps + i);
+      if constexpr (!DIAG) b[k] = ld_amp<Real>(amps + (i ^ g.xmask));
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) add(index(p0 + k * stride), a[k], DIAG ? a[k] : b[k]);
   }
-  block_reduce_store<2 + PauliGroup::MAX_TERMS>(v, partials + (2 + PauliGroup::MAX_TERMS) * (size_t)blockIdx.x);
+  for (; p0 < count; p0 += stride) {
+    const uint64_t i = index(p0);
+    const V2<Real> a = ld_amp<Real>(amps + i);
+    add(i, a, DIAG ? a : ld_amp<Real>(amps + (i ^ g.xmask)));
+  }
+  if constexpr (!DIAG) {  // both members of each pair
+#pragma unroll
+    for (int k = 0; k < NT; ++k) v[2 + k] *= 2.0;
+  }
+  block_reduce_store<NV>(v, partials + NV * (size_t)blockIdx.x);
+}
+
+template <typename Real, int NT>
+static cudaError_t launch_pauli_t(const V2<Real>* amps, uint32_t n, const PauliGroup& g, double* partials,
+                                  uint32_t nblocks, double* out, cudaStream_t s) {
+  const uint64_t len = 1ull << n;
+  if (g.xmask == 0)
+    pauli_group_kernel<Real, true, NT><<<nblocks, RB, 0, s>>>(amps, len, g, 0, partials);
+  else
+    pauli_group_kernel<Real, false, NT>
+        <<<nblocks, RB, 0, s>>>(amps, len / 2, g, 63u - (uint32_t)__builtin_clzll(g.xmask), partials);
+  finish_kernel<2 + NT><<<1, 32 * (2 + NT), 0, s>>>(partials, nblocks, out);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_pauli_group(const void* amps, int precision, uint32_t n, const PauliGroup& g, double* partials,
                                uint32_t nblocks, double* out, cudaStream_t s) {
-  const uint64_t len = 1ull << n;
-  constexpr int NV = 2 + PauliGroup::MAX_TERMS;
   if (g.count == 0 || g.count > (uint32_t)PauliGroup::MAX_TERMS) return cudaErrorInvalidValue;
-  const bool diag = g.xmask == 0;
-  if (precision == ALEPH_B200_F64) {
-    if (diag) pauli_group_kernel<double, true><<<nblocks, RB, 0, s>>>((const double2*)amps, len, g, partials);
-    else pauli_group_kernel<double, false><<<nblocks, RB, 0, s>>>((const double2*)amps, len, g, partials);
-  } else {
-    if (diag) pauli_group_kernel<float, true><<<nblocks, RB, 0, s>>>((const float2*)amps, len, g, partials);
-    else pauli_group_kernel<float, false><<<nblocks, RB, 0, s>>>((const float2*)amps, len, g, partials);
+  // accumulators for 1, 2, 4, 8 or 16 terms
+  uint32_t slots = 1;
+  while (slots < g.count) slots *= 2;
+  const bool f64 = precision == ALEPH_B200_F64;
+  switch (slots) {
+#define AB_PAULI(nt)                                                                                    \
+  case nt:                                                                                              \
+    return f64 ? launch_pauli_t<double, nt>((const double2*)amps, n, g, partials, nblocks, out, s)      \
+               : launch_pauli_t<float, nt>((const float2*)amps, n, g, partials, nblocks, out, s);
+    AB_PAULI(1)
+    AB_PAULI(2)
+    AB_PAULI(4)
+    AB_PAULI(8)
+    AB_PAULI(16)
+#undef AB_PAULI
   }
-  finish_kernel<NV><<<1, 32, 0, s>>>(partials, nblocks, out);
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;
+}
+
+// One Pauli string: [sum |a|^2, non-finite count, Re <psi|P|psi>].
+cudaError_t launch_expectation(const void* amps, int precision, uint32_t n, uint64_t xmask, uint64_t zmask,
+                               uint32_t ny, double* partials, uint32_t nblocks, double* out3, cudaStream_t s) {
+  PauliGroup g{};
+  g.xmask = xmask;
+  g.count = 1;
+  g.zmask[0] = zmask;
+  g.ny[0] = ny;
+  return launch_pauli_group(amps, precision, n, g, partials, nblocks, out3, s);
 }
 
 // ---- marginal probabilities ------------------------------------------------------
-// k <= 10: per-block shared-memory histograms, summed by a second kernel.
+// out[o] = sum of |a_i|^2 over the basis states i whose selected qubits spell
+// o. Lanes are qubits 0..4, so every load is one run of 32 amplitudes. A warp
+// fixes the selected qubits above 4 (a pattern) and adds over the unselected
+// ones above 4 in its own registers; at the end a shuffle tree adds over the
+// unselected lane qubits. Where the patterns alone would leave the chip idle, the
+// unselected qubits' top `split_bits` are split over warps: 8 of a CTA meet in
+// shared memory, and a second kernel adds the CTAs' partial tables. No atomics,
+// one read of the state, and the norm comes with it. (At n = 23 FP64 a histogram
+// of shared-memory atomics took 150 us for 6 qubits and a thread per output 2.8 ms
+// for 12; both take 24 us now.)
+struct Marginal {
+  uint32_t k, lane_sel;  // selected count; mask of the selected lane qubits
+  uint32_t lanes;        // active lanes (32, or 2^n below 5 qubits)
+  uint32_t pat_bits, split_bits;
+  uint64_t pat_mask, split_mask, loop_mask;  // qubits above 4: selected / split / added in the loop
+  uint64_t loops;
+  uint8_t qubits[64];
+};
+
+__device__ __forceinline__ uint64_t deposit(uint64_t x, uint64_t mask) {  // bits of x into the set bits of mask
+  uint64_t r = 0;
+  while (mask && x) {
+    const uint64_t low = mask & (~mask + 1);
+    if (x & 1) r |= low;
+    x >>= 1;
+    mask ^= low;
+  }
+  return r;
+}
+
 template <typename Real>
-__global__ void __launch_bounds__(RB) hist_kernel(const V2<Real>* __restrict__ amps, uint64_t len,
-                                                  const uint32_t* __restrict__ qubits, uint32_t k,
-                                                  double* __restrict__ partials) {
-  extern __shared__ double hist[];
-  const uint32_t dim = 1u << k;
-  for (uint32_t i = threadIdx.x; i < dim; i += RB) hist[i] = 0.0;
-  __shared__ uint32_t qs[16];
-  if (threadIdx.x < k) qs[threadIdx.x] = qubits[threadIdx.x];
-  __syncthreads();
+__global__ void __launch_bounds__(RB) marginal_kernel(const V2<Real>* __restrict__ amps, const Marginal m,
+                                                      uint64_t items, double* __restrict__ tables,
+                                                      double* __restrict__ norm_partials) {
+  __shared__ double red[RB / 32][32];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool meet = m.split_bits >= 3;  // the CTA's warps are eight splits of one pattern
+  const bool on = lane < m.lanes;
+  uint32_t o_lane = 0;
+  for (uint32_t t = 0; t < m.k; ++t)
+    if (m.qubits[t] < 5) o_lane |= ((lane >> m.qubits[t]) & 1) << t;
   double v[2] = {0.0, 0.0};
-  for (uint64_t i = (uint64_t)blockIdx.x * RB + threadIdx.x; i < len; i += (uint64_t)gridDim.x * RB) {
-    const double p = abs2<Real>(ld_amp<Real>(amps + i));
-    if (!isfinite(p)) {
-      v[1] += 1.0;
-      continue;
+  const uint64_t warps = 1ull << (m.pat_bits + m.split_bits);
+  for (uint64_t item = blockIdx.x; item < items; item += gridDim.x) {
+    const uint64_t id = item * (RB / 32) + w;
+    double s = 0.0;
+    const uint64_t pat = id >> m.split_bits, split = id & ((1ull << m.split_bits) - 1);
+    const uint64_t fixed = deposit(pat, m.pat_mask);
+    if (id < warps && on) {
+      const V2<Real>* base = amps + (fixed | deposit(split, m.split_mask) | lane);
+      uint64_t x = 0;
+      auto next = [&] { x = ((x | ~m.loop_mask) + 1) & m.loop_mask; };
+      double bad = 0.0;
+      auto add = [&](double p) {
+        if (isfinite(p)) s += p;
+        else bad += 1.0;
+      };
+      uint64_t r = 0;
+      for (; r + 4 <= m.loops; r += 4) {  // four loads in flight (see norm_kernel)
+        V2<Real> a[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a[k] = ld_amp<Real>(base + x);
+          next();
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) add(abs2<Real>(a[k]));
+      }
+      for (; r < m.loops; ++r) {
+        add(abs2<Real>(ld_amp<Real>(base + x)));
+        next();
+      }
+      v[0] += s;
+      v[1] += bad;
     }
-    v[0] += p;
-    uint32_t o = 0;
-    for (uint32_t q = 0; q < k; ++q) o |= (uint32_t)((i >> qs[q]) & 1) << q;
-    atomicAdd(&hist[o], p);
+#pragma unroll
+    for (int b = 0; b < 5; ++b) {
+      const double other = __shfl_xor_sync(0xffffffffu, s, 1 << b);
+      if (!((m.lane_sel >> b) & 1)) s += other;
+    }
+    bool writes = id < warps && on && (lane & ~m.lane_sel) == 0;
+    uint64_t table = split;
+    if (meet) {
+      __syncthreads();  // the previous item's sums have been read
+      red[w][lane] = s;
+      __syncthreads();
+      s = 0.0;
+#pragma unroll
+      for (int x = 0; x < RB / 32; ++x) s += red[x][lane];
+      writes = writes && w == 0;
+      table = split >> 3;
+    }
+    if (writes) {
+      uint64_t o = o_lane;
+      for (uint32_t t = 0; t < m.k; ++t)
+        if (m.qubits[t] >= 5) o |= ((fixed >> m.qubits[t]) & 1) << t;
+      tables[(table << m.k) + o] = s;
+    }
   }
   __syncthreads();
-  double* out = partials + (size_t)blockIdx.x * (dim + 2);
-  for (uint32_t i = threadIdx.x; i < dim; i += RB) out[2 + i] = hist[i];
-  block_reduce_store<2>(v, out);
+  block_reduce_store<2>(v, norm_partials + 2 * (size_t)blockIdx.x);
 }
 
-__global__ void hist_finish_kernel(const double* __restrict__ partials, uint32_t nblocks, uint32_t dim,
-                                   double* __restrict__ out, double* __restrict__ norm_out) {
-  for (uint32_t o = blockIdx.x * blockDim.x + threadIdx.x; o < dim + 2; o += gridDim.x * blockDim.x) {
+// out[o] = sum over the tables, a warp per output in a fixed order.
+__global__ void __launch_bounds__(256) marginal_sum_kernel(const double* __restrict__ tables, uint32_t ntables,
+                                                           uint64_t dim, double* __restrict__ out) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint64_t o = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5); o < dim; o += (uint64_t)gridDim.x * 8) {
     double s = 0.0;
-    for (uint32_t b = 0; b < nblocks; ++b) s += partials[(size_t)b * (dim + 2) + o];
-    if (o < 2) norm_out[o] = s;
-    else out[o - 2] = s;
+    for (uint32_t t = lane; t < ntables; t += 32) s += tables[(uint64_t)t * dim + o];
+    for (int x = 16; x; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+    if (lane == 0) out[o] = s;
   }
 }
 
-// k > 10: one thread per output entry sums its pre-images in index order.
-template <typename Real>
-__global__ void marginal_kernel(const V2<Real>* __restrict__ amps, uint32_t n, const uint32_t* __restrict__ qubits,
-                                uint32_t k, double* __restrict__ out) {
-  uint64_t qmask = 0;
-  for (uint32_t q = 0; q < k; ++q) qmask |= 1ull << qubits[q];
-  const uint64_t dim = 1ull << k, rest = 1ull << (n - k);
-  for (uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; o < dim; o += (uint64_t)gridDim.x * blockDim.x) {
-    uint64_t fixed = 0;
-    for (uint32_t q = 0; q < k; ++q) fixed |= ((o >> q) & 1) << qubits[q];
-    double s = 0.0;
-    for (uint64_t r = 0; r < rest; ++r) {
-      // deposit r into the non-selected qubits
-      uint64_t x = fixed, rr = r;
-      for (uint32_t pos = 0; rr != 0 && pos < n; ++pos) {
-        if ((qmask >> pos) & 1) continue;
-        x |= (rr & 1) << pos;
-        rr >>= 1;
-      }
-      s += abs2<Real>(ld_amp<Real>(amps + x));
-    }
-    out[o] = s;
+namespace {
+struct MarginalPlan {
+  Marginal m;
+  uint64_t items;
+  uint32_t blocks, tables;
+};
+MarginalPlan plan_marginal(uint32_t n, const uint32_t* qubits, uint32_t k, int sm_count) {
+  MarginalPlan P{};
+  Marginal& m = P.m;
+  m.k = k;
+  m.lanes = n < 5 ? 1u << n : 32u;
+  uint64_t sel = 0;
+  for (uint32_t t = 0; t < k; ++t) {
+    sel |= 1ull << qubits[t];
+    m.qubits[t] = (uint8_t)qubits[t];
   }
+  m.lane_sel = (uint32_t)(sel & 31u) | (n < 5 ? 31u & ~((1u << n) - 1) : 0u);  // absent lane qubits: nothing to add
+  const uint64_t high = n > 5 ? ((1ull << n) - 1) & ~31ull : 0ull;
+  m.pat_mask = sel & high;
+  m.pat_bits = (uint32_t)__builtin_popcountll(m.pat_mask);
+  uint64_t rest = high & ~sel;
+  const uint32_t rest_bits = (uint32_t)__builtin_popcountll(rest);
+  // about 2^13 warps: 55 per SM, a little under what an SM holds
+  m.split_bits = m.pat_bits < 13 ? (rest_bits < 13 - m.pat_bits ? rest_bits : 13 - m.pat_bits) : 0;
+  for (uint32_t b = 0; b < m.split_bits; ++b) {
+    const uint64_t top = 1ull << (63 - __builtin_clzll(rest));
+    m.split_mask |= top;
+    rest ^= top;
+  }
+  m.loop_mask = rest;
+  m.loops = 1ull << (rest_bits - m.split_bits);
+  const uint64_t warps = 1ull << (m.pat_bits + m.split_bits);
+  P.items = (warps + RB / 32 - 1) / (RB / 32);
+  P.blocks = (uint32_t)(P.items < (uint64_t)sm_count * 8 ? P.items : (uint64_t)sm_count * 8);
+  P.tables = m.split_bits >= 3 ? 1u << (m.split_bits - 3) : 1u << m.split_bits;
+  return P;
+}
+}  // namespace
+
+size_t probabilities_scratch_bytes(uint32_t n, const uint32_t* qubits, uint32_t k, int sm_count) {
+  const MarginalPlan P = plan_marginal(n, qubits, k, sm_count);
+  return ((size_t)2 * P.blocks + (P.tables > 1 ? (size_t)P.tables << k : 0)) * 8;
 }
 
-cudaError_t launch_probabilities(const void* amps, int precision, uint32_t n, const uint32_t* qubits_dev, uint32_t k,
-                                 double* partials, uint32_t nblocks, double* out, double* norm_out, cudaStream_t s) {
-  const uint64_t len = 1ull << n;
-  if (k <= 10) {
-    const uint32_t dim = 1u << k;
-    const size_t sh = sizeof(double) * dim;
-    if (precision == ALEPH_B200_F64)
-      hist_kernel<double><<<nblocks, RB, sh, s>>>((const double2*)amps, len, qubits_dev, k, partials);
-    else
-      hist_kernel<float><<<nblocks, RB, sh, s>>>((const float2*)amps, len, qubits_dev, k, partials);
-    hist_finish_kernel<<<(dim + 2 + 255) / 256, 256, 0, s>>>(partials, nblocks, dim, out, norm_out);
-  } else {
-    launch_norm(amps, precision, n, partials, nblocks, norm_out, s);
-    const uint64_t dim = 1ull << k;
-    const uint64_t b = (dim + 255) / 256;
-    const unsigned blocks = (unsigned)(b > 148ull * 16 ? 148ull * 16 : b);
-    if (precision == ALEPH_B200_F64)
-      marginal_kernel<double><<<blocks, 256, 0, s>>>((const double2*)amps, n, qubits_dev, k, out);
-    else
-      marginal_kernel<float><<<blocks, 256, 0, s>>>((const float2*)amps, n, qubits_dev, k, out);
+cudaError_t launch_probabilities(const void* amps, int precision, uint32_t n, const uint32_t* qubits, uint32_t k,
+                                 double* scratch, double* out, double* norm_out, int sm_count, cudaStream_t s) {
+  const MarginalPlan P = plan_marginal(n, qubits, k, sm_count);
+  double* partials = scratch;
+  double* tables = P.tables > 1 ? scratch + 2 * (size_t)P.blocks : out;
+  if (precision == ALEPH_B200_F64)
+    marginal_kernel<double><<<P.blocks, RB, 0, s>>>((const double2*)amps, P.m, P.items, tables, partials);
+  else
+    marginal_kernel<float><<<P.blocks, RB, 0, s>>>((const float2*)amps, P.m, P.items, tables, partials);
+  if (P.tables > 1) {
+    const uint64_t dim = 1ull << k, b = (dim + 7) / 8;
+    marginal_sum_kernel<<<(unsigned)(b < 4096 ? b : 4096), 256, 0, s>>>(tables, P.tables, dim, out);
   }
+  finish_kernel<2><<<1, 64, 0, s>>>(partials, P.blocks, norm_out);
   return cudaGetLastError();
 }
 
