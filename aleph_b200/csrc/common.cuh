@@ -87,7 +87,8 @@ __device__ __forceinline__ double poly_phase(const PolyTables& t, uint32_t first
   return phi;
 }
 
-// Apply one diagonal op to an amplitude at global index g.
+// Apply one diagonal op to an amplitude at global index g (coefficients in
+// global or shared memory).
 template <typename Real>
 __device__ __forceinline__ V2<Real> apply_diag_op(const Op& op, V2<Real> a, uint64_t g, const V2<Real>* coef,
                                                   const PolyTables& poly) {
@@ -96,13 +97,13 @@ __device__ __forceinline__ V2<Real> apply_diag_op(const Op& op, V2<Real> a, uint
     case OP_NEG:
       return ((g & op.mask) == op.mask) ? cneg<Real>(a) : a;
     case OP_CPHASE:
-      return ((g & op.mask) == op.mask) ? cmul<Real>(ld_coef<Real>(coef + op.coef), a) : a;
+      return ((g & op.mask) == op.mask) ? cmul<Real>(coef[op.coef], a) : a;
     case OP_DIAG: {
       uint32_t idx = 0;
 #pragma unroll
       for (int i = 0; i < 3; ++i)
         if (i < op.nq) idx = (idx << 1) | (uint32_t)((g >> op.q[i]) & 1);
-      return cmul<Real>(ld_coef<Real>(coef + op.coef + idx), a);
+      return cmul<Real>(coef[op.coef + idx], a);
     }
     case OP_POLY: {
       const double phi = poly_phase(poly, (uint32_t)op.mask, op.aux, g);

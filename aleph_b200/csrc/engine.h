@@ -221,8 +221,9 @@ cudaError_t launch_init_zero_state(void* amps, uint32_t n, int precision, cudaSt
 // dev_error: set to ALEPH_B200_DEVICE_FAILURE by a pass kernel whose bounded copy wait expires.
 cudaError_t launch_tile_pass(void* amps, int precision, const TilePass& p, const Op* ops, const void* coef,
                              PolyTables poly, int* dev_error, int sm_count, cudaStream_t s);
+// coef_end: one past the last op's coefficients (the ops' coefficients are contiguous, in op order).
 cudaError_t launch_smem_pass(void* amps, int precision, uint32_t n, const Op* ops, uint32_t op_count,
-                             const void* coef, PolyTables poly, cudaStream_t s);
+                             const void* coef, uint32_t coef_end, PolyTables poly, cudaStream_t s);
 cudaError_t launch_kq_pass(void* amps, int precision, uint32_t n, const Op* op_dev, const Op& op_host,
                            const void* coef, cudaStream_t s);
 cudaError_t launch_block_pass(void* amps, const BlockPass& p, const uint8_t* images, const Op* ops,

@@ -15,84 +15,160 @@
 namespace ab {
 
 // ---- whole state in shared memory (n <= 12) ---------------------------------
-template <typename Real>
-__device__ void smem_apply_op(V2<Real>* sm, uint32_t n, const Op& op, const V2<Real>* coef, const PolyTables& poly) {
-  const uint64_t len = 1ull << n;
-  const V2<Real>* m = coef + op.coef;
-  if (is_diag_type(op.type)) {
-    for (uint64_t i = threadIdx.x; i < len; i += blockDim.x) sm[i] = apply_diag_op<Real>(op, sm[i], i, coef, poly);
-    return;
+// One CTA applies the whole op list; a barrier separates ops that move
+// amplitudes between threads. The list is latency-bound: at n = 10 an op is 256
+// quartets of arithmetic, about 0.2 us, and reading each op and its coefficients
+// from global memory when it is due cost 1.5 us more (146 us for the 86 gates of a
+// depth-4 Ry + CNOT ansatz in FP64). So ops and coefficients come to shared memory
+// in groups, one read each; runs of diagonal ops stay in registers without a
+// barrier; and the planner merges gates into 4x4s to halve the barriers.
+constexpr uint32_t SMEM_OPS = 64;        // ops per staged group
+constexpr uint32_t SMEM_COEFS = 2048;    // coefficients per staged group (one 5-qubit unitary is 1024)
+
+template <typename Real, int K>
+__device__ __forceinline__ void smem_dense(V2<Real>* sm, uint64_t groups, const Op& op, const V2<Real>* m) {
+  constexpr uint32_t DIM = 1u << K;
+  uint32_t sorted[K], bit[K];
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    sorted[i] = op.q[i];
+    bit[i] = 1u << op.q[K - 1 - i];  // matrix bit i <-> qubit q[K-1-i]
   }
-  const int k = op.type == OP_2Q ? 2 : (op.type == OP_KQ ? op.nq : 1);
-  uint32_t sorted[6];
-  for (int i = 0; i < k; ++i) sorted[i] = op.q[i];
-  for (int i = 1; i < k; ++i)
-    for (int j = i; j > 0 && sorted[j - 1] > sorted[j]; --j) {
-      uint32_t t = sorted[j];
-      sorted[j] = sorted[j - 1];
-      sorted[j - 1] = t;
-    }
-  const uint32_t dim = 1u << k;
-  const uint64_t groups = len >> k;
-  for (uint64_t gi = threadIdx.x; gi < groups; gi += blockDim.x) {
-    uint64_t base = gi;
-    for (int i = 0; i < k; ++i) base = insert_zero(base, sorted[i]);
+#pragma unroll
+  for (int i = 1; i < K; ++i)
+#pragma unroll
+    for (int j = i; j > 0; --j)
+      if (sorted[j - 1] > sorted[j]) {
+        const uint32_t t = sorted[j];
+        sorted[j] = sorted[j - 1];
+        sorted[j - 1] = t;
+      }
+  for (uint32_t gi = threadIdx.x; gi < groups; gi += blockDim.x) {
+    uint32_t base = gi;
+#pragma unroll
+    for (int i = 0; i < K; ++i) base = (uint32_t)insert_zero(base, sorted[i]);
     if ((base & op.ctrl) != op.ctrl) continue;
-    // offsets[c]: matrix bit p <-> qubit q[k-1-p]
-    auto off = [&](uint32_t c) {
-      uint64_t o = 0;
-      for (int p = 0; p < k; ++p)
-        if ((c >> p) & 1) o |= 1ull << op.q[k - 1 - p];
+    auto at = [&](uint32_t c) {
+      uint32_t o = base;
+#pragma unroll
+      for (int i = 0; i < K; ++i)
+        if ((c >> i) & 1) o |= bit[i];
       return o;
     };
-    if (op.type == OP_X) {
-      const uint64_t i1 = base | (1ull << op.q[0]);
-      V2<Real> t = sm[base];
-      sm[base] = sm[i1];
-      sm[i1] = t;
-      continue;
+    V2<Real> x[DIM];
+#pragma unroll
+    for (uint32_t c = 0; c < DIM; ++c) x[c] = sm[at(c)];
+#pragma unroll(DIM <= 8 ? (int)DIM : 1)
+    for (uint32_t r = 0; r < DIM; ++r) {
+      V2<Real> acc = cmul<Real>(m[r * DIM], x[0]);
+#pragma unroll
+      for (uint32_t c = 1; c < DIM; ++c) {
+        const V2<Real> u = m[r * DIM + c];
+        acc.x = fma(u.x, x[c].x, acc.x);
+        acc.y = fma(u.x, x[c].y, acc.y);
+        acc.x = fma(-u.y, x[c].y, acc.x);
+        acc.y = fma(u.y, x[c].x, acc.y);
+      }
+      sm[at(r)] = acc;
     }
-    V2<Real> x[32];
-    for (uint32_t c = 0; c < dim; ++c) x[c] = sm[base | off(c)];
-    for (uint32_t r = 0; r < dim; ++r) {
-      V2<Real> acc = mk<Real>(0, 0);
-      for (uint32_t c = 0; c < dim; ++c) acc = cadd<Real>(acc, cmul<Real>(ld_coef<Real>(m + r * dim + c), x[c]));
-      sm[base | off(r)] = acc;
+  }
+}
+
+template <typename Real>
+__device__ __forceinline__ void smem_apply_op(V2<Real>* sm, uint64_t len, const Op& op, const V2<Real>* m) {
+  switch (op.type == OP_KQ ? 8 + op.nq : op.type) {
+    case OP_X: {
+      const uint32_t bit = 1u << op.q[0];
+      for (uint32_t gi = threadIdx.x; gi < len / 2; gi += blockDim.x) {
+        const uint32_t i0 = (uint32_t)insert_zero(gi, op.q[0]);
+        if ((i0 & op.ctrl) != op.ctrl) continue;
+        const V2<Real> t = sm[i0];
+        sm[i0] = sm[i0 | bit];
+        sm[i0 | bit] = t;
+      }
+      break;
     }
+    case OP_1Q: smem_dense<Real, 1>(sm, len >> 1, op, m); break;
+    case OP_2Q: smem_dense<Real, 2>(sm, len >> 2, op, m); break;
+    case 8 + 3: smem_dense<Real, 3>(sm, len >> 3, op, m); break;
+    case 8 + 4: smem_dense<Real, 4>(sm, len >> 4, op, m); break;
+    case 8 + 5: smem_dense<Real, 5>(sm, len >> 5, op, m); break;
   }
 }
 
 template <typename Real>
 __global__ void __launch_bounds__(512) smem_kernel(V2<Real>* __restrict__ amps, uint32_t n, const Op* __restrict__ ops,
                                                    uint32_t op_count, const V2<Real>* __restrict__ coef,
-                                                   const PolyTables poly) {
+                                                   uint32_t coef_end, const PolyTables poly) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  V2<Real>* sm = reinterpret_cast<V2<Real>*>(smem_raw);
-  const uint64_t len = 1ull << n;
-  for (uint64_t i = threadIdx.x; i < len; i += blockDim.x) sm[i] = ld_amp<Real>(amps + i);
-  __syncthreads();
-  for (uint32_t o = 0; o < op_count; ++o) {
-    const Op op = ops[o];
-    smem_apply_op<Real>(sm, n, op, coef, poly);
+  V2<Real>* cf = reinterpret_cast<V2<Real>*>(smem_raw);
+  V2<Real>* sm = cf + SMEM_COEFS;
+  __shared__ Op group[SMEM_OPS + 1];
+  const uint32_t len = 1u << n;
+  for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) sm[i] = ld_amp<Real>(amps + i);
+  for (uint32_t o0 = 0; o0 < op_count;) {
+    // stage up to SMEM_OPS ops (and the next one, whose coefficients follow theirs)
+    uint32_t cnt = min(SMEM_OPS, op_count - o0);
+    const uint32_t words = min(cnt + 1, op_count - o0) * (uint32_t)(sizeof(Op) / 4);
     __syncthreads();
+    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x)
+      reinterpret_cast<uint32_t*>(group)[i] = reinterpret_cast<const uint32_t*>(ops + o0)[i];
+    __syncthreads();
+    const uint32_t c0 = group[0].coef;
+    auto end_of = [&](uint32_t c) { return o0 + c < op_count ? group[c].coef : coef_end; };
+    while (cnt > 1 && end_of(cnt) - c0 > SMEM_COEFS) cnt >>= 1;
+    const uint32_t nc = end_of(cnt) - c0;
+    for (uint32_t i = threadIdx.x; i < nc; i += blockDim.x) cf[i] = ld_coef<Real>(coef + c0 + i);
+    __syncthreads();
+    for (uint32_t k = 0; k < cnt;) {
+      if (is_diag_type(group[k].type)) {  // a run of diagonal ops: every thread keeps its amplitudes
+        uint32_t e = k + 1;
+        while (e < cnt && is_diag_type(group[e].type)) ++e;
+        for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) {
+          V2<Real> a = sm[i];
+          for (uint32_t x = k; x < e; ++x) a = apply_diag_op<Real>(group[x], a, i, cf - c0, poly);
+          sm[i] = a;
+        }
+        k = e;
+      } else {
+        smem_apply_op<Real>(sm, len, group[k], cf + (group[k].coef - c0));
+        ++k;
+      }
+      __syncthreads();
+    }
+    o0 += cnt;
   }
-  for (uint64_t i = threadIdx.x; i < len; i += blockDim.x) st_amp<Real>(amps + i, sm[i]);
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) st_amp<Real>(amps + i, sm[i]);
+}
+
+template <typename Real>
+static cudaError_t launch_smem_t(V2<Real>* amps, uint32_t n, const Op* ops, uint32_t op_count, const V2<Real>* coef,
+                                 uint32_t coef_end, PolyTables poly, cudaStream_t s) {
+  const size_t bytes = (((size_t)1 << n) + SMEM_COEFS) * sizeof(V2<Real>);
+  static uint64_t ready = 0;  // devices with the shared-memory opt-in
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= 64 || !((ready >> dev) & 1)) {
+    const int most = (int)(((1u << 12) + SMEM_COEFS) * sizeof(V2<Real>));
+    e = cudaFuncSetAttribute(smem_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e != cudaSuccess) return e;
+    if (dev < 64) ready |= 1ull << dev;
+  }
+  // a quartet per thread: fewer warps than that idle the SM, more only slow the barriers
+  const uint32_t quartets = n > 2 ? 1u << (n - 2) : 1u;
+  const uint32_t threads = quartets < 64 ? 64 : quartets > 512 ? 512 : quartets;
+  smem_kernel<Real><<<1, threads, bytes, s>>>(amps, n, ops, op_count, coef, coef_end, poly);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_smem_pass(void* amps, int precision, uint32_t n, const Op* ops, uint32_t op_count,
-                             const void* coef, PolyTables poly, cudaStream_t s) {
+                             const void* coef, uint32_t coef_end, PolyTables poly, cudaStream_t s) {
   if (n > 12) return cudaErrorInvalidValue;
-  const size_t bytes = (precision == ALEPH_B200_F64 ? 16 : 8) << n;
-  if (precision == ALEPH_B200_F64) {
-    if (bytes > 48 * 1024)
-      cudaFuncSetAttribute(smem_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    smem_kernel<double><<<1, 512, bytes, s>>>((double2*)amps, n, ops, op_count, (const double2*)coef, poly);
-  } else {
-    if (bytes > 48 * 1024)
-      cudaFuncSetAttribute(smem_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    smem_kernel<float><<<1, 512, bytes, s>>>((float2*)amps, n, ops, op_count, (const float2*)coef, poly);
-  }
-  return cudaGetLastError();
+  if (precision == ALEPH_B200_F64)
+    return launch_smem_t<double>((double2*)amps, n, ops, op_count, (const double2*)coef, coef_end, poly, s);
+  return launch_smem_t<float>((float2*)amps, n, ops, op_count, (const float2*)coef, coef_end, poly, s);
 }
 
 // ---- dense k-qubit op on arbitrary qubits (UnitaryKq, k = 3..5) --------------

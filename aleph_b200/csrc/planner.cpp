@@ -580,7 +580,12 @@ bool fusable_type(const Lowered& L) {
 
 }  // namespace
 
-std::vector<const Lowered*> fuse_pairs(const std::vector<const Lowered*>& seg, std::deque<Lowered>& store) {
+// barrier_cost: what an op that moves amplitudes costs beside its arithmetic
+// (shared-memory passes: a barrier and its latency); 0 in tile passes.
+std::vector<const Lowered*> fuse_pairs(const std::vector<const Lowered*>& seg, std::deque<Lowered>& store,
+                                       int barrier_cost = 0) {
+  const int min_cost = barrier_cost ? 17 + barrier_cost : kFuseMinCost;
+  auto gate_cost = [&](const Lowered& L) { return tile_cost(L) + (L.nondiag ? barrier_cost : 0); };
   struct Block {
     uint32_t a, b;
     Cx m[16];
@@ -598,7 +603,7 @@ std::vector<const Lowered*> fuse_pairs(const std::vector<const Lowered*>& seg, s
     if (k < 0) return;
     Block& B = blocks[(size_t)k];
     open[B.a] = open[B.b] = -1;
-    if (B.cost >= kFuseMinCost) {
+    if (B.cost >= min_cost) {
       store.emplace_back();
       Lowered& F = store.back();
       std::memset(&F.op, 0, sizeof(Op));
@@ -642,7 +647,7 @@ std::vector<const Lowered*> fuse_pairs(const std::vector<const Lowered*>& seg, s
         Block& B = blocks[(size_t)k];
         fold_into_4x4(*L, B.a, B.b, B.m);
         B.members.push_back(L);
-        B.cost += tile_cost(*L);
+        B.cost += gate_cost(*L);
       } else {
         out.push_back(L);
         waiting[q].push_back(out.size() - 1);
@@ -655,7 +660,7 @@ std::vector<const Lowered*> fuse_pairs(const std::vector<const Lowered*>& seg, s
         Block& B = blocks[(size_t)open[lo]];
         fold_into_4x4(*L, B.a, B.b, B.m);
         B.members.push_back(L);
-        B.cost += tile_cost(*L);
+        B.cost += gate_cost(*L);
         continue;
       }
       close(lo);
@@ -670,14 +675,14 @@ std::vector<const Lowered*> fuse_pairs(const std::vector<const Lowered*>& seg, s
           const Lowered* W = out[idx];
           fold_into_4x4(*W, B.a, B.b, B.m);
           B.members.push_back(W);
-          B.cost += tile_cost(*W);
+          B.cost += gate_cost(*W);
           out[idx] = nullptr;
         }
         waiting[q].clear();
       }
       fold_into_4x4(*L, B.a, B.b, B.m);
       B.members.push_back(L);
-      B.cost += tile_cost(*L);
+      B.cost += gate_cost(*L);
       blocks.push_back(std::move(B));
       open[hi] = open[lo] = (int)blocks.size() - 1;
       continue;
@@ -695,6 +700,55 @@ std::vector<const Lowered*> fuse_pairs(const std::vector<const Lowered*>& seg, s
   for (const Lowered* L : out)
     if (L) compact.push_back(L);
   return compact;
+}
+
+// Shared-memory passes: after pair fusion, two dense one-qubit gates in a row
+// become one op, their product on one qubit or their 4x4 on two (one barrier
+// for two).
+constexpr int kBarrierCost = 16;
+std::vector<const Lowered*> fuse_for_smem(const std::vector<const Lowered*>& seg, std::deque<Lowered>& store) {
+  const std::vector<const Lowered*> in = fuse_pairs(seg, store, kBarrierCost);
+  auto plain_1q = [](const Lowered* L) { return L->op.type == OP_1Q && L->op.ctrl == 0; };
+  std::vector<const Lowered*> out;
+  out.reserve(in.size());
+  for (const Lowered* L : in) {
+    if (out.empty() || !plain_1q(L) || !plain_1q(out.back())) {
+      out.push_back(L);
+      continue;
+    }
+    const Lowered* W = out.back();
+    const uint32_t a = W->op.q[0], b = L->op.q[0];
+    store.emplace_back();
+    Lowered& F = store.back();
+    std::memset(&F.op, 0, sizeof(Op));
+    F.record = W->record;
+    F.gates = (W->gates ? W->gates : 1) + (L->gates ? L->gates : 1);
+    F.diag = 0;
+    F.nondiag = (1ull << a) | (1ull << b);
+    if (a == b) {
+      const Cx* u = reinterpret_cast<const Cx*>(W->coef.data());
+      const Cx* v = reinterpret_cast<const Cx*>(L->coef.data());
+      Cx m[4];
+      for (int r = 0; r < 2; ++r)
+        for (int c = 0; c < 2; ++c) m[2 * r + c] = add(mul(v[2 * r], u[c]), mul(v[2 * r + 1], u[2 + c]));
+      F.op.type = OP_1Q;
+      F.op.nq = 1;
+      F.op.q[0] = (uint8_t)a;
+      push_coef(&F, m, 4);
+    } else {
+      Cx m[16];
+      for (int i = 0; i < 16; ++i) m[i] = Cx{(i % 5) == 0 ? 1.0 : 0.0, 0.0};
+      fold_into_4x4(*W, a, b, m);
+      fold_into_4x4(*L, a, b, m);
+      F.op.type = OP_2Q;
+      F.op.nq = 2;
+      F.op.q[0] = (uint8_t)a;
+      F.op.q[1] = (uint8_t)b;
+      push_coef(&F, m, 16);
+    }
+    out.back() = &F;
+  }
+  return out;
 }
 
 int plan_segment_tiles(const std::vector<const Lowered*>& seg, uint32_t n, uint32_t R, Plan* P) {
@@ -1120,11 +1174,13 @@ int build_plan(const std::vector<Lowered>& ops, uint32_t n, const PlanOptions& o
       ps.kind = PASS_SMEM;
       ps.tile.n = n;
       ps.tile.op_begin = (uint32_t)P->ops.size();
-      for (const Lowered* L : seg) append_op(P, *L, L->op);
+      std::deque<Lowered> fused;
+      const std::vector<const Lowered*> list = o.pair_fusion ? fuse_for_smem(seg, fused) : seg;
+      for (const Lowered* L : list) append_op(P, *L, L->op);
       ps.tile.op_count = (uint32_t)P->ops.size() - ps.tile.op_begin;
       ps.record = seg.front()->record;
       ps.gates = (uint32_t)seg.size();
-      count_ops(seg, &ps);
+      count_ops(list, &ps);
       P->passes.push_back(ps);
     } else {
       // a 2-qubit gate may need two register qubits: R >= 2 unless only one high qubit exists
