@@ -282,7 +282,11 @@ struct BlockArgs {
   int* err;
   uint32_t n;
   uint32_t bq[6];
-  uint64_t tmask;                       // tile qubits: block + column qubits
+  // The non-tile qubits as runs of consecutive positions: tile index bits
+  // [dep_src, dep_src + len) land on qubits [dep_dst, dep_dst + len). At most
+  // 14: the 13 tile qubits leave at most 14 gaps.
+  uint32_t n_dep;
+  uint32_t dep_src[14], dep_mask[14], dep_dst[14];
   uint32_t nruns, run_bytes, run_stride;  // contiguous runs of a tile; stage bytes between runs
   // Per block row j: byte offset in a stage and global offset. Kept in the
   // kernel-parameter (constant) bank so the unrolled per-element loops of the
@@ -323,12 +327,9 @@ __global__ void __launch_bounds__(blk::THREADS, 1) block_kernel(const __grid_con
   __shared__ uint64_t fold_cmask[MAX_POST];
   __shared__ int8_t fold_rbit[MAX_POST], fold_col[MAX_POST];
   __shared__ float2 fold_c0[MAX_POST], fold_c1[MAX_POST];
-  __shared__ Op other_ops[MAX_POST];
+  __shared__ Op post_ops[MAX_POST];
+  __shared__ int8_t other_ops[MAX_POST];  // indices in post_ops
   __shared__ int n_neg_sh, n_other_sh, n_fold_sh;
-  // The non-tile qubits as runs of consecutive positions: tile index bits
-  // [dep_src, dep_src + len) land on qubits [dep_dst, dep_dst + len).
-  __shared__ uint32_t dep_src[16], dep_mask[16], dep_dst[16];
-  __shared__ int n_dep_sh;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t n = a.n;
@@ -337,7 +338,6 @@ __global__ void __launch_bounds__(blk::THREADS, 1) block_kernel(const __grid_con
   // ---- tile geometry (computed on the host) ---------------------------------
   uint64_t bmask = 0;
   for (int j = 0; j < 6; ++j) bmask |= 1ull << a.bq[j];
-  const uint64_t tmask = a.tmask;
   const uint32_t nruns = a.nruns, run_bytes = a.run_bytes, run_stride = a.run_stride;
   if (tid < NCOL) {
     Lcol[tid] = a.coloff[tid];
@@ -356,64 +356,14 @@ __global__ void __launch_bounds__(blk::THREADS, 1) block_kernel(const __grid_con
     }
     fence_barrier_init();
     abort_sh = 0;
-    int nd = 0;
-    for (uint32_t q = 0, src = 0; q < n;) {
-      if ((tmask >> q) & 1) {
-        ++q;
-        continue;
-      }
-      uint32_t len = 0;
-      while (q + len < n && !((tmask >> (q + len)) & 1)) ++len;
-      dep_src[nd] = src;
-      dep_mask[nd] = (1u << len) - 1;  // len <= n - 13 <= 27
-      dep_dst[nd] = q;
-      ++nd;
-      src += len;
-      q += len;
-    }
-    n_dep_sh = nd;  // at most 14: the 13 tile qubits leave at most 14 gaps
-    int nn = 0, no = 0, nf = 0;
-    const uint32_t cnt = a.post_count < (uint32_t)MAX_POST ? a.post_count : (uint32_t)MAX_POST;
-    for (uint32_t o = 0; o < cnt; ++o) {
-      const Op op = a.post[o];
-      if (op.type == OP_NEG) {
-        uint64_t rows = 0;
-        for (int j = 0; j < 64; ++j) {
-          uint64_t gr = 0;
-          for (int b = 0; b < 6; ++b)
-            if ((j >> b) & 1) gr |= 1ull << a.bq[b];
-          if ((gr & op.mask & bmask) == (op.mask & bmask)) rows |= 1ull << j;
-        }
-        neg_rows[nn] = rows;
-        neg_cmask[nn] = op.mask & ~bmask;
-        ++nn;
-      } else if (FOLD && op.type == OP_CPHASE && __popcll(op.mask & bmask) <= 1) {
-        // a phase on a corner: at most one block qubit, the rest a column condition
-        const uint64_t rm = op.mask & bmask;
-        int rb = -1;
-        for (int b = 0; b < 6; ++b)
-          if (rm == (1ull << a.bq[b])) rb = b;
-        fold_cmask[nf] = op.mask & ~bmask;
-        fold_rbit[nf] = (int8_t)rb;
-        fold_col[nf] = -1;
-        fold_c0[nf] = fold_c1[nf] = a.coef[op.coef];
-        ++nf;
-      } else if (FOLD && op.type == OP_DIAG && op.nq == 1 && !((bmask >> op.q[0]) & 1) && !(op.ctrl & bmask)) {
-        // a one-qubit diagonal on a column qubit (controls on columns too)
-        fold_cmask[nf] = op.ctrl;
-        fold_rbit[nf] = -1;
-        fold_col[nf] = (int8_t)op.q[0];
-        fold_c0[nf] = a.coef[op.coef];
-        fold_c1[nf] = a.coef[op.coef + 1];
-        ++nf;
-      } else {
-        other_ops[no++] = op;
-      }
-    }
-    n_neg_sh = nn;
-    n_other_sh = no;
-    n_fold_sh = nf;
   }
+  // Post ops: staged with one read each, then classified by one warp, a lane per
+  // op, each class in op order. (One thread reading them one after the other
+  // and forming the 64-row masks bit by bit took about 4 us per op before the
+  // first tile; at n = 19, where a CTA has at most one tile, that was a third of the pass.)
+  const uint32_t cnt = a.post_count < (uint32_t)MAX_POST ? a.post_count : (uint32_t)MAX_POST;
+  for (uint32_t i = tid; i < cnt * (uint32_t)(sizeof(Op) / 4); i += THREADS)
+    reinterpret_cast<uint32_t*>(post_ops)[i] = reinterpret_cast<const uint32_t*>(a.post)[i];
   if (warp == 0) {
     tmem_alloc(smem_u32(&tmem_base_sh), TMEM_COLS);
     tmem_relinquish();
@@ -422,13 +372,68 @@ __global__ void __launch_bounds__(blk::THREADS, 1) block_kernel(const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_base_sh;
+  // The epilogue warps classify the post ops; the loads, conversions and MMAs of the first tile run meanwhile.
+  if (warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS) {
+    if (warp == EPI_WARP0) {
+      int nn = 0, no = 0, nf = 0;
+      for (uint32_t o0 = 0; o0 < cnt; o0 += 32) {
+        const uint32_t o = o0 + lane;
+        const bool on = o < cnt;
+        const Op op = post_ops[on ? o : 0];
+        const uint64_t rm = op.mask & bmask;
+        const bool neg = on && op.type == OP_NEG;
+        // a phase on a corner: at most one block qubit, the rest a column condition
+        const bool corner = FOLD && on && op.type == OP_CPHASE && __popcll(rm) <= 1;
+        // a one-qubit diagonal on a column qubit (controls on columns too)
+        const bool diag1 = FOLD && on && op.type == OP_DIAG && op.nq == 1 && !((bmask >> op.q[0]) & 1) && !(op.ctrl & bmask);
+        const bool other = on && !neg && !corner && !diag1;
+        const unsigned bn = __ballot_sync(0xffffffffu, neg), bf = __ballot_sync(0xffffffffu, corner || diag1),
+                       bo = __ballot_sync(0xffffffffu, other);
+        const unsigned below = (1u << lane) - 1u;
+        if (neg) {
+          // rows whose bits cover the op's block qubits: the AND of one 64-row pattern per qubit
+          uint64_t rows = ~0ull;
+#pragma unroll
+          for (int b = 0; b < 6; ++b) {
+            constexpr uint64_t pat[6] = {0xAAAAAAAAAAAAAAAAull, 0xCCCCCCCCCCCCCCCCull, 0xF0F0F0F0F0F0F0F0ull,
+                                         0xFF00FF00FF00FF00ull, 0xFFFF0000FFFF0000ull, 0xFFFFFFFF00000000ull};
+            if ((rm >> a.bq[b]) & 1) rows &= pat[b];
+          }
+          const int k = nn + __popc(bn & below);
+          neg_rows[k] = rows;
+          neg_cmask[k] = op.mask & ~bmask;
+        } else if (corner || diag1) {
+          int rb = -1;
+          for (int b = 0; b < 6; ++b)
+            if (corner && rm == (1ull << a.bq[b])) rb = b;
+          const int k = nf + __popc(bf & below);
+          fold_cmask[k] = corner ? op.mask & ~bmask : op.ctrl;
+          fold_rbit[k] = (int8_t)rb;
+          fold_col[k] = corner ? (int8_t)-1 : (int8_t)op.q[0];
+          fold_c0[k] = a.coef[op.coef];
+          fold_c1[k] = a.coef[op.coef + (corner ? 0 : 1)];
+        } else if (other) {
+          other_ops[no + __popc(bo & below)] = (int8_t)o;
+        }
+        nn += __popc(bn);
+        nf += __popc(bf);
+        no += __popc(bo);
+      }
+      if (lane == 0) {
+        n_neg_sh = nn;
+        n_other_sh = no;
+        n_fold_sh = nf;
+      }
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(32 * EPI_WARPS) : "memory");  // the epilogue warps only
+  }
 
   const uint64_t ntiles = 1ull << (n - 13);
-  const int n_dep = n_dep_sh;
+  const int n_dep = (int)a.n_dep;
   auto tile_base = [&](uint64_t t) -> uint64_t {  // deposit a tile index into the non-tile qubits
     const uint32_t tt = (uint32_t)t;              // n - 13 <= 27 bits
     uint64_t base = 0;
-    for (int k = 0; k < n_dep; ++k) base |= (uint64_t)((tt >> dep_src[k]) & dep_mask[k]) << dep_dst[k];
+    for (int k = 0; k < n_dep; ++k) base |= (uint64_t)((tt >> a.dep_src[k]) & a.dep_mask[k]) << a.dep_dst[k];
     return base;
   };
   const uint64_t first = blockIdx.x, stride = gridDim.x;
@@ -632,7 +637,7 @@ __global__ void __launch_bounds__(blk::THREADS, 1) block_kernel(const __grid_con
                 for (int r = 0; r < 8; ++r) {
                   float2 y = eo[r * 32 + lane];
                   const uint64_t g = a.grow[j0 + r];
-                  for (int o = 0; o < n_other; ++o) y = apply_diag_op<float>(other_ops[o], y, gc | g, a.coef, a.poly);
+                  for (int o = 0; o < n_other; ++o) y = apply_diag_op<float>(post_ops[other_ops[o]], y, gc | g, a.coef, a.poly);
                   __stcs(pc + g, y);
                 }
               }
@@ -680,22 +685,19 @@ __global__ void __launch_bounds__(blk::THREADS, 1) block_kernel(const __grid_con
 namespace {
 
 // Bank-conflict degree of one warp's 8-byte shared-memory accesses at byte
-// offsets off[0..32): the most distinct 4-byte words any of the 32 banks
-// serves (2 is the minimum: 256 bytes take two 128-byte wavefronts).
+// offsets off[0..32) (multiples of 8): the most distinct 4-byte words any of
+// the 32 banks serves (2 is the minimum: 256 bytes take two 128-byte
+// wavefronts). An access covers one even bank and the next, so the even banks decide.
 int conflict_degree(const uint32_t* off) {
+  uint32_t words[16][32];
+  int count[16] = {};
   int worst = 0;
-  for (uint32_t bank = 0; bank < 32; ++bank) {
-    uint32_t words[64];
-    int nw = 0;
-    for (int t = 0; t < 32; ++t)
-      for (uint32_t h = 0; h < 2; ++h) {
-        const uint32_t w = off[t] / 4 + h;
-        if (w % 32 != bank) continue;
-        bool seen = false;
-        for (int k = 0; k < nw; ++k) seen = seen || words[k] == w;
-        if (!seen) words[nw++] = w;
-      }
-    worst = nw > worst ? nw : worst;
+  for (int t = 0; t < 32; ++t) {
+    const uint32_t w = off[t] / 8, bank = w % 16;
+    bool seen = false;
+    for (int k = 0; k < count[bank]; ++k) seen = seen || words[bank][k] == w;
+    if (!seen) words[bank][count[bank]++] = w;
+    worst = count[bank] > worst ? count[bank] : worst;
   }
   return worst;
 }
@@ -708,8 +710,10 @@ int conflict_degree(const uint32_t* off) {
 // non-block qubits under the block plus the ones above a one-qubit gap after
 // it (so that those columns index runs, which the pad skews across banks).
 // The candidate and pad with the fewest bank conflicts for the 32 columns of
-// a warp win (ties: the first, natural and unpadded).
-void set_tile_geometry(uint32_t n, const uint32_t* bq, BlockArgs* a) {
+// a warp win (ties: the first, natural and unpadded). Returns the tile qubits.
+// Every launch computes this; the tables are built by doubling (they and a slower
+// conflict count took longer on the host than a pass does on the device at n = 19).
+uint64_t set_tile_geometry(uint32_t n, const uint32_t* bq, BlockArgs* a) {
   using namespace blk;
   uint64_t bmask = 0;
   uint32_t bmax = 0;
@@ -764,7 +768,6 @@ void set_tile_geometry(uint32_t n, const uint32_t* bq, BlockArgs* a) {
   for (int k = 0; k < 7; ++k) tmask |= 1ull << cols[k];
   uint32_t c = 0;
   while (c < 13 && ((tmask >> c) & 1)) ++c;
-  a->tmask = tmask;
   a->nruns = 1u << (13 - c);
   a->run_bytes = 8u << c;
   a->run_stride = a->run_bytes + best_pad;
@@ -772,40 +775,42 @@ void set_tile_geometry(uint32_t n, const uint32_t* bq, BlockArgs* a) {
     const uint32_t pos = (uint32_t)__builtin_popcountll(tmask & ((1ull << q) - 1));
     return pos < c ? 8u << pos : a->run_stride << (pos - c);
   };
-  for (uint32_t j = 0; j < 64; ++j) {
-    uint32_t ro = 0;
-    uint64_t gr = 0;
-    for (int b = 0; b < 6; ++b)
-      if ((j >> b) & 1) {
-        ro += stride(bq[b]);
-        gr |= 1ull << bq[b];
-      }
-    a->rowoff[j] = ro;
-    a->grow[j] = gr;
-  }
-  for (uint32_t col = 0; col < (uint32_t)NCOL; ++col) {
-    uint32_t co = 0;
-    uint64_t gc = 0;
-    for (int k = 0; k < 7; ++k)
-      if ((col >> k) & 1) {
-        co += stride(cols[k]);
-        gc |= 1ull << cols[k];
-      }
-    a->coloff[col] = co;
-    a->gcol[col] = gc;
-  }
-  for (uint32_t r = 0; r < (uint32_t)MAX_RUNS; ++r) {  // run r: its bits -> the tile qubits from c up
-    uint64_t off = 0;
-    if (r < a->nruns) {
-      uint32_t bit = 0;
-      for (uint32_t q = c; q < n; ++q)
-        if ((tmask >> q) & 1) {
-          if ((r >> bit) & 1) off |= 1ull << q;
-          ++bit;
-        }
+  // offsets are sums over index bits: table[x] = table[x without its top bit] + that bit's offset
+  a->rowoff[0] = a->coloff[0] = 0;
+  a->grow[0] = a->gcol[0] = a->runoff[0] = 0;
+  for (int b = 0; b < 6; ++b)
+    for (uint32_t x = 0, w = 1u << b; x < w; ++x) {
+      a->rowoff[w + x] = a->rowoff[x] + stride(bq[b]);
+      a->grow[w + x] = a->grow[x] | 1ull << bq[b];
     }
-    a->runoff[r] = off;
+  for (int b = 0; b < 7; ++b)
+    for (uint32_t x = 0, w = 1u << b; x < w; ++x) {
+      a->coloff[w + x] = a->coloff[x] + stride(cols[b]);
+      a->gcol[w + x] = a->gcol[x] | 1ull << cols[b];
+    }
+  uint32_t runs = 1;  // run r: its bits -> the tile qubits from c up
+  for (uint32_t q = c; q < n; ++q)
+    if ((tmask >> q) & 1) {
+      for (uint32_t x = 0; x < runs; ++x) a->runoff[runs + x] = a->runoff[x] | 1ull << q;
+      runs *= 2;
+    }
+  for (uint32_t r = runs; r < (uint32_t)MAX_RUNS; ++r) a->runoff[r] = 0;
+  a->n_dep = 0;
+  for (uint32_t q = 0, src = 0; q < n;) {
+    if ((tmask >> q) & 1) {
+      ++q;
+      continue;
+    }
+    uint32_t len = 0;
+    while (q + len < n && !((tmask >> (q + len)) & 1)) ++len;
+    const uint32_t k = a->n_dep++;
+    a->dep_src[k] = src;
+    a->dep_mask[k] = (1u << len) - 1;  // len <= n - 13 <= 27
+    a->dep_dst[k] = q;
+    src += len;
+    q += len;
   }
+  return tmask;
 }
 
 // The tensor map of a tile box (BlockArgs::tmap), for two geometries:
@@ -821,13 +826,13 @@ void set_tile_geometry(uint32_t n, const uint32_t* bq, BlockArgs* a) {
 // Leaves trank = 0 (per-run bulk copies) for any other geometry, for more
 // than 5 dimensions, or when the driver's encoder is unavailable or refuses
 // the map.
-void set_tensor_map(uint32_t n, void* amps, BlockArgs* a) {
+void set_tensor_map(uint32_t n, void* amps, uint64_t tmask, BlockArgs* a) {
   using namespace blk;
   a->trank = 0;
   uint64_t bmask = 0;
   for (int j = 0; j < 6; ++j) bmask |= 1ull << a->bq[j];
   const bool high = !(bmask & 0x7F) && a->nruns == 64 && a->run_bytes == 1024 && a->run_stride == 1024;
-  const bool low = bmask == 0x3F && a->tmask == 0x3FBFull && a->nruns == 128 && a->run_bytes == 512 &&
+  const bool low = bmask == 0x3F && tmask == 0x3FBFull && a->nruns == 128 && a->run_bytes == 512 &&
                    a->run_stride == 528 && n >= 14;
   if (!high && !low) return;
   typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -913,8 +918,8 @@ cudaError_t launch_block_pass(void* amps, const BlockPass& p, const uint8_t* ima
   a.err = dev_error;
   a.n = p.n;
   for (int j = 0; j < 6; ++j) a.bq[j] = p.bq[j];
-  set_tile_geometry(p.n, p.bq, &a);
-  set_tensor_map(p.n, amps, &a);
+  const uint64_t tmask = set_tile_geometry(p.n, p.bq, &a);
+  set_tensor_map(p.n, amps, tmask, &a);
   static uint64_t attr_devices = 0;  // devices on which the shared-memory opt-in is done
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
