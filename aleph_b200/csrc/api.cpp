@@ -184,13 +184,13 @@ int execute(aleph_b200_handle* h, aleph_b200_state* st, const Plan& P, const dou
     coef32.resize(P.coef.size());
     for (size_t i = 0; i < P.coef.size(); ++i) coef32[i] = (float)P.coef[i];
   }
-  const size_t b_ops = al(P.ops.size() * sizeof(Op));
+  const size_t b_ops = al(P.ops.size() * sizeof(Op)), b_ph = al(P.phases.size() * sizeof(WidePhase));
   const size_t b_coef = al(P.coef.size() * (f64 ? 8 : 4));
   const size_t b_pa = al(P.poly_angle.size() * 8), b_po = al(P.poly_off.size() * 4), b_pc = al(P.poly_cnt.size() * 4),
                b_pd = al(P.poly_conds.size() * 8);
   const size_t b_u = al((size_t)ucap * 8), b_s = al(64), b_o = al(P.n_measures + 1);
   const size_t b_img = al(P.block_images.size());
-  const size_t total = b_img + b_ops + b_coef + b_pa + b_po + b_pc + b_pd + b_u + b_s + b_o;
+  const size_t total = b_img + b_ops + b_ph + b_coef + b_pa + b_po + b_pc + b_pd + b_u + b_s + b_o;
   if (int r = ensure(h, buf, total)) return r;
   std::vector<uint8_t> img(reuse ? 0 : total, 0);
   size_t off = 0;
@@ -202,6 +202,7 @@ int execute(aleph_b200_handle* h, aleph_b200_state* st, const Plan& P, const dou
   };
   const size_t o_img = put(P.block_images.data(), P.block_images.size(), b_img);
   const size_t o_ops = put(P.ops.data(), P.ops.size() * sizeof(Op), b_ops);
+  const size_t o_ph = put(P.phases.data(), P.phases.size() * sizeof(WidePhase), b_ph);
   const size_t o_coef = f64 ? put(P.coef.data(), P.coef.size() * 8, b_coef) : put(coef32.data(), P.coef.size() * 4, b_coef);
   const size_t o_pa = put(P.poly_angle.data(), P.poly_angle.size() * 8, b_pa);
   const size_t o_po = put(P.poly_off.data(), P.poly_off.size() * 4, b_po);
@@ -277,6 +278,13 @@ int execute(aleph_b200_handle* h, aleph_b200_state* st, const Plan& P, const dou
         h->stats.passes++;
         h->stats.algorithmic_bytes += 2 * len * bpa;
         break;
+      case PASS_WIDE:
+        e = launch_wide_pass(st->amps, st->precision, ps.wide, (const WidePhase*)(base + o_ph), d.ops, d.coef, d.poly,
+                             h->stream);
+        h->stats.tile_passes++;
+        h->stats.passes++;
+        h->stats.algorithmic_bytes += 2 * len * bpa;
+        break;
       case PASS_SMEM: {
         const size_t next = (size_t)ps.tile.op_begin + ps.tile.op_count;
         const uint32_t coef_end = next < P.ops.size() ? P.ops[next].coef : (uint32_t)(P.coef.size() / 2);
@@ -316,10 +324,10 @@ int execute(aleph_b200_handle* h, aleph_b200_state* st, const Plan& P, const dou
     h->stats.kernel_launches++;
     h->stats.gates_planned += ps.gates;
     {
-      const uint32_t* qs = ps.kind == PASS_BLOCK ? ps.block.bq : ps.tile.hq;
-      const uint32_t nq = ps.kind == PASS_BLOCK ? 6 : ps.kind == PASS_TILE ? ps.tile.R : 0;
+      const uint32_t* qs = ps.kind == PASS_BLOCK ? ps.block.bq : ps.kind == PASS_WIDE ? ps.wide.free_q : ps.tile.hq;
+      const uint32_t nq = ps.kind == PASS_BLOCK ? 6 : ps.kind == PASS_WIDE ? 8 : ps.kind == PASS_TILE ? ps.tile.R : 0;
       const double bytes = ps.kind == PASS_MEASURE ? 3 * len * bpa : 2 * len * bpa;
-      CK(record_end(pk, (uint32_t)ps.kind, ps.gates, nq, qs, ps.kind == PASS_BLOCK ? ps.block.post_count : 0, bytes),
+      CK(record_end(pk, ps.kind == PASS_WIDE ? PASS_TILE : (uint32_t)ps.kind, ps.gates, nq, qs, ps.kind == PASS_BLOCK ? ps.block.post_count : 0, bytes),
          "event record");
       if (rec) {
         aleph_b200_pass_record& r = h->records.back();
@@ -550,7 +558,8 @@ int aleph_b200_apply_gate(aleph_b200_handle* h, aleph_b200_state* st, const alep
     ops[0] = std::move(L);
   }
   Plan P;
-  if (int s = build_plan(ops, n, h->opts, &P)) return set_error(h, s, "optimization pipeline failed: planner");
+  if (int s = build_plan(ops, n, st->precision == ALEPH_B200_F64, h->opts, &P))
+    return set_error(h, s, "optimization pipeline failed: planner");
   return execute(h, st, P, nullptr, 0, nullptr, nullptr);
 }
 
@@ -731,7 +740,7 @@ static int stream_impl(aleph_b200_handle* h, aleph_b200_state* st, const aleph_b
   std::vector<Lowered> ops;
   if (int r = lower_stream(h, st->n, in, count, pools, &ops)) return r;
   Plan P;
-  if (int s = build_plan(ops, st->n, h->opts, &P)) return set_error(h, s, "optimization pipeline failed: planner");
+  if (int s = build_plan(ops, st->n, st->precision == ALEPH_B200_F64, h->opts, &P)) return set_error(h, s, "optimization pipeline failed: planner");
   return run_plan(h, st, P, mu, n_mu, outcomes, outcomes_cap, n_outcomes, used_out);
 }
 
@@ -764,7 +773,7 @@ int aleph_b200_compile(aleph_b200_handle* h, uint32_t num_qubits, const aleph_b2
   aleph_b200_plan* p = new (std::nothrow) aleph_b200_plan();
   if (!p) return set_error(h, ALEPH_B200_DEVICE_FAILURE, "host allocation failed");
   p->n = num_qubits;
-  if (int s = build_plan(ops, num_qubits, h->opts, &p->P)) {
+  if (int s = build_plan(ops, num_qubits, h->precision == ALEPH_B200_F64, h->opts, &p->P)) {
     delete p;
     return set_error(h, s, "optimization pipeline failed: planner");
   }
@@ -1034,7 +1043,7 @@ int aleph_b200_paged_run(aleph_b200_handle* h, uint32_t n, const aleph_b200_inst
     {
       std::vector<Lowered> ops;
       if (int r = lower_stream(h, nl, local.data(), local.size(), pools, &ops)) return fail(r);
-      if (int s = build_plan(ops, nl, h->opts, &P)) return fail(set_error(h, s, "optimization pipeline failed: planner"));
+      if (int s = build_plan(ops, nl, h->precision == ALEPH_B200_F64, h->opts, &P)) return fail(set_error(h, s, "optimization pipeline failed: planner"));
       P.renormalize = false;
     }
     bool uploaded = false;
@@ -1334,7 +1343,7 @@ int aleph_b200_apply_diagonal_phase(aleph_b200_handle* h, aleph_b200_state* st, 
   aleph_b200_error_info e{};
   if (lower_diagonal_phase(terms, n_terms, conds, n_conds, &ops[0], &e)) return report(h, e);
   Plan P;
-  if (int s = build_plan(ops, st->n, h->opts, &P)) return set_error(h, s, "optimization pipeline failed: planner");
+  if (int s = build_plan(ops, st->n, st->precision == ALEPH_B200_F64, h->opts, &P)) return set_error(h, s, "optimization pipeline failed: planner");
   return execute(h, st, P, nullptr, 0, nullptr, nullptr);
 }
 
@@ -1986,18 +1995,18 @@ int aleph_b200_describe_plan(uint32_t num_qubits, const aleph_b200_plan_config* 
   std::vector<Lowered> ops;
   if (int r = lower_stream(&tmp, num_qubits, in, count, pools, &ops)) return r;
   Plan P;
-  if (int s = build_plan(ops, num_qubits, tmp.opts, &P)) return s;
+  if (int s = build_plan(ops, num_qubits, config->precision == ALEPH_B200_F64, tmp.opts, &P)) return s;
   const double bpa = config->precision == ALEPH_B200_F64 ? 16.0 : 8.0;
   const double len = (double)(1ull << num_qubits);
   *n_passes = P.passes.size();
   for (size_t k = 0; k < P.passes.size() && k < cap; ++k) {
     const Pass& ps = P.passes[k];
     aleph_b200_pass_record r{};
-    r.kind = (uint32_t)ps.kind;
+    r.kind = ps.kind == PASS_WIDE ? PASS_TILE : (uint32_t)ps.kind;
     r.gates = ps.gates;
     r.n = num_qubits;
-    const uint32_t* qs = ps.kind == PASS_BLOCK ? ps.block.bq : ps.tile.hq;
-    r.nq = ps.kind == PASS_BLOCK ? 6 : ps.kind == PASS_TILE ? ps.tile.R : 0;
+    const uint32_t* qs = ps.kind == PASS_BLOCK ? ps.block.bq : ps.kind == PASS_WIDE ? ps.wide.free_q : ps.tile.hq;
+    r.nq = ps.kind == PASS_BLOCK ? 6 : ps.kind == PASS_WIDE ? 8 : ps.kind == PASS_TILE ? ps.tile.R : 0;
     for (uint32_t j = 0; j < r.nq && j < 8; ++j) r.qubits[j] = qs[j];
     r.post_ops = ps.kind == PASS_BLOCK ? ps.block.post_count : 0;
     r.lane_ops = ps.lane_ops;

@@ -25,6 +25,9 @@ enum OpType : uint8_t {
   OP_POLY = 6,    // DiagonalPhase: amp *= exp(i*phi(x)), terms [mask, mask+aux)
   OP_KQ = 7,      // dense 2^k x 2^k, k = nq (3..5), q MSB-first (coef: 4^k complex)
   OP_NEG = 8,     // amp = -amp where every bit of `mask` is 1 (CZ, CCZ, Z fast path)
+  // wide tile pass only: `aux` records follow, each with a thread condition `mask`
+  OP_SIGNS = 9,   // sign flips: record `aux` = the registers it flips (bit r: register r)
+  OP_PHASES = 10, // phases (`coef`) whose product scales the registers with bit `a` set (a > 4: all)
 };
 
 struct Op {
@@ -63,6 +66,27 @@ struct TilePass {
   uint32_t occupancy;  // resident 128-thread blocks per SM the kernel variant targets (2..4; 0 = default)
 };
 
+// Wide tile pass: a CTA's tile is 2^12 amplitudes over qubits 0..3 and eight
+// others; ops run in phases, each with kWideRegs of the twelve in registers.
+constexpr uint32_t kWideBits = 12;
+constexpr uint32_t kWideRegs = 5;                       // register qubits of a phase
+constexpr uint32_t kWideThreadBits = kWideBits - kWideRegs;
+struct WidePass {
+  uint32_t n;
+  uint32_t phase_begin, phase_count;  // the first and the last phase have qubits 0..3 on lanes 0..3
+  uint32_t op_begin, op_count;
+  uint32_t free_q[8];  // the eight other tile qubits, ascending
+  // the non-tile qubits as runs of consecutive positions (tile index bits
+  // [dep_src, ...) land on qubits [dep_dst, ...)): at most 9
+  uint32_t n_dep;
+  uint32_t dep_src[9], dep_mask[9], dep_dst[9];
+};
+struct WidePhase {
+  uint32_t op_begin, op_count;  // dense ops: Op::a / Op::b = 5 + register bit
+  uint16_t ts[kWideThreadBits], rs[kWideRegs];  // shared-memory slot offset of each thread-index / register bit (XORed)
+  uint8_t tq[kWideThreadBits], rq[kWideRegs];   // qubit of each thread-index / register bit
+};
+
 // Tensor-core dense-block pass (TC32): a 2^6 x 2^6 complex matrix on the
 // qubits bq[0..6) (ascending; bq[j] = bit j of the block row index), with
 // diagonal ops applied before (pre) and after (post) the block product.
@@ -85,6 +109,7 @@ enum PassKind : uint8_t {
   PASS_MEASURE = 4,
   PASS_BLOCK = 5,
   PASS_PERMUTE = 7,
+  PASS_WIDE = 8,  // reported as PASS_TILE in pass records
 };
 
 constexpr uint32_t kMaxQubits = 40;
@@ -92,6 +117,7 @@ constexpr uint32_t kMaxQubits = 40;
 struct Pass {
   PassKind kind;
   TilePass tile;       // PASS_TILE (also op range for PASS_SMEM / PASS_KQ)
+  WidePass wide;       // PASS_WIDE
   BlockPass block;     // PASS_BLOCK
   uint32_t qubit;      // PASS_MEASURE
   // PASS_PERMUTE: an involution of the qubit positions; the pass maps
@@ -129,6 +155,7 @@ struct Lowered {
 struct Plan {
   std::vector<Pass> passes;
   std::vector<Op> ops;
+  std::vector<WidePhase> phases;
   std::vector<double> coef;  // complex pairs
   // OP_POLY tables
   std::vector<double> poly_angle;
@@ -222,6 +249,10 @@ cudaError_t launch_init_zero_state(void* amps, uint32_t n, int precision, cudaSt
 cudaError_t launch_tile_pass(void* amps, int precision, const TilePass& p, const Op* ops, const void* coef,
                              PolyTables poly, int* dev_error, int sm_count, cudaStream_t s);
 // coef_end: one past the last op's coefficients (the ops' coefficients are contiguous, in op order).
+cudaError_t launch_wide_pass(void* amps, int precision, const WidePass& p, const WidePhase* phases, const Op* ops,
+                             const void* coef, PolyTables poly, cudaStream_t s);
+// Fills a phase's layout (ts, rs, tq, rq) for the tile bits `regs` in registers.
+void wide_layout(const uint8_t* tile_qubits, uint32_t regs, bool io, bool f64, WidePhase* P);
 cudaError_t launch_smem_pass(void* amps, int precision, uint32_t n, const Op* ops, uint32_t op_count,
                              const void* coef, uint32_t coef_end, PolyTables poly, cudaStream_t s);
 cudaError_t launch_kq_pass(void* amps, int precision, uint32_t n, const Op* op_dev, const Op& op_host,
@@ -326,6 +357,7 @@ int lower_gate(const aleph_b200_instr& g, uint32_t n, const double* pool, uint64
 int lower_diagonal_phase(const aleph_b200_phase_term* terms, uint64_t n_terms, const uint64_t* conds, uint64_t n_conds,
                          Lowered* out, aleph_b200_error_info* err);
 const char* gate_name(uint32_t kind);
-int build_plan(const std::vector<Lowered>& ops, uint32_t n, const PlanOptions& o, Plan* plan);
+// f64: the state's precision (shared-memory layouts of wide tile passes).
+int build_plan(const std::vector<Lowered>& ops, uint32_t n, bool f64, const PlanOptions& o, Plan* plan);
 
 }  // namespace ab

@@ -874,6 +874,266 @@ int plan_segment_tiles(const std::vector<const Lowered*>& seg, uint32_t n, uint3
   return ALEPH_B200_OK;
 }
 
+// ---- wide tile passes ------------------------------------------------------------
+// The ops of `pending` that fit one pass (or one phase of it), in order: an op
+// joins if it commutes past every op left behind and acts non-diagonally only on
+// qubits of the set. The set is `have` plus up to `room` qubits taken first come.
+struct WideTake {
+  uint64_t set = 0;
+  std::vector<const Lowered*> take, rest;
+  double score = 0.0;  // arithmetic taken, older ops counting more (see BlockTake)
+};
+
+double wide_weight(const Lowered& L) {  // arithmetic, and a little for every op's own overhead
+  return 2.0 + tile_cost(L);
+}
+
+void wide_take(const std::vector<const Lowered*>& pending, uint64_t have, uint32_t room, uint32_t base, WideTake* out) {
+  uint64_t set = have, blocked_full = 0, blocked_diag = 0;
+  for (const Lowered* L : pending) {
+    bool ok = L->op.type != OP_KQ && !(L->nondiag & (blocked_full | blocked_diag)) && !(L->diag & blocked_full);
+    const uint64_t need = L->nondiag & ~set;
+    const uint32_t count = (uint32_t)__builtin_popcountll(need);
+    if (ok && count > room) ok = false;
+    if (ok) {
+      set |= need;
+      room -= count;
+      out->take.push_back(L);
+      if (L->nondiag) out->score += wide_weight(*L) / (1.0 + (double)(L->record - base) / 256.0);
+    } else {
+      blocked_full |= L->nondiag;
+      blocked_diag |= L->diag;
+      out->rest.push_back(L);
+    }
+  }
+  out->set = set;
+}
+
+// The best of the first-come set and of every window of consecutive qubits
+// (on a brickwall the windows follow the light cone).
+WideTake wide_best(const std::vector<const Lowered*>& pending, uint64_t have, uint32_t room, const uint8_t* qubits,
+                   uint32_t nq) {
+  const uint32_t base = pending.front()->record;
+  WideTake best;
+  wide_take(pending, have, room, base, &best);
+  for (uint32_t a = 0; a + room <= nq; ++a) {
+    uint64_t window = have;
+    for (uint32_t k = 0; k < room; ++k) window |= 1ull << qubits[a + k];
+    WideTake c;
+    wide_take(pending, window, 0, base, &c);
+    if (c.score > best.score) best = std::move(c);
+  }
+  return best;
+}
+
+// Appends the ops of one phase, `reg_of[q]` the register bit of qubit q (255:
+// none). Sign flips and corner phases with at most one register qubit are
+// collected into groups: such an op joins the last group if it commutes with the
+// dense ops after it. A group costs one sweep over the registers per class however
+// many ops it holds (the QFT's passes hold some 20 phases per dense gate; one at
+// a time, each cost half a sweep and its predicates).
+void emit_wide_phase(const std::vector<const Lowered*>& ops, const uint8_t* reg_of, uint32_t n, Plan* P) {
+  struct Group {
+    std::vector<const Lowered*> signs, phases[6];
+    bool empty() const {
+      for (const auto& c : phases)
+        if (!c.empty()) return false;
+      return signs.empty();
+    }
+  };
+  struct Item {
+    const Lowered* op = nullptr;  // null: group `group`
+    size_t group = 0;
+  };
+  std::vector<Group> groups;
+  std::vector<Item> items;
+  uint64_t after = 0;  // qubits acted on non-diagonally after the last group
+  auto split = [&](uint64_t m, uint64_t* rest, uint32_t* regs) {
+    *rest = m;
+    *regs = 0;
+    for (uint32_t q = 0; q < n; ++q)
+      if (((m >> q) & 1) && reg_of[q] != 255) {
+        *regs |= 1u << reg_of[q];
+        *rest &= ~(1ull << q);
+      }
+  };
+  for (const Lowered* L : ops) {
+    uint64_t rest = 0;
+    uint32_t regs = 0;
+    if (L->op.type == OP_NEG || L->op.type == OP_CPHASE) split(L->op.mask, &rest, &regs);
+    const bool sign = L->op.type == OP_NEG;
+    const bool phase = L->op.type == OP_CPHASE && __builtin_popcount(regs) <= 1;
+    if (!sign && !phase) {
+      items.push_back(Item{L, 0});
+      if (L->nondiag) after |= L->nondiag;
+      continue;
+    }
+    if (groups.empty() || (L->diag & after)) {
+      groups.emplace_back();
+      items.push_back(Item{nullptr, groups.size() - 1});
+      after = 0;
+    }
+    Group& G = groups.back();
+    if (sign) G.signs.push_back(L);
+    else G.phases[regs ? (uint32_t)__builtin_ctz(regs) : 5u].push_back(L);
+  }
+  auto group_op = [&](uint8_t type, uint8_t cls, size_t count) {
+    Op op;
+    std::memset(&op, 0, sizeof(Op));
+    op.type = type;
+    op.a = cls;
+    op.aux = (uint32_t)count;
+    op.coef = (uint32_t)(P->coef.size() / 2);
+    P->ops.push_back(op);
+  };
+  for (const Item& it : items) {
+    if (!it.op) {
+      const Group& G = groups[it.group];
+      if (!G.signs.empty()) {
+        group_op(OP_SIGNS, 0, G.signs.size());
+        for (const Lowered* L : G.signs) {
+          Op op = L->op;
+          uint32_t regs = 0, flips = 0;
+          split(L->op.mask, &op.mask, &regs);
+          for (uint32_t r = 0; r < 32; ++r)
+            if ((r & regs) == regs) flips |= 1u << r;
+          append_op(P, *L, op);
+          P->ops.back().aux = flips;
+        }
+      }
+      for (uint32_t c = 0; c < 6; ++c) {
+        if (G.phases[c].empty()) continue;
+        group_op(OP_PHASES, (uint8_t)c, G.phases[c].size());
+        for (const Lowered* L : G.phases[c]) {
+          Op op = L->op;
+          uint32_t regs = 0;
+          split(L->op.mask, &op.mask, &regs);
+          append_op(P, *L, op);
+        }
+      }
+      continue;
+    }
+    const Lowered* L = it.op;
+    Op op = L->op;
+    uint32_t regs = 0;
+    if (op.type == OP_CPHASE) {
+      split(op.mask, &op.mask, &regs);
+      op.creg = (uint8_t)regs;
+      op.ctrl = 0;
+    } else if (op.type != OP_POLY) {
+      split(op.ctrl, &op.ctrl, &regs);
+      op.creg = (uint8_t)regs;
+    }
+    if (op.type == OP_DIAG) {
+      op.dsrc = 0;
+      for (int i = 0; i < op.nq; ++i)
+        if (reg_of[op.q[i]] != 255) {
+          op.dsrc |= (uint8_t)(1u << i);
+          op.q[3 + i] = reg_of[op.q[i]];
+        }
+    }
+    if (op.type == OP_1Q || op.type == OP_X) {
+      op.a = (uint8_t)(5 + reg_of[op.q[0]]);
+    } else if (op.type == OP_2Q) {
+      op.a = (uint8_t)(5 + reg_of[op.q[0]]);
+      op.b = (uint8_t)(5 + reg_of[op.q[1]]);
+      if (op.a < op.b) {
+        Lowered tmp = *L;
+        swap_2q_operands(tmp.coef);
+        std::swap(op.q[0], op.q[1]);
+        std::swap(op.a, op.b);
+        append_op(P, tmp, op);
+        continue;
+      }
+    }
+    append_op(P, *L, op);
+  }
+}
+
+int plan_segment_wide(const std::vector<const Lowered*>& seg, uint32_t n, bool f64, uint32_t R, Plan* P) {
+  std::vector<const Lowered*> pending = seg;
+  uint8_t all[kMaxQubits];
+  for (uint32_t q = 0; q < n; ++q) all[q] = (uint8_t)q;
+  while (!pending.empty()) {
+    if (pending.front()->op.type == OP_KQ) {
+      const std::vector<const Lowered*> one{pending.front()};
+      if (int s = plan_segment_tiles(one, n, R, P)) return s;
+      pending.erase(pending.begin());
+      continue;
+    }
+    WideTake T = wide_best(pending, 0xFull, kWideBits - 4, all + 4, n - 4);
+    if (T.take.empty()) return ALEPH_B200_OPTIMIZATION;
+    // the tile: the chosen qubits, padded with the lowest unused ones
+    uint64_t set = T.set;
+    for (uint32_t q = 4; q < n && __builtin_popcountll(set) < (int)kWideBits; ++q) set |= 1ull << q;
+    Pass ps{};
+    ps.kind = PASS_WIDE;
+    WidePass& W = ps.wide;
+    W.n = n;
+    uint8_t tile[kWideBits];
+    uint32_t k = 0;
+    for (uint32_t q = 0; q < n; ++q) {
+      if ((set >> q) & 1) {
+        if (k >= 4) W.free_q[k - 4] = q;
+        tile[k++] = (uint8_t)q;
+      }
+    }
+    for (uint32_t q = 0, src = 0; q < n;) {
+      if ((set >> q) & 1) {
+        ++q;
+        continue;
+      }
+      uint32_t len = 0;
+      while (q + len < n && !((set >> (q + len)) & 1)) ++len;
+      W.dep_src[W.n_dep] = src;
+      W.dep_mask[W.n_dep] = (1u << len) - 1;  // len <= 28
+      W.dep_dst[W.n_dep] = q;
+      ++W.n_dep;
+      src += len;
+      q += len;
+    }
+    // phases: sets of kWideRegs tile qubits, until the pass's ops are spent
+    W.phase_begin = (uint32_t)P->phases.size();
+    W.op_begin = (uint32_t)P->ops.size();
+    std::vector<const Lowered*> left = T.take;
+    auto add_phase = [&](uint32_t regs, bool io, const std::vector<const Lowered*>& ops) {
+      WidePhase ph{};
+      wide_layout(tile, regs, io, f64, &ph);
+      uint8_t reg_of[kMaxQubits];
+      std::memset(reg_of, 255, sizeof(reg_of));
+      for (uint32_t j = 0; j < kWideRegs; ++j) reg_of[ph.rq[j]] = (uint8_t)j;
+      ph.op_begin = (uint32_t)P->ops.size();
+      emit_wide_phase(ops, reg_of, n, P);
+      ph.op_count = (uint32_t)P->ops.size() - ph.op_begin;
+      P->phases.push_back(ph);
+    };
+    constexpr uint32_t kIoRegs = ((1u << kWideRegs) - 1) << kWideThreadBits;  // the top tile bits: lanes take bits 0..4
+    bool first = true;
+    while (!left.empty()) {
+      WideTake F = wide_best(left, 0, kWideRegs, tile, kWideBits);
+      if (F.take.empty()) return ALEPH_B200_OPTIMIZATION;
+      uint32_t regs = 0;
+      for (uint32_t b = 0; b < kWideBits; ++b)
+        if ((F.set >> tile[b]) & 1) regs |= 1u << b;
+      for (int b = (int)kWideBits - 1; b >= 0 && __builtin_popcount(regs) < (int)kWideRegs; --b) regs |= 1u << b;
+      const bool low = (regs & 0xFu) != 0, last = F.rest.empty();
+      if (first && low) add_phase(kIoRegs, true, {});
+      add_phase(regs, !low && (first || last), F.take);
+      if (last && low) add_phase(kIoRegs, true, {});
+      first = false;
+      left.swap(F.rest);
+    }
+    W.phase_count = (uint32_t)P->phases.size() - W.phase_begin;
+    W.op_count = (uint32_t)P->ops.size() - W.op_begin;
+    ps.record = T.take.front()->record;
+    for (const Lowered* L : T.take) ps.gates += L->gates ? L->gates : 1;
+    count_ops(T.take, &ps);
+    P->passes.push_back(ps);
+    pending.swap(T.rest);
+  }
+  return ALEPH_B200_OK;
+}
+
 // ---- tensor-core dense blocks ------------------------------------------------
 // Apply a lowered op to a vector over the block qubits bq[0..6) (index bit b
 // <-> qubit bq[b]); the op's qubits must all be block qubits, except for the
@@ -1163,7 +1423,7 @@ std::vector<std::vector<uint8_t>> split_into_involutions(const std::vector<uint3
   return out;
 }
 
-int build_plan(const std::vector<Lowered>& ops, uint32_t n, const PlanOptions& o, Plan* P) {
+int build_plan(const std::vector<Lowered>& ops, uint32_t n, bool f64, const PlanOptions& o, Plan* P) {
   P->renormalize = o.renormalize;
   std::vector<const Lowered*> seg;
   int status = ALEPH_B200_OK;
@@ -1188,7 +1448,12 @@ int build_plan(const std::vector<Lowered>& ops, uint32_t n, const PlanOptions& o
       if (o.tensor_blocks && n >= 13) status = plan_segment_blocks(seg, n, R, o.block_window_search, P);
       else if (o.pair_fusion) {
         std::deque<Lowered> fused;
-        status = plan_segment_tiles(fuse_pairs(seg, fused), n, R, P);
+        const std::vector<const Lowered*> list = fuse_pairs(seg, fused);
+        // Wide tiles unless a key of the warp-tile planner was changed (tile_r,
+        // tile_occupancy, pair_fusion, relabel_swaps compare its parts) or the
+        // state is smaller than one wide tile.
+        const bool wide = n >= kWideBits && o.tile_r == 5 && o.tile_occupancy == 0 && o.relabel_swaps;
+        status = wide ? plan_segment_wide(list, n, f64, R, P) : plan_segment_tiles(list, n, R, P);
       } else {
         status = plan_segment_tiles(seg, n, R, P);
       }
