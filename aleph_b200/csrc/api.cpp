@@ -425,7 +425,7 @@ int aleph_b200_destroy(aleph_b200_handle* h) {
   if (!h) return ALEPH_B200_OK;
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
-  for (Scratch* s : {&h->reduce, &h->plan_buf, &h->sample, &h->status, &h->qaoa.dev, &h->qaoa.state, &h->qaoa.cuts})
+  for (Scratch* s : {&h->reduce, &h->plan_buf, &h->sample, &h->status, &h->qaoa.dev, &h->qaoa.state, &h->qaoa.tables})
     if (s->ptr) cudaFree(s->ptr);
   for (Scratch& s : h->state_pool) cudaFree(s.ptr);
   if (h->qaoa.exec) cudaGraphExecDestroy(h->qaoa.exec);
@@ -1209,7 +1209,6 @@ int aleph_b200_qaoa_sweep(aleph_b200_handle* h, uint32_t p, const aleph_b200_qao
   // each edge's CNOT(i, j) operands, then the Rz / Rx angles
   const int prec = h->precision == ALEPH_B200_F64 ? ALEPH_B200_F64 : ALEPH_B200_F32;
   const uint32_t smem_n = qaoa_smem_max_n(prec);
-  uint32_t nmax_stream = 0;
   for (uint32_t k = 0; k < n_sets; ++k) {
     const aleph_b200_qaoa_set& s = sets[k];
     aleph_b200_error_info e{};
@@ -1243,27 +1242,95 @@ int aleph_b200_qaoa_sweep(aleph_b200_handle* h, uint32_t p, const aleph_b200_qao
         std::snprintf(e.kind, sizeof(e.kind), j < p ? "rz" : "rx");
         return report(h, e);
       }
-    if (s.num_qubits > smem_n && s.num_qubits > nmax_stream) nmax_stream = s.num_qubits;
   }
   if (int r = bind(h)) return r;
   auto& Q = h->qaoa;
-  // streamed sets: one state slice and one cut slice per CTA, within a memory budget
-  const uint64_t slice = nmax_stream ? (1ull << nmax_stream) : 0;
   const size_t bpa = prec == ALEPH_B200_F64 ? 16 : 8;
-  int grid = h->sm_count * qaoa_ctas_per_sm(prec);
-  if (slice) {
-    const uint64_t budget = 48ull << 30;
-    const uint64_t per_cta = slice * (bpa + 1);
-    if ((uint64_t)grid * per_cta > budget) grid = (int)(budget / per_cta);
-    if (grid < 1) grid = 1;
+  const int grid = h->sm_count * qaoa_ctas_per_sm(prec);
+  // The queue: streamed sets, largest first, in waves that share a half of the
+  // state buffer (512 MiB, or the largest set); in a wave pass by pass, so that
+  // a set's next pass comes long after its previous one; then the small sets,
+  // which fill the last wave's tail.
+  std::vector<uint32_t> order(n_sets);
+  for (uint32_t k = 0; k < n_sets; ++k) order[k] = k;
+  std::stable_sort(order.begin(), order.end(),
+                   [&](uint32_t x, uint32_t y) { return sets[x].num_qubits > sets[y].num_qubits; });
+  uint32_t n_streamed = 0;
+  while (n_streamed < n_sets && sets[order[n_streamed]].num_qubits > smem_n) ++n_streamed;
+  uint64_t half = n_streamed ? std::max<uint64_t>((512ull << 20) / bpa, 1ull << sets[order[0]].num_qubits) : 0;  // amplitudes
+  std::vector<QaoaGroup> groups;
+  groups.reserve((size_t)n_streamed * (p + 1) + (n_sets - n_streamed));
+  uint64_t items = 0;
+  uint32_t n_waves = 0, n_partials = 0, prev_wave_items[2] = {0, 0};
+  uint64_t used_half = 0;
+  for (uint32_t s0 = 0; s0 < n_streamed; ++n_waves) {
+    uint32_t s1 = s0;
+    uint64_t amps = 0, tiles = 0;
+    while (s1 < n_streamed && amps + (1ull << sets[order[s1]].num_qubits) <= half) {
+      amps += 1ull << sets[order[s1]].num_qubits;
+      tiles += 1ull << (sets[order[s1]].num_qubits - kQaoaTileBits);
+      ++s1;
+    }
+    used_half = std::max(used_half, amps);
+    // several items per CTA and pass; up to 8 tiles an item spread its set-up
+    const uint32_t per = (uint32_t)std::min<uint64_t>(8, std::max<uint64_t>(1, tiles / (4 * (uint64_t)grid)));
+    uint32_t wave_items = 0;
+    for (uint32_t k = 0; k <= p; ++k) {
+      uint64_t off = (n_waves & 1) * half;
+      for (uint32_t j = s0; j < s1; ++j) {
+        const uint32_t n = sets[order[j]].num_qubits;
+        QaoaGroup g{};
+        g.first_item = (uint32_t)items;
+        g.set = order[j];
+        g.pass = k;
+        g.ntiles = 1u << (n - kQaoaTileBits);
+        g.tiles_per_item = per;
+        g.slot = j;
+        g.state_off = off;
+        const uint32_t cnt = (g.ntiles + per - 1) / per;
+        g.done_idx = 2 + j;
+        g.wave_idx = 2 + n_streamed + n_waves;
+        if (k) {
+          g.wait_idx = g.done_idx;
+          g.wait_val = k * cnt;
+        } else if (n_waves >= 2) {  // the half's previous wave is done with it
+          g.wait_idx = g.wave_idx - 2;
+          g.wait_val = prev_wave_items[n_waves & 1];
+        }
+        if (k == p) {
+          g.part0 = n_partials;
+          n_partials += cnt;
+          wave_items += cnt;
+        }
+        groups.push_back(g);
+        items += cnt;
+        off += 1ull << n;
+      }
+    }
+    prev_wave_items[n_waves & 1] = wave_items;
+    s0 = s1;
   }
-  // device input region: sets | order | edges | angles | out | counter
-  const size_t b_sets = al((size_t)n_sets * sizeof(aleph_b200_qaoa_set)), b_order = al((size_t)n_sets * 4),
+  for (uint32_t j = n_streamed; j < n_sets; ++j) {
+    QaoaGroup g{};
+    g.first_item = (uint32_t)items++;
+    g.set = order[j];
+    g.pass = kQaoaSmall;
+    groups.push_back(g);
+  }
+  if (items > 0x7fffffffull) return set_error(h, ALEPH_B200_INVALID_ARGUMENT, "qaoa sweep has too many tiles");
+  const uint64_t state_amps = n_waves > 1 ? half + used_half : used_half;
+  // device region: sets | streamed | edges | angles | groups (uploaded), out | error, counters
+  const size_t b_sets = al((size_t)n_sets * sizeof(aleph_b200_qaoa_set)), b_str = al((size_t)n_streamed * 4),
                b_edges = al((size_t)n_edge_pairs * 8), b_ang = al((size_t)n_sets * 2 * p * 8),
-               b_out = al((size_t)n_sets * 8), b_cnt = al(4);
-  const size_t in_bytes = b_sets + b_order + b_edges + b_ang;
+               b_grp = al(groups.size() * sizeof(QaoaGroup)), b_out = al((size_t)n_sets * 8 + 8),
+               b_cnt = al(((size_t)2 + n_streamed + n_waves) * 4);
+  const size_t in_bytes = b_sets + b_str + b_edges + b_ang + b_grp;
   const size_t total = in_bytes + b_out + b_cnt;
-  const uint64_t key[6] = {(uint64_t)prec, n_sets, p, n_edge_pairs, (uint64_t)grid, slice};
+  const size_t out_bytes = (size_t)n_sets * 8 + 8;
+  const QaoaSizes z = qaoa_sizes(prec, n_streamed, p);
+  const size_t b_tab = al(z.tables), b_msk = al(z.masks), b_phs = al(z.phases);
+  const uint64_t key[10] = {(uint64_t)prec, n_sets, p, n_edge_pairs, (uint64_t)n_streamed, n_waves, groups.size(), items,
+                            state_amps, n_partials};
   const bool same = Q.exec && std::memcmp(key, Q.key, sizeof(key)) == 0;
   if (!same) {
     if (Q.exec) {
@@ -1271,9 +1338,9 @@ int aleph_b200_qaoa_sweep(aleph_b200_handle* h, uint32_t p, const aleph_b200_qao
       Q.exec = nullptr;
     }
     if (int r = ensure(h, Q.dev, total)) return r;
-    if (slice) {
-      if (int r = ensure(h, Q.state, (size_t)grid * slice * bpa)) return r;
-      if (int r = ensure(h, Q.cuts, (size_t)grid * slice)) return r;
+    if (n_streamed) {
+      if (int r = ensure(h, Q.state, (size_t)state_amps * bpa)) return r;
+      if (int r = ensure(h, Q.tables, b_tab + b_msk + b_phs + (size_t)n_partials * 8)) return r;
     }
     if (Q.host_in_bytes < in_bytes) {
       if (Q.host_in) cudaFreeHost(Q.host_in);
@@ -1282,39 +1349,50 @@ int aleph_b200_qaoa_sweep(aleph_b200_handle* h, uint32_t p, const aleph_b200_qao
       CK(cudaHostAlloc(&Q.host_in, in_bytes, cudaHostAllocDefault), "pinned staging");
       Q.host_in_bytes = in_bytes;
     }
-    if (Q.host_out_bytes < b_out) {
+    if (Q.host_out_bytes < out_bytes) {
       if (Q.host_out) cudaFreeHost(Q.host_out);
       Q.host_out = nullptr;
       Q.host_out_bytes = 0;
-      CK(cudaHostAlloc(&Q.host_out, b_out, cudaHostAllocDefault), "pinned staging");
-      Q.host_out_bytes = b_out;
+      CK(cudaHostAlloc(&Q.host_out, out_bytes, cudaHostAllocDefault), "pinned staging");
+      Q.host_out_bytes = out_bytes;
     }
   }
   // stage this call's inputs (the graph copies the staging area as it is at replay)
   uint8_t* hin = (uint8_t*)Q.host_in;
+  const size_t o_str = b_sets, o_edges = o_str + b_str, o_ang = o_edges + b_edges, o_grp = o_ang + b_ang;
   std::memcpy(hin, sets, (size_t)n_sets * sizeof(aleph_b200_qaoa_set));
-  {
-    std::vector<uint32_t> order(n_sets);
-    for (uint32_t k = 0; k < n_sets; ++k) order[k] = k;
-    std::stable_sort(order.begin(), order.end(),
-                     [&](uint32_t x, uint32_t y) { return sets[x].num_qubits > sets[y].num_qubits; });
-    std::memcpy(hin + b_sets, order.data(), (size_t)n_sets * 4);
-  }
-  if (n_edge_pairs) std::memcpy(hin + b_sets + b_order, edges, (size_t)n_edge_pairs * 8);
-  std::memcpy(hin + b_sets + b_order + b_edges, angles, (size_t)n_sets * 2 * p * 8);
+  if (n_streamed) std::memcpy(hin + o_str, order.data(), (size_t)n_streamed * 4);
+  if (n_edge_pairs) std::memcpy(hin + o_edges, edges, (size_t)n_edge_pairs * 8);
+  std::memcpy(hin + o_ang, angles, (size_t)n_sets * 2 * p * 8);
+  std::memcpy(hin + o_grp, groups.data(), groups.size() * sizeof(QaoaGroup));
   char* d = (char*)Q.dev.ptr;
   if (!same) {
-    // capture: inputs up, counter cleared, the persistent sweep, results down
+    // capture: inputs up, results and counters cleared, tables, the persistent sweep, results down
+    QaoaLaunch L{};
+    L.sets = (const aleph_b200_qaoa_set*)d;
+    L.streamed = (const uint32_t*)(d + o_str);
+    L.edges = (const uint32_t*)(d + o_edges);
+    L.angles = (const double*)(d + o_ang);
+    L.groups = (const QaoaGroup*)(d + o_grp);
+    L.out = (double*)(d + in_bytes);
+    L.error = (int*)(d + in_bytes + (size_t)n_sets * 8);
+    L.counters = (uint32_t*)(d + in_bytes + b_out);
+    char* t = (char*)Q.tables.ptr;
+    L.state = Q.state.ptr;
+    L.tables = t;
+    L.masks = t + b_tab;
+    L.phases = t + b_tab + b_msk;
+    L.partials = (double*)(t + b_tab + b_msk + b_phs);
+    L.n_groups = (uint32_t)groups.size();
+    L.n_items = (uint32_t)items;
+    L.n_streamed = n_streamed;
+    L.p = p;
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "graph capture");
     cudaError_t e = cudaMemcpyAsync(d, hin, in_bytes, cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d + in_bytes + b_out, 0, 4, h->stream);
-    if (e == cudaSuccess)
-      e = launch_qaoa_sweep(prec, (const aleph_b200_qaoa_set*)d, (const uint32_t*)(d + b_sets + b_order),
-                            (const double*)(d + b_sets + b_order + b_edges), (const uint32_t*)(d + b_sets),
-                            (uint32_t*)(d + in_bytes + b_out), (double*)(d + in_bytes), Q.state.ptr,
-                            (uint8_t*)Q.cuts.ptr, slice, n_sets, p, grid, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(Q.host_out, d + in_bytes, (size_t)n_sets * 8, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d + in_bytes, 0, b_out + b_cnt, h->stream);
+    if (e == cudaSuccess) e = launch_qaoa_sweep(prec, L, grid, h->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(Q.host_out, d + in_bytes, out_bytes, cudaMemcpyDeviceToHost, h->stream);
     const cudaError_t ec = cudaStreamEndCapture(h->stream, &g);
     if (e == cudaSuccess) e = ec;
     if (e == cudaSuccess) e = cudaGraphInstantiate(&Q.exec, g, 0);
@@ -1328,10 +1406,13 @@ int aleph_b200_qaoa_sweep(aleph_b200_handle* h, uint32_t p, const aleph_b200_qao
   }
   CK(cudaGraphLaunch(Q.exec, h->stream), "qaoa sweep graph launch");
   CK(cudaStreamSynchronize(h->stream), "stream synchronize");
+  int32_t failed = 0;
+  std::memcpy(&failed, (const char*)Q.host_out + (size_t)n_sets * 8, 4);
+  if (failed) return set_error(h, ALEPH_B200_DEVICE_FAILURE, "device operation failed: qaoa sweep wait expired");
   std::memcpy(expectations, Q.host_out, (size_t)n_sets * 8);
-  h->stats.kernel_launches += 1;
+  h->stats.kernel_launches += n_streamed ? 3 : 1;
   h->stats.h2d_bytes += in_bytes;
-  h->stats.d2h_bytes += (size_t)n_sets * 8;
+  h->stats.d2h_bytes += out_bytes;
   return ALEPH_B200_OK;
 }
 

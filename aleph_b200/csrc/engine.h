@@ -224,14 +224,14 @@ struct Handle {
   std::vector<aleph_b200_pass_record> records;
   // batched QAOA sweep: device buffers, pinned staging and the captured graph
   struct Qaoa {
-    Scratch dev;           // sets | order | edges | angles | out | counter
-    Scratch state;         // per-CTA state slices (streamed sets)
-    Scratch cuts;          // per-CTA cut(z) slices
+    Scratch dev;           // sets | streamed | edges | angles | groups | out | error | counters
+    Scratch state;         // the two state halves (streamed sets)
+    Scratch tables;        // per streamed set: cut tables, masks, phases; then partial sums
     void* host_in = nullptr;   // pinned staging of the device input region
     void* host_out = nullptr;  // pinned staging of the results
     size_t host_in_bytes = 0, host_out_bytes = 0;
     cudaGraphExec_t exec = nullptr;
-    uint64_t key[6] = {0, 0, 0, 0, 0, 0};  // layout the graph was captured for
+    uint64_t key[10] = {};  // layout the graph was captured for
   } qaoa;
 };
 
@@ -310,13 +310,46 @@ cudaError_t mlp_adam(float* params, const float* grads, float* m, float* v, size
                      cudaStream_t s);
 
 // batched QAOA sweep (kernels_qaoa.cu): sets with n <= qaoa_smem_max_n run in
-// shared memory; larger ones stream through per-CTA slices of slice_amps.
+// shared memory, one CTA each; larger ones stream in tiles of 2^13 amplitudes.
+// The queue is a list of groups (one pass of one streamed set, or one small
+// set), each a run of items; items are handed out in order.
+constexpr uint32_t kQaoaSmall = 0xffffffffu;  // QaoaGroup::pass of a small set
+constexpr uint32_t kQaoaTileBits = 13;
+struct QaoaGroup {
+  uint32_t first_item;
+  uint32_t set;             // index in the caller's order
+  uint32_t pass;            // 0..p, or kQaoaSmall
+  uint32_t ntiles, tiles_per_item;
+  uint32_t slot;            // streamed sets: index of the set's tables
+  uint64_t state_off;       // amplitudes into the state buffer
+  uint32_t wait_idx, wait_val;  // counter that must reach wait_val first (0: none)
+  uint32_t done_idx, wave_idx;  // counters of finished items: the set's, and the wave's (last pass)
+  uint32_t part0;           // last pass: first partial sum
+  uint32_t pad;
+};
+struct QaoaLaunch {
+  const aleph_b200_qaoa_set* sets;
+  const uint32_t* edges;
+  const double* angles;
+  const QaoaGroup* groups;
+  const uint32_t* streamed;  // slot -> set
+  uint32_t* counters;        // [0] next item, [1] abort, then the groups' counters; zero at launch
+  double* out;
+  void* state;
+  void* tables;
+  void* masks;
+  void* phases;
+  double* partials;
+  int* error;                // set to ALEPH_B200_DEVICE_FAILURE when a bounded wait expires
+  uint32_t n_groups, n_items, n_streamed, p;
+};
+struct QaoaSizes {
+  size_t tables, masks, phases;  // bytes
+};
+QaoaSizes qaoa_sizes(int precision, uint32_t n_streamed, uint32_t p);
 uint32_t qaoa_smem_max_n(int precision);
 int qaoa_ctas_per_sm(int precision);
-cudaError_t launch_qaoa_sweep(int precision, const aleph_b200_qaoa_set* sets, const uint32_t* edges,
-                              const double* angles, const uint32_t* order, uint32_t* next, double* out,
-                              void* scratch, uint8_t* cuts, uint64_t slice_amps, uint32_t n_sets, uint32_t p,
-                              int grid, cudaStream_t s);
+cudaError_t launch_qaoa_sweep(int precision, const QaoaLaunch& q, int grid, cudaStream_t s);
 
 // FP64 issue rate (kernels_peak.cu): DFMA chains only, no memory traffic
 cudaError_t launch_dfma_peak(double* out, uint32_t blocks, uint32_t iters, cudaStream_t s);

@@ -9,24 +9,40 @@
 // every qubit. The output is <C> = sum_z |psi_z|^2 cut(z), the expectation of
 // H_C = sum_edges 1/2 (I - Z_i Z_j) (ansatz.rs:100-117), reduced in FP64.
 //
-// One CTA per SM pulls sets from a queue (largest first). A state of at most
-// SMEM_N qubits lives in shared memory for the whole circuit. A larger one
-// lives in the CTA's slice of a device buffer and is streamed in tiles of
-// 2^13 amplitudes, two passes per layer: pass A over contiguous chunks
-// (qubits 0..12: cost phase + mixer), pass B over tiles spanning the qubits
-// 13..n-1 (mixer). The first pass generates |+>^n instead of reading it; the
-// last pass only reads and accumulates <C>. A pass loads a tile into
-// registers (32 amplitudes a thread, every load in flight at once), mixes the
-// register and lane bits there, and at most one trip through shared memory
-// mixes the warp bits.
+// A state of at most SMEM_N qubits lives in one CTA's shared memory for the
+// whole circuit. A larger one is streamed in tiles of 2^13 amplitudes, and its
+// tiles are spread over all CTAs: a set's passes are work items in one queue.
 //
-// cut(z) per amplitude: within a pass-A chunk z = (t << 13) | lo and
-// cut(z) = cutT[lo] + (edges among the high qubits cut by t) + X0[lo & 127] +
-// X1[lo >> 7], where cutT counts the edges among qubits 0..12 (per set) and
-// X0 / X1 the edges between a low and a high qubit (per chunk). The first
-// cost layer also stores cut(z) as one byte per amplitude, which the final
-// pass B reads. Multiple edges between the same pair count once each, as the
-// repeated gadgets do.
+// Passes. The mixer of a layer is a product of Rx on every qubit, so its parts
+// on the low qubits 0..12 (A) and on the high ones 13..n-1 (B) commute; a cost
+// layer is diagonal and needs whole amplitudes only. So the layers alternate which
+// part they start with, and two halves meet in one pass:
+//     A: cost 1, low 1 | B: high 1, cost 2, high 2 | A: low 2, cost 3, low 3 | ...
+// p + 1 passes over the state for p layers, where one pass per part takes 2p. The
+// first pass generates |+>^n, the last one accumulates <C> and writes nothing. An
+// A tile is a contiguous chunk; a B tile spans the high qubits and the lowest
+// c = 26 - n ones.
+//
+// In a tile, bits 8..12 are mixed in registers and bits 0..4 by lane shuffles
+// (layout 1), one trip through shared memory brings bits 5..7 into registers
+// (layout 2), where the cost phase is applied and the next layer's part starts,
+// and a second trip brings bits 8..12 back.
+//
+// cut(z) of a tile amplitude i: T[i] (edges inside the tile's qubits, a table per
+// set and tile kind, built once by prep_kernel) + edges among the tile's fixed
+// qubits (a constant) + X0[i & 127] + X1[i >> 7] (edges between the two, rebuilt
+// per tile from neighbour masks). Multiple edges between the same pair count
+// once each, as the repeated gadgets do (the masks come in bit planes).
+//
+// Queue. Items are handed out in order: wave by wave, pass by pass, set by set. The
+// sets of a wave share one half of the state buffer; a wave starts once the wave
+// before the last has finished with that half, and a pass of a set once the
+// set's previous pass has. An item waits only for items before it in the queue, and
+// those are held by CTAs that already run, so the queue cannot lock up; every
+// wait is bounded all the same.
+//
+// Measured (384 FP32 sets, n = 12..22, p = 4): one CTA per set with 2p passes took
+// 39 ms, most of it the last n = 22 sets on one CTA each.
 
 #include "common.cuh"
 
@@ -41,23 +57,34 @@ constexpr int MAX_EDGES = 128;
 template <typename Real>
 struct Cfg {
   static constexpr int SMEM_N = 13;  // states kept in shared memory (the tile size)
-  static constexpr uint32_t SMEM_BYTES = (1u << SMEM_N) * sizeof(V2<Real>);
   // FP32 tiles (64 KiB) leave room for two CTAs per SM, which overlap one
   // CTA's tile loads with the other's arithmetic
   static constexpr int CTAS_PER_SM = sizeof(Real) == 4 ? 2 : 1;
+};
+
+// Per streamed set and tile kind (0: A, 1: B): the neighbour masks in bit planes.
+constexpr int PLANES = 8;  // multiplicities up to 128 edges
+struct Masks {
+  uint16_t cross[TILE_BITS][PLANES];  // tile bit -> neighbours among the fixed qubits
+  uint16_t fixed[TILE_BITS][PLANES];  // fixed qubit -> neighbours among the fixed qubits
+  uint32_t planes;                    // planes in use
+  uint32_t pad;
 };
 
 struct Args {
   const aleph_b200_qaoa_set* sets;
   const uint32_t* edges;   // (u, v) pairs
   const double* angles;    // per set: gamma[0..p), beta[0..p)
-  const uint32_t* order;   // set indices, largest first
-  uint32_t* next;          // work counter (zero at launch)
+  const QaoaGroup* groups; // the queue, in order
+  uint32_t* counters;      // [0] next item, [1] abort, then the groups' counters
   double* out;
-  void* scratch;           // per-CTA state slices for the streamed sets
-  uint8_t* cuts;           // per-CTA cut(z) slices
-  uint64_t slice_amps;
-  uint32_t n_sets, p;
+  void* scratch;           // the two state halves (V2<Real>)
+  uint8_t* tables;         // per streamed set: T of kind 0, T of kind 1
+  Masks* masks;            // per streamed set: kind 0, kind 1
+  void* phases;            // per streamed set and layer: exp(-i gamma (m - 2k)), k = 0..m
+  double* partials;        // last-pass items
+  uint32_t n_groups, n_items, p;
+  int* error;
 };
 
 // Rx(2 beta) on tile-local bit k of every pair in S[0..len): (a, b) -> (c a - i s b, c b - i s a).
@@ -155,24 +182,6 @@ __device__ __forceinline__ void rx_lanes(V2<Real> (&v)[NR], uint32_t mask, Real 
   }
 }
 
-// One read of the tile in shared memory in the layout lane = tile bits 0..4,
-// register = bits 5..7, warp and loop = bits 8..12: Rx on the register bits
-// set in mask3, then emit(i, amplitude) for each of this thread's 32 indices.
-template <typename Real, typename Emit>
-__device__ __forceinline__ void shared_sweep(const V2<Real>* S, uint32_t mask3, Real c, Real s, Emit&& emit) {
-  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint32_t hi = (w | (uint32_t)j << 3) << 8;
-    V2<Real> u[8];
-#pragma unroll
-    for (int r = 0; r < 8; ++r) u[r] = S[hi | (uint32_t)r << 5 | lane];
-    rx_regs<Real, 8>(u, mask3, c, s);
-#pragma unroll
-    for (int r = 0; r < 8; ++r) emit(hi | (uint32_t)r << 5 | lane, u[r]);
-  }
-}
-
 __device__ __forceinline__ double block_sum(double v, double* red) {
   for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
@@ -184,183 +193,323 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
   return s;
 }
 
+// Tile bit of qubit q for tile kind B (c lowest qubits, then 13..n-1), or 16 + its fixed index.
+__device__ __forceinline__ uint32_t place(uint32_t kind, uint32_t n, uint32_t q) {
+  const uint32_t c = 2 * TILE_BITS - n;
+  if (kind == 0) return q < TILE_BITS ? q : 16 + (q - TILE_BITS);
+  return q < c ? q : q < TILE_BITS ? 16 + (q - c) : q - TILE_BITS + c;
+}
+
+// One CTA per streamed set and tile kind: masks, the table T, and (kind 0) the layers' phases.
+template <typename Real>
+__global__ void __launch_bounds__(THREADS) prep_kernel(Args a, const uint32_t* __restrict__ streamed) {
+  __shared__ uint32_t mult[2 * TILE_BITS][2 * TILE_BITS];  // edge multiplicities: tile bits, then fixed qubits
+  __shared__ uint16_t tt[TILE_BITS][PLANES];
+  __shared__ uint32_t used;
+  const uint32_t slot = blockIdx.x >> 1, kind = blockIdx.x & 1, tid = threadIdx.x;
+  const aleph_b200_qaoa_set cs = a.sets[streamed[slot]];
+  const uint32_t n = cs.num_qubits, m = cs.num_edges;
+  for (uint32_t i = tid; i < 4 * TILE_BITS * TILE_BITS; i += THREADS) (&mult[0][0])[i] = 0;
+  if (tid == 0) used = 1;
+  __syncthreads();
+  for (uint32_t e = tid; e < m; e += THREADS) {
+    uint32_t u = place(kind, n, a.edges[2 * (cs.edge_offset + e)]), v = place(kind, n, a.edges[2 * (cs.edge_offset + e) + 1]);
+    u = u < 16 ? u : u - 16 + TILE_BITS;
+    v = v < 16 ? v : v - 16 + TILE_BITS;
+    atomicAdd(&mult[u][v], 1u);
+    atomicAdd(&mult[v][u], 1u);
+  }
+  __syncthreads();
+  Masks& M = a.masks[2 * slot + kind];
+  for (uint32_t i = tid; i < TILE_BITS * PLANES; i += THREADS) {
+    const uint32_t q = i / PLANES, b = i % PLANES;
+    uint32_t x = 0, y = 0, z = 0;
+    for (uint32_t f = 0; f < TILE_BITS; ++f) {
+      x |= ((mult[q][TILE_BITS + f] >> b) & 1u) << f;
+      y |= ((mult[TILE_BITS + q][TILE_BITS + f] >> b) & 1u) << f;
+      z |= ((mult[q][f] >> b) & 1u) << f;
+    }
+    M.cross[q][b] = (uint16_t)x;
+    M.fixed[q][b] = (uint16_t)y;
+    tt[q][b] = (uint16_t)z;
+    if (x | y | z) atomicMax(&used, b + 1);
+  }
+  __syncthreads();
+  const uint32_t np = used;
+  if (tid == 0) M.planes = np;
+  uint8_t* T = a.tables + (2 * (size_t)slot + kind) * TILE;
+  for (uint32_t z = tid; z < TILE; z += THREADS) {
+    uint32_t c = 0;
+    for (uint32_t b = 0; b < np; ++b)
+#pragma unroll
+      for (uint32_t q = 0; q < TILE_BITS; ++q)
+        if ((z >> q) & 1u) c += (uint32_t)__popc(tt[q][b] & ~z) << b;
+    T[z] = (uint8_t)c;
+  }
+  if (kind == 0) {
+    const double* gam = a.angles + (size_t)streamed[slot] * 2 * a.p;
+    V2<Real>* ph = (V2<Real>*)a.phases + (size_t)slot * a.p * (MAX_EDGES + 1);
+    for (uint32_t i = tid; i < a.p * (m + 1); i += THREADS) {
+      const uint32_t l = i / (m + 1), k = i % (m + 1);
+      double sn, cn;
+      sincos(-gam[l] * ((double)m - 2.0 * (double)k), &sn, &cn);
+      ph[(size_t)l * (MAX_EDGES + 1) + k] = mk<Real>((Real)cn, (Real)sn);
+    }
+  }
+}
+
+// <C> of the streamed sets: their last pass's partial sums, in item order.
+__global__ void __launch_bounds__(32) total_kernel(Args a) {
+  const QaoaGroup g = a.groups[blockIdx.x];
+  if (g.pass != a.p) return;  // small sets (kQaoaSmall) write their result themselves
+  double s = 0.0;
+  const uint32_t items = (g.ntiles + g.tiles_per_item - 1) / g.tiles_per_item;
+  for (uint32_t i = threadIdx.x; i < items; i += 32) s += a.partials[g.part0 + i];
+  for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (threadIdx.x == 0) a.out[g.set] = s;
+}
+
+template <typename Real>
+struct Shared {
+  V2<Real> S[TILE];
+  V2<Real> ph[MAX_EDGES + 1];  // cost-layer phase by cut value
+  double red[THREADS / 32];
+  alignas(16) uint8_t cutT[TILE];  // filled by 16-byte copies
+  uint8_t X0[2][128], X1[2][64];
+  uint32_t ch[2];
+  Masks masks;
+  uint8_t eu[MAX_EDGES], ev[MAX_EDGES];
+  uint32_t item[2], group[2];
+  int ok;
+};
+
 template <typename Real>
 __global__ void __launch_bounds__(THREADS, Cfg<Real>::CTAS_PER_SM) sweep_kernel(Args a) {
   extern __shared__ __align__(16) uint8_t qsm[];
-  V2<Real>* S = (V2<Real>*)qsm;
-  __shared__ uint8_t eu[MAX_EDGES], ev[MAX_EDGES];
-  __shared__ uint8_t cutT[1 << TILE_BITS];
-  __shared__ uint8_t X0[128], X1[64];
-  __shared__ V2<Real> ph[MAX_EDGES + 1];  // cost-layer phase by cut value
-  __shared__ double red[THREADS / 32];
-  __shared__ uint32_t s_idx, s_ch;
-  const uint32_t tid = threadIdx.x;
-  V2<Real>* X = (V2<Real>*)a.scratch + (uint64_t)blockIdx.x * a.slice_amps;
-  uint8_t* CG = a.cuts + (uint64_t)blockIdx.x * a.slice_amps;
+  Shared<Real>& sh = *(Shared<Real>*)qsm;
+  V2<Real>* S = sh.S;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
 
-  for (;;) {
-    if (tid == 0) s_idx = atomicAdd(a.next, 1u);
-    __syncthreads();
-    const uint32_t idx = s_idx;
-    __syncthreads();
-    if (idx >= a.n_sets) break;
-    const uint32_t ci = a.order[idx];
-    const aleph_b200_qaoa_set cs = a.sets[ci];
-    const uint32_t n = cs.num_qubits, m = cs.num_edges;
-    for (uint32_t e = tid; e < m; e += THREADS) {
-      eu[e] = (uint8_t)a.edges[2 * (cs.edge_offset + e)];
-      ev[e] = (uint8_t)a.edges[2 * (cs.edge_offset + e) + 1];
-    }
-    __syncthreads();
-    const bool in_smem = n <= (uint32_t)Cfg<Real>::SMEM_N;
-    const uint32_t lb = in_smem ? n : (uint32_t)TILE_BITS;  // cutT covers qubits 0..lb-1
-    for (uint32_t z = tid; z < (1u << lb); z += THREADS) {
-      uint32_t c = 0;
-      for (uint32_t e = 0; e < m; ++e)
-        if (eu[e] < lb && ev[e] < lb) c += ((z >> eu[e]) ^ (z >> ev[e])) & 1u;
-      cutT[z] = (uint8_t)c;
-    }
-    const double* gam = a.angles + (size_t)ci * 2 * a.p;
-    const double* bet = gam + a.p;
-    const uint64_t len = 1ull << n;
-    const Real amp0 = (Real)rsqrt((double)len);  // |+>^n
-    auto set_phases = [&](double gamma) {  // ph[k] = exp(-i gamma (m - 2k))
-      __syncthreads();
-      for (uint32_t k = tid; k <= m; k += THREADS) {
-        double sn, cn;
-        sincos(-gamma * ((double)m - 2.0 * (double)k), &sn, &cn);
-        ph[k] = mk<Real>((Real)cn, (Real)sn);
+  // warp 0: the next item and its group (the last one whose first item is not past it)
+  auto fetch = [&](int at) {
+    uint32_t idx = 0;
+    if (lane == 0) idx = atomicAdd(a.counters, 1u);
+    idx = __shfl_sync(0xffffffffu, idx, 0);
+    uint32_t lo = 0, hi = a.n_groups;  // groups[lo].first_item <= idx < groups[hi].first_item
+    if (idx < a.n_items)
+      while (hi - lo > 1) {
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint32_t g = lo + step * (lane + 1);
+        const bool past = g >= hi || a.groups[g].first_item > idx;
+        const uint32_t first = __ffs(__ballot_sync(0xffffffffu, past)) - 1;  // lane 31 is always past
+        hi = min(hi, lo + step * (first + 1));
+        lo += step * first;
       }
-      __syncthreads();
-    };
+    if (lane == 0) {
+      sh.item[at] = idx;
+      sh.group[at] = lo;
+    }
+  };
+  if (w == 0) fetch(0);
+  for (int at = 0;; at ^= 1) {
+    __syncthreads();
+    const uint32_t idx = sh.item[at];
+    if (idx >= a.n_items) break;
+    const QaoaGroup g = a.groups[sh.group[at]];
+    const aleph_b200_qaoa_set cs = a.sets[g.set];
+    const uint32_t n = cs.num_qubits, m = cs.num_edges;
+    const double* bet = a.angles + (size_t)g.set * 2 * a.p + a.p;
+    const Real amp0 = (Real)rsqrt((double)(1ull << n));  // |+>^n
     double acc = 0.0;
 
-    if (in_smem) {
+    if (g.pass == kQaoaSmall) {
       // ---- whole state in shared memory ----
-      const uint32_t L = (uint32_t)len;
+      if (w == 0) fetch(at ^ 1);
+      const double* gam = bet - a.p;
+      for (uint32_t e = tid; e < m; e += THREADS) {
+        sh.eu[e] = (uint8_t)a.edges[2 * (cs.edge_offset + e)];
+        sh.ev[e] = (uint8_t)a.edges[2 * (cs.edge_offset + e) + 1];
+      }
+      __syncthreads();
+      const uint32_t L = 1u << n;
+      for (uint32_t z = tid; z < L; z += THREADS) {
+        uint32_t c = 0;
+        for (uint32_t e = 0; e < m; ++e) c += ((z >> sh.eu[e]) ^ (z >> sh.ev[e])) & 1u;
+        sh.cutT[z] = (uint8_t)c;
+      }
       for (uint32_t i = tid; i < L; i += THREADS) S[i] = mk<Real>(amp0, (Real)0);
       for (uint32_t l = 0; l < a.p; ++l) {
-        set_phases(gam[l]);
-        for (uint32_t i = tid; i < L; i += THREADS) S[i] = cmul<Real>(ph[cutT[i]], S[i]);
+        __syncthreads();
+        for (uint32_t k = tid; k <= m; k += THREADS) {  // ph[k] = exp(-i gamma (m - 2k))
+          double sn, cn;
+          sincos(-gam[l] * ((double)m - 2.0 * (double)k), &sn, &cn);
+          sh.ph[k] = mk<Real>((Real)cn, (Real)sn);
+        }
+        __syncthreads();
+        for (uint32_t i = tid; i < L; i += THREADS) S[i] = cmul<Real>(sh.ph[sh.cutT[i]], S[i]);
         double sb, cb;
         sincos(bet[l], &sb, &cb);
         mixer_range<Real>(S, L, 0, n, (Real)cb, (Real)sb);
       }
       for (uint32_t i = tid; i < L; i += THREADS) {
         const double x = (double)S[i].x, y = (double)S[i].y;
-        acc += (x * x + y * y) * (double)cutT[i];
+        acc += (x * x + y * y) * (double)sh.cutT[i];
       }
-    } else {
-      // ---- streamed through this CTA's state slice ----
-      const uint32_t c = 2 * TILE_BITS - n;                 // pass B: low run bits (n <= 26)
-      const uint32_t maskB = (TILE - 1) & ~((1u << c) - 1);  // pass B mixes tile bits c..12
-      const uint64_t ntiles = len >> TILE_BITS;
-      V2<Real> v[REGS];  // the register sweep's amplitudes (see load_chunk / load_tile)
-      for (uint32_t l = 0; l < a.p; ++l) {
-        set_phases(gam[l]);
-        double sb, cb;
-        sincos(bet[l], &sb, &cb);
-        const Real rc = (Real)cb, rs = (Real)sb;
-        // pass A: contiguous chunks, cost phase + mixer on qubits 0..12.
-        // Chunk constants: cut edges among the high qubits, and the low/high
-        // cross-edge tables.
-        auto chunk_tables = [&](uint32_t t) {
-          if (tid == 0) {
-            uint32_t ch = 0;
-            for (uint32_t e = 0; e < m; ++e)
-              if (eu[e] >= TILE_BITS && ev[e] >= TILE_BITS)
-                ch += (uint32_t)(((t >> (eu[e] - TILE_BITS)) ^ (t >> (ev[e] - TILE_BITS))) & 1u);
-            s_ch = ch;
-          }
-          if (tid < 192) {
-            const uint32_t base = tid < 128 ? 0u : 7u, v = tid < 128 ? tid : tid - 128;
-            uint32_t x = 0;
-            for (uint32_t e = 0; e < m; ++e) {
-              const uint32_t u0 = eu[e], v0 = ev[e];
-              const bool ul = u0 < TILE_BITS, vl = v0 < TILE_BITS;
-              if (ul == vl) continue;  // not a low/high cross edge
-              const uint32_t lo_q = ul ? u0 : v0, hi_q = ul ? v0 : u0;
-              if (lo_q < base || lo_q >= base + (base ? 6u : 7u)) continue;
-              const uint32_t zb = (v >> (lo_q - base)) & 1u, hb = (uint32_t)(t >> (hi_q - TILE_BITS)) & 1u;
-              x += zb ^ hb;
-            }
-            if (tid < 128) X0[v] = (uint8_t)x;
-            else X1[v] = (uint8_t)x;
-          }
-        };
-        // this thread's 32 amplitudes i = tid | r << 8 of chunk t, every load in flight at once
-        // (slice offsets fit in 32 bits: n <= 26)
-        auto load_chunk = [&](uint32_t t) {
-          if (l == 0) {
-#pragma unroll
-            for (int r = 0; r < REGS; ++r) v[r] = mk<Real>(amp0, (Real)0);
-          } else {
-#pragma unroll
-            for (int r = 0; r < REGS; ++r) v[r] = X[(t << TILE_BITS) | tid | (uint32_t)r << 8];
-          }
-        };
-        // Software pipeline: chunk t+1's loads and tables are issued once chunk
-        // t sits in shared memory, and are in flight during its shared sweep.
-        chunk_tables(0);
-        load_chunk(0);
-        for (uint32_t t = 0; t < (uint32_t)ntiles; ++t) {
-          __syncthreads();  // chunk t's tables are visible; chunk t-1's shared sweep is done
-          const uint32_t ch = s_ch;
-          const uint32_t g0 = t << TILE_BITS;
-          const uint32_t x0 = X0[tid & 127];
-#pragma unroll
-          for (int r = 0; r < REGS; ++r) {
-            const uint32_t i = tid | (uint32_t)r << 8;
-            const uint32_t cut = cutT[i] + ch + x0 + X1[i >> 7];
-            if (l == 0) CG[g0 + i] = (uint8_t)cut;
-            v[r] = cmul<Real>(ph[cut], v[r]);
-          }
-          rx_regs<Real, REGS>(v, 0x1fu, rc, rs);   // tile bits 8..12
-          rx_lanes<Real, REGS>(v, 0x1fu, rc, rs);  // tile bits 0..4
-#pragma unroll
-          for (int r = 0; r < REGS; ++r) S[tid | (uint32_t)r << 8] = v[r];
-          __syncthreads();
-          if (t + 1 < (uint32_t)ntiles) {
-            chunk_tables(t + 1);
-            load_chunk(t + 1);
-          }
-          // shared-memory sweep: tile bits 5..7, straight back to the chunk
-          shared_sweep<Real>(S, 0x7u, rc, rs, [&](uint32_t i, const V2<Real>& u) { X[g0 + i] = u; });
-        }
-        __syncthreads();  // pass A's stores are visible to every thread of the CTA
-        // pass B: tiles over {qubits 0..c-1} + {qubits 13..n-1}; tile index -> qubits c..12
-        const bool last = l + 1 == a.p;
-        const uint32_t lowm = (1u << c) - 1;
-        auto gidx = [&](uint32_t t, uint32_t i) -> uint32_t {
-          return (i & lowm) | t << c | (i >> c) << TILE_BITS;
-        };
-        auto load_tile = [&](uint32_t t) {
-#pragma unroll
-          for (int r = 0; r < REGS; ++r) v[r] = X[gidx(t, tid | (uint32_t)r << 8)];
-        };
-        load_tile(0);
-        for (uint32_t t = 0; t < (uint32_t)ntiles; ++t) {
-          rx_regs<Real, REGS>(v, maskB >> 8, rc, rs);
-          rx_lanes<Real, REGS>(v, maskB & 0x1fu, rc, rs);
-          __syncthreads();  // the previous tile's shared-memory sweep is done
-#pragma unroll
-          for (int r = 0; r < REGS; ++r) S[tid | (uint32_t)r << 8] = v[r];
-          __syncthreads();
-          if (t + 1 < (uint32_t)ntiles) load_tile(t + 1);
-          shared_sweep<Real>(S, (maskB >> 5) & 0x7u, rc, rs, [&](uint32_t i, const V2<Real>& u) {
-            if (last) {
-              const double x = (double)u.x, y = (double)u.y;
-              acc += (x * x + y * y) * (double)CG[gidx(t, i)];
-            } else {
-              X[gidx(t, i)] = u;
-            }
-          });
-        }
+      const double tot = block_sum(acc, sh.red);
+      if (tid == 0) a.out[g.set] = tot;
+      continue;
+    }
+
+    // ---- tiles [t0, t1) of one pass of a streamed set ----
+    const uint32_t kind = g.pass & 1u, k = g.pass;
+    const uint32_t chunk = idx - g.first_item;
+    const uint32_t t0 = chunk * g.tiles_per_item, t1 = min(g.ntiles, t0 + g.tiles_per_item);
+    const bool pre = k > 0, last = k == a.p;
+    const uint32_t c = 2 * TILE_BITS - n, lowm = (1u << c) - 1;
+    const uint32_t mix = kind == 0 ? TILE - 1 : (TILE - 1) & ~lowm;  // tile bits mixed by this pass
+    V2<Real>* X = (V2<Real>*)a.scratch + g.state_off;
+    // state offset of tile amplitude i (offsets fit in 32 bits: n <= 26)
+    auto at_tile = [&](uint32_t t, uint32_t i) -> uint32_t {
+      return kind == 0 ? (t << TILE_BITS) | i : (i & lowm) | t << c | (i >> c) << TILE_BITS;
+    };
+    Real pc = 1, ps = 0, nc = 1, ns = 0;  // Rx of the finishing and of the starting layer
+    {
+      double sn, cn;
+      if (pre) {
+        sincos(bet[k - 1], &sn, &cn);
+        pc = (Real)cn;
+        ps = (Real)sn;
+      }
+      if (!last) {
+        sincos(bet[k], &sn, &cn);
+        nc = (Real)cn;
+        ns = (Real)sn;
       }
     }
-    const double tot = block_sum(acc, red);
-    if (tid == 0) a.out[ci] = tot;
+    {
+      const uint4* T = (const uint4*)(a.tables + (2 * (size_t)g.slot + kind) * TILE);
+      for (uint32_t i = tid; i < TILE / 16; i += THREADS) ((uint4*)sh.cutT)[i] = T[i];
+      const uint32_t* M = (const uint32_t*)(a.masks + 2 * (size_t)g.slot + kind);
+      for (uint32_t i = tid; i < sizeof(Masks) / 4; i += THREADS) ((uint32_t*)&sh.masks)[i] = M[i];
+      if (!last) {
+        const V2<Real>* ph = (const V2<Real>*)a.phases + ((size_t)g.slot * a.p + k) * (MAX_EDGES + 1);
+        for (uint32_t i = tid; i <= m; i += THREADS) sh.ph[i] = ph[i];
+      }
+    }
+    if (tid == 0) {  // what this item reads (or overwrites) is complete
+      sh.ok = 1;
+      volatile uint32_t* cnt = a.counters + g.wait_idx;
+      if (g.wait_val && *cnt < g.wait_val) {
+        const uint64_t start = globaltimer_ns();
+        for (uint32_t spin = 1; *cnt < g.wait_val; ++spin) {
+          __nanosleep(64);
+          if ((spin & 63) == 0 && (*(volatile uint32_t*)(a.counters + 1) || globaltimer_ns() - start > 10 * kWaitDeadlineNs)) {
+            sh.ok = 0;
+            break;
+          }
+        }
+      }
+      __threadfence();
+    }
     __syncthreads();
+    if (!sh.ok) {
+      if (tid == 0) {
+        atomicExch(a.counters + 1, 1u);
+        atomicExch(a.error, ALEPH_B200_DEVICE_FAILURE);
+      }
+      return;
+    }
+    if (w == 0) fetch(at ^ 1);
+    // the cut contributions of a tile's fixed qubits (bits of t)
+    auto tile_tables = [&](uint32_t t, int b) {
+      const uint32_t np = sh.masks.planes;
+      if (tid < 192) {
+        const uint32_t first = tid < 128 ? 0u : 7u, v = tid < 128 ? tid : tid - 128, bits = tid < 128 ? 7u : 6u;
+        uint32_t x = 0;
+        for (uint32_t pl = 0; pl < np; ++pl)
+          for (uint32_t q = 0; q < bits; ++q) {
+            const uint32_t f = sh.masks.cross[first + q][pl];
+            x += (uint32_t)__popc(f & (((v >> q) & 1u) ? ~t : t)) << pl;
+          }
+        if (tid < 128) sh.X0[b][v] = (uint8_t)x;
+        else sh.X1[b][v] = (uint8_t)x;
+      } else if (tid == 192) {
+        uint32_t x = 0;
+        for (uint32_t pl = 0; pl < np; ++pl)
+          for (uint32_t f = 0; f < TILE_BITS; ++f)
+            if ((t >> f) & 1u) x += (uint32_t)__popc(sh.masks.fixed[f][pl] & ~t) << pl;
+        sh.ch[b] = x;
+      }
+    };
+    V2<Real> v[REGS];
+    for (uint32_t t = t0; t < t1; ++t) {
+      const int b = t & 1;
+      tile_tables(t, b);
+      if (pre) {
+#pragma unroll
+        for (int r = 0; r < REGS; ++r) v[r] = ld_amp<Real>(X + at_tile(t, tid | (uint32_t)r << 8));
+        rx_regs<Real, REGS>(v, mix >> 8, pc, ps);
+        rx_lanes<Real, REGS>(v, mix & 0x1fu, pc, ps);
+        __syncthreads();  // the previous tile's layout-1 reads are done
+#pragma unroll
+        for (int r = 0; r < REGS; ++r) S[tid | (uint32_t)r << 8] = v[r];
+      }
+      __syncthreads();  // the tile and its tables are visible
+      // layout 2: lane = tile bits 0..4, register = bits 5..7, warp and loop = bits 8..12
+      const uint32_t ch = sh.ch[b];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t hi = (w | (uint32_t)j << 3) << 8;
+        V2<Real> u[8];
+        if (pre) {
+#pragma unroll
+          for (int r = 0; r < 8; ++r) u[r] = S[hi | (uint32_t)r << 5 | lane];
+          rx_regs<Real, 8>(u, (mix >> 5) & 0x7u, pc, ps);
+        }
+        uint32_t cut[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const uint32_t i = hi | (uint32_t)r << 5 | lane;
+          cut[r] = sh.cutT[i] + ch + sh.X0[b][i & 127] + sh.X1[b][i >> 7];
+        }
+        if (last) {
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            const double x = (double)u[r].x, y = (double)u[r].y;
+            acc += (x * x + y * y) * (double)cut[r];
+          }
+        } else {
+#pragma unroll
+          for (int r = 0; r < 8; ++r) {
+            const V2<Real> f = sh.ph[cut[r]];
+            u[r] = pre ? cmul<Real>(f, u[r]) : mk<Real>(f.x * amp0, f.y * amp0);
+          }
+          rx_regs<Real, 8>(u, (mix >> 5) & 0x7u, nc, ns);
+          rx_lanes<Real, 8>(u, mix & 0x1fu, nc, ns);
+#pragma unroll
+          for (int r = 0; r < 8; ++r) S[hi | (uint32_t)r << 5 | lane] = u[r];
+        }
+      }
+      if (!last) {
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < REGS; ++r) v[r] = S[tid | (uint32_t)r << 8];
+        rx_regs<Real, REGS>(v, mix >> 8, nc, ns);
+#pragma unroll
+        for (int r = 0; r < REGS; ++r) st_amp<Real>(X + at_tile(t, tid | (uint32_t)r << 8), v[r]);
+        if (!pre) __syncthreads();  // the next tile writes shared memory at once
+      }
+    }
+    if (last) {
+      const double tot = block_sum(acc, sh.red);
+      if (tid == 0) a.partials[g.part0 + chunk] = tot;
+    }
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      atomicAdd(a.counters + g.done_idx, 1u);
+      if (last) atomicAdd(a.counters + g.wave_idx, 1u);
+    }
   }
 }
 
@@ -374,29 +523,53 @@ int qaoa_ctas_per_sm(int precision) {
   return precision == ALEPH_B200_F64 ? qaoa::Cfg<double>::CTAS_PER_SM : qaoa::Cfg<float>::CTAS_PER_SM;
 }
 
-cudaError_t launch_qaoa_sweep(int precision, const aleph_b200_qaoa_set* sets, const uint32_t* edges,
-                              const double* angles, const uint32_t* order, uint32_t* next, double* out,
-                              void* scratch, uint8_t* cuts, uint64_t slice_amps, uint32_t n_sets, uint32_t p,
-                              int grid, cudaStream_t s) {
-  qaoa::Args a{sets, edges, angles, order, next, out, scratch, cuts, slice_amps, n_sets, p};
-  static uint64_t attr_devices[2] = {0, 0};  // per precision: devices with the shared-memory opt-in
+QaoaSizes qaoa_sizes(int precision, uint32_t n_streamed, uint32_t p) {
+  const size_t amp = precision == ALEPH_B200_F64 ? sizeof(double2) : sizeof(float2);
+  QaoaSizes z;
+  z.tables = (size_t)n_streamed * 2 * qaoa::TILE;
+  z.masks = (size_t)n_streamed * 2 * sizeof(qaoa::Masks);
+  z.phases = (size_t)n_streamed * p * (qaoa::MAX_EDGES + 1) * amp;
+  return z;
+}
+
+template <typename Real>
+static cudaError_t launch_qaoa_t(const qaoa::Args& a, const uint32_t* streamed, uint32_t n_streamed, int grid,
+                                 cudaStream_t s) {
+  constexpr int bytes = (int)sizeof(qaoa::Shared<Real>);
+  static uint64_t attr_devices = 0;  // devices with the shared-memory opt-in
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  const int k = precision == ALEPH_B200_F64 ? 1 : 0;
-  if (dev >= 64 || !((attr_devices[k] >> dev) & 1)) {
-    e = k ? cudaFuncSetAttribute(qaoa::sweep_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 qaoa::Cfg<double>::SMEM_BYTES)
-          : cudaFuncSetAttribute(qaoa::sweep_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 qaoa::Cfg<float>::SMEM_BYTES);
+  if (dev >= 64 || !((attr_devices >> dev) & 1)) {
+    e = cudaFuncSetAttribute(qaoa::sweep_kernel<Real>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    if (dev < 64) attr_devices[k] |= 1ull << dev;
+    if (dev < 64) attr_devices |= 1ull << dev;
   }
-  if (k)
-    qaoa::sweep_kernel<double><<<grid, qaoa::THREADS, qaoa::Cfg<double>::SMEM_BYTES, s>>>(a);
-  else
-    qaoa::sweep_kernel<float><<<grid, qaoa::THREADS, qaoa::Cfg<float>::SMEM_BYTES, s>>>(a);
+  if (n_streamed) qaoa::prep_kernel<Real><<<2 * n_streamed, qaoa::THREADS, 0, s>>>(a, streamed);
+  qaoa::sweep_kernel<Real><<<grid, qaoa::THREADS, bytes, s>>>(a);
+  if (n_streamed) qaoa::total_kernel<<<a.n_groups, 32, 0, s>>>(a);
   return cudaGetLastError();
+}
+
+cudaError_t launch_qaoa_sweep(int precision, const QaoaLaunch& q, int grid, cudaStream_t s) {
+  qaoa::Args a;
+  a.sets = q.sets;
+  a.edges = q.edges;
+  a.angles = q.angles;
+  a.groups = q.groups;
+  a.counters = q.counters;
+  a.out = q.out;
+  a.scratch = q.state;
+  a.tables = (uint8_t*)q.tables;
+  a.masks = (qaoa::Masks*)q.masks;
+  a.phases = q.phases;
+  a.partials = q.partials;
+  a.n_groups = q.n_groups;
+  a.n_items = q.n_items;
+  a.p = q.p;
+  a.error = q.error;
+  return precision == ALEPH_B200_F64 ? launch_qaoa_t<double>(a, q.streamed, q.n_streamed, grid, s)
+                                     : launch_qaoa_t<float>(a, q.streamed, q.n_streamed, grid, s);
 }
 
 }  // namespace ab
