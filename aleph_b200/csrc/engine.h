@@ -146,6 +146,7 @@ struct Lowered {
   bool is_permute = false;
   std::vector<uint8_t> sigma;
   uint32_t gates = 0;
+  bool absorbed = false;  // its gates are counted by another op
   // OP_POLY terms (DiagonalPhase): angle, condition count, condition masks
   std::vector<double> poly_angle;
   std::vector<uint32_t> poly_cnt;

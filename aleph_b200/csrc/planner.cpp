@@ -559,6 +559,9 @@ int tile_cost(const Lowered& L) {
 
 constexpr int kFuseMinCost = 24;
 
+// Source gates that an op stands for.
+uint32_t gates_of(const Lowered& L) { return L.absorbed ? 0 : L.gates ? L.gates : 1; }
+
 // The 4x4 of an op on qubits {a (matrix MSB), b (LSB)}, right-multiplied into m:
 // m := op * m.
 void fold_into_4x4(const Lowered& L, uint32_t a, uint32_t b, Cx* m) {
@@ -579,6 +582,191 @@ bool fusable_type(const Lowered& L) {
 }
 
 }  // namespace
+
+// ---- diagonal cores (wide tile passes) ------------------------------------------
+// Gate sequences on two or three qubits often multiply out to a diagonal: the
+// CX Rz CX of a ZZ rotation, a Toffoli in CX + T without the H around it. As
+// written they move amplitudes and tie their qubits to a pass; as a diagonal
+// they are sign flips and corner phases, which act on any qubit and are grouped.
+//
+// Gates are gathered greedily into blocks of at most three qubits (a block
+// owns its qubits until a gate joins them to others). Of a closed block, the core
+// runs from each qubit's first to its last gate on several qubits; the
+// one-qubit gates outside it stay. A core that multiplies out to a diagonal (to
+// rounding) is replaced by its corner phases when those cost less than its gates,
+// an amplitude-moving gate counted as 8. The phases of all cores on no qubit are one op
+// at the end.
+std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& seg, std::deque<Lowered>& store) {
+  struct Block {
+    uint64_t qubits = 0;
+    std::vector<size_t> members;  // indices in seg, ascending
+  };
+  // Ops with the place they go to (sorted at the end, so that gates that stay keep
+  // their order): a gate's own index in seg; for corner phases, the last of the
+  // first core gates on their qubits, which is behind all that earlier blocks did there.
+  std::vector<std::pair<size_t, const Lowered*>> out;
+  out.reserve(seg.size());
+  std::vector<Block> blocks;  // open ones; few at a time
+  Cx global{1.0, 0.0};
+  uint32_t last_record = 0;
+  auto width = [](const Lowered& L) { return __builtin_popcountll(L.nondiag | L.diag); };
+  auto corner = [&](size_t at, uint64_t mask, Cx c, uint32_t record, uint32_t gates) {
+    store.emplace_back();
+    Lowered& F = store.back();
+    std::memset(&F.op, 0, sizeof(Op));
+    F.op.mask = mask;
+    F.nondiag = 0;
+    F.diag = mask;
+    F.record = record;
+    F.gates = gates;
+    F.absorbed = gates == 0;
+    if (c.re == -1.0) {
+      F.op.type = OP_NEG;
+    } else {
+      F.op.type = OP_CPHASE;
+      push_coef(&F, &c, 1);
+    }
+    out.emplace_back(at, &F);
+  };
+  auto emit = [&](const Block& B) {
+    size_t first[64], last[64];
+    for (auto& x : first) x = SIZE_MAX;
+    for (auto& x : last) x = 0;
+    uint32_t multi = 0;
+    for (size_t k = 0; k < B.members.size(); ++k) {
+      const Lowered& L = *seg[B.members[k]];
+      if (width(L) < 2) continue;
+      ++multi;
+      for (uint64_t t = L.nondiag | L.diag; t; t &= t - 1) {
+        const int q = __builtin_ctzll(t);
+        first[q] = std::min(first[q], k);
+        last[q] = k;
+      }
+    }
+    auto plain = [&] {
+      for (size_t m : B.members) out.emplace_back(m, seg[m]);
+    };
+    if (multi < 2) return plain();
+    uint32_t bq[6] = {60, 61, 62, 63, 59, 58}, nb = 0;
+    for (uint64_t t = B.qubits; t; t &= t - 1) bq[nb++] = (uint32_t)__builtin_ctzll(t);
+    const uint32_t dim = 1u << nb;
+    std::vector<size_t> before, after;
+    std::vector<const Lowered*> core;
+    size_t place = 0;  // behind everything that came before the block on any of the core's qubits
+    for (uint32_t q = 0; q < 64; ++q)
+      if (first[q] != SIZE_MAX) place = std::max(place, B.members[first[q]]);
+    int cost = 0;
+    uint32_t gates = 0;
+    for (size_t k = 0; k < B.members.size(); ++k) {
+      const Lowered* L = seg[B.members[k]];
+      if (width(*L) < 2) {
+        const uint64_t t = L->nondiag | L->diag;
+        const int q = t ? __builtin_ctzll(t) : 0;
+        if (first[q] == SIZE_MAX || k < first[q] || k > last[q]) {
+          // a qubit without multi-qubit gates keeps its order: everything on it comes first
+          (first[q] == SIZE_MAX || k < first[q] ? before : after).push_back(B.members[k]);
+          continue;
+        }
+      }
+      core.push_back(L);
+      cost += L->nondiag ? std::max(8, tile_cost(*L)) : tile_cost(*L);
+      gates += gates_of(*L);
+    }
+    const double tol = 1e-15 * (double)(core.size() + 2);
+    Cx d[8];
+    for (uint32_t c = 0; c < dim; ++c) {
+      Cx s[64];
+      for (auto& x : s) x = Cx{0, 0};
+      s[c] = Cx{1.0, 0.0};
+      for (const Lowered* L : core) apply_local(*L, bq, s);
+      for (uint32_t r = 0; r < dim; ++r)
+        if (r != c && std::hypot(s[r].re, s[r].im) > tol) return plain();
+      const double len = std::hypot(s[c].re, s[c].im);
+      if (std::fabs(len - 1.0) > 4 * tol) return plain();
+      d[c] = Cx{s[c].re / len, s[c].im / len};
+    }
+    // corner phases: c_S = prod over T in S of d_T^(+-1), sign by the parity of |S| - |T|
+    Cx cs[8];
+    bool used[8];
+    int price = 0;
+    for (uint32_t S = 0; S < dim; ++S) {
+      Cx c{1.0, 0.0};
+      for (uint32_t T = 0; T < dim; ++T)
+        if ((T & S) == T) c = mul(c, (__builtin_popcount(S ^ T) & 1) ? conj(d[T]) : d[T]);
+      const double snap = 8 * tol;
+      if (std::fabs(c.im) <= snap) c = Cx{c.re > 0 ? 1.0 : -1.0, 0.0};
+      else if (std::fabs(c.re) <= snap) c = Cx{0.0, c.im > 0 ? 1.0 : -1.0};
+      cs[S] = c;
+      used[S] = S != 0 && !is_one(c);
+      if (used[S]) price += c.re == -1.0 ? 1 : 2;
+    }
+    if (price >= cost) return plain();
+    for (size_t m : before) out.emplace_back(m, seg[m]);
+    const uint32_t record = core.front()->record;
+    bool any = false;
+    for (uint32_t S = 1; S < dim; ++S) {
+      if (!used[S]) continue;
+      uint64_t mask = 0;
+      for (uint32_t b = 0; b < nb; ++b)
+        if ((S >> b) & 1) mask |= 1ull << bq[b];
+      corner(place, mask, cs[S], record, any ? 0 : gates);
+      any = true;
+    }
+    if (!any) corner(place, 0, Cx{1.0, 0.0}, record, gates);  // the identity, kept for its gate count
+    global = mul(global, cs[0]);
+    last_record = record;
+    for (size_t m : after) out.emplace_back(std::max(m, place), seg[m]);
+  };
+  auto close = [&](size_t k) {
+    const Block B = std::move(blocks[k]);
+    blocks.erase(blocks.begin() + (long)k);
+    emit(B);
+  };
+  for (size_t i = 0; i < seg.size(); ++i) {
+    const Lowered& L = *seg[i];
+    const uint64_t touched = L.nondiag | L.diag;
+    const bool small = fusable_type(L) && touched && __builtin_popcountll(touched) <= 3;
+    // close touched blocks, the widest first, until the rest and this gate fit three qubits
+    for (;;) {
+      uint64_t all = touched;
+      size_t widest = SIZE_MAX;
+      for (size_t k = 0; k < blocks.size(); ++k) {
+        if (!(blocks[k].qubits & touched)) continue;
+        all |= blocks[k].qubits;
+        if (widest == SIZE_MAX ||
+            __builtin_popcountll(blocks[k].qubits) > __builtin_popcountll(blocks[widest].qubits))
+          widest = k;
+      }
+      if (widest == SIZE_MAX || (small && __builtin_popcountll(all) <= 3)) break;
+      close(widest);
+    }
+    if (!small) {
+      out.emplace_back(i, &L);
+      continue;
+    }
+    Block B;
+    for (size_t k = 0; k < blocks.size();) {
+      if (blocks[k].qubits & touched) {
+        B.qubits |= blocks[k].qubits;
+        B.members.insert(B.members.end(), blocks[k].members.begin(), blocks[k].members.end());
+        blocks.erase(blocks.begin() + (long)k);
+      } else {
+        ++k;
+      }
+    }
+    std::sort(B.members.begin(), B.members.end());
+    B.qubits |= touched;
+    B.members.push_back(i);
+    blocks.push_back(std::move(B));
+  }
+  while (!blocks.empty()) close(0);
+  if (!is_one(global)) corner(SIZE_MAX, 0, global, last_record, 0);
+  std::stable_sort(out.begin(), out.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
+  std::vector<const Lowered*> ops;
+  ops.reserve(out.size());
+  for (const auto& o : out) ops.push_back(o.second);
+  return ops;
+}
 
 // barrier_cost: what an op that moves amplitudes costs beside its arithmetic
 // (shared-memory passes: a barrier and its latency); 0 in tile passes.
@@ -616,7 +804,7 @@ std::vector<const Lowered*> fuse_pairs(const std::vector<const Lowered*>& seg, s
       F.diag = 0;
       F.record = B.record;
       F.gates = 0;
-      for (const Lowered* L : B.members) F.gates += L->gates ? L->gates : 1;
+      for (const Lowered* L : B.members) F.gates += gates_of(*L);
       out.push_back(&F);
       waiting[B.a].clear();
       waiting[B.b].clear();
@@ -722,7 +910,7 @@ std::vector<const Lowered*> fuse_for_smem(const std::vector<const Lowered*>& seg
     Lowered& F = store.back();
     std::memset(&F.op, 0, sizeof(Op));
     F.record = W->record;
-    F.gates = (W->gates ? W->gates : 1) + (L->gates ? L->gates : 1);
+    F.gates = gates_of(*W) + gates_of(*L);
     F.diag = 0;
     F.nondiag = (1ull << a) | (1ull << b);
     if (a == b) {
@@ -866,7 +1054,7 @@ int plan_segment_tiles(const std::vector<const Lowered*>& seg, uint32_t n, uint3
     ps.tile = tp;
     ps.record = take.empty() ? 0 : take.front()->record;
     ps.gates = 0;
-    for (const Lowered* L : take) ps.gates += L->gates ? L->gates : 1;
+    for (const Lowered* L : take) ps.gates += gates_of(*L);
     count_ops(take, &ps);
     P->passes.push_back(ps);
     pending.swap(rest);
@@ -899,7 +1087,7 @@ void wide_take(const std::vector<const Lowered*>& pending, uint64_t have, uint32
       set |= need;
       room -= count;
       out->take.push_back(L);
-      if (L->nondiag) out->score += wide_weight(*L) / (1.0 + (double)(L->record - base) / 256.0);
+      if (L->nondiag) out->score += wide_weight(*L) / (1.0 + (L->record > base ? (double)(L->record - base) / 256.0 : 0.0));
     } else {
       blocked_full |= L->nondiag;
       blocked_diag |= L->diag;
@@ -1126,7 +1314,7 @@ int plan_segment_wide(const std::vector<const Lowered*>& seg, uint32_t n, bool f
     W.phase_count = (uint32_t)P->phases.size() - W.phase_begin;
     W.op_count = (uint32_t)P->ops.size() - W.op_begin;
     ps.record = T.take.front()->record;
-    for (const Lowered* L : T.take) ps.gates += L->gates ? L->gates : 1;
+    for (const Lowered* L : T.take) ps.gates += gates_of(*L);
     count_ops(T.take, &ps);
     P->passes.push_back(ps);
     pending.swap(T.rest);
@@ -1448,12 +1636,12 @@ int build_plan(const std::vector<Lowered>& ops, uint32_t n, bool f64, const Plan
       if (o.tensor_blocks && n >= 13) status = plan_segment_blocks(seg, n, R, o.block_window_search, P);
       else if (o.pair_fusion) {
         std::deque<Lowered> fused;
-        const std::vector<const Lowered*> list = fuse_pairs(seg, fused);
         // Wide tiles unless a key of the warp-tile planner was changed (tile_r,
         // tile_occupancy, pair_fusion, relabel_swaps compare its parts) or the
         // state is smaller than one wide tile.
         const bool wide = n >= kWideBits && o.tile_r == 5 && o.tile_occupancy == 0 && o.relabel_swaps;
-        status = wide ? plan_segment_wide(list, n, f64, R, P) : plan_segment_tiles(list, n, R, P);
+        status = wide ? plan_segment_wide(fuse_pairs(diagonal_cores(seg, fused), fused), n, f64, R, P)
+                      : plan_segment_tiles(fuse_pairs(seg, fused), n, R, P);
       } else {
         status = plan_segment_tiles(seg, n, R, P);
       }
