@@ -140,6 +140,21 @@ int ensure(aleph_b200_handle* h, Scratch& s, size_t bytes) {
   return 0;
 }
 
+// The reduction scratch: a header with the ticket of the blocks that finished
+// (zero between reductions; see kernels_readout.cu), then the partial sums.
+int ensure_reduce(aleph_b200_handle* h, size_t bytes) {
+  if (h->reduce.bytes >= bytes + kReduceHeader) return 0;
+  if (int r = ensure(h, h->reduce, bytes + kReduceHeader)) return r;
+  const cudaError_t e = cudaMemsetAsync(h->reduce.ptr, 0, kReduceHeader, h->stream);
+  if (e != cudaSuccess) {  // never leave an unset ticket behind
+    cudaFree(h->reduce.ptr);
+    h->reduce = Scratch{};
+    return cuda_fail(h, e, "scratch clear");
+  }
+  return 0;
+}
+double* reduce_area(aleph_b200_handle* h) { return (double*)((char*)h->reduce.ptr + kReduceHeader); }
+
 // Every host<->device copy of the engine goes through here so that the
 // stats count the bytes that cross PCIe/C2C.
 cudaError_t copy_async(aleph_b200_handle* h, void* dst, const void* src, size_t bytes, cudaMemcpyKind kind,
@@ -234,7 +249,7 @@ int execute(aleph_b200_handle* h, aleph_b200_state* st, const Plan& P, const dou
 
   const uint32_t nb = reduce_blocks(st->n, h->sm_count);
   if (P.n_measures) {
-    if (int r = ensure(h, h->reduce, (size_t)nb * 3 * 8 + 256)) return r;
+    if (int r = ensure_reduce(h, (size_t)nb * 3 * 8 + 256)) return r;
   }
   const double bpa = f64 ? 16.0 : 8.0;
   const double len = (double)(1ull << st->n);
@@ -301,10 +316,10 @@ int execute(aleph_b200_handle* h, aleph_b200_state* st, const Plan& P, const dou
         h->stats.algorithmic_bytes += 2 * len * bpa;
         break;
       case PASS_MEASURE:
-        e = launch_measure_pass(st->amps, st->precision, st->n, ps.qubit, (double*)h->reduce.ptr, nb, d.uniforms,
+        e = launch_measure_pass(st->amps, st->precision, st->n, ps.qubit, reduce_area(h), nb, d.uniforms,
                                 n_uniforms, d.status, d.outcomes + mi, h->stream);
         ++mi;
-        h->stats.kernel_launches += 3;
+        h->stats.kernel_launches += 1;
         h->stats.algorithmic_bytes += 3 * len * bpa;
         break;
       case PASS_BLOCK:
@@ -343,13 +358,13 @@ int execute(aleph_b200_handle* h, aleph_b200_state* st, const Plan& P, const dou
   bool any_block = false;
   for (const Pass& ps : P.passes) any_block |= ps.kind == PASS_BLOCK;
   if (any_block && P.renormalize) {
-    if (int r = ensure(h, h->reduce, (size_t)nb * 3 * 8 + 256)) return r;
-    double* part = (double*)h->reduce.ptr;
+    if (int r = ensure_reduce(h, (size_t)nb * 3 * 8 + 256)) return r;
+    double* part = reduce_area(h);
     CK(record_begin(pk), "event record");
     CK(launch_renormalize(st->amps, st->precision, st->n, part, nb, part + 3 * (size_t)nb, h->stream), "renormalize");
     CK(record_end(pk, 6, 0, 0, nullptr, 0, 3 * len * bpa), "event record");
     ++pk;
-    h->stats.kernel_launches += 3;
+    h->stats.kernel_launches += 2;
     h->stats.algorithmic_bytes += 3 * len * bpa;
   }
   if (rec) {
@@ -1492,11 +1507,11 @@ static int check_norm(aleph_b200_handle* h, aleph_b200_state* st, const double* 
 
 static int check_norm_host(aleph_b200_handle* h, aleph_b200_state* st, double* norm_out) {
   const uint32_t nb = reduce_blocks(st->n, h->sm_count);
-  if (int r = ensure(h, h->reduce, (size_t)nb * 3 * 8 + 256)) return r;
-  double* part = (double*)h->reduce.ptr;
+  if (int r = ensure_reduce(h, (size_t)nb * 3 * 8 + 256)) return r;
+  double* part = reduce_area(h);
   double* out2 = part + 3 * (size_t)nb;
   CK(launch_norm(st->amps, st->precision, st->n, part, nb, out2, h->stream), "norm");
-  h->stats.kernel_launches += 2;
+  h->stats.kernel_launches += 1;
   double res[2];
   CK(copy_async(h, res, out2, 16, cudaMemcpyDeviceToHost, h->stream), "norm readback");
   CK(cudaStreamSynchronize(h->stream), "stream synchronize");
@@ -1532,7 +1547,7 @@ int aleph_b200_sample(aleph_b200_handle* h, aleph_b200_state* st, uint32_t shots
   CK(copy_async(h, dvar, variates, vb, cudaMemcpyHostToDevice, h->stream), "variates upload");
   CK(launch_sample(st->amps, st->precision, st->n, shots, mode, dvar, dout, base, sb, dstatus, h->sm_count, h->stream),
      "sample");
-  h->stats.kernel_launches += mode == ALEPH_B200_SAMPLE_ALIAS ? 7 : 5;
+  h->stats.kernel_launches += mode == ALEPH_B200_SAMPLE_ALIAS ? 12 : 11;
   int32_t status[4];
   CK(copy_async(h, status, dstatus, 16, cudaMemcpyDeviceToHost, h->stream), "status readback");
   CK(copy_async(h, out, dout, vb, cudaMemcpyDeviceToHost, h->stream), "sample readback");
@@ -1612,7 +1627,7 @@ int aleph_b200_sample_cumulative_noalloc(aleph_b200_handle* h, aleph_b200_state*
   CK(launch_sample(st->amps, st->precision, st->n, shots, ALEPH_B200_SAMPLE_CUMULATIVE, dvar, dout, base, sb, dstatus,
                    h->sm_count, h->stream),
      "sample");
-  h->stats.kernel_launches += shots ? 5 : 3;
+  h->stats.kernel_launches += shots ? 11 : 5;
   int32_t status[4];
   CK(copy_async(h, status, dstatus, 16, cudaMemcpyDeviceToHost, h->stream), "status readback");
   if (shots) CK(copy_async(h, out, dout, vb, cudaMemcpyDeviceToHost, h->stream), "sample readback");
@@ -1632,7 +1647,7 @@ int aleph_b200_expectation(aleph_b200_handle* h, aleph_b200_state* st, const uin
   if (!h || !st || !out || (nt && (!qubits || !paulis))) return ALEPH_B200_INVALID_ARGUMENT;
   if (int r = bind(h)) return r;
   const uint32_t nb = reduce_blocks(st->n, h->sm_count);
-  if (int r = ensure(h, h->reduce, (size_t)nb * 3 * 8 + 256)) return r;
+  if (int r = ensure_reduce(h, (size_t)nb * 3 * 8 + 256)) return r;
   uint64_t xm = 0, zm = 0;
   uint32_t ny = 0;
   bool bad_pauli = false;
@@ -1646,7 +1661,7 @@ int aleph_b200_expectation(aleph_b200_handle* h, aleph_b200_state* st, const uin
       default: bad_pauli = true;
     }
   }
-  double* part = (double*)h->reduce.ptr;
+  double* part = reduce_area(h);
   double* out3 = part + 3 * (size_t)nb;
   const bool valid_q = [&] {
     for (uint32_t t = 0; t < nt; ++t)
@@ -1656,7 +1671,7 @@ int aleph_b200_expectation(aleph_b200_handle* h, aleph_b200_state* st, const uin
   CK(launch_expectation(st->amps, st->precision, st->n, valid_q ? xm : 0, valid_q ? zm : 0, ny, part, nb, out3,
                         h->stream),
      "expectation");
-  h->stats.kernel_launches += 2;
+  h->stats.kernel_launches += 1;
   double res[3];
   CK(copy_async(h, res, out3, 24, cudaMemcpyDeviceToHost, h->stream), "expectation readback");
   CK(cudaStreamSynchronize(h->stream), "stream synchronize");
@@ -1751,13 +1766,13 @@ int aleph_b200_expectation_sum(aleph_b200_handle* h, aleph_b200_state* st, const
   }
   constexpr size_t NV = 2 + PauliGroup::MAX_TERMS;
   const uint32_t nb = reduce_blocks(st->n, h->sm_count);
-  if (int r = ensure(h, h->reduce, ((size_t)nb + chunks.size()) * NV * 8 + 256)) return r;
-  double* part = (double*)h->reduce.ptr;
+  if (int r = ensure_reduce(h, ((size_t)nb + chunks.size()) * NV * 8 + 256)) return r;
+  double* part = reduce_area(h);
   double* res = part + NV * (size_t)nb;
   for (size_t c = 0; c < chunks.size(); ++c)
     CK(launch_pauli_group(st->amps, st->precision, st->n, chunks[c], part, nb, res + NV * c, h->stream),
        "Pauli sum");
-  h->stats.kernel_launches += 2 * chunks.size();
+  h->stats.kernel_launches += chunks.size();
   std::vector<double> host(NV * chunks.size());
   CK(copy_async(h, host.data(), res, host.size() * 8, cudaMemcpyDeviceToHost, h->stream), "Pauli sum readback");
   CK(cudaStreamSynchronize(h->stream), "stream synchronize");
@@ -1833,14 +1848,14 @@ int aleph_b200_probabilities(aleph_b200_handle* h, aleph_b200_state* st, const u
     return ALEPH_B200_OK;
   }
   const size_t dim = (size_t)1 << k;
-  if (int r = ensure(h, h->reduce, probabilities_scratch_bytes(st->n, qubits, k, h->sm_count) + 256)) return r;
+  if (int r = ensure_reduce(h, probabilities_scratch_bytes(st->n, qubits, k, h->sm_count) + 256)) return r;
   if (int r = ensure(h, h->sample, dim * 8 + 256)) return r;
   double* dnorm = (double*)h->sample.ptr;  // the norm's two sums, then the marginal
   double* dout = dnorm + 2;
-  CK(launch_probabilities(st->amps, st->precision, st->n, qubits, k, (double*)h->reduce.ptr, dout, dnorm, h->sm_count,
+  CK(launch_probabilities(st->amps, st->precision, st->n, qubits, k, reduce_area(h), dout, dnorm, h->sm_count,
                           h->stream),
      "probabilities");
-  h->stats.kernel_launches += 3;
+  h->stats.kernel_launches += 2;
   // a small marginal comes back with the norm in one copy
   const size_t head = dim <= 4096 ? dim + 2 : 2;
   std::vector<double> host(head);
@@ -1876,14 +1891,14 @@ int aleph_b200_fp64_rate(aleph_b200_handle* h, double* tflops) {
   if (!h || !tflops) return ALEPH_B200_INVALID_ARGUMENT;
   if (int r = bind(h)) return r;
   const uint32_t blocks = (uint32_t)h->sm_count * 8, iters = 20000;
-  if (int r = ensure(h, h->reduce, (size_t)blocks * 256 * 8 + 256)) return r;
+  if (int r = ensure_reduce(h, (size_t)blocks * 256 * 8 + 256)) return r;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CK(cudaEventCreate(&e0), "event");
   cudaError_t ce = cudaEventCreate(&e1);
   float best = 0.f;
   for (int k = 0; k < 4 && ce == cudaSuccess; ++k) {  // one warm-up launch, then three timed
     ce = cudaEventRecord(e0, h->stream);
-    if (ce == cudaSuccess) ce = launch_dfma_peak((double*)h->reduce.ptr, blocks, iters, h->stream);
+    if (ce == cudaSuccess) ce = launch_dfma_peak(reduce_area(h), blocks, iters, h->stream);
     if (ce == cudaSuccess) ce = cudaEventRecord(e1, h->stream);
     if (ce == cudaSuccess) ce = cudaEventSynchronize(e1);
     float ms = 0.f;
@@ -1947,10 +1962,10 @@ int aleph_b200_state_memory(aleph_b200_handle* h, aleph_b200_state* st, void** d
 int aleph_b200_scale_state(aleph_b200_handle* h, aleph_b200_state* st, double factor) {
   if (!h || !st || !(factor > 0.0) || !std::isfinite(factor)) return ALEPH_B200_INVALID_ARGUMENT;
   if (int r = bind(h)) return r;
-  if (int r = ensure(h, h->reduce, 256)) return r;
+  if (int r = ensure_reduce(h, 256)) return r;
   const double norm2 = 1.0 / (factor * factor);  // the rescale kernel multiplies by 1 / sqrt(norm2)
-  CK(copy_async(h, h->reduce.ptr, &norm2, sizeof(norm2), cudaMemcpyHostToDevice, h->stream), "scale upload");
-  CK(launch_rescale(st->amps, st->precision, st->n, (const double*)h->reduce.ptr, h->stream), "rescale");
+  CK(copy_async(h, reduce_area(h), &norm2, sizeof(norm2), cudaMemcpyHostToDevice, h->stream), "scale upload");
+  CK(launch_rescale(st->amps, st->precision, st->n, reduce_area(h), h->stream), "rescale");
   CK(cudaStreamSynchronize(h->stream), "stream synchronize");
   h->stats.kernel_launches += 1;
   return ALEPH_B200_OK;
@@ -1967,11 +1982,11 @@ int aleph_b200_norm_sqr(aleph_b200_handle* h, aleph_b200_state* st, double* out)
   if (!h || !st || !out) return ALEPH_B200_INVALID_ARGUMENT;
   if (int r = bind(h)) return r;
   const uint32_t nb = reduce_blocks(st->n, h->sm_count);
-  if (int r = ensure(h, h->reduce, (size_t)nb * 3 * 8 + 256)) return r;
-  double* part = (double*)h->reduce.ptr;
+  if (int r = ensure_reduce(h, (size_t)nb * 3 * 8 + 256)) return r;
+  double* part = reduce_area(h);
   double* out2 = part + 3 * (size_t)nb;
   CK(launch_norm(st->amps, st->precision, st->n, part, nb, out2, h->stream), "norm");
-  h->stats.kernel_launches += 2;
+  h->stats.kernel_launches += 1;
   double res[2];
   CK(copy_async(h, res, out2, 16, cudaMemcpyDeviceToHost, h->stream), "norm readback");
   CK(cudaStreamSynchronize(h->stream), "stream synchronize");

@@ -274,7 +274,10 @@ cudaError_t launch_permute_pass(void* amps, int precision, uint32_t n, const uin
 // pass P_sigma maps psi(j) -> psi(sigma(j)). At most two; none for the identity.
 std::vector<std::vector<uint8_t>> split_into_involutions(const std::vector<uint32_t>& pi);
 
-// readout (kernels_readout.cu)
+// readout (kernels_readout.cu). `partials` is the area behind a reduction
+// scratch's header (kReduceHeader bytes, zero before the first use): the blocks of
+// a reduction take tickets there, and the last one adds the partial sums.
+constexpr size_t kReduceHeader = 256;
 // partial sums: out[0] = sum |a|^2, out[1] = count of non-finite |a|^2
 cudaError_t launch_norm(const void* amps, int precision, uint32_t n, double* partials, uint32_t nblocks,
                         double* out2, cudaStream_t s);
@@ -369,8 +372,9 @@ cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t 
 // cudaGetSymbolAddress, with the target device current.
 constexpr size_t kFixedSampleScratchBytes = (size_t)8 << 20;
 // ... plus room for the chunk functions of the exact resolution, which do not
-// count against that limit: 20 bytes per 2048 amplitudes at n = 28.
-constexpr size_t kFixedChunkFnBytes = (((size_t)1 << kExactCumulativeMaxN) / 2048) * 20 + 4096;
+// count against that limit: 20 bytes per 2048 amplitudes at n = 28, and 36 KiB of
+// range totals and segments.
+constexpr size_t kFixedChunkFnBytes = (((size_t)1 << kExactCumulativeMaxN) / 2048) * 20 + (64 << 10);
 size_t sample_chunk_fn_bytes(uint32_t n);
 cudaError_t fixed_sample_scratch_address(void** out);
 

@@ -45,31 +45,56 @@ __device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* out)
   }
 }
 
-// Sum over the blocks of one of NV partials: every lane of a warp adds a
+// Sum over the blocks of one of NV partials by a warp: every lane adds a
 // strided share (four loads in flight), then a shuffle tree; the order is fixed.
 // (One thread adding 1184 partials in order took 65 us, as long as a sweep
-// over 2^25 complex64 amplitudes; a warp takes 4 us.)
+// over 2^25 complex64 amplitudes.)
 template <int NV>
 __device__ __forceinline__ double sum_partials(const double* __restrict__ partials, uint32_t nblocks, int k) {
   double s[4] = {0.0, 0.0, 0.0, 0.0};
   uint32_t b = threadIdx.x & 31;
   for (; b + 96 < nblocks; b += 128) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) s[u] += partials[(size_t)(b + 32 * u) * NV + k];
+    for (int u = 0; u < 4; ++u) s[u] += __ldcg(partials + (size_t)(b + 32 * u) * NV + k);
   }
-  for (; b < nblocks; b += 32) s[0] += partials[(size_t)b * NV + k];
+  for (; b < nblocks; b += 32) s[0] += __ldcg(partials + (size_t)b * NV + k);
   double x = (s[0] + s[1]) + (s[2] + s[3]);
   for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
   return x;
 }
 
-// partials[b*NV + k] -> out[k], one warp per k.
+// Stores this block's sums; the block that finishes last then adds all blocks'
+// and returns true with the totals in tot (valid for every thread). The
+// ticket returns to zero by itself. A kernel of its own for the totals cost
+// 4 us and a launch after every sweep.
 template <int NV>
-__global__ void __launch_bounds__(32 * NV) finish_kernel(const double* __restrict__ partials, uint32_t nblocks,
-                                                         double* __restrict__ out) {
-  const int k = threadIdx.x >> 5;
-  const double s = sum_partials<NV>(partials, nblocks, k);
-  if ((threadIdx.x & 31) == 0) out[k] = s;
+__device__ __forceinline__ bool reduce_grid(double (&v)[NV], double* partials, double (&tot)[NV]) {
+  __shared__ double all[NV];
+  __shared__ bool last;
+  block_reduce_store<NV>(v, partials + NV * (size_t)blockIdx.x);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    uint32_t* ticket = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(partials) - kReduceHeader);
+    last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return false;
+  for (int k = threadIdx.x >> 5; k < NV; k += RB / 32) {
+    const double s = sum_partials<NV>(partials, gridDim.x, k);
+    if ((threadIdx.x & 31) == 0) all[k] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) tot[k] = all[k];
+  return true;
+}
+template <int NV>
+__device__ __forceinline__ void reduce_grid_to(double (&v)[NV], double* partials, double* out) {
+  double tot[NV];
+  if (reduce_grid<NV>(v, partials, tot) && threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) out[k] = tot[k];
 }
 
 template <typename Real>
@@ -81,7 +106,7 @@ __device__ __forceinline__ double abs2(V2<Real> a) {
 // ---- norm: [sum |a|^2, non-finite count] ------------------------------------
 template <typename Real>
 __global__ void __launch_bounds__(RB) norm_kernel(const V2<Real>* __restrict__ amps, uint64_t len,
-                                                  double* __restrict__ partials) {
+                                                  double* partials, double* __restrict__ out2) {
   double v[2] = {0.0, 0.0};
   // four independent loads per step keep enough bytes in flight for the
   // 8-byte complex64 amplitudes (one load per step left the pass latency-bound)
@@ -103,23 +128,33 @@ __global__ void __launch_bounds__(RB) norm_kernel(const V2<Real>* __restrict__ a
     if (isfinite(p)) v[0] += p;
     else v[1] += 1.0;
   }
-  block_reduce_store<2>(v, partials + 2 * blockIdx.x);
+  reduce_grid_to<2>(v, partials, out2);
 }
 
 cudaError_t launch_norm(const void* amps, int precision, uint32_t n, double* partials, uint32_t nblocks, double* out2,
                         cudaStream_t s) {
   const uint64_t len = 1ull << n;
-  if (precision == ALEPH_B200_F64) norm_kernel<double><<<nblocks, RB, 0, s>>>((const double2*)amps, len, partials);
-  else norm_kernel<float><<<nblocks, RB, 0, s>>>((const float2*)amps, len, partials);
-  finish_kernel<2><<<1, 64, 0, s>>>(partials, nblocks, out2);
+  if (precision == ALEPH_B200_F64) norm_kernel<double><<<nblocks, RB, 0, s>>>((const double2*)amps, len, partials, out2);
+  else norm_kernel<float><<<nblocks, RB, 0, s>>>((const float2*)amps, len, partials, out2);
   return cudaGetLastError();
 }
 
 // ---- measurement ---------------------------------------------------------------
-// [p0, p1, non-finite count]
+// What a measurement's decision needs and writes.
+struct Decision {
+  uint32_t qubit, n_uniforms;
+  const double* uniforms;
+  int32_t* status;
+  double* dec;
+  uint8_t* outcome_slot;
+  double tol;
+};
+__device__ void measure_decide(const double* sums, const Decision& d);
+
+// [p0, p1, non-finite count], and the decision by the last block.
 template <typename Real>
 __global__ void __launch_bounds__(RB) branch_kernel(const V2<Real>* __restrict__ amps, uint64_t len, uint64_t qb,
-                                                    double* __restrict__ partials) {
+                                                    double* partials, const Decision d) {
   double v[3] = {0.0, 0.0, 0.0};
   auto add = [&](uint64_t i, double p) {
     if (!isfinite(p)) v[2] += 1.0;
@@ -136,26 +171,21 @@ __global__ void __launch_bounds__(RB) branch_kernel(const V2<Real>* __restrict__
     for (int k = 0; k < 4; ++k) add(i + k * stride, abs2<Real>(a[k]));
   }
   for (; i < len; i += stride) add(i, abs2<Real>(ld_amp<Real>(amps + i)));
-  block_reduce_store<3>(v, partials + 3 * blockIdx.x);
+  double tot[3];
+  if (reduce_grid<3>(v, partials, tot) && threadIdx.x == 0) measure_decide(tot, d);
 }
 
 // status[0]: error code (0 ok), status[1]: uniforms consumed, status[2]: failing qubit;
 // dec[0] = outcome (0/1), dec[1] = 1/norm scale; dval[0] = reported probability.
-// One warp per sum of the block partials, then one thread decides.
-__global__ void __launch_bounds__(96) measure_decide_kernel(const double* __restrict__ partials, uint32_t nblocks,
-                                                            uint32_t qubit, const double* __restrict__ uniforms,
-                                                            uint32_t n_uniforms, int32_t* status, double* dec,
-                                                            uint8_t* outcome_slot, double tol) {
-  __shared__ double sums[3];
-  const double part = sum_partials<3>(partials, nblocks, threadIdx.x >> 5);
-  if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = part;
-  __syncthreads();
-  if (threadIdx.x != 0) return;
+__device__ void measure_decide(const double* sums, const Decision& d) {
+  double* dec = d.dec;
+  int32_t* status = d.status;
+  const uint32_t qubit = d.qubit;
   dec[0] = -1.0;  // "skip collapse" unless a decision is made below
   if (status[0] != 0) return;  // an earlier instruction failed: do nothing further
   const double p0r = sums[0], p1r = sums[1], bad = sums[2];
   const double total = p0r + p1r;
-  if (bad > 0.0 || !isfinite(total) || fabs(total - 1.0) > tol) {
+  if (bad > 0.0 || !isfinite(total) || fabs(total - 1.0) > d.tol) {
     status[0] = ALEPH_B200_INVALID_STATE;
     status[2] = (int32_t)qubit;
     return;
@@ -177,18 +207,18 @@ __global__ void __launch_bounds__(96) measure_decide_kernel(const double* __rest
     p = p0;
   } else {
     const uint32_t used = (uint32_t)status[1];
-    if (used >= n_uniforms) {
+    if (used >= d.n_uniforms) {
       status[0] = ALEPH_B200_INVALID_ARGUMENT;
       status[2] = (int32_t)qubit;
       return;
     }
-    outcome = uniforms[used] < p1;
+    outcome = d.uniforms[used] < p1;
     status[1] = (int32_t)(used + 1);
     p = outcome ? p1 : p0;
   }
   dec[0] = outcome ? 1.0 : 0.0;
   dec[1] = sqrt(p);
-  if (outcome_slot) *outcome_slot = outcome ? 1 : 0;
+  if (d.outcome_slot) *d.outcome_slot = outcome ? 1 : 0;
 }
 
 // The kept half is read, divided and written; the other half is only written.
@@ -233,10 +263,11 @@ cudaError_t launch_measure_pass(void* amps, int precision, uint32_t n, uint32_t 
   const uint64_t len = 1ull << n;
   const uint64_t qb = 1ull << qubit;
   double* dec = partials + 3 * (size_t)nblocks;
-  if (precision == ALEPH_B200_F64) branch_kernel<double><<<nblocks, RB, 0, s>>>((const double2*)amps, len, qb, partials);
-  else branch_kernel<float><<<nblocks, RB, 0, s>>>((const float2*)amps, len, qb, partials);
-  measure_decide_kernel<<<1, 96, 0, s>>>(partials, nblocks, qubit, uniforms, n_uniforms, status, dec, outcome_slot,
-                                         norm_tolerance(len, precision));
+  const Decision d{qubit, n_uniforms, uniforms, status, dec, outcome_slot, norm_tolerance(len, precision)};
+  if (precision == ALEPH_B200_F64)
+    branch_kernel<double><<<nblocks, RB, 0, s>>>((const double2*)amps, len, qb, partials, d);
+  else
+    branch_kernel<float><<<nblocks, RB, 0, s>>>((const float2*)amps, len, qb, partials, d);
   const uint64_t pairs = len / 2, b = (pairs + 255) / 256;
   const unsigned blocks = (unsigned)(b > 148ull * 32 ? 148ull * 32 : b);
   if (precision == ALEPH_B200_F64) collapse_kernel<double><<<blocks, 256, 0, s>>>((double2*)amps, pairs, qubit, dec);
@@ -256,64 +287,77 @@ cudaError_t launch_measure_pass(void* amps, int precision, uint32_t n, uint32_t 
 // member read everything twice: 93 us a group at n = 23 FP64 against 28 us
 // now, with the terms unrolled to the group's size and not to 16.)
 // partials per block: [sum |a|^2, non-finite count, term 0 .. NT-1].
+//
+// Signs: an index is a warp-uniform part plus a lane part on disjoint bits, so the
+// parity of a term's mask splits the same way. Each lane forms one term's uniform
+// parity and a ballot hands all of them to the warp as one word.
 template <typename Real, bool DIAG, int NT>
 __global__ void __launch_bounds__(RB) pauli_group_kernel(const V2<Real>* __restrict__ amps, uint64_t count,
-                                                         const PauliGroup g, uint32_t pivot,
-                                                         double* __restrict__ partials) {
+                                                         const PauliGroup g, uint32_t pivot, double* partials,
+                                                         double* __restrict__ out) {
   constexpr int NV = 2 + NT, U = 4;
   double v[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) v[k] = 0.0;
   const uint64_t stride = (uint64_t)gridDim.x * RB;
-  auto add = [&](uint64_t i, V2<Real> a, V2<Real> b) {
+  const uint32_t lane = threadIdx.x & 31;
+  auto index = [&](uint64_t p) { return DIAG ? p : insert_zero(p, pivot); };
+  uint64_t my_z = 0;  // this lane's term
+  uint32_t lane_word = 0, swap = 0;  // per term: parity of the lane part; i^ny takes the imaginary part
+#pragma unroll
+  for (int k = 0; k < NT; ++k) {
+    if (k >= (int)g.count) break;
+    if ((int)lane == k) my_z = g.zmask[k];
+    const uint32_t y = DIAG ? 0u : g.ny[k] & 3;
+    // i^ny: ny & 3 = 0, 1, 2, 3 keeps re, -im, -re, im; the sign mask applies to j = i ^ xmask
+    const uint32_t flip = (y == 1 || y == 2) ^ (__popcll(g.zmask[k] & g.xmask) & 1);
+    lane_word |= ((__popcll(g.zmask[k] & index(lane)) & 1) ^ flip) << k;
+    swap |= (y & 1) << k;
+  }
+  auto add = [&](uint32_t word, V2<Real> a, V2<Real> b) {
     const double p = abs2<Real>(a), q = DIAG ? 0.0 : abs2<Real>(b);
     if (!isfinite(p) || !isfinite(q)) {
       v[1] += 1.0;
       return;
     }
     v[0] += p + q;
-    if constexpr (DIAG) {  // no X/Y factor: Re conj(a) a = |a|^2 and ny = 0
+    const double re = DIAG ? p : (double)a.x * b.x + (double)a.y * b.y;  // conj(a) * b
+    const double im = DIAG ? 0.0 : (double)a.x * b.y - (double)a.y * b.x;
 #pragma unroll
-      for (int k = 0; k < NT; ++k)
-        if (k < (int)g.count) v[2 + k] += (__popcll(g.zmask[k] & i) & 1) ? -p : p;
-    } else {
-      const uint64_t j = i ^ g.xmask;
-      const double re = (double)a.x * b.x + (double)a.y * b.y;  // conj(a) * b
-      const double im = (double)a.x * b.y - (double)a.y * b.x;
-#pragma unroll
-      for (int k = 0; k < NT; ++k)
-        if (k < (int)g.count) {
-          // i^ny: ny & 3 = 0, 1, 2, 3 keeps re, -im, -re, im
-          const uint32_t y = g.ny[k] & 3;
-          double t = (y & 1) ? im : re;
-          if ((y == 1 || y == 2) != (bool)(__popcll(g.zmask[k] & j) & 1)) t = -t;
-          v[2 + k] += t;
-        }
-    }
+    for (int k = 0; k < NT; ++k)
+      if (k < (int)g.count) {
+        const double t = !DIAG && ((swap >> k) & 1) ? im : re;
+        v[2 + k] += __hiloint2double(__double2hiint(t) ^ (int)((word << (31 - k)) & 0x80000000u), __double2loint(t));
+      }
   };
-  auto index = [&](uint64_t p) { return DIAG ? p : insert_zero(p, pivot); };
-  uint64_t p0 = (uint64_t)blockIdx.x * RB + threadIdx.x;
-  for (; p0 + (U - 1) * stride < count; p0 += U * stride) {  // loads in flight (see norm_kernel)
+  // the word of a warp whose first index is p: count and stride are multiples of 32, or there is one warp
+  auto word_at = [&](uint64_t p) {
+    return __ballot_sync(0xffffffffu, __popcll(my_z & index(p)) & 1) ^ lane_word;
+  };
+  uint64_t p0 = (uint64_t)blockIdx.x * RB + (threadIdx.x & ~31u);  // the warp's first
+  for (; p0 + (U - 1) * stride + 31 < count; p0 += U * stride) {  // loads in flight (see norm_kernel)
     V2<Real> a[U], b[U];
 #pragma unroll
     for (int k = 0; k < U; ++k) {
-      const uint64_t i = index(p0 + k * stride);
+      const uint64_t i = index(p0 + k * stride) | index(lane);
       a[k] = ld_amp<Real>(amps + i);
       if constexpr (!DIAG) b[k] = ld_amp<Real>(amps + (i ^ g.xmask));
     }
 #pragma unroll
-    for (int k = 0; k < U; ++k) add(index(p0 + k * stride), a[k], DIAG ? a[k] : b[k]);
+    for (int k = 0; k < U; ++k) add(word_at(p0 + k * stride), a[k], DIAG ? a[k] : b[k]);
   }
   for (; p0 < count; p0 += stride) {
-    const uint64_t i = index(p0);
+    const uint32_t word = word_at(p0);
+    if (p0 + lane >= count) continue;
+    const uint64_t i = index(p0) | index(lane);
     const V2<Real> a = ld_amp<Real>(amps + i);
-    add(i, a, DIAG ? a : ld_amp<Real>(amps + (i ^ g.xmask)));
+    add(word, a, DIAG ? a : ld_amp<Real>(amps + (i ^ g.xmask)));
   }
   if constexpr (!DIAG) {  // both members of each pair
 #pragma unroll
     for (int k = 0; k < NT; ++k) v[2 + k] *= 2.0;
   }
-  block_reduce_store<NV>(v, partials + NV * (size_t)blockIdx.x);
+  reduce_grid_to<NV>(v, partials, out);
 }
 
 template <typename Real, int NT>
@@ -321,11 +365,10 @@ static cudaError_t launch_pauli_t(const V2<Real>* amps, uint32_t n, const PauliG
                                   uint32_t nblocks, double* out, cudaStream_t s) {
   const uint64_t len = 1ull << n;
   if (g.xmask == 0)
-    pauli_group_kernel<Real, true, NT><<<nblocks, RB, 0, s>>>(amps, len, g, 0, partials);
+    pauli_group_kernel<Real, true, NT><<<nblocks, RB, 0, s>>>(amps, len, g, 0, partials, out);
   else
     pauli_group_kernel<Real, false, NT>
-        <<<nblocks, RB, 0, s>>>(amps, len / 2, g, 63u - (uint32_t)__builtin_clzll(g.xmask), partials);
-  finish_kernel<2 + NT><<<1, 32 * (2 + NT), 0, s>>>(partials, nblocks, out);
+        <<<nblocks, RB, 0, s>>>(amps, len / 2, g, 63u - (uint32_t)__builtin_clzll(g.xmask), partials, out);
   return cudaGetLastError();
 }
 
@@ -396,7 +439,7 @@ __device__ __forceinline__ uint64_t deposit(uint64_t x, uint64_t mask) {  // bit
 template <typename Real>
 __global__ void __launch_bounds__(RB) marginal_kernel(const V2<Real>* __restrict__ amps, const Marginal m,
                                                       uint64_t items, double* __restrict__ tables,
-                                                      double* __restrict__ norm_partials) {
+                                                      double* norm_partials, double* __restrict__ norm_out) {
   __shared__ double red[RB / 32][32];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const bool meet = m.split_bits >= 3;  // the CTA's warps are eight splits of one pattern
@@ -463,7 +506,7 @@ __global__ void __launch_bounds__(RB) marginal_kernel(const V2<Real>* __restrict
     }
   }
   __syncthreads();
-  block_reduce_store<2>(v, norm_partials + 2 * (size_t)blockIdx.x);
+  reduce_grid_to<2>(v, norm_partials, norm_out);
 }
 
 // out[o] = sum over the tables, a warp per output in a fixed order.
@@ -528,14 +571,13 @@ cudaError_t launch_probabilities(const void* amps, int precision, uint32_t n, co
   double* partials = scratch;
   double* tables = P.tables > 1 ? scratch + 2 * (size_t)P.blocks : out;
   if (precision == ALEPH_B200_F64)
-    marginal_kernel<double><<<P.blocks, RB, 0, s>>>((const double2*)amps, P.m, P.items, tables, partials);
+    marginal_kernel<double><<<P.blocks, RB, 0, s>>>((const double2*)amps, P.m, P.items, tables, partials, norm_out);
   else
-    marginal_kernel<float><<<P.blocks, RB, 0, s>>>((const float2*)amps, P.m, P.items, tables, partials);
+    marginal_kernel<float><<<P.blocks, RB, 0, s>>>((const float2*)amps, P.m, P.items, tables, partials, norm_out);
   if (P.tables > 1) {
     const uint64_t dim = 1ull << k, b = (dim + 7) / 8;
     marginal_sum_kernel<<<(unsigned)(b < 4096 ? b : 4096), 256, 0, s>>>(tables, P.tables, dim, out);
   }
-  finish_kernel<2><<<1, 64, 0, s>>>(partials, P.blocks, norm_out);
   return cudaGetLastError();
 }
 

@@ -18,8 +18,8 @@
 //   sequential running sum (for n <= 28), so the outcome equals the
 //   sequential CPU result. The running sum, too, is evaluated in parallel.
 //
-// Measured on B200: alias table and 1024 shots at n = 22 FP64 0.78 ms (234 ms
-// with the chain on one lane); 4096 cumulative shots at n = 26 FP32 1.0 ms (458
+// Measured on B200: alias table and 1024 shots at n = 22 FP64 0.71 ms (234 ms
+// with the chain on one lane); 4096 cumulative shots at n = 26 FP32 0.76 ms (458
 // ms with the sum on one lane).
 
 #include <cmath>
@@ -386,8 +386,8 @@ __global__ void __launch_bounds__(128) alias_spec_kernel(AliasScratch s, uint32_
   stage_chunk(s, m, i0, j0, ns, nl, o);
   const double unit = s.cunit[c];
   double V = s.cbase[c] + (double)lane * unit;
-  const long long one = 1ll << 52;
-  long long margin = (long long)fmin(fabs(V - 1.0) * kUnits, 0x1p60);
+  const double start = fmin(fabs(V - 1.0) * kUnits, 0x1p60);
+  uint32_t near = 0xffffffffu;  // least distance of an S to its binade's ends, units of 2^-32 of the binade
   int smax = 0;
   uint32_t is = 0, il = 0;
   double va = o.a[0], vb = o.b[0];
@@ -398,17 +398,17 @@ __global__ void __launch_bounds__(128) alias_spec_kernel(AliasScratch s, uint32_
     il += small ? 0u : 1u;
     va = o.a[is];  // is, il <= len <= CH_MAX: inside the arrays whatever this lane decided
     vb = o.b[il];
-    const long long bits = __double_as_longlong(S);
-    const long long mant = bits & (one - 1);
-    const int hi = (int)(bits >> 32);
-    // distance to the binade's ends, at least this many units of 2^-52 (S >= 1 always)
-    long long d = one - mant;
-    if (hi >= 0x40000000) d = min(d, mant);
-    margin = min(margin, d);
+    // the top 32 mantissa bits: S is at least that far above its binade's lower end
+    // (which binds from 2 up; S >= 1 always) and at least the complement below the upper one
+    const int hi = __double2hiint(S);
+    const uint32_t top = __funnelshift_l((uint32_t)__double2loint(S), (uint32_t)hi, 12);
+    near = min(near, hi >= 0x40000000 ? min(top, ~top) : ~top);
     smax = max(smax, hi);
     V = __dsub_rn(S, 1.0);
   }
   const bool ok = is == ns && il == nl;  // this lane popped what the prefix sums predicted
+  // in units of 2^-52, rounded down: a binade spans 2^52 units or more
+  long long margin = min((long long)start, (long long)near << 20);
   for (int x = 16; x; x >>= 1) {
     margin = min(margin, __shfl_xor_sync(0xffffffffu, margin, x));
     smax = max(smax, __shfl_xor_sync(0xffffffffu, smax, x));
@@ -434,14 +434,14 @@ struct Entry {
 constexpr long long kMoved = 1ll << 28;
 __device__ __forceinline__ bool enter_chunk(double V, double base, double unit, long long margin, long long max_moved,
                                             Entry* e, long long* left) {
-  const double q = (V - base) / unit;  // exact: a power of two, and V close to base on its grid
+  const int g = exponent_of(unit) + 52;
+  if (g < 0 || g > 30) return false;
+  const double q = (V - base) * pow2(52 - g);  // over unit, a power of two: exact, with V close to base on its grid
   if (!(fabs(q) < 0x1p30)) return false;
   const long long qi = (long long)q;
   if ((double)qi != q) return false;  // not on this chunk's grid
   const int r = (int)(qi & 31);
   const long long D = qi - r;
-  const int g = exponent_of(unit) + 52;
-  if (g < 0 || g > 30) return false;
   const long long moved = (D < 0 ? -D : D) << g;  // units of 2^-52
   *left = margin - moved;
   if (*left <= 0 || moved > max_moved) return false;
@@ -753,6 +753,11 @@ struct CumScratch {
   uint32_t* amb;     // shots: ambiguous shot ids
   double* ck;        // exact mode: sequential sum at the end of every SEQ_CH chunk
   double* seq;       // exact mode: [sequential total, last positive index (bits)]
+  double* part;      // PREFIX_T range totals of the block prefix
+  // exact mode: the chunks in up to PREFIX_T segments: function, binade, start (< 0: not walked whole)
+  SeqFn* sfn;
+  int* sfe;
+  double* sstart;
   SeqFn* fn;         // exact mode: the chunk as a function of the start's parity
   int* fe;           // exact mode: its binade (kNoBinade: crosses one; kAnyBinade: adds nothing)
 };
@@ -788,19 +793,30 @@ __global__ void cum_blocks_kernel(const V2<Real>* __restrict__ amps, uint64_t le
   }
 }
 
-// Exclusive prefix of the block sums, one CTA of PREFIX_T threads: thread t
-// sums a contiguous range, the range totals are scanned in shared memory, and
-// each thread writes its range's prefixes. The draws treat this prefix as an
-// approximation (guard band E below), so its rounding order is free.
+// Exclusive prefix of the block sums: PREFIX_T contiguous ranges are added in
+// order, their totals are scanned, and each range's prefixes are written in
+// order. The draws treat this prefix as an approximation (guard band E below), so
+// its rounding order is free, but it is kept. The ranges are spread over CTAs
+// of one warp: on one SM the strided reads alone took 50 us at n = 26.
 constexpr uint32_t PREFIX_T = 1024;
+constexpr uint32_t RANGE_T = 32;  // threads per CTA of the range kernels
+__device__ __forceinline__ void range_of(uint32_t n, uint32_t t, uint32_t* b0, uint32_t* b1) {
+  const uint32_t per = (n + PREFIX_T - 1) / PREFIX_T;
+  *b0 = min(n, t * per);
+  *b1 = min(n, *b0 + per);
+}
+__global__ void __launch_bounds__(RANGE_T) cum_range_kernel(CumScratch c, uint32_t nb) {
+  const uint32_t t = blockIdx.x * RANGE_T + threadIdx.x;
+  uint32_t b0, b1;
+  range_of(nb, t, &b0, &b1);
+  double s = 0.0;
+  for (uint32_t b = b0; b < b1; ++b) s += c.bsum[b];
+  c.part[t] = s;
+}
 __global__ void __launch_bounds__(PREFIX_T) cum_prefix_kernel(CumScratch c, uint32_t nb) {
   __shared__ double part[PREFIX_T];
   const uint32_t t = threadIdx.x;
-  const uint32_t per = (nb + PREFIX_T - 1) / PREFIX_T;
-  const uint32_t b0 = min(nb, t * per), b1 = min(nb, b0 + per);
-  double s = 0.0;
-  for (uint32_t b = b0; b < b1; ++b) s += c.bsum[b];
-  part[t] = s;
+  part[t] = c.part[t];
   __syncthreads();
   for (uint32_t off = 1; off < PREFIX_T; off <<= 1) {  // inclusive Hillis-Steele scan
     const double v = t >= off ? part[t - off] : 0.0;
@@ -808,15 +824,21 @@ __global__ void __launch_bounds__(PREFIX_T) cum_prefix_kernel(CumScratch c, uint
     part[t] += v;
     __syncthreads();
   }
-  double run = t ? part[t - 1] : 0.0;
+  c.part[t] = part[t];
+  if (t == PREFIX_T - 1) {
+    c.bsum[nb] = part[PREFIX_T - 1];
+    c.norm[0] = part[PREFIX_T - 1];
+  }
+}
+__global__ void __launch_bounds__(RANGE_T) cum_spread_kernel(CumScratch c, uint32_t nb) {
+  const uint32_t t = blockIdx.x * RANGE_T + threadIdx.x;
+  uint32_t b0, b1;
+  range_of(nb, t, &b0, &b1);
+  double run = t ? c.part[t - 1] : 0.0;
   for (uint32_t b = b0; b < b1; ++b) {
     const double x = c.bsum[b];
     c.bsum[b] = run;
     run += x;
-  }
-  if (t == PREFIX_T - 1) {
-    c.bsum[nb] = part[PREFIX_T - 1];
-    c.norm[0] = part[PREFIX_T - 1];
   }
 }
 
@@ -1017,89 +1039,111 @@ __global__ void __launch_bounds__(256) cum_fn_kernel(const V2<Real>* __restrict_
   }
 }
 
-// Applies a chunk's (or segment's) function to *S; false when S is not in its
-// binade at both ends.
-__device__ __forceinline__ bool seq_step(double* S, int e, const SeqFn& f) {
+// A sum as its mantissa (units of 2^(e-52)) and binade.
+struct SeqSum {
+  long long mant;
+  int e;
+};
+__device__ __forceinline__ SeqSum seq_sum(double S) {
+  const long long bits = __double_as_longlong(S);
+  return SeqSum{(bits & ((1ll << 52) - 1)) | (1ll << 52), (int)((bits >> 52) & 0x7ff) - 1023};
+}
+__device__ __forceinline__ double seq_value(const SeqSum& s) {
+  return __longlong_as_double(((long long)(s.e + 1023) << 52) | (s.mant & ((1ll << 52) - 1)));
+}
+// Applies a chunk's (or segment's) function; false when the sum does not stay in its binade.
+__device__ __forceinline__ bool seq_step(SeqSum* s, int e, const SeqFn& f) {
   if (e == kAnyBinade) return true;
-  const long long bits = __double_as_longlong(*S);
-  if (e == kNoBinade || (int)((bits >> 52) & 0x7ff) - 1023 != e) return false;
-  const long long off = (bits & 1) ? f.o1 : f.o0;
-  const long long mant = (bits & ((1ll << 52) - 1)) | (1ll << 52);
-  if (mant + off >= kSeqOver) return false;
-  *S = seq_add(*S, off, __longlong_as_double((long long)(e - 52 + 1023) << 52));
+  if (e != s->e) return false;
+  const long long m = s->mant + ((s->mant & 1) ? f.o1 : f.o0);
+  if (m >= kSeqOver) return false;
+  s->mant = m;
   return true;
 }
 
+// The chunks of each segment composed: one binade, or kNoBinade.
+__global__ void __launch_bounds__(RANGE_T) cum_compose_kernel(CumScratch c, uint32_t nch) {
+  if (*c.namb == 0) return;
+  const uint32_t t = blockIdx.x * RANGE_T + threadIdx.x;
+  uint32_t c0, c1;
+  range_of(nch, t, &c0, &c1);
+  SeqFn f{0, 0};
+  int e = kAnyBinade;
+  for (uint32_t k = c0; k < c1; ++k) {
+    const int ek = c.fe[k];
+    const SeqFn fk = c.fn[k];
+    if (ek == kAnyBinade) continue;
+    if (e == kAnyBinade) {
+      e = ek;
+      f = fk;
+    } else if (ek == e && e != kNoBinade) {
+      f = seq_then(f, fk);
+    } else {
+      e = kNoBinade;
+    }
+  }
+  c.sfn[t] = f;
+  c.sfe[t] = e;
+  c.sstart[t] = -1.0;
+}
+
 constexpr uint32_t WALK_T = 1024;
+static_assert(WALK_T == PREFIX_T && 2 * WALK_T == SEQ_CH, "a thread per segment, and two elements of a crossing chunk");
+// chunks per segment at most (n = kExactCumulativeMaxN)
+constexpr uint32_t kWalkChunks = (uint32_t)(((uint64_t)1 << kExactCumulativeMaxN) / SEQ_CH / WALK_T);
 template <typename Real>
 __global__ void __launch_bounds__(WALK_T) cum_walk_kernel(const V2<Real>* __restrict__ amps, uint64_t len,
                                                           uint32_t nch, CumScratch c) {
   __shared__ SeqFn sfn[WALK_T];
   __shared__ int se[WALK_T];
-  __shared__ double sstart[WALK_T];
-  __shared__ bool swalked[WALK_T];
   __shared__ SeqFn wtot[32];
+  __shared__ SeqFn cfn[kWalkChunks];  // the chunks of the segment at hand
+  __shared__ int cfe[kWalkChunks];
   __shared__ double S_sh;
   __shared__ uint32_t seg_sh, ch_sh, first_sh;
   if (*c.namb == 0) return;
   const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
   const uint32_t per = (nch + WALK_T - 1) / WALK_T;
-  const uint32_t c0 = min(nch, t * per), c1 = min(nch, c0 + per);
-  {
-    SeqFn f{0, 0};
-    int e = kAnyBinade;
-    for (uint32_t k = c0; k < c1; ++k) {
-      const int ek = c.fe[k];
-      if (ek == kAnyBinade) continue;
-      if (e == kAnyBinade) {
-        e = ek;
-        f = c.fn[k];
-      } else if (ek == e) {
-        f = seq_then(f, c.fn[k]);
-      } else {
-        e = kNoBinade;
-      }
-      if (e == kNoBinade) break;
-    }
-    sfn[t] = f;
-    se[t] = e;
-    swalked[t] = false;
-  }
+  sfn[t] = c.sfn[t];
+  se[t] = c.sfe[t];
   if (t == 0) {
     S_sh = 0.0;
     seg_sh = 0;
   }
   __syncthreads();
-  const uint32_t nseg = per ? (nch + per - 1) / per : 0;
+  const uint32_t nseg = (nch + per - 1) / per;
   for (;;) {
     if (t == 0) {  // as many whole segments as hold
-      double S = S_sh;
+      SeqSum S = seq_sum(S_sh);
       uint32_t g = seg_sh;
       for (; g < nseg; ++g) {
-        const double at = S;
+        const SeqSum at = S;
         if (!seq_step(&S, se[g], sfn[g])) break;
-        sstart[g] = at;
-        swalked[g] = true;
+        c.sstart[g] = S_sh > 0.0 ? seq_value(at) : 0.0;
       }
-      S_sh = S;
+      if (S_sh > 0.0) S_sh = seq_value(S);
       seg_sh = g;
       ch_sh = g * per;
     }
     __syncthreads();
     const uint32_t g = seg_sh;
     if (g >= nseg) break;
-    const uint32_t end = min(nch, (g + 1) * per);
+    const uint32_t first = g * per, end = min(nch, first + per);
+    for (uint32_t k = first + t; k < end; k += WALK_T) {
+      cfe[k - first] = c.fe[k];
+      cfn[k - first] = c.fn[k];
+    }
     for (;;) {  // its chunks one by one
       __syncthreads();
       if (t == 0) {
-        double S = S_sh;
+        SeqSum S = seq_sum(S_sh);
+        const bool zero = !(S_sh > 0.0);
         uint32_t k = ch_sh;
         for (; k < end; ++k) {
-          const int ek = c.fe[k];
-          if (!seq_step(&S, ek, ek == kNoBinade || ek == kAnyBinade ? SeqFn{0, 0} : c.fn[k])) break;
-          c.ck[k] = S;
+          if (!seq_step(&S, cfe[k - first], cfn[k - first])) break;
+          c.ck[k] = zero ? 0.0 : seq_value(S);
         }
-        S_sh = S;
+        if (!zero) S_sh = seq_value(S);
         ch_sh = k;
       }
       __syncthreads();
@@ -1120,61 +1164,54 @@ __global__ void __launch_bounds__(WALK_T) cum_walk_kernel(const V2<Real>* __rest
         if (S < kSeqMin) {  // near zero: the next positive element by itself
           if (a0 && p0 > 0.0) stop = 2 * t;
           else if (a1 && p1 > 0.0) stop = 2 * t + 1;
+          if (stop < SEQ_CH) atomicMin(&first_sh, stop);
+          __syncthreads();
+          if (first_sh == SEQ_CH) break;
         } else {
-          const long long bits = __double_as_longlong(S);
-          const int ex = (int)((bits >> 52) & 0x7ff) - 1023;
-          const double scale = __longlong_as_double((long long)(52 - ex + 1023) << 52);
-          const double unit = __longlong_as_double((long long)(ex - 52 + 1023) << 52);
+          const SeqSum q = seq_sum(S);
+          const double scale = __longlong_as_double((long long)(52 - q.e + 1023) << 52);
           bool tie = false;
           const SeqFn f0 = a0 ? seq_fn(p0, scale, &tie) : SeqFn{0, 0}, f1 = a1 ? seq_fn(p1, scale, &tie) : SeqFn{0, 0};
-          SeqFn f = seq_then(f0, f1);
-          SeqFn inc = f;
+          SeqFn inc = seq_then(f0, f1);
+          auto scan = [&](SeqFn x) {  // inclusive over the warp, in order
 #pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            SeqFn x;
-            x.o0 = __shfl_up_sync(0xffffffffu, inc.o0, o);
-            x.o1 = __shfl_up_sync(0xffffffffu, inc.o1, o);
-            if (lane >= (uint32_t)o) inc = seq_then(x, inc);
-          }
+            for (int o = 1; o < 32; o <<= 1) {
+              SeqFn y;
+              y.o0 = __shfl_up_sync(0xffffffffu, x.o0, o);
+              y.o1 = __shfl_up_sync(0xffffffffu, x.o1, o);
+              if (lane >= (uint32_t)o) x = seq_then(y, x);
+            }
+            return x;
+          };
+          inc = scan(inc);
           if (lane == 31) wtot[w] = inc;
-          SeqFn ex_lane;  // exclusive within the warp
-          ex_lane.o0 = __shfl_up_sync(0xffffffffu, inc.o0, 1);
-          ex_lane.o1 = __shfl_up_sync(0xffffffffu, inc.o1, 1);
-          if (lane == 0) ex_lane = SeqFn{0, 0};
+          SeqFn ex;  // exclusive within the warp
+          ex.o0 = __shfl_up_sync(0xffffffffu, inc.o0, 1);
+          ex.o1 = __shfl_up_sync(0xffffffffu, inc.o1, 1);
+          if (lane == 0) ex = SeqFn{0, 0};
           __syncthreads();
-          SeqFn pre{0, 0};
-          for (uint32_t x = 0; x < w; ++x) pre = seq_then(pre, wtot[x]);
-          pre = seq_then(pre, ex_lane);
-          const bool odd = bits & 1;
-          const long long mant = (bits & ((1ll << 52) - 1)) | (1ll << 52);
-          // sums of up to 2048 marked elements stay below 2^64
-          const long long m0 = mant + (odd ? pre.o1 : pre.o0);
-          const long long g0 = (m0 & 1) ? f0.o1 : f0.o0;
-          const long long m1 = m0 + g0;
-          const long long g1 = (m1 & 1) ? f1.o1 : f1.o0;
+          if (w == 0) wtot[lane] = scan(wtot[lane]);
+          __syncthreads();
+          const SeqFn pre = seq_then(w ? wtot[w - 1] : SeqFn{0, 0}, ex);
+          // at the first element that leaves the binade all sums before it are below 2^53
+          const long long m0 = q.mant + ((q.mant & 1) ? pre.o1 : pre.o0);
+          const long long m1 = m0 + ((m0 & 1) ? f0.o1 : f0.o0);
+          const long long m2 = m1 + ((m1 & 1) ? f1.o1 : f1.o0);
           if (a0 && m1 >= kSeqOver) {
             stop = 2 * t;
-            before = seq_add(S, m0 - mant, unit);
-          } else if (a1 && m1 + g1 >= kSeqOver) {
+            before = seq_value(SeqSum{m0, q.e});
+          } else if (a1 && m2 >= kSeqOver) {
             stop = 2 * t + 1;
-            before = seq_add(S, m1 - mant, unit);
+            before = seq_value(SeqSum{m1, q.e});
           }
           if (stop < SEQ_CH) atomicMin(&first_sh, stop);
           __syncthreads();
           if (first_sh == SEQ_CH) {  // the rest stays in the binade
-            if (t == WALK_T - 1) S_sh = seq_add(S, m1 + g1 - mant, unit);
-            __syncthreads();
+            if (t == WALK_T - 1) S_sh = seq_value(SeqSum{m2, q.e});
             break;
           }
-          if (stop == first_sh) S_sh = __dadd_rn(before, (stop & 1) ? p1 : p0);
-          pos = first_sh + 1;
-          __syncthreads();
-          continue;
         }
-        if (stop < SEQ_CH) atomicMin(&first_sh, stop);
-        __syncthreads();
-        if (first_sh == SEQ_CH) break;
-        if (stop == first_sh) S_sh = __dadd_rn(S, (stop & 1) ? p1 : p0);
+        if (stop == first_sh) S_sh = __dadd_rn(before, (stop & 1) ? p1 : p0);
         pos = first_sh + 1;
         __syncthreads();
       }
@@ -1188,15 +1225,22 @@ __global__ void __launch_bounds__(WALK_T) cum_walk_kernel(const V2<Real>* __rest
     if (t == 0) seg_sh = g + 1;
     __syncthreads();
   }
-  if (t < nseg && swalked[t]) {  // the checkpoints inside the walked segments
-    double S = sstart[t];
-    for (uint32_t k = c0; k < c1; ++k) {
-      const int ek = c.fe[k];
-      if (ek != kAnyBinade) seq_step(&S, ek, c.fn[k]);
-      c.ck[k] = S;
-    }
-  }
   if (t == 0) c.seq[0] = S_sh;
+}
+
+// The checkpoints inside the segments that were walked whole.
+__global__ void __launch_bounds__(RANGE_T) cum_expand_kernel(CumScratch c, uint32_t nch) {
+  if (*c.namb == 0) return;
+  const uint32_t t = blockIdx.x * RANGE_T + threadIdx.x;
+  uint32_t c0, c1;
+  range_of(nch, t, &c0, &c1);
+  const double start = c.sstart[t];
+  if (start < 0.0) return;
+  SeqSum S = seq_sum(start);
+  for (uint32_t k = c0; k < c1; ++k) {
+    seq_step(&S, c.fe[k], c.fn[k]);
+    c.ck[k] = start > 0.0 ? seq_value(S) : 0.0;
+  }
 }
 
 // One warp per ambiguous shot.
@@ -1237,7 +1281,7 @@ __global__ void __launch_bounds__(128) cum_exact_kernel(const V2<Real>* __restri
 size_t sample_chunk_fn_bytes(uint32_t n) {
   const uint64_t len = 1ull << n;
   const uint64_t nch = n <= EXACT_MAX_N ? (len + SEQ_CH - 1) / SEQ_CH : 0;
-  return nch * (sizeof(SeqFn) + 4) + 32;
+  return nch * (sizeof(SeqFn) + 4) + PREFIX_T * (8 + sizeof(SeqFn) + 4 + 8) + 128;
 }
 
 namespace {
@@ -1352,11 +1396,17 @@ cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t 
   c.ck = (double*)p; p += (size_t)nch * 8;
   c.fn = (SeqFn*)align_up(p, 16); p = (char*)(c.fn + nch);
   c.fe = (int*)p; p += (size_t)nch * 4;
+  c.part = (double*)align_up(p, 16); p = (char*)(c.part + PREFIX_T);
+  c.sfn = (SeqFn*)align_up(p, 16); p = (char*)(c.sfn + PREFIX_T);
+  c.sstart = (double*)p; p += PREFIX_T * 8;
+  c.sfe = (int*)p; p += PREFIX_T * 4;
   if ((size_t)(p - (char*)scratch) > scratch_bytes) return cudaErrorInvalidValue;
   cudaMemsetAsync(c.norm, 0, 48, st);  // norm, namb, seq
   if (f64) cum_blocks_kernel<double><<<nb, 256, 0, st>>>((const double2*)amps, len, c);
   else cum_blocks_kernel<float><<<nb, 256, 0, st>>>((const float2*)amps, len, c);
+  cum_range_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nb);
   cum_prefix_kernel<<<1, PREFIX_T, 0, st>>>(c, nb);
+  cum_spread_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nb);
   check_norm_kernel<<<1, 32, 0, st>>>(c.norm, norm_tolerance(len, precision), status);
   if (shots) {
     const unsigned wb = (shots + 3) / 4;  // a warp per shot
@@ -1368,11 +1418,15 @@ cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t 
     if (n <= EXACT_MAX_N) {
       if (f64) {
         cum_fn_kernel<double><<<nch, 256, 0, st>>>((const double2*)amps, len, c);
+        cum_compose_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nch);
         cum_walk_kernel<double><<<1, WALK_T, 0, st>>>((const double2*)amps, len, nch, c);
+        cum_expand_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nch);
         cum_exact_kernel<double><<<wb, 128, 0, st>>>((const double2*)amps, len, c, u, out, status);
       } else {
         cum_fn_kernel<float><<<nch, 256, 0, st>>>((const float2*)amps, len, c);
+        cum_compose_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nch);
         cum_walk_kernel<float><<<1, WALK_T, 0, st>>>((const float2*)amps, len, nch, c);
+        cum_expand_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nch);
         cum_exact_kernel<float><<<wb, 128, 0, st>>>((const float2*)amps, len, c, u, out, status);
       }
     }
