@@ -2,6 +2,8 @@
 #pragma once
 
 #include <cstdint>
+#include <utility>
+
 #include <cuda_runtime.h>
 
 #include "engine.h"
@@ -123,6 +125,29 @@ __device__ __forceinline__ bool is_diag_type(uint8_t t) {
 __device__ __forceinline__ uint64_t insert_zero(uint64_t x, uint32_t pos) {
   const uint64_t lo = x & ((1ull << pos) - 1);
   return ((x >> pos) << (pos + 1)) | lo;
+}
+
+// Programmatic dependent launch: a pass kernel lets the next one start at once
+// (its blocks take free SMs, set up and wait), and touches the state only after
+// the kernel before it has completed.
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launches `kern` so that it may start before the previous kernel of the stream ends.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_overlapped(void (*kern)(Params...), unsigned grid, unsigned threads, size_t smem,
+                                     cudaStream_t s, Args&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
 // Nanoseconds of the GPU's global timer.

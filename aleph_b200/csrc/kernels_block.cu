@@ -334,6 +334,7 @@ __global__ void __launch_bounds__(blk::THREADS, 1) block_kernel(const __grid_con
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t n = a.n;
   volatile int* abort_flag = &abort_sh;
+  grid_launch_next();  // the next pass may set up on SMs this one leaves free
 
   // ---- tile geometry (computed on the host) ---------------------------------
   uint64_t bmask = 0;
@@ -444,6 +445,9 @@ __global__ void __launch_bounds__(blk::THREADS, 1) block_kernel(const __grid_con
       mbar_expect_tx(bar_w, W_BYTES);
       bulk_load(sbase + OFF_W, a.image, W_BYTES, bar_w);
     }
+    // the state is touched from here on (every store follows a load of this warp);
+    // operands, post ops and tables come from the plan, which no kernel writes
+    grid_wait_previous();
     uint32_t i = 0;
     for (uint64_t t = first; t < ntiles; t += stride, ++i) {
       const uint32_t s = i & 1, ph = (i >> 1) & 1;
@@ -933,11 +937,7 @@ cudaError_t launch_block_pass(void* amps, const BlockPass& p, const uint8_t* ima
   }
   const uint64_t ntiles = 1ull << (p.n - 13);
   const unsigned grid = (unsigned)(ntiles < (uint64_t)sm_count ? ntiles : (uint64_t)sm_count);
-  if (p.fold)
-    block_kernel<true><<<grid, blk::THREADS, blk::SMEM_BYTES, s>>>(a);
-  else
-    block_kernel<false><<<grid, blk::THREADS, blk::SMEM_BYTES, s>>>(a);
-  return cudaGetLastError();
+  return launch_overlapped(p.fold ? block_kernel<true> : block_kernel<false>, grid, blk::THREADS, blk::SMEM_BYTES, s, a);
 }
 
 // Host helper: lay out a 128x128 real matrix (row-major doubles, W[r][k]) as
