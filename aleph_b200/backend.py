@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import ctypes as ct
 from dataclasses import dataclass
+from itertools import chain
 
 import numpy as np
 
@@ -350,17 +351,19 @@ class B200SvBackend:
         if gam.shape != bet.shape:
             raise ValueError("gammas and betas must have the same shape")
         p = gam.shape[1]
-        sets = (abi.QaoaSet * max(1, count))()
-        pool = []
-        for k, (nq, edges) in enumerate(graphs):
-            sets[k].num_qubits, sets[k].num_edges, sets[k].edge_offset = nq, len(edges), len(pool) // 2
-            for (i, j) in edges:
-                pool += [int(i), int(j)]
-        edges_arr = np.ascontiguousarray(np.asarray(pool, dtype=np.uint32))
+        # whole columns at once: a 384-graph batch holds some 12,000 edges
+        lens = [len(edges) for _, edges in graphs]
+        sets = np.zeros(max(1, count), dtype=np.dtype(abi.QaoaSet))
+        sets["num_qubits"][:count] = [nq for nq, _ in graphs]
+        sets["num_edges"][:count] = lens
+        sets["edge_offset"][:count] = np.cumsum([0] + lens[:-1]) if count else 0
+        edges_arr = np.fromiter(chain.from_iterable(chain.from_iterable(edges for _, edges in graphs)), dtype=np.uint32)
+        if edges_arr.size != 2 * sum(lens):
+            raise ValueError("an edge is a pair of qubits")
         ang = np.ascontiguousarray(np.concatenate([gam, bet], axis=1))
         out = np.zeros(max(1, count), dtype=np.float64)
         self._check(self.lib.aleph_b200_qaoa_sweep(
-            self.handle, p, sets, count, edges_arr.ctypes.data_as(ct.POINTER(ct.c_uint32)) if edges_arr.size else None,
+            self.handle, p, sets.ctypes.data_as(ct.POINTER(abi.QaoaSet)), count, edges_arr.ctypes.data_as(ct.POINTER(ct.c_uint32)) if edges_arr.size else None,
             edges_arr.size // 2, ang.ctypes.data_as(ct.POINTER(ct.c_double)), out.ctypes.data_as(ct.POINTER(ct.c_double))))
         return out[:count]
 
