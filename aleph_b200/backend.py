@@ -13,6 +13,7 @@ from __future__ import annotations
 import ctypes as ct
 from dataclasses import dataclass
 from itertools import chain
+from operator import index
 
 import numpy as np
 
@@ -354,16 +355,21 @@ class B200SvBackend:
         # whole columns at once: a 384-graph batch holds some 12,000 edges
         lens = [len(edges) for _, edges in graphs]
         sets = np.zeros(max(1, count), dtype=np.dtype(abi.QaoaSet))
-        sets["num_qubits"][:count] = [nq for nq, _ in graphs]
+        sets["num_qubits"][:count] = [index(nq) & 0xFFFFFFFF for nq, _ in graphs]
         sets["num_edges"][:count] = lens
         sets["edge_offset"][:count] = np.cumsum([0] + lens[:-1]) if count else 0
-        edges_arr = np.fromiter(chain.from_iterable(chain.from_iterable(edges for _, edges in graphs)), dtype=np.uint32)
-        if edges_arr.size != 2 * sum(lens):
+        pairs = list(chain.from_iterable(edges for _, edges in graphs))
+        if set(map(len, pairs)) - {2}:
             raise ValueError("an edge is a pair of qubits")
+        ends = np.fromiter(chain.from_iterable(pairs), dtype=np.int64, count=2 * len(pairs))
+        if ends.size and (ends.min() < 0 or ends.max() > 0xFFFFFFFF):
+            raise OverflowError("an edge's qubit is out of range")
+        edges_arr = ends.astype(np.uint32)
         ang = np.ascontiguousarray(np.concatenate([gam, bet], axis=1))
         out = np.zeros(max(1, count), dtype=np.float64)
         self._check(self.lib.aleph_b200_qaoa_sweep(
-            self.handle, p, sets.ctypes.data_as(ct.POINTER(abi.QaoaSet)), count, edges_arr.ctypes.data_as(ct.POINTER(ct.c_uint32)) if edges_arr.size else None,
+            self.handle, p, sets.ctypes.data_as(ct.POINTER(abi.QaoaSet)), count,
+            edges_arr.ctypes.data_as(ct.POINTER(ct.c_uint32)) if edges_arr.size else None,
             edges_arr.size // 2, ang.ctypes.data_as(ct.POINTER(ct.c_double)), out.ctypes.data_as(ct.POINTER(ct.c_double))))
         return out[:count]
 
