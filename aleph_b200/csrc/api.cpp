@@ -350,7 +350,7 @@ int execute(aleph_b200_handle* h, aleph_b200_state* st, const Plan& P, const dou
         r.dense_ops = ps.dense_ops;
         r.diag_ops = ps.diag_ops;
         r.fma_per_amp = ps.fma_per_amp;
-        r.variant = ps.kind == PASS_TILE ? ps.tile.occupancy : 0;
+        r.variant = ps.kind == PASS_TILE ? ps.tile.occupancy : ps.kind == PASS_WIDE && ps.wide.R == 4 ? 3 : 0;
       }
     }
     ++pk;
@@ -2109,7 +2109,7 @@ int aleph_b200_describe_plan(uint32_t num_qubits, const aleph_b200_plan_config* 
     r.dense_ops = ps.dense_ops;
     r.diag_ops = ps.diag_ops;
     r.fma_per_amp = ps.fma_per_amp;
-    r.variant = ps.kind == PASS_TILE ? ps.tile.occupancy : 0;
+    r.variant = ps.kind == PASS_TILE ? ps.tile.occupancy : ps.kind == PASS_WIDE && ps.wide.R == 4 ? 3 : 0;
     r.bytes = (ps.kind == PASS_MEASURE ? 3 : 2) * len * bpa;
     out[k] = r;
   }

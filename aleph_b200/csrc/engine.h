@@ -36,7 +36,8 @@ struct Op {
   uint8_t a, b;    // tile slots of q[0] / q[1] (tile kernel); see TilePass
   uint8_t q[6];    // global target qubits, MSB-first
   uint8_t creg;    // tile kernel: control / mask bits that are register qubits (R-bit mask)
-  uint8_t dsrc;    // tile kernel, OP_DIAG: bit i set -> table bit i comes from register slot q[3+i]
+  uint8_t dsrc;    // tile kernel, OP_DIAG: bit i set -> table bit i comes from register slot q[3+i];
+                   // wide tile pass, OP_1Q / OP_2Q without controls: WideMatrix
   uint64_t ctrl;   // global control mask: op acts where (x & ctrl) == ctrl
                    // (tile kernel: only the bits outside the register qubits)
   uint64_t mask;   // OP_CPHASE / OP_NEG: qubit mask (tile kernel: bits outside the
@@ -45,6 +46,14 @@ struct Op {
   uint32_t aux;    // OP_POLY: term count
 };
 static_assert(sizeof(Op) == 40, "Op layout");
+
+// Forms of a dense matrix (Op::dsrc): uncontrolled ones in a wide tile pass, any in
+// a shared-memory pass (WIDE_REAL only, coefficients as they are); 0: complex
+// coefficients. In a wide pass, FP32 coefficients of the other forms are duplicated, (x, x).
+enum WideMatrix : uint8_t {
+  WIDE_REAL = 1,    // imaginary parts zero (FP32: one (re, re) per entry)
+  WIDE_PAIRED = 2,  // FP32 only: (re, re) and (im, im) per entry
+};
 
 // Diagonal-phase polynomial tables (OP_POLY), device-resident per plan.
 struct PolyTables {
@@ -67,12 +76,13 @@ struct TilePass {
 };
 
 // Wide tile pass: a CTA's tile is 2^12 amplitudes over qubits 0..3 and eight
-// others; ops run in phases, each with kWideRegs of the twelve in registers.
+// others; ops run in phases, each with R of the twelve in registers (32 or 16
+// amplitudes per thread, 128 or 256 threads).
 constexpr uint32_t kWideBits = 12;
-constexpr uint32_t kWideRegs = 5;                       // register qubits of a phase
-constexpr uint32_t kWideThreadBits = kWideBits - kWideRegs;
 struct WidePass {
   uint32_t n;
+  uint32_t R;  // 5 or 4
+  uint32_t full;  // the pass has phases, tables or real matrices
   uint32_t phase_begin, phase_count;  // the first and the last phase have qubits 0..3 on lanes 0..3
   uint32_t op_begin, op_count;
   uint32_t free_q[8];  // the eight other tile qubits, ascending
@@ -83,8 +93,8 @@ struct WidePass {
 };
 struct WidePhase {
   uint32_t op_begin, op_count;  // dense ops: Op::a / Op::b = 5 + register bit
-  uint16_t ts[kWideThreadBits], rs[kWideRegs];  // shared-memory slot offset of each thread-index / register bit (XORed)
-  uint8_t tq[kWideThreadBits], rq[kWideRegs];   // qubit of each thread-index / register bit
+  uint16_t ts[8], rs[5];  // shared-memory slot offset of each thread-index / register bit (XORed)
+  uint8_t tq[8], rq[5];   // qubit of each thread-index / register bit
 };
 
 // Tensor-core dense-block pass (TC32): a 2^6 x 2^6 complex matrix on the
@@ -253,7 +263,7 @@ cudaError_t launch_tile_pass(void* amps, int precision, const TilePass& p, const
 cudaError_t launch_wide_pass(void* amps, int precision, const WidePass& p, const WidePhase* phases, const Op* ops,
                              const void* coef, PolyTables poly, cudaStream_t s);
 // Fills a phase's layout (ts, rs, tq, rq) for the tile bits `regs` in registers.
-void wide_layout(const uint8_t* tile_qubits, uint32_t regs, bool io, bool f64, WidePhase* P);
+void wide_layout(const uint8_t* tile_qubits, uint32_t R, uint32_t regs, bool io, bool f64, WidePhase* P);
 cudaError_t launch_smem_pass(void* amps, int precision, uint32_t n, const Op* ops, uint32_t op_count,
                              const void* coef, uint32_t coef_end, PolyTables poly, cudaStream_t s);
 cudaError_t launch_kq_pass(void* amps, int precision, uint32_t n, const Op* op_dev, const Op& op_host,

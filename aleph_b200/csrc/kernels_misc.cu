@@ -25,7 +25,7 @@ namespace ab {
 constexpr uint32_t SMEM_OPS = 64;        // ops per staged group
 constexpr uint32_t SMEM_COEFS = 2048;    // coefficients per staged group (one 5-qubit unitary is 1024)
 
-template <typename Real, int K>
+template <typename Real, int K, bool REAL = false>
 __device__ __forceinline__ void smem_dense(V2<Real>* sm, uint64_t groups, const Op& op, const V2<Real>* m) {
   constexpr uint32_t DIM = 1u << K;
   uint32_t sorted[K], bit[K];
@@ -60,14 +60,16 @@ __device__ __forceinline__ void smem_dense(V2<Real>* sm, uint64_t groups, const 
     for (uint32_t c = 0; c < DIM; ++c) x[c] = sm[at(c)];
 #pragma unroll(DIM <= 8 ? (int)DIM : 1)
     for (uint32_t r = 0; r < DIM; ++r) {
-      V2<Real> acc = cmul<Real>(m[r * DIM], x[0]);
+      V2<Real> acc = REAL ? mk<Real>(m[r * DIM].x * x[0].x, m[r * DIM].x * x[0].y) : cmul<Real>(m[r * DIM], x[0]);
 #pragma unroll
       for (uint32_t c = 1; c < DIM; ++c) {
         const V2<Real> u = m[r * DIM + c];
         acc.x = fma(u.x, x[c].x, acc.x);
         acc.y = fma(u.x, x[c].y, acc.y);
-        acc.x = fma(-u.y, x[c].y, acc.x);
-        acc.y = fma(u.y, x[c].x, acc.y);
+        if constexpr (!REAL) {
+          acc.x = fma(-u.y, x[c].y, acc.x);
+          acc.y = fma(u.y, x[c].x, acc.y);
+        }
       }
       sm[at(r)] = acc;
     }
@@ -88,11 +90,55 @@ __device__ __forceinline__ void smem_apply_op(V2<Real>* sm, uint64_t len, const 
       }
       break;
     }
-    case OP_1Q: smem_dense<Real, 1>(sm, len >> 1, op, m); break;
-    case OP_2Q: smem_dense<Real, 2>(sm, len >> 2, op, m); break;
+    case OP_1Q:
+      if (op.dsrc == WIDE_REAL) smem_dense<Real, 1, true>(sm, len >> 1, op, m);
+      else smem_dense<Real, 1>(sm, len >> 1, op, m);
+      break;
+    case OP_2Q:
+      if (op.dsrc == WIDE_REAL) smem_dense<Real, 2, true>(sm, len >> 2, op, m);
+      else smem_dense<Real, 2>(sm, len >> 2, op, m);
+      break;
     case 8 + 3: smem_dense<Real, 3>(sm, len >> 3, op, m); break;
     case 8 + 4: smem_dense<Real, 4>(sm, len >> 4, op, m); break;
     case 8 + 5: smem_dense<Real, 5>(sm, len >> 5, op, m); break;
+  }
+}
+
+// A run of diagonal ops on the amplitudes this thread owns: each op is decoded
+// once for four amplitudes held in registers, without branches.
+template <typename Real>
+__device__ __forceinline__ void smem_diag_run(V2<Real>* sm, uint32_t len, const Op* ops, uint32_t count,
+                                              const V2<Real>* coef, const PolyTables& poly) {
+  constexpr int PER = 4;
+  for (uint32_t i0 = threadIdx.x; i0 < len; i0 += PER * blockDim.x) {
+    V2<Real> a[PER];
+    uint32_t at[PER];
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      at[k] = i0 + k * blockDim.x;
+      a[k] = sm[at[k] < len ? at[k] : i0];
+    }
+#pragma unroll 2
+    for (uint32_t x = 0; x < count; ++x) {
+      const uint32_t type = ops[x].type;
+      const uint32_t mask = (uint32_t)(ops[x].mask | ops[x].ctrl);
+      if (type == OP_NEG || type == OP_CPHASE) {
+        const bool neg = type == OP_NEG;
+        const V2<Real> c = neg ? mk<Real>(1, 0) : coef[ops[x].coef];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+          const V2<Real> y = neg ? cneg<Real>(a[k]) : cmul<Real>(c, a[k]);
+          const bool on = (at[k] & mask) == mask;
+          a[k] = mk<Real>(on ? y.x : a[k].x, on ? y.y : a[k].y);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < PER; ++k) a[k] = apply_diag_op<Real>(ops[x], a[k], at[k], coef, poly);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+      if (at[k] < len) sm[at[k]] = a[k];
   }
 }
 
@@ -124,11 +170,7 @@ __global__ void __launch_bounds__(512) smem_kernel(V2<Real>* __restrict__ amps, 
       if (is_diag_type(group[k].type)) {  // a run of diagonal ops: every thread keeps its amplitudes
         uint32_t e = k + 1;
         while (e < cnt && is_diag_type(group[e].type)) ++e;
-        for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) {
-          V2<Real> a = sm[i];
-          for (uint32_t x = k; x < e; ++x) a = apply_diag_op<Real>(group[x], a, i, cf - c0, poly);
-          sm[i] = a;
-        }
+        smem_diag_run<Real>(sm, len, group + k, e - k, cf - c0, poly);
         k = e;
       } else {
         smem_apply_op<Real>(sm, len, group[k], cf + (group[k].coef - c0));

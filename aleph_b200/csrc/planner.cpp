@@ -559,6 +559,13 @@ int tile_cost(const Lowered& L) {
 
 constexpr int kFuseMinCost = 24;
 
+// Every coefficient's imaginary part is exactly zero.
+bool real_matrix(const Lowered& L) {
+  for (size_t c = 1; c < L.coef.size(); c += 2)
+    if (L.coef[c] != 0.0) return false;
+  return true;
+}
+
 // Source gates that an op stands for.
 uint32_t gates_of(const Lowered& L) { return L.absorbed ? 0 : L.gates ? L.gates : 1; }
 
@@ -583,7 +590,7 @@ bool fusable_type(const Lowered& L) {
 
 }  // namespace
 
-// ---- diagonal cores (wide tile passes) ------------------------------------------
+// ---- diagonal cores -------------------------------------------------------------------------------
 // Gate sequences on two or three qubits often multiply out to a diagonal: the
 // CX Rz CX of a ZZ rotation, a Toffoli in CX + T without the H around it. As
 // written they move amplitudes and tie their qubits to a pass; as a diagonal
@@ -592,11 +599,17 @@ bool fusable_type(const Lowered& L) {
 // Gates are gathered greedily into blocks of at most three qubits (a block
 // owns its qubits until a gate joins them to others). Of a closed block, the core
 // runs from each qubit's first to its last gate on several qubits; the
-// one-qubit gates outside it stay. A core that multiplies out to a diagonal (to
-// rounding) is replaced by its corner phases when those cost less than its gates,
+// one-qubit gates outside it stay. A core of X-like and diagonal gates whose moves
+// cancel is replaced by its corner phases when those cost less than its gates,
 // an amplitude-moving gate counted as 8. The phases of all cores on no qubit are one op
 // at the end.
-std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& seg, std::deque<Lowered>& store) {
+//
+// In shared-memory passes (`smem`) a run of gates on one pair of qubits costs one 4x4,
+// about what two phases cost there, so only cores cheaper than their runs at that
+// price are taken: the CCZ of a Toffoli (six runs, one sign flip) is, a ZZ rotation (one
+// run, three phases) is not (n = 8 FP32 QAOA, p = 2: 48 us with it, 38 without).
+std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& seg, std::deque<Lowered>& store,
+                                           bool smem = false) {
   struct Block {
     uint64_t qubits = 0;
     std::vector<size_t> members;  // indices in seg, ascending
@@ -628,6 +641,29 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
     }
     out.emplace_back(at, &F);
   };
+  // A gate that stays, at `at`. A table diagonal on one qubit (with up to two
+  // controls) becomes its corner phases too: the one on the qubits' ones and the
+  // one on the controls alone, which without controls joins the global phase.
+  auto keep = [&](size_t at, size_t m) {
+    const Lowered& L = *seg[m];
+    if (L.op.type != OP_DIAG || L.op.nq != 1) {
+      out.emplace_back(at, &L);
+      return;
+    }
+    const Cx* d = reinterpret_cast<const Cx*>(L.coef.data());
+    const double l0 = std::hypot(d[0].re, d[0].im), l1 = std::hypot(d[1].re, d[1].im);
+    if (std::fabs(l0 - 1.0) > 1e-15 || std::fabs(l1 - 1.0) > 1e-15) {  // not unimodular to rounding: keep the table
+      out.emplace_back(at, &L);
+      return;
+    }
+    corner(at, L.op.ctrl | 1ull << L.op.q[0], mul(d[1], conj(d[0])), L.record, gates_of(L));
+    if (L.op.ctrl) {
+      if (!is_one(d[0])) corner(at, L.op.ctrl, d[0], L.record, 0);
+    } else {
+      global = mul(global, d[0]);
+      last_record = L.record;
+    }
+  };
   auto emit = [&](const Block& B) {
     size_t first[64], last[64];
     for (auto& x : first) x = SIZE_MAX;
@@ -644,7 +680,7 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
       }
     }
     auto plain = [&] {
-      for (size_t m : B.members) out.emplace_back(m, seg[m]);
+      for (size_t m : B.members) keep(m, m);
     };
     if (multi < 2) return plain();
     uint32_t bq[6] = {60, 61, 62, 63, 59, 58}, nb = 0;
@@ -657,6 +693,7 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
       if (first[q] != SIZE_MAX) place = std::max(place, B.members[first[q]]);
     int cost = 0;
     uint32_t gates = 0;
+    bool monomial = true;  // a core with a dense member is left alone
     for (size_t k = 0; k < B.members.size(); ++k) {
       const Lowered* L = seg[B.members[k]];
       if (width(*L) < 2) {
@@ -668,22 +705,47 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
           continue;
         }
       }
+      if (L->op.type != OP_X && L->nondiag) monomial = false;
       core.push_back(L);
       cost += L->nondiag ? std::max(8, tile_cost(*L)) : tile_cost(*L);
       gates += gates_of(*L);
     }
+    if (!monomial) return plain();
+    // The core as a map of basis states with phases: its members are X-like or diagonal.
     const double tol = 1e-15 * (double)(core.size() + 2);
+    auto local = [&](uint64_t m) {  // qubit mask -> bits of the block's index
+      uint32_t r = 0;
+      for (uint32_t b = 0; b < nb; ++b) r |= (uint32_t)((m >> bq[b]) & 1) << b;
+      return r;
+    };
+    uint32_t to[8];
     Cx d[8];
     for (uint32_t c = 0; c < dim; ++c) {
-      Cx s[64];
-      for (auto& x : s) x = Cx{0, 0};
-      s[c] = Cx{1.0, 0.0};
-      for (const Lowered* L : core) apply_local(*L, bq, s);
-      for (uint32_t r = 0; r < dim; ++r)
-        if (r != c && std::hypot(s[r].re, s[r].im) > tol) return plain();
-      const double len = std::hypot(s[c].re, s[c].im);
-      if (std::fabs(len - 1.0) > 4 * tol) return plain();
-      d[c] = Cx{s[c].re / len, s[c].im / len};
+      to[c] = c;
+      d[c] = Cx{1.0, 0.0};
+    }
+    for (const Lowered* L : core) {
+      const Op& op = L->op;
+      const Cx* k = reinterpret_cast<const Cx*>(L->coef.data());
+      const uint32_t ctrl = local(op.ctrl), mask = local(op.mask), bit = local(1ull << op.q[0]);
+      for (uint32_t c = 0; c < dim; ++c) {
+        const uint32_t x = to[c];
+        if (op.type == OP_X) {
+          if ((x & ctrl) == ctrl) to[c] = x ^ bit;
+        } else if (op.type == OP_DIAG) {
+          if ((x & ctrl) != ctrl) continue;
+          uint32_t idx = 0;
+          for (int i = 0; i < op.nq; ++i) idx = (idx << 1) | ((x & local(1ull << op.q[i])) ? 1u : 0u);
+          d[c] = mul(k[idx], d[c]);
+        } else if ((x & mask) == mask) {
+          d[c] = op.type == OP_NEG ? neg(d[c]) : mul(k[0], d[c]);
+        }
+      }
+    }
+    for (uint32_t c = 0; c < dim; ++c) {
+      const double len = std::hypot(d[c].re, d[c].im);
+      if (to[c] != c || std::fabs(len - 1.0) > tol) return plain();
+      d[c] = Cx{d[c].re / len, d[c].im / len};
     }
     // corner phases: c_S = prod over T in S of d_T^(+-1), sign by the parity of |S| - |T|
     Cx cs[8];
@@ -700,8 +762,22 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
       used[S] = S != 0 && !is_one(c);
       if (used[S]) price += c.re == -1.0 ? 1 : 2;
     }
+    if (smem) {
+      int runs = 0;
+      uint64_t pair = 0;
+      for (const Lowered* L : core) {
+        const uint64_t q = L->nondiag | L->diag;
+        if (runs == 0 || __builtin_popcountll(pair | q) > 2) {
+          ++runs;
+          pair = q;
+        } else {
+          pair |= q;
+        }
+      }
+      cost = 2 * runs;
+    }
     if (price >= cost) return plain();
-    for (size_t m : before) out.emplace_back(m, seg[m]);
+    for (size_t m : before) keep(m, m);
     const uint32_t record = core.front()->record;
     bool any = false;
     for (uint32_t S = 1; S < dim; ++S) {
@@ -715,7 +791,7 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
     if (!any) corner(place, 0, Cx{1.0, 0.0}, record, gates);  // the identity, kept for its gate count
     global = mul(global, cs[0]);
     last_record = record;
-    for (size_t m : after) out.emplace_back(std::max(m, place), seg[m]);
+    for (size_t m : after) keep(std::max(m, place), m);
   };
   auto close = [&](size_t k) {
     const Block B = std::move(blocks[k]);
@@ -741,7 +817,7 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
       close(widest);
     }
     if (!small) {
-      out.emplace_back(i, &L);
+      keep(i, i);
       continue;
     }
     Block B;
@@ -1120,7 +1196,7 @@ WideTake wide_best(const std::vector<const Lowered*>& pending, uint64_t have, ui
 // dense ops after it. A group costs one sweep over the registers per class however
 // many ops it holds (the QFT's passes hold some 20 phases per dense gate; one at
 // a time, each cost half a sweep and its predicates).
-void emit_wide_phase(const std::vector<const Lowered*>& ops, const uint8_t* reg_of, uint32_t n, Plan* P) {
+void emit_wide_phase(const std::vector<const Lowered*>& ops, const uint8_t* reg_of, uint32_t n, bool f64, Plan* P) {
   struct Group {
     std::vector<const Lowered*> signs, phases[6];
     bool empty() const {
@@ -1220,32 +1296,46 @@ void emit_wide_phase(const std::vector<const Lowered*>& ops, const uint8_t* reg_
           op.q[3 + i] = reg_of[op.q[i]];
         }
     }
-    if (op.type == OP_1Q || op.type == OP_X) {
+    if (op.type == OP_X) op.a = (uint8_t)(5 + reg_of[op.q[0]]);
+    if (op.type == OP_1Q || op.type == OP_2Q) {
+      Lowered M = *L;
       op.a = (uint8_t)(5 + reg_of[op.q[0]]);
-    } else if (op.type == OP_2Q) {
-      op.a = (uint8_t)(5 + reg_of[op.q[0]]);
-      op.b = (uint8_t)(5 + reg_of[op.q[1]]);
-      if (op.a < op.b) {
-        Lowered tmp = *L;
-        swap_2q_operands(tmp.coef);
-        std::swap(op.q[0], op.q[1]);
-        std::swap(op.a, op.b);
-        append_op(P, tmp, op);
-        continue;
+      if (op.type == OP_2Q) {
+        op.b = (uint8_t)(5 + reg_of[op.q[1]]);
+        if (op.a < op.b) {
+          swap_2q_operands(M.coef);
+          std::swap(op.q[0], op.q[1]);
+          std::swap(op.a, op.b);
+        }
       }
+      if (L->op.ctrl == 0) {
+        const bool real = real_matrix(M);
+        op.dsrc = real ? WIDE_REAL : f64 ? 0 : WIDE_PAIRED;
+        if (!f64) {  // duplicated for paired arithmetic
+          std::vector<double> dup;
+          for (size_t c = 0; c < M.coef.size(); c += 2) {
+            dup.insert(dup.end(), 2, M.coef[c]);
+            if (!real) dup.insert(dup.end(), 2, M.coef[c + 1]);
+          }
+          M.coef = std::move(dup);
+        }
+      }
+      append_op(P, M, op);
+      continue;
     }
     append_op(P, *L, op);
   }
 }
 
-int plan_segment_wide(const std::vector<const Lowered*>& seg, uint32_t n, bool f64, uint32_t R, Plan* P) {
+// R: register qubits of a phase, 4 or 5.
+int plan_segment_wide(const std::vector<const Lowered*>& seg, uint32_t n, bool f64, uint32_t tile_r, uint32_t R, Plan* P) {
   std::vector<const Lowered*> pending = seg;
   uint8_t all[kMaxQubits];
   for (uint32_t q = 0; q < n; ++q) all[q] = (uint8_t)q;
   while (!pending.empty()) {
     if (pending.front()->op.type == OP_KQ) {
       const std::vector<const Lowered*> one{pending.front()};
-      if (int s = plan_segment_tiles(one, n, R, P)) return s;
+      if (int s = plan_segment_tiles(one, n, tile_r, P)) return s;
       pending.erase(pending.begin());
       continue;
     }
@@ -1258,6 +1348,7 @@ int plan_segment_wide(const std::vector<const Lowered*>& seg, uint32_t n, bool f
     ps.kind = PASS_WIDE;
     WidePass& W = ps.wide;
     W.n = n;
+    W.R = R;
     uint8_t tile[kWideBits];
     uint32_t k = 0;
     for (uint32_t q = 0; q < n; ++q) {
@@ -1280,30 +1371,30 @@ int plan_segment_wide(const std::vector<const Lowered*>& seg, uint32_t n, bool f
       src += len;
       q += len;
     }
-    // phases: sets of kWideRegs tile qubits, until the pass's ops are spent
+    // phases: sets of R tile qubits, until the pass's ops are spent
     W.phase_begin = (uint32_t)P->phases.size();
     W.op_begin = (uint32_t)P->ops.size();
     std::vector<const Lowered*> left = T.take;
     auto add_phase = [&](uint32_t regs, bool io, const std::vector<const Lowered*>& ops) {
       WidePhase ph{};
-      wide_layout(tile, regs, io, f64, &ph);
+      wide_layout(tile, W.R, regs, io, f64, &ph);
       uint8_t reg_of[kMaxQubits];
       std::memset(reg_of, 255, sizeof(reg_of));
-      for (uint32_t j = 0; j < kWideRegs; ++j) reg_of[ph.rq[j]] = (uint8_t)j;
+      for (uint32_t j = 0; j < W.R; ++j) reg_of[ph.rq[j]] = (uint8_t)j;
       ph.op_begin = (uint32_t)P->ops.size();
-      emit_wide_phase(ops, reg_of, n, P);
+      emit_wide_phase(ops, reg_of, n, f64, P);
       ph.op_count = (uint32_t)P->ops.size() - ph.op_begin;
       P->phases.push_back(ph);
     };
-    constexpr uint32_t kIoRegs = ((1u << kWideRegs) - 1) << kWideThreadBits;  // the top tile bits: lanes take bits 0..4
+    const uint32_t kIoRegs = ((1u << W.R) - 1) << (kWideBits - W.R);  // the top tile bits: lanes take bits 0..4
     bool first = true;
     while (!left.empty()) {
-      WideTake F = wide_best(left, 0, kWideRegs, tile, kWideBits);
+      WideTake F = wide_best(left, 0, W.R, tile, kWideBits);
       if (F.take.empty()) return ALEPH_B200_OPTIMIZATION;
       uint32_t regs = 0;
       for (uint32_t b = 0; b < kWideBits; ++b)
         if ((F.set >> tile[b]) & 1) regs |= 1u << b;
-      for (int b = (int)kWideBits - 1; b >= 0 && __builtin_popcount(regs) < (int)kWideRegs; --b) regs |= 1u << b;
+      for (int b = (int)kWideBits - 1; b >= 0 && __builtin_popcount(regs) < (int)W.R; --b) regs |= 1u << b;
       const bool low = (regs & 0xFu) != 0, last = F.rest.empty();
       if (first && low) add_phase(kIoRegs, true, {});
       add_phase(regs, !low && (first || last), F.take);
@@ -1313,6 +1404,16 @@ int plan_segment_wide(const std::vector<const Lowered*>& seg, uint32_t n, bool f
     }
     W.phase_count = (uint32_t)P->phases.size() - W.phase_begin;
     W.op_count = (uint32_t)P->ops.size() - W.op_begin;
+    W.full = 0;
+    for (uint32_t i = W.op_begin; i < W.op_begin + W.op_count; ++i) {
+      const Op& op = P->ops[i];
+      if (op.type == OP_SIGNS) {  // its records follow
+        i += op.aux;
+        continue;
+      }
+      const bool dense = op.type == OP_1Q || op.type == OP_2Q;
+      if (dense ? op.dsrc == WIDE_REAL : op.type != OP_X) W.full = 1;
+    }
     ps.record = T.take.front()->record;
     for (const Lowered* L : T.take) ps.gates += gates_of(*L);
     count_ops(T.take, &ps);
@@ -1427,8 +1528,9 @@ struct BlockTake {
   double score(uint32_t base) const {
     if (take.empty()) return 0.0;
     double s = 0.0;
-    for (const Lowered* L : take) s += 1.0 / (1.0 + (double)(L->record - base) / 64.0);
-    for (const Lowered* L : post) s += 1.0 / (1.0 + (double)(L->record - base) / 64.0);
+    auto weight = [&](const Lowered* L) { return 1.0 / (1.0 + (L->record > base ? (double)(L->record - base) : 0.0) / 64.0); };
+    for (const Lowered* L : take) s += weight(L);
+    for (const Lowered* L : post) s += weight(L);
     return s;
   }
 };
@@ -1569,7 +1671,8 @@ int plan_segment_blocks(const std::vector<const Lowered*>& seg, uint32_t n, uint
         ps.block.fold = 1;
     }
     ps.record = take.front()->record;
-    ps.gates = (uint32_t)(take.size() + post.size());
+    for (const Lowered* L : take) ps.gates += gates_of(*L);
+    for (const Lowered* L : post) ps.gates += gates_of(*L);
     count_ops(take, &ps);
     ps.lane_ops = 0;  // a block has no lane shuffles
     ps.diag_ops += (uint32_t)post.size();
@@ -1623,8 +1726,12 @@ int build_plan(const std::vector<Lowered>& ops, uint32_t n, bool f64, const Plan
       ps.tile.n = n;
       ps.tile.op_begin = (uint32_t)P->ops.size();
       std::deque<Lowered> fused;
-      const std::vector<const Lowered*> list = o.pair_fusion ? fuse_for_smem(seg, fused) : seg;
-      for (const Lowered* L : list) append_op(P, *L, L->op);
+      const std::vector<const Lowered*> list = o.pair_fusion ? fuse_for_smem(diagonal_cores(seg, fused, true), fused) : seg;
+      for (const Lowered* L : list) {
+        Op op = L->op;
+        if ((op.type == OP_1Q || op.type == OP_2Q) && real_matrix(*L)) op.dsrc = WIDE_REAL;
+        append_op(P, *L, op);
+      }
       ps.tile.op_count = (uint32_t)P->ops.size() - ps.tile.op_begin;
       ps.record = seg.front()->record;
       ps.gates = (uint32_t)seg.size();
@@ -1633,14 +1740,20 @@ int build_plan(const std::vector<Lowered>& ops, uint32_t n, bool f64, const Plan
     } else {
       // a 2-qubit gate may need two register qubits: R >= 2 unless only one high qubit exists
       const uint32_t R = std::min<uint32_t>(std::max<uint32_t>(o.tile_r, 2), std::min<uint32_t>(5, n - 5));
-      if (o.tensor_blocks && n >= 13) status = plan_segment_blocks(seg, n, R, o.block_window_search, P);
-      else if (o.pair_fusion) {
+      if (o.tensor_blocks && n >= 13) {
+        // diagonal cores follow a block as its post ops instead of ending it
         std::deque<Lowered> fused;
-        // Wide tiles unless a key of the warp-tile planner was changed (tile_r,
-        // tile_occupancy, pair_fusion, relabel_swaps compare its parts) or the
-        // state is smaller than one wide tile.
-        const bool wide = n >= kWideBits && o.tile_r == 5 && o.tile_occupancy == 0 && o.relabel_swaps;
-        status = wide ? plan_segment_wide(fuse_pairs(diagonal_cores(seg, fused), fused), n, f64, R, P)
+        status = plan_segment_blocks(o.pair_fusion ? diagonal_cores(seg, fused) : seg, n, R, o.block_window_search, P);
+      } else if (o.pair_fusion) {
+        std::deque<Lowered> fused;
+        // Wide tiles in the default configuration (five register qubits), and with four
+        // for tile_r = 4, which the learned planner may choose: FP64 measured at n = 25
+        // and 26, QFT passes 1.0 to 1.2 times faster, brickwall 1.35 times slower, FP32
+        // 1.2 times slower; other values of the warp-tile keys (and pair_fusion or
+        // relabel_swaps off) compare the parts of the warp-tile planner, and a state
+        // smaller than one wide tile has no choice.
+        const bool wide = n >= kWideBits && o.relabel_swaps && ((o.tile_r == 5 && o.tile_occupancy == 0) || o.tile_r == 4);
+        status = wide ? plan_segment_wide(fuse_pairs(diagonal_cores(seg, fused), fused), n, f64, R, o.tile_r == 4 ? 4 : 5, P)
                       : plan_segment_tiles(fuse_pairs(seg, fused), n, R, P);
       } else {
         status = plan_segment_tiles(seg, n, R, P);

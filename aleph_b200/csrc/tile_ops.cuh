@@ -194,6 +194,170 @@ __device__ __forceinline__ void reg_2q_blocked(V2<Real> (&v)[1 << R], const V2<R
   }
 }
 
+// ---- real matrices (Ry, H, and the 4x4s they fuse to with CNOTs and CZs) -----
+// Half the multiply-adds of the complex forms: both components of an amplitude
+// see the same real matrix. Uncontrolled, coefficients as complex numbers with
+// zero imaginary parts.
+template <typename Real, int R, int J>
+__device__ __forceinline__ void reg_1q_real(V2<Real> (&v)[1 << R], const V2<Real>* m) {
+  const Real m0 = ld_coef<Real>(m).x, m1 = ld_coef<Real>(m + 1).x, m2 = ld_coef<Real>(m + 2).x,
+             m3 = ld_coef<Real>(m + 3).x;
+#pragma unroll
+  for (int r = 0; r < (1 << R); ++r) {
+    if (r & (1 << J)) continue;
+    const int r1 = r | (1 << J);
+    const V2<Real> a = v[r], b = v[r1];
+    v[r] = mk<Real>(fma(m1, b.x, m0 * a.x), fma(m1, b.y, m0 * a.y));
+    v[r1] = mk<Real>(fma(m3, b.x, m2 * a.x), fma(m3, b.y, m2 * a.y));
+  }
+}
+
+template <typename Real, int R>
+__device__ __forceinline__ void dispatch_reg_real(int j, V2<Real> (&v)[1 << R], const V2<Real>* m) {
+  switch (j) {
+    case 0: if constexpr (R > 0) reg_1q_real<Real, R, 0>(v, m); break;
+    case 1: if constexpr (R > 1) reg_1q_real<Real, R, 1>(v, m); break;
+    case 2: if constexpr (R > 2) reg_1q_real<Real, R, 2>(v, m); break;
+    case 3: if constexpr (R > 3) reg_1q_real<Real, R, 3>(v, m); break;
+    case 4: if constexpr (R > 4) reg_1q_real<Real, R, 4>(v, m); break;
+  }
+}
+
+// A real 4x4 on register bits JA > JB, QB quartets per coefficient row (see reg_2q_blocked).
+template <typename Real, int R, int JA, int JB, int QB>
+__device__ __forceinline__ void reg_2q_real(V2<Real> (&v)[1 << R], const V2<Real>* m) {
+  constexpr int NQ = 1 << (R - 2);
+  constexpr int A = 1 << JA, B = 1 << JB;
+#pragma unroll
+  for (int q0 = 0; q0 < NQ; q0 += QB) {
+    V2<Real> o[QB][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const Real c0 = ld_coef<Real>(m + 4 * k).x, c1 = ld_coef<Real>(m + 4 * k + 1).x,
+                 c2 = ld_coef<Real>(m + 4 * k + 2).x, c3 = ld_coef<Real>(m + 4 * k + 3).x;
+#pragma unroll
+      for (int j = 0; j < QB; ++j) {
+        const int r = quartet_base<R, JA, JB>(q0 + j);
+        o[j][k].x = fma(c3, v[r | A | B].x, fma(c2, v[r | A].x, fma(c1, v[r | B].x, c0 * v[r].x)));
+        o[j][k].y = fma(c3, v[r | A | B].y, fma(c2, v[r | A].y, fma(c1, v[r | B].y, c0 * v[r].y)));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < QB; ++j) {
+      const int r = quartet_base<R, JA, JB>(q0 + j);
+      v[r] = o[j][0];
+      v[r | B] = o[j][1];
+      v[r | A] = o[j][2];
+      v[r | A | B] = o[j][3];
+    }
+  }
+}
+
+template <typename Real, int R, int QB>
+__device__ __forceinline__ void dispatch_reg_2q_real(int ja, int jb, V2<Real> (&v)[1 << R], const V2<Real>* m) {
+#define AB_RR(a, b)                                                    \
+  case (a)*8 + (b):                                                    \
+    if constexpr (R > (a)) reg_2q_real<Real, R, (a), (b), QB>(v, m);   \
+    break;
+  switch (ja * 8 + jb) {
+    AB_RR(1, 0) AB_RR(2, 0) AB_RR(2, 1) AB_RR(3, 0) AB_RR(3, 1)
+    AB_RR(3, 2) AB_RR(4, 0) AB_RR(4, 1) AB_RR(4, 2) AB_RR(4, 3)
+  }
+#undef AB_RR
+}
+
+// ---- paired FP32 arithmetic ----------------------------------------------------
+// An FP32 amplitude is one register pair, and a matrix entry c acts on it as
+// (cx, cx) * (re, im) + (cy, cy) * (-im, re): two paired multiply-adds for both
+// components, half the instructions of the scalar form. The coefficients come
+// duplicated, (cx, cx) then (cy, cy) per entry; a real matrix has (cx, cx) only.
+__device__ __forceinline__ float2 times_i(float2 x) { return make_float2(-x.y, x.x); }
+
+template <int R, int J, bool REAL>
+__device__ __forceinline__ void reg_1q_f32x2(float2 (&v)[1 << R], const float2* m) {
+  constexpr int S = REAL ? 1 : 2;
+  float2 c[4 * S];
+#pragma unroll
+  for (int k = 0; k < 4 * S; ++k) c[k] = ld_coef<float>(m + k);
+#pragma unroll
+  for (int r = 0; r < (1 << R); ++r) {
+    if (r & (1 << J)) continue;
+    const int r1 = r | (1 << J);
+    const float2 a = v[r], b = v[r1];
+    float2 o0 = __fmul2_rn(c[0], a), o1 = __fmul2_rn(c[2 * S], a);
+    if constexpr (!REAL) {
+      const float2 ia = times_i(a), ib = times_i(b);
+      o0 = __ffma2_rn(c[1], ia, o0);
+      o1 = __ffma2_rn(c[2 * S + 1], ia, o1);
+      o0 = __ffma2_rn(c[S + 1], ib, o0);
+      o1 = __ffma2_rn(c[3 * S + 1], ib, o1);
+    }
+    v[r] = __ffma2_rn(c[S], b, o0);
+    v[r1] = __ffma2_rn(c[3 * S], b, o1);
+  }
+}
+
+template <int R, bool REAL>
+__device__ __forceinline__ void dispatch_1q_f32x2(int j, float2 (&v)[1 << R], const float2* m) {
+  switch (j) {
+    case 0: if constexpr (R > 0) reg_1q_f32x2<R, 0, REAL>(v, m); break;
+    case 1: if constexpr (R > 1) reg_1q_f32x2<R, 1, REAL>(v, m); break;
+    case 2: if constexpr (R > 2) reg_1q_f32x2<R, 2, REAL>(v, m); break;
+    case 3: if constexpr (R > 3) reg_1q_f32x2<R, 3, REAL>(v, m); break;
+    case 4: if constexpr (R > 4) reg_1q_f32x2<R, 4, REAL>(v, m); break;
+  }
+}
+
+// A 4x4 on register bits JA > JB, QB quartets per coefficient row (see reg_2q_blocked).
+template <int R, int JA, int JB, int QB, bool REAL>
+__device__ __forceinline__ void reg_2q_f32x2(float2 (&v)[1 << R], const float2* m) {
+  constexpr int NQ = 1 << (R - 2), S = REAL ? 1 : 2;
+  constexpr int A = 1 << JA, B = 1 << JB;
+#pragma unroll
+  for (int q0 = 0; q0 < NQ; q0 += QB) {
+    float2 o[QB][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      float2 c[4 * S];
+#pragma unroll
+      for (int e = 0; e < 4 * S; ++e) c[e] = ld_coef<float>(m + 4 * S * k + e);
+#pragma unroll
+      for (int j = 0; j < QB; ++j) {
+        const int r = quartet_base<R, JA, JB>(q0 + j);
+        const float2 x[4] = {v[r], v[r | B], v[r | A], v[r | A | B]};
+        float2 t = __fmul2_rn(c[0], x[0]);
+#pragma unroll
+        for (int e = 1; e < 4; ++e) t = __ffma2_rn(c[S * e], x[e], t);
+        if constexpr (!REAL)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) t = __ffma2_rn(c[S * e + 1], times_i(x[e]), t);
+        o[j][k] = t;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < QB; ++j) {
+      const int r = quartet_base<R, JA, JB>(q0 + j);
+      v[r] = o[j][0];
+      v[r | B] = o[j][1];
+      v[r | A] = o[j][2];
+      v[r | A | B] = o[j][3];
+    }
+  }
+}
+
+template <int R, int QB, bool REAL>
+__device__ __forceinline__ void dispatch_2q_f32x2(int ja, int jb, float2 (&v)[1 << R], const float2* m) {
+#define AB_RR(a, b)                                                       \
+  case (a)*8 + (b):                                                       \
+    if constexpr (R > (a)) reg_2q_f32x2<R, (a), (b), QB, REAL>(v, m);     \
+    break;
+  switch (ja * 8 + jb) {
+    AB_RR(1, 0) AB_RR(2, 0) AB_RR(2, 1) AB_RR(3, 0) AB_RR(3, 1)
+    AB_RR(3, 2) AB_RR(4, 0) AB_RR(4, 1) AB_RR(4, 2) AB_RR(4, 3)
+  }
+#undef AB_RR
+}
+
 // ---- diagonal ops -------------------------------------------------------------
 template <typename Real, int R>
 __device__ __forceinline__ void diag_ops(const Op& op, V2<Real> (&v)[1 << R], uint64_t gl, const uint64_t (&hb)[5],

@@ -355,22 +355,26 @@ int aleph_b200_last_error(const aleph_b200_handle* h, char* buf, uint64_t len);
 int aleph_b200_last_error_info(const aleph_b200_handle* h, aleph_b200_error_info* out);
 
 /* ---- planner tuning (the autotuner's knobs) ----
- * keys: "tile_r" (register qubits per warp tile, 1..5), "smem_max_n" (states
- * with n <= this run as one shared-memory pass, 0..12), "record_passes"
- * (0/1: time every pass of later gate streams with CUDA events),
+ * keys: "tile_r" (register qubits per thread, 1..5; 5 and 4 choose wide tile
+ * passes for n >= 12 where the keys below leave them on, else warp tiles),
+ * "smem_max_n" (states with n <= this run as one shared-memory pass, 0..12),
+ * "record_passes" (0/1: time every pass of later gate streams with CUDA events),
  * "relabel_swaps" (0/1, default 1: an uncontrolled SWAP of a state larger
  * than smem_max_n relabels qubits instead of moving data, and one or two
- * in-place permutation passes settle the labels at the end of the stream),
+ * in-place permutation passes settle the labels at the end of the stream;
+ * 0 also chooses warp tiles),
  * "paged_local_qubits" (0..40, default 0: the most qubits one device tile
  * group of an out-of-core run may hold; 0 lets free device memory decide),
- * "tile_occupancy" (0 or 2..4: the tile kernel variant, resident 128-thread
- * blocks per SM), "tensor_blocks" (TC32 handles, 0/1), "block_window_search"
- * (0/1), "renormalize" (0/1, default 1: a TC32 gate stream with tensor-core
- * blocks rescales the state to norm 1 at its end; 0 for states that are one
- * slice of a larger state, whose norm is not 1), "pair_fusion" (0/1,
- * default 1: in warp-tile passes a gate on two qubits and the one-qubit
- * gates next to it on those qubits run as one 4x4 when that saves
- * arithmetic). */
+ * "tile_occupancy" (0 or 2..4: the warp-tile kernel variant, resident
+ * 128-thread blocks per SM; with "tile_r" 5, any but 0 chooses warp tiles),
+ * "tensor_blocks" (TC32 handles, 0/1), "block_window_search" (0/1),
+ * "renormalize" (0/1, default 1: a TC32 gate stream with tensor-core blocks
+ * rescales the state to norm 1 at its end; 0 for states that are one slice
+ * of a larger state, whose norm is not 1), "pair_fusion" (0/1,
+ * default 1: a gate on two qubits and the one-qubit gates next to it on
+ * those qubits run as one 4x4 when that saves arithmetic, and gate sequences
+ * on at most three qubits that multiply out to a diagonal run as phases; 0
+ * also chooses warp tiles). */
 int aleph_b200_set_tuning(aleph_b200_handle* h, const char* key, int64_t value);
 
 /* ---- per-pass timing records (training data of the learned fusion planner) ---- */
@@ -386,7 +390,8 @@ typedef struct aleph_b200_pass_record {
   uint32_t lane_ops;    /* tile pass: non-diagonal ops on the lane qubits 0..4 (shuffles)  */
   uint32_t dense_ops;   /* non-diagonal ops the pass applies (a block: the fused gates)    */
   uint32_t diag_ops;    /* diagonal ops the pass applies (phases, CZ-like, DiagonalPhase)  */
-  uint32_t variant;     /* kernel variant (tile pass: blocks per SM)                       */
+  uint32_t variant;     /* kernel variant (warp tiles: blocks per SM; wide tiles: 0, or 3
+                           with tile_r 4)                                                  */
   uint32_t fma_per_amp; /* tile pass: real multiply-adds per amplitude (8 per dense one-qubit
                            op, 16 per dense 4x4, 4 per diagonal phase; controls ignored)   */
   double ms;            /* device time of the pass (CUDA events on the handle's stream)    */
@@ -404,7 +409,7 @@ typedef struct aleph_b200_plan_config {
   uint32_t block_window_search;  /* TC32: also try every 6-qubit window      */
   uint32_t tile_occupancy;       /* tile kernel variant: 0 (default) or 2..4 */
   uint32_t keep_swaps;           /* 1: SWAP records run as gates; 0: relabel */
-  uint32_t no_pair_fusion;       /* 1: tile passes apply every gate as given */
+  uint32_t no_pair_fusion;       /* 1: warp tiles, every gate applied as given */
 } aleph_b200_plan_config;
 int aleph_b200_describe_plan(uint32_t num_qubits, const aleph_b200_plan_config* config, const aleph_b200_instr* instrs,
                              uint64_t count, const aleph_b200_pools* pools, aleph_b200_pass_record* out, uint64_t cap,

@@ -1,8 +1,10 @@
 """Edges of the passes and reductions against the oracle or a dense restatement:
 wide tiles (smallest states, every class of grouped diagonal, controls on and
-off the tile, gate sequences replaced by the diagonal they multiply out to), shared-memory passes longer than one staged group, tensor-core
-passes with more post ops than a warp has lanes, marginals and Pauli strings on
-lane, pattern and split qubits, sweeps over several waves.
+off the tile, real and complex matrices with 16 and 32 amplitudes per thread,
+gate sequences replaced by the diagonal they multiply out to), shared-memory
+passes longer than one staged group, tensor-core passes with more post ops than
+a warp has lanes, marginals and Pauli strings on lane, pattern and split qubits,
+sweeps over several waves.
 
 Tolerances: FP64 amplitudes 1e-12 and FP32 1e-5 as in the parity tests; FP64
 reductions 1e-12 (sums of at most 2^17 terms of a normalised state), FP32 states
@@ -68,6 +70,40 @@ def test_wide_tiles_match_the_oracle(n, precision, seed):
     assert len(describe_plan(n, c.instructions, precision, smem_max_n=0)[0]["qubits"]) == 8  # a wide tile
     want, _ = oracle.run(n, c.instructions)
     assert np.abs(run_engine(c, precision, smem_max_n=0) - want).max() <= TOL[precision]
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("tile_r", [4, 5])
+@pytest.mark.parametrize("n,phases", [(12, False), (12, True), (13, False), (16, True)])
+def test_wide_tiles_real_and_complex_matrices(n, phases, tile_r, precision):
+    """One- and two-qubit matrices, real and complex, with and without controls; the
+    passes without phases run the smaller kernel."""
+    rng = np.random.default_rng(n + tile_r)
+    c = C.Circuit(n)
+    for _ in range(120):
+        q = [int(x) for x in rng.choice(n, 4, replace=False)]
+        t = float(rng.uniform(-np.pi, np.pi))
+        kind = int(rng.integers(0, 8 if phases else 6))
+        if kind == 0:
+            c.add(C.Ry(t), q[:1], controls=q[1:1 + int(rng.integers(0, 2))])
+        elif kind == 1:
+            c.add(C.U3(t, 0.4, 1.1), q[:1], controls=q[1:1 + int(rng.integers(0, 3))])
+        elif kind == 2:  # a real pair: fused to one real 4x4
+            c.add(C.Ry(t), q[:1]).add(C.H(), q[1:2]).add(C.Cnot(), q[:2]).add(C.Ry(-t), q[1:2])
+        elif kind == 3:
+            c.add(C.Rx(t), q[:1]).add(C.Cz(), q[:2]).add(C.U3(t, 0.2, 0.1), q[1:2])
+        elif kind == 4:
+            c.add(C.Cnot(), q[:2])
+        elif kind == 5:
+            c.add(C.Swap(), q[:2], controls=q[2:3])
+        elif kind == 6:
+            c.add(C.Phase(t), q[:1], controls=q[1:3])
+        else:
+            c.add(C.Unitary2qDiag(np.exp(1j * rng.uniform(0, 6, 4))), q[:2])
+    passes = describe_plan(n, c.instructions, precision, smem_max_n=0, tile_r=tile_r)
+    assert all(len(p["qubits"]) == 8 and p["variant"] == (3 if tile_r == 4 else 0) for p in passes if p["kind"] == 1)
+    want, _ = oracle.run(n, c.instructions)
+    assert np.abs(run_engine(c, precision, smem_max_n=0, tile_r=tile_r) - want).max() <= TOL[precision]
 
 
 def test_wide_plans_keep_every_gate():
