@@ -19,7 +19,7 @@
 // At those two warps per scheduler a pass of 4x4s is bound by latency (n = 27 FP64:
 // FP64 pipe 43%, issue 37%). Measured against warp tiles: n = 27 depth-20 FP64
 // brickwall 44.5 -> 36.5 ms, n = 25 FP64 QFT 8.0 -> 4.6 ms, n = 22 FP32 Grover
-// 4.06 -> 1.72 ms (the last two with grouped phases and diagonal cores).
+// 4.06 -> 1.06 ms (the last two with grouped phases and diagonal cores).
 //
 // Bank conflicts: amplitude i of the tile sits at slot i ^ f(i >> 3) (FP64; i >> 4
 // in FP32) with f linear over bits; the host orders a phase's lane qubits so

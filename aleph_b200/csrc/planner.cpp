@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstring>
 #include <thread>
+#include <unordered_map>
 
 #include "engine.h"
 
@@ -841,6 +842,108 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
   std::vector<const Lowered*> ops;
   ops.reserve(out.size());
   for (const auto& o : out) ops.push_back(o.second);
+  return ops;
+}
+
+// After the cores: phases on the same qubits with nothing between that moves
+// one of them become one (T and Tdg cancel), and H, a sign flip on t and others,
+// H on t become an X on t controlled by the others. A CX + T Toffoli is then one
+// exact move instead of two roundings by sqrt(1/2) and some phases, each of which
+// shortens an FP32 state a little in the same direction.
+// Measured: n = 22 FP32 Grover 1697 -> 1060 us (19 -> 14 passes), its error against
+// 64 bits 1.3e-5 -> 2.4e-6.
+std::vector<const Lowered*> cancel_phases(const std::vector<const Lowered*>& seg, std::deque<Lowered>& store) {
+  std::vector<const Lowered*> ops = seg;
+  std::unordered_map<uint64_t, size_t> phase;  // mask -> its last phase op, while it can still be joined
+  size_t h[64];                                // per qubit: an H with only phases since; SIZE_MAX: none
+  std::vector<size_t> since[64];               // those phases
+  for (auto& x : h) x = SIZE_MAX;
+  auto is_phase = [](const Lowered& L) {
+    return fusable_type(L) && (L.op.type == OP_NEG || L.op.type == OP_CPHASE) && !L.nondiag && L.op.mask && L.diag == L.op.mask;
+  };
+  auto is_h = [](const Lowered& L) {
+    if (!fusable_type(L) || L.op.type != OP_1Q || L.op.ctrl || L.coef.size() < 4 * sizeof(Cx) / sizeof(L.coef[0])) return false;
+    const Cx* m = reinterpret_cast<const Cx*>(L.coef.data());
+    const double s = std::sqrt(0.5);
+    for (int k = 0; k < 4; ++k)
+      if (m[k].im != 0.0 || std::fabs(m[k].re - (k == 3 ? -s : s)) > 1e-15) return false;
+    return true;
+  };
+  auto coef = [](const Lowered& L) { return L.op.type == OP_NEG ? Cx{-1.0, 0.0} : *reinterpret_cast<const Cx*>(L.coef.data()); };
+  for (size_t i = 0; i < ops.size(); ++i) {
+    const Lowered& L = *ops[i];
+    const uint64_t touched = L.nondiag | L.diag;
+    if (is_phase(L)) {
+      const auto it = phase.find(L.op.mask);
+      if (it != phase.end()) {  // join the earlier one, here
+        const Lowered& E = *ops[it->second];
+        Cx c = mul(coef(E), coef(L));
+        if (std::fabs(c.im) <= 4e-15) c = Cx{c.re > 0 ? 1.0 : -1.0, 0.0};
+        store.emplace_back();
+        Lowered& F = store.back();
+        std::memset(&F.op, 0, sizeof(Op));
+        F.record = L.record;
+        F.gates = gates_of(E) + gates_of(L);
+        F.absorbed = F.gates == 0;
+        F.op.mask = F.diag = L.op.mask;
+        F.nondiag = 0;
+        if (c.re == -1.0) {
+          F.op.type = OP_NEG;
+        } else {
+          F.op.type = OP_CPHASE;
+          push_coef(&F, &c, 1);
+        }
+        const bool gone = is_one(c);
+        if (gone) F.op.mask = F.diag = 0;  // the identity, kept for its gate count
+        // an H before the earlier phase sees the joined one instead
+        for (uint64_t t = L.op.mask; t; t &= t - 1) {
+          auto& list = since[__builtin_ctzll(t)];
+          list.erase(std::remove(list.begin(), list.end(), it->second), list.end());
+          if (!gone) list.push_back(i);
+        }
+        ops[it->second] = nullptr;
+        ops[i] = &F;
+        if (gone) phase.erase(it);
+        else it->second = i;
+        continue;
+      }
+      phase[L.op.mask] = i;
+      for (uint64_t t = L.op.mask; t; t &= t - 1) since[__builtin_ctzll(t)].push_back(i);
+      continue;
+    }
+    const int q = touched ? __builtin_ctzll(touched) : 0;
+    if (is_h(L) && h[q] != SIZE_MAX && since[q].size() == 1 && ops[since[q][0]]->op.type == OP_NEG &&
+        ops[since[q][0]]->op.mask != touched) {
+      const size_t at = since[q][0];
+      const Lowered& N = *ops[at];
+      const uint64_t others = N.op.mask & ~touched;
+      store.emplace_back();
+      Lowered& F = store.back();
+      std::memset(&F.op, 0, sizeof(Op));
+      F.record = N.record;
+      F.gates = gates_of(*ops[h[q]]) + gates_of(N) + gates_of(L);
+      F.absorbed = F.gates == 0;
+      F.op.type = OP_X;
+      F.op.nq = 1;
+      F.op.q[0] = (uint8_t)q;
+      F.op.ctrl = F.diag = others;
+      F.nondiag = touched;
+      ops[h[q]] = ops[i] = nullptr;
+      phase.erase(N.op.mask);
+      for (uint64_t t = others; t; t &= t - 1) h[__builtin_ctzll(t)] = SIZE_MAX;  // the flip is gone from their runs
+      ops[at] = &F;
+      h[q] = SIZE_MAX;
+    } else {
+      for (uint64_t t = touched; t; t &= t - 1) h[__builtin_ctzll(t)] = SIZE_MAX;
+      if (is_h(L)) {
+        h[q] = i;
+        since[q].clear();
+      }
+    }
+    if (L.nondiag)
+      for (auto it = phase.begin(); it != phase.end();) it = it->first & L.nondiag ? phase.erase(it) : std::next(it);
+  }
+  ops.erase(std::remove(ops.begin(), ops.end(), nullptr), ops.end());
   return ops;
 }
 
@@ -1753,7 +1856,7 @@ int build_plan(const std::vector<Lowered>& ops, uint32_t n, bool f64, const Plan
         // relabel_swaps off) compare the parts of the warp-tile planner, and a state
         // smaller than one wide tile has no choice.
         const bool wide = n >= kWideBits && o.relabel_swaps && ((o.tile_r == 5 && o.tile_occupancy == 0) || o.tile_r == 4);
-        status = wide ? plan_segment_wide(fuse_pairs(diagonal_cores(seg, fused), fused), n, f64, R, o.tile_r == 4 ? 4 : 5, P)
+        status = wide ? plan_segment_wide(fuse_pairs(cancel_phases(diagonal_cores(seg, fused), fused), fused), n, f64, R, o.tile_r == 4 ? 4 : 5, P)
                       : plan_segment_tiles(fuse_pairs(seg, fused), n, R, P);
       } else {
         status = plan_segment_tiles(seg, n, R, P);
