@@ -567,6 +567,10 @@ bool real_matrix(const Lowered& L) {
   return true;
 }
 
+// |c| = 1 to rounding. A TiledBlock's matrices are taken as they are, so a
+// diagonal's entries need not be phases.
+bool unimodular(Cx c) { return std::fabs(std::hypot(c.re, c.im) - 1.0) <= 1e-15; }
+
 // Source gates that an op stands for.
 uint32_t gates_of(const Lowered& L) { return L.absorbed ? 0 : L.gates ? L.gates : 1; }
 
@@ -652,8 +656,7 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
       return;
     }
     const Cx* d = reinterpret_cast<const Cx*>(L.coef.data());
-    const double l0 = std::hypot(d[0].re, d[0].im), l1 = std::hypot(d[1].re, d[1].im);
-    if (std::fabs(l0 - 1.0) > 1e-15 || std::fabs(l1 - 1.0) > 1e-15) {  // not unimodular to rounding: keep the table
+    if (!unimodular(d[0]) || !unimodular(d[1])) {  // keep the table
       out.emplace_back(at, &L);
       return;
     }
@@ -875,9 +878,11 @@ std::vector<const Lowered*> cancel_phases(const std::vector<const Lowered*>& seg
     const uint64_t touched = L.nondiag | L.diag;
     if (is_phase(L)) {
       const auto it = phase.find(L.op.mask);
-      if (it != phase.end()) {  // join the earlier one, here
+      if (it != phase.end() && unimodular(coef(*ops[it->second])) && unimodular(coef(L))) {  // join the earlier one, here
         const Lowered& E = *ops[it->second];
         Cx c = mul(coef(E), coef(L));
+        const double len = std::hypot(c.re, c.im);
+        c = Cx{c.re / len, c.im / len};
         if (std::fabs(c.im) <= 4e-15) c = Cx{c.re > 0 ? 1.0 : -1.0, 0.0};
         store.emplace_back();
         Lowered& F = store.back();

@@ -1,0 +1,46 @@
+"""Diagonal gates that the planner joins, cancels or multiplies out, against the
+oracle: entries that are no phases, phases next to +1 and -1, and long runs of
+small rotations. Every circuit runs on a wide plan (n = 14), a shared-memory one
+(n = 10) and, in TC32, on block passes.
+
+Tolerances: FP64 1e-12 and FP32 / TC32 1e-5 on the amplitudes, as in the parity
+tests."""
+import numpy as np
+import pytest
+
+from aleph_b200 import circuit as C
+from aleph_b200.backend import B200SvBackend
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"f64": 1e-12, "f32": 1e-5, "tc32": 1e-5}
+
+
+def check(n, insts, precision):
+    want, _ = oracle.run(n, insts)
+    be = B200SvBackend(seed=0, precision=precision)
+    if precision == "tc32":
+        be.set_tuning("renormalize", 0)  # the blocks are not unitary
+    st = be.allocate(n)
+    be.apply_stream(st, insts)
+    assert np.abs(be.statevector(st) - want).max() <= TOL[precision]
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32", "tc32"])
+@pytest.mark.parametrize("n", [10, 14])
+@pytest.mark.parametrize("pair", [(0.5, 0.5), (2.0, 0.25), (0.0, 0.0), (-1.0, 0.5), (0.5j, 0.5j), (1 + 1e-9, 1.0)])
+def test_diagonals_that_are_no_phases_keep_their_modulus(pair, n, precision):
+    # a TiledBlock's matrices are taken without a unitarity check
+    def diag(c, q):
+        return C.GateInstance(C.Unitary1q(np.diag([1.0, c])), [q])
+
+    def cdiag(c, q):
+        return C.GateInstance(C.Unitary1q(np.diag([1.0, c])), [q[1]], [q[0]])
+
+    insts = [C.GateInstance(C.H(), [q]) for q in range(3)]
+    insts.append(C.TiledBlock([diag(pair[0], 0), diag(pair[1], 0), cdiag(pair[0], [1, 2]), cdiag(pair[1], [1, 2])], 15))
+    insts.append(C.GateInstance(C.H(), [0]))
+    insts.append(C.TiledBlock([C.GateInstance(C.Cnot(), [0, 1]), diag(pair[0], 1), diag(pair[1], 1),
+                               C.GateInstance(C.Cnot(), [0, 1])], 15))
+    check(n, insts, precision)
