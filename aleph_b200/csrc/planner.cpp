@@ -195,6 +195,7 @@ double unitarity_deviation(const Cx* m, int dim) {
 
 bool is_zero(Cx a) { return a.re == 0.0 && a.im == 0.0; }
 bool is_one(Cx a) { return a.re == 1.0 && a.im == 0.0; }
+bool is_minus_one(Cx a) { return a.re == -1.0 && a.im == 0.0; }  // re alone rounds to -1 up to 1e-8 away from it
 
 void push_coef(Lowered* L, const Cx* c, int count) {
   for (int i = 0; i < count; ++i) {
@@ -229,7 +230,7 @@ void lower_matrix(const Cx* m, int dim, const uint32_t* tq, uint64_t ctrl, Lower
     if (corner) {
       op.mask = tmask | ctrl;
       op.ctrl = 0;
-      if (c.re == -1.0 && c.im == 0.0) {
+      if (is_minus_one(c)) {
         op.type = OP_NEG;
       } else {
         op.type = OP_CPHASE;
@@ -638,7 +639,7 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
     F.record = record;
     F.gates = gates;
     F.absorbed = gates == 0;
-    if (c.re == -1.0) {
+    if (is_minus_one(c)) {
       F.op.type = OP_NEG;
     } else {
       F.op.type = OP_CPHASE;
@@ -764,7 +765,7 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
       else if (std::fabs(c.re) <= snap) c = Cx{0.0, c.im > 0 ? 1.0 : -1.0};
       cs[S] = c;
       used[S] = S != 0 && !is_one(c);
-      if (used[S]) price += c.re == -1.0 ? 1 : 2;
+      if (used[S]) price += is_minus_one(c) ? 1 : 2;
     }
     if (smem) {
       int runs = 0;
@@ -892,7 +893,7 @@ std::vector<const Lowered*> cancel_phases(const std::vector<const Lowered*>& seg
         F.absorbed = F.gates == 0;
         F.op.mask = F.diag = L.op.mask;
         F.nondiag = 0;
-        if (c.re == -1.0) {
+        if (is_minus_one(c)) {
           F.op.type = OP_NEG;
         } else {
           F.op.type = OP_CPHASE;

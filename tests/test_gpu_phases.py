@@ -44,3 +44,18 @@ def test_diagonals_that_are_no_phases_keep_their_modulus(pair, n, precision):
     insts.append(C.TiledBlock([C.GateInstance(C.Cnot(), [0, 1]), diag(pair[0], 1), diag(pair[1], 1),
                                C.GateInstance(C.Cnot(), [0, 1])], 15))
     check(n, insts, precision)
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32", "tc32"])
+@pytest.mark.parametrize("n", [10, 14])
+@pytest.mark.parametrize("eps", [1e-8, -1e-10, 3e-12, 0.0])
+def test_phases_next_to_a_sign_flip(eps, n, precision):
+    # cos(pi - 1e-8) rounds to -1: the angle is in the imaginary part alone
+    insts = [C.GateInstance(C.H(), [q]) for q in range(4)]
+    insts += [C.GateInstance(C.Rz(np.pi - eps), [0]), C.GateInstance(C.CRz(np.pi - eps), [1, 2])]
+    insts += [C.GateInstance(C.Phase(1.0), [3]), C.GateInstance(C.Phase(np.pi - 1.0 - eps), [3])]
+    insts += [C.GateInstance(C.H(), [q]) for q in range(4)]
+    insts += [C.GateInstance(C.Cnot(), [0, 1]), C.GateInstance(C.Rz(np.pi / 2 - eps), [1]),
+              C.GateInstance(C.Cnot(), [0, 1]), C.GateInstance(C.Cnot(), [0, 2]), C.GateInstance(C.Cnot(), [0, 2])]
+    insts += [C.GateInstance(C.Phase(np.pi - eps), [2], [0])]
+    check(n, insts, precision)
