@@ -572,6 +572,15 @@ bool real_matrix(const Lowered& L) {
 // diagonal's entries need not be phases.
 bool unimodular(Cx c) { return std::fabs(std::hypot(c.re, c.im) - 1.0) <= 1e-15; }
 
+// A phase, exactly +-1 or +-i where it lies within `tol` of that. tol is what the
+// rounding of the phase's own product can have moved it by, so that no angle is
+// dropped that its gates had.
+Cx snapped(Cx c, double tol) {
+  if (std::fabs(c.im) <= tol) return Cx{c.re > 0 ? 1.0 : -1.0, 0.0};
+  if (std::fabs(c.re) <= tol) return Cx{0.0, c.im > 0 ? 1.0 : -1.0};
+  return c;
+}
+
 // Source gates that an op stands for.
 uint32_t gates_of(const Lowered& L) { return L.absorbed ? 0 : L.gates ? L.gates : 1; }
 
@@ -729,8 +738,10 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
       to[c] = c;
       d[c] = Cx{1.0, 0.0};
     }
+    uint32_t phases = 0;  // members whose products round
     for (const Lowered* L : core) {
       const Op& op = L->op;
+      phases += op.type == OP_CPHASE || op.type == OP_DIAG;
       const Cx* k = reinterpret_cast<const Cx*>(L->coef.data());
       const uint32_t ctrl = local(op.ctrl), mask = local(op.mask), bit = local(1ull << op.q[0]);
       for (uint32_t c = 0; c < dim; ++c) {
@@ -760,10 +771,7 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
       Cx c{1.0, 0.0};
       for (uint32_t T = 0; T < dim; ++T)
         if ((T & S) == T) c = mul(c, (__builtin_popcount(S ^ T) & 1) ? conj(d[T]) : d[T]);
-      const double snap = 8 * tol;
-      if (std::fabs(c.im) <= snap) c = Cx{c.re > 0 ? 1.0 : -1.0, 0.0};
-      else if (std::fabs(c.re) <= snap) c = Cx{0.0, c.im > 0 ? 1.0 : -1.0};
-      cs[S] = c;
+      cs[S] = c = snapped(c, std::min(0x1p-49, 0x1p-52 * (double)(2 + phases)));
       used[S] = S != 0 && !is_one(c);
       if (used[S]) price += is_minus_one(c) ? 1 : 2;
     }
@@ -883,8 +891,7 @@ std::vector<const Lowered*> cancel_phases(const std::vector<const Lowered*>& seg
         const Lowered& E = *ops[it->second];
         Cx c = mul(coef(E), coef(L));
         const double len = std::hypot(c.re, c.im);
-        c = Cx{c.re / len, c.im / len};
-        if (std::fabs(c.im) <= 4e-15) c = Cx{c.re > 0 ? 1.0 : -1.0, 0.0};
+        c = snapped(Cx{c.re / len, c.im / len}, 0x1p-52);  // one product
         store.emplace_back();
         Lowered& F = store.back();
         std::memset(&F.op, 0, sizeof(Op));

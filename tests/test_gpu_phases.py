@@ -59,3 +59,15 @@ def test_phases_next_to_a_sign_flip(eps, n, precision):
               C.GateInstance(C.Cnot(), [0, 1]), C.GateInstance(C.Cnot(), [0, 2]), C.GateInstance(C.Cnot(), [0, 2])]
     insts += [C.GateInstance(C.Phase(np.pi - eps), [2], [0])]
     check(n, insts, precision)
+
+
+@pytest.mark.parametrize("n", [10, 14])
+@pytest.mark.parametrize("angle,count", [(1e-14, 3000), (3e-13, 40), (1e-15, 2000)])
+def test_long_runs_of_small_rotations_add_up(angle, count, n):
+    # ZZ rotations and phases on the same qubits: each is far below the tolerance, their sum is not
+    insts = [C.GateInstance(C.H(), [q]) for q in range(3)]
+    for _ in range(count):
+        insts += [C.GateInstance(C.Cnot(), [0, 1]), C.GateInstance(C.Rz(angle), [1]), C.GateInstance(C.Cnot(), [0, 1]),
+                  C.GateInstance(C.Phase(angle), [2])]
+    insts += [C.GateInstance(C.H(), [q]) for q in range(3)]
+    check(n, insts, "f64")
