@@ -765,12 +765,29 @@ int aleph_b200_apply_gate_stream(aleph_b200_handle* h, aleph_b200_state* st, con
   return stream_impl(h, st, in, count, pools, mu, n_mu, outcomes, outcomes_cap, n_outcomes, nullptr);
 }
 
+// A plan's coefficients are laid out for one precision (wide passes pair them
+// for FP32). The handle's own form is planned at compile time, the other one
+// when a state of that precision first comes to execute.
 struct aleph_b200_plan {
   uint32_t n = 0;
-  Plan P;
-  Scratch buf;
-  bool uploaded = false;
+  std::vector<Lowered> ops;
+  PlanOptions opts;  // the handle's at compile time
+  struct Form {
+    Plan P;
+    Scratch buf;
+    bool planned = false, uploaded = false;
+  } form[2];  // FP32 states, FP64 states
 };
+
+static int plan_form(aleph_b200_handle* h, aleph_b200_plan* p, bool f64) {
+  aleph_b200_plan::Form& F = p->form[f64];
+  if (F.planned) return 0;
+  F.P = Plan();
+  if (int s = build_plan(p->ops, p->n, f64, p->opts, &F.P))
+    return set_error(h, s, "optimization pipeline failed: planner");
+  F.planned = true;
+  return 0;
+}
 
 int aleph_b200_compile(aleph_b200_handle* h, uint32_t num_qubits, const aleph_b200_instr* in, uint64_t count,
                        const aleph_b200_pools* pools, aleph_b200_plan** out) {
@@ -788,9 +805,11 @@ int aleph_b200_compile(aleph_b200_handle* h, uint32_t num_qubits, const aleph_b2
   aleph_b200_plan* p = new (std::nothrow) aleph_b200_plan();
   if (!p) return set_error(h, ALEPH_B200_DEVICE_FAILURE, "host allocation failed");
   p->n = num_qubits;
-  if (int s = build_plan(ops, num_qubits, h->precision == ALEPH_B200_F64, h->opts, &p->P)) {
+  p->ops = std::move(ops);
+  p->opts = h->opts;
+  if (int s = plan_form(h, p, h->precision == ALEPH_B200_F64)) {
     delete p;
-    return set_error(h, s, "optimization pipeline failed: planner");
+    return s;
   }
   *out = p;
   return ALEPH_B200_OK;
@@ -803,17 +822,21 @@ int aleph_b200_execute(aleph_b200_handle* h, aleph_b200_state* st, aleph_b200_pl
   if (plan->n != st->n)
     return set_error(h, ALEPH_B200_INVALID_ARGUMENT, "plan compiled for %u qubits, state has %u", plan->n, st->n);
   if (int r = bind(h)) return r;
-  return run_plan(h, st, plan->P, mu, n_mu, outcomes, outcomes_cap, n_outcomes, nullptr, &plan->buf, &plan->uploaded);
+  const bool f64 = st->precision == ALEPH_B200_F64;
+  if (int r = plan_form(h, plan, f64)) return r;
+  aleph_b200_plan::Form& F = plan->form[f64];
+  return run_plan(h, st, F.P, mu, n_mu, outcomes, outcomes_cap, n_outcomes, nullptr, &F.buf, &F.uploaded);
 }
 
 int aleph_b200_plan_free(aleph_b200_handle* h, aleph_b200_plan* plan) {
   if (!plan) return ALEPH_B200_OK;
-  if (plan->buf.ptr) {
+  if (plan->form[0].buf.ptr || plan->form[1].buf.ptr) {
     if (h) {
       cudaSetDevice(h->device);
       cudaStreamSynchronize(h->stream);
     }
-    cudaFree(plan->buf.ptr);
+    for (auto& F : plan->form)
+      if (F.buf.ptr) cudaFree(F.buf.ptr);
   }
   delete plan;
   return ALEPH_B200_OK;

@@ -1856,7 +1856,7 @@ int build_plan(const std::vector<Lowered>& ops, uint32_t n, bool f64, const Plan
     } else {
       // a 2-qubit gate may need two register qubits: R >= 2 unless only one high qubit exists
       const uint32_t R = std::min<uint32_t>(std::max<uint32_t>(o.tile_r, 2), std::min<uint32_t>(5, n - 5));
-      if (o.tensor_blocks && n >= 13) {
+      if (o.tensor_blocks && !f64 && n >= 13) {  // blocks act on FP32 states
         // diagonal cores follow a block as its post ops instead of ending it
         std::deque<Lowered> fused;
         status = plan_segment_blocks(o.pair_fusion ? diagonal_cores(seg, fused) : seg, n, R, o.block_window_search, P);
