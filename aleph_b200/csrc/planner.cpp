@@ -198,10 +198,8 @@ bool is_one(Cx a) { return a.re == 1.0 && a.im == 0.0; }
 bool is_minus_one(Cx a) { return a.re == -1.0 && a.im == 0.0; }  // re alone rounds to -1 up to 1e-8 away from it
 
 void push_coef(Lowered* L, const Cx* c, int count) {
-  for (int i = 0; i < count; ++i) {
-    L->coef.push_back(c[i].re);
-    L->coef.push_back(c[i].im);
-  }
+  const double* d = reinterpret_cast<const double*>(c);
+  L->coef.insert(L->coef.end(), d, d + 2 * count);
 }
 
 // Lower a validated dense matrix with MSB-first targets to the cheapest op.
@@ -545,8 +543,6 @@ void swap_2q_operands(std::vector<double>& c) {
 // again on their qubits (so a CZ between two already-absorbed layers leaves
 // the next layer to the next block). This is the idea of Fuse2q
 // (crates/aleph-ir/src/passes/fuse_2q.rs) with a cost rule for register tiles.
-void apply_local(const Lowered& L, const uint32_t* bq, Cx* s);
-
 namespace {
 
 int tile_cost(const Lowered& L) {
@@ -584,19 +580,61 @@ Cx snapped(Cx c, double tol) {
 // Source gates that an op stands for.
 uint32_t gates_of(const Lowered& L) { return L.absorbed ? 0 : L.gates ? L.gates : 1; }
 
-// The 4x4 of an op on qubits {a (matrix MSB), b (LSB)}, right-multiplied into m:
-// m := op * m.
+// The 4x4 of an op on qubits {a (matrix MSB), b (LSB)}, left-multiplied into m:
+// m := op * m. At most 64 complex products; the plan of a state that fits one SM
+// is made of these, and it is made again for every new set of angles.
 void fold_into_4x4(const Lowered& L, uint32_t a, uint32_t b, Cx* m) {
-  const uint32_t bq[6] = {b, a, 60, 61, 62, 63};  // local bit 0 = b, bit 1 = a
-  Cx out[16];
-  for (uint32_t c = 0; c < 4; ++c) {
-    Cx s[64];
-    for (auto& x : s) x = Cx{0, 0};
-    for (uint32_t r = 0; r < 4; ++r) s[r] = m[r * 4 + c];
-    apply_local(L, bq, s);
-    for (uint32_t r = 0; r < 4; ++r) out[r * 4 + c] = s[r];
+  const Op& op = L.op;
+  const Cx* c = reinterpret_cast<const Cx*>(L.coef.data());
+  auto rows = [&](uint64_t q) { return (uint32_t)(((q >> b) & 1) | (((q >> a) & 1) << 1)); };  // qubit mask -> row bits
+  switch (op.type) {
+    case OP_NEG:
+    case OP_CPHASE: {
+      const uint32_t mask = rows(op.mask);
+      const Cx f = op.type == OP_NEG ? Cx{-1, 0} : c[0];
+      for (uint32_t r = 0; r < 4; ++r)
+        if ((r & mask) == mask)
+          for (uint32_t k = 0; k < 4; ++k) m[r * 4 + k] = mul(f, m[r * 4 + k]);
+      return;
+    }
+    case OP_DIAG: {
+      const uint32_t ctrl = rows(op.ctrl);
+      for (uint32_t r = 0; r < 4; ++r) {
+        if ((r & ctrl) != ctrl) continue;
+        uint32_t idx = 0;
+        for (int i = 0; i < op.nq; ++i) idx = (idx << 1) | (op.q[i] == a ? r >> 1 : r & 1);
+        for (uint32_t k = 0; k < 4; ++k) m[r * 4 + k] = mul(c[idx], m[r * 4 + k]);
+      }
+      return;
+    }
+    case OP_X:
+    case OP_1Q: {
+      const uint32_t bit = rows(1ull << op.q[0]), ctrl = rows(op.ctrl);
+      for (uint32_t r = 0; r < 4; ++r) {
+        if ((r & bit) || (r & ctrl) != ctrl) continue;
+        Cx *x = m + r * 4, *y = m + (r | bit) * 4;
+        for (uint32_t k = 0; k < 4; ++k) {
+          const Cx u = x[k], v = y[k];
+          x[k] = op.type == OP_X ? v : add(mul(c[0], u), mul(c[1], v));
+          y[k] = op.type == OP_X ? u : add(mul(c[2], u), mul(c[3], v));
+        }
+      }
+      return;
+    }
+    default: {  // OP_2Q, operands in either order
+      const uint32_t hi = rows(1ull << op.q[0]), lo = rows(1ull << op.q[1]);
+      const uint32_t at[4] = {0, lo, hi, hi | lo};
+      Cx out[16];
+      for (uint32_t r = 0; r < 4; ++r)
+        for (uint32_t k = 0; k < 4; ++k) {
+          Cx acc = mul(c[r * 4], m[at[0] * 4 + k]);
+          for (uint32_t t = 1; t < 4; ++t) acc = add(acc, mul(c[r * 4 + t], m[at[t] * 4 + k]));
+          out[at[r] * 4 + k] = acc;
+        }
+      for (int i = 0; i < 16; ++i) m[i] = out[i];
+      return;
+    }
   }
-  for (int i = 0; i < 16; ++i) m[i] = out[i];
 }
 
 bool fusable_type(const Lowered& L) {
@@ -627,18 +665,22 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
                                            bool smem = false) {
   struct Block {
     uint64_t qubits = 0;
-    std::vector<size_t> members;  // indices in seg, ascending
+    std::vector<size_t> members;  // indices in seg, ascending; empty: no block
   };
   // Ops with the place they go to (sorted at the end, so that gates that stay keep
   // their order): a gate's own index in seg; for corner phases, the last of the
   // first core gates on their qubits, which is behind all that earlier blocks did there.
   std::vector<std::pair<size_t, const Lowered*>> out;
   out.reserve(seg.size());
-  std::vector<Block> blocks;  // open ones; few at a time
+  std::vector<Block> blocks;         // open ones; each owns its qubits
+  int owner[64];                     // per qubit: its block, or -1
+  std::fill(owner, owner + 64, -1);
+  bool changed = false;  // some op goes out in another form or place than it came
   Cx global{1.0, 0.0};
   uint32_t last_record = 0;
   auto width = [](const Lowered& L) { return __builtin_popcountll(L.nondiag | L.diag); };
   auto corner = [&](size_t at, uint64_t mask, Cx c, uint32_t record, uint32_t gates) {
+    changed = true;
     store.emplace_back();
     Lowered& F = store.back();
     std::memset(&F.op, 0, sizeof(Op));
@@ -678,48 +720,57 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
       last_record = L.record;
     }
   };
+  std::vector<size_t> before, after;
+  std::vector<const Lowered*> core;
   auto emit = [&](const Block& B) {
-    size_t first[64], last[64];
-    for (auto& x : first) x = SIZE_MAX;
-    for (auto& x : last) x = 0;
+    uint32_t bq[3] = {0, 0, 0}, nb = 0;
+    for (uint64_t t = B.qubits; t; t &= t - 1) bq[nb++] = (uint32_t)__builtin_ctzll(t);
+    const uint32_t dim = 1u << nb;
+    auto local = [&](uint64_t m) {  // qubit mask -> bits of the block's index
+      uint32_t r = 0;
+      for (uint32_t b = 0; b < nb; ++b) r |= (uint32_t)((m >> bq[b]) & 1) << b;
+      return r;
+    };
+    size_t first[3] = {SIZE_MAX, SIZE_MAX, SIZE_MAX}, last[3] = {0, 0, 0};  // per qubit: its gates on several qubits
     uint32_t multi = 0;
     for (size_t k = 0; k < B.members.size(); ++k) {
       const Lowered& L = *seg[B.members[k]];
       if (width(L) < 2) continue;
       ++multi;
-      for (uint64_t t = L.nondiag | L.diag; t; t &= t - 1) {
-        const int q = __builtin_ctzll(t);
-        first[q] = std::min(first[q], k);
-        last[q] = k;
-      }
+      const uint32_t on = local(L.nondiag | L.diag);
+      for (uint32_t b = 0; b < nb; ++b)
+        if ((on >> b) & 1) {
+          first[b] = std::min(first[b], k);
+          last[b] = k;
+        }
     }
     auto plain = [&] {
       for (size_t m : B.members) keep(m, m);
     };
     if (multi < 2) return plain();
-    uint32_t bq[6] = {60, 61, 62, 63, 59, 58}, nb = 0;
-    for (uint64_t t = B.qubits; t; t &= t - 1) bq[nb++] = (uint32_t)__builtin_ctzll(t);
-    const uint32_t dim = 1u << nb;
-    std::vector<size_t> before, after;
-    std::vector<const Lowered*> core;
+    before.clear();
+    after.clear();
+    core.clear();
     size_t place = 0;  // behind everything that came before the block on any of the core's qubits
-    for (uint32_t q = 0; q < 64; ++q)
-      if (first[q] != SIZE_MAX) place = std::max(place, B.members[first[q]]);
+    for (uint32_t b = 0; b < nb; ++b)
+      if (first[b] != SIZE_MAX) place = std::max(place, B.members[first[b]]);
     int cost = 0;
     uint32_t gates = 0;
     bool monomial = true;  // a core with a dense member is left alone
     for (size_t k = 0; k < B.members.size(); ++k) {
       const Lowered* L = seg[B.members[k]];
       if (width(*L) < 2) {
-        const uint64_t t = L->nondiag | L->diag;
-        const int q = t ? __builtin_ctzll(t) : 0;
-        if (first[q] == SIZE_MAX || k < first[q] || k > last[q]) {
+        const int b = __builtin_ctz(local(L->nondiag | L->diag));
+        if (first[b] == SIZE_MAX || k < first[b] || k > last[b]) {
           // a qubit without multi-qubit gates keeps its order: everything on it comes first
-          (first[q] == SIZE_MAX || k < first[q] ? before : after).push_back(B.members[k]);
+          (first[b] == SIZE_MAX || k < first[b] ? before : after).push_back(B.members[k]);
           continue;
         }
       }
-      if (L->op.type != OP_X && L->nondiag) monomial = false;
+      if (L->op.type != OP_X && L->nondiag) {
+        monomial = false;
+        break;
+      }
       core.push_back(L);
       cost += L->nondiag ? std::max(8, tile_cost(*L)) : tile_cost(*L);
       gates += gates_of(*L);
@@ -727,11 +778,6 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
     if (!monomial) return plain();
     // The core as a map of basis states with phases: its members are X-like or diagonal.
     const double tol = 1e-15 * (double)(core.size() + 2);
-    auto local = [&](uint64_t m) {  // qubit mask -> bits of the block's index
-      uint32_t r = 0;
-      for (uint32_t b = 0; b < nb; ++b) r |= (uint32_t)((m >> bq[b]) & 1) << b;
-      return r;
-    };
     uint32_t to[8];
     Cx d[8];
     for (uint32_t c = 0; c < dim; ++c) {
@@ -806,49 +852,72 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
     last_record = record;
     for (size_t m : after) keep(std::max(m, place), m);
   };
-  auto close = [&](size_t k) {
-    const Block B = std::move(blocks[k]);
-    blocks.erase(blocks.begin() + (long)k);
-    emit(B);
+  auto release = [&](Block& B) {
+    for (uint64_t t = B.qubits; t; t &= t - 1) owner[__builtin_ctzll(t)] = -1;
+    B.qubits = 0;
+    B.members.clear();
   };
+  auto close = [&](int k) {
+    emit(blocks[(size_t)k]);
+    release(blocks[(size_t)k]);
+  };
+  std::vector<size_t> merged;
   for (size_t i = 0; i < seg.size(); ++i) {
     const Lowered& L = *seg[i];
     const uint64_t touched = L.nondiag | L.diag;
     const bool small = fusable_type(L) && touched && __builtin_popcountll(touched) <= 3;
-    // close touched blocks, the widest first, until the rest and this gate fit three qubits
+    // close touched blocks, the widest first (the older of two), until the rest and this gate fit three qubits
+    int mine = -1;  // the touched block that stays open and is widened
     for (;;) {
       uint64_t all = touched;
-      size_t widest = SIZE_MAX;
-      for (size_t k = 0; k < blocks.size(); ++k) {
-        if (!(blocks[k].qubits & touched)) continue;
-        all |= blocks[k].qubits;
-        if (widest == SIZE_MAX ||
-            __builtin_popcountll(blocks[k].qubits) > __builtin_popcountll(blocks[widest].qubits))
-          widest = k;
+      int widest = -1;
+      for (uint64_t t = touched; t; t &= t - 1) {
+        const int k = owner[__builtin_ctzll(t)];
+        if (k < 0 || k == widest) continue;
+        const Block& B = blocks[(size_t)k];
+        all |= B.qubits;
+        if (widest >= 0) {
+          const Block& W = blocks[(size_t)widest];
+          const int wide = __builtin_popcountll(B.qubits), most = __builtin_popcountll(W.qubits);
+          if (wide < most || (wide == most && B.members.back() >= W.members.back())) continue;
+        }
+        widest = k;
       }
-      if (widest == SIZE_MAX || (small && __builtin_popcountll(all) <= 3)) break;
+      mine = widest;
+      if (widest < 0 || (small && __builtin_popcountll(all) <= 3)) break;
       close(widest);
     }
     if (!small) {
       keep(i, i);
       continue;
     }
-    Block B;
-    for (size_t k = 0; k < blocks.size();) {
-      if (blocks[k].qubits & touched) {
-        B.qubits |= blocks[k].qubits;
-        B.members.insert(B.members.end(), blocks[k].members.begin(), blocks[k].members.end());
-        blocks.erase(blocks.begin() + (long)k);
-      } else {
-        ++k;
+    if (mine < 0) {
+      for (mine = 0; mine < (int)blocks.size() && !blocks[(size_t)mine].members.empty();) ++mine;
+      if (mine == (int)blocks.size()) blocks.emplace_back();
+    }
+    Block& M = blocks[(size_t)mine];
+    for (uint64_t t = touched; t; t &= t - 1) {
+      const int k = owner[__builtin_ctzll(t)];
+      if (k >= 0 && k != mine) {  // join it: at most twice in a block's life
+        Block& B = blocks[(size_t)k];
+        merged.resize(M.members.size() + B.members.size());
+        std::merge(M.members.begin(), M.members.end(), B.members.begin(), B.members.end(), merged.begin());
+        M.members.swap(merged);
+        const uint64_t q = B.qubits;
+        release(B);
+        M.qubits |= q;
       }
     }
-    std::sort(B.members.begin(), B.members.end());
-    B.qubits |= touched;
-    B.members.push_back(i);
-    blocks.push_back(std::move(B));
+    M.qubits |= touched;
+    for (uint64_t t = M.qubits; t; t &= t - 1) owner[__builtin_ctzll(t)] = mine;
+    M.members.push_back(i);
   }
-  while (!blocks.empty()) close(0);
+  std::sort(blocks.begin(), blocks.end(), [](const Block& x, const Block& y) {  // by their last gates
+    return (x.members.empty() ? 0 : x.members.back()) < (y.members.empty() ? 0 : y.members.back());
+  });
+  for (const Block& B : blocks)
+    if (!B.members.empty()) emit(B);
+  if (!changed) return seg;
   if (!is_one(global)) corner(SIZE_MAX, 0, global, last_record, 0);
   std::stable_sort(out.begin(), out.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
   std::vector<const Lowered*> ops;
@@ -865,11 +934,13 @@ std::vector<const Lowered*> diagonal_cores(const std::vector<const Lowered*>& se
 // Measured: n = 22 FP32 Grover 1697 -> 1060 us (19 -> 14 passes), its error against
 // 64 bits 1.3e-5 -> 2.4e-6.
 std::vector<const Lowered*> cancel_phases(const std::vector<const Lowered*>& seg, std::deque<Lowered>& store) {
-  std::vector<const Lowered*> ops = seg;
-  std::unordered_map<uint64_t, size_t> phase;  // mask -> its last phase op, while it can still be joined
+  // A mask's last phase op can still be joined while no op behind it moves one of
+  // the mask's qubits.
+  std::unordered_map<uint64_t, size_t> phase;  // mask -> its last phase op, counted from 1
+  size_t moved[64] = {};                       // per qubit: the last op that moves it, counted from 1
   size_t h[64];                                // per qubit: an H with only phases since; SIZE_MAX: none
   std::vector<size_t> since[64];               // those phases
-  for (auto& x : h) x = SIZE_MAX;
+  std::fill(h, h + 64, SIZE_MAX);
   auto is_phase = [](const Lowered& L) {
     return fusable_type(L) && (L.op.type == OP_NEG || L.op.type == OP_CPHASE) && !L.nondiag && L.op.mask && L.diag == L.op.mask;
   };
@@ -882,13 +953,18 @@ std::vector<const Lowered*> cancel_phases(const std::vector<const Lowered*>& seg
     return true;
   };
   auto coef = [](const Lowered& L) { return L.op.type == OP_NEG ? Cx{-1.0, 0.0} : *reinterpret_cast<const Cx*>(L.coef.data()); };
+  if (std::none_of(seg.begin(), seg.end(), [&](const Lowered* L) { return is_phase(*L); })) return seg;
+  std::vector<const Lowered*> ops = seg;
   for (size_t i = 0; i < ops.size(); ++i) {
     const Lowered& L = *ops[i];
     const uint64_t touched = L.nondiag | L.diag;
     if (is_phase(L)) {
-      const auto it = phase.find(L.op.mask);
-      if (it != phase.end() && unimodular(coef(*ops[it->second])) && unimodular(coef(L))) {  // join the earlier one, here
-        const Lowered& E = *ops[it->second];
+      size_t& last = phase[L.op.mask];
+      for (uint64_t t = L.op.mask; t; t &= t - 1)
+        if (last <= moved[__builtin_ctzll(t)]) last = 0;
+      if (last && unimodular(coef(*ops[last - 1])) && unimodular(coef(L))) {  // join the earlier one, here
+        const size_t e = last - 1;
+        const Lowered& E = *ops[e];
         Cx c = mul(coef(E), coef(L));
         const double len = std::hypot(c.re, c.im);
         c = snapped(Cx{c.re / len, c.im / len}, 0x1p-52);  // one product
@@ -910,18 +986,20 @@ std::vector<const Lowered*> cancel_phases(const std::vector<const Lowered*>& seg
         if (gone) F.op.mask = F.diag = 0;  // the identity, kept for its gate count
         // an H before the earlier phase sees the joined one instead
         for (uint64_t t = L.op.mask; t; t &= t - 1) {
-          auto& list = since[__builtin_ctzll(t)];
-          list.erase(std::remove(list.begin(), list.end(), it->second), list.end());
+          const int q = __builtin_ctzll(t);
+          if (h[q] == SIZE_MAX) continue;
+          auto& list = since[q];
+          list.erase(std::remove(list.begin(), list.end(), e), list.end());
           if (!gone) list.push_back(i);
         }
-        ops[it->second] = nullptr;
+        ops[e] = nullptr;
         ops[i] = &F;
-        if (gone) phase.erase(it);
-        else it->second = i;
+        last = gone ? 0 : i + 1;
         continue;
       }
-      phase[L.op.mask] = i;
-      for (uint64_t t = L.op.mask; t; t &= t - 1) since[__builtin_ctzll(t)].push_back(i);
+      last = i + 1;
+      for (uint64_t t = L.op.mask; t; t &= t - 1)
+        if (h[__builtin_ctzll(t)] != SIZE_MAX) since[__builtin_ctzll(t)].push_back(i);
       continue;
     }
     const int q = touched ? __builtin_ctzll(touched) : 0;
@@ -942,7 +1020,6 @@ std::vector<const Lowered*> cancel_phases(const std::vector<const Lowered*>& seg
       F.op.ctrl = F.diag = others;
       F.nondiag = touched;
       ops[h[q]] = ops[i] = nullptr;
-      phase.erase(N.op.mask);
       for (uint64_t t = others; t; t &= t - 1) h[__builtin_ctzll(t)] = SIZE_MAX;  // the flip is gone from their runs
       ops[at] = &F;
       h[q] = SIZE_MAX;
@@ -953,8 +1030,7 @@ std::vector<const Lowered*> cancel_phases(const std::vector<const Lowered*>& seg
         since[q].clear();
       }
     }
-    if (L.nondiag)
-      for (auto it = phase.begin(); it != phase.end();) it = it->first & L.nondiag ? phase.erase(it) : std::next(it);
+    for (uint64_t t = L.nondiag; t; t &= t - 1) moved[__builtin_ctzll(t)] = i + 1;
   }
   ops.erase(std::remove(ops.begin(), ops.end(), nullptr), ops.end());
   return ops;
@@ -966,23 +1042,56 @@ std::vector<const Lowered*> fuse_pairs(const std::vector<const Lowered*>& seg, s
                                        int barrier_cost = 0) {
   const int min_cost = barrier_cost ? 17 + barrier_cost : kFuseMinCost;
   auto gate_cost = [&](const Lowered& L) { return tile_cost(L) + (L.nondiag ? barrier_cost : 0); };
+  // Lists (a block's members, the gates waiting on a qubit) are links in one
+  // array: no allocation for each.
+  struct Link {
+    size_t at;  // an index in seg (members) or in out (waiting)
+    int next;
+  };
+  struct List {
+    int head = -1, tail = -1;
+  };
+  std::vector<Link> links;
+  links.reserve(2 * seg.size());
+  auto append = [&](List& l, size_t at) {
+    links.push_back(Link{at, -1});
+    const int k = (int)links.size() - 1;
+    if (l.tail >= 0) links[(size_t)l.tail].next = k;
+    else l.head = k;
+    l.tail = k;
+  };
   struct Block {
     uint32_t a, b;
     Cx m[16];
-    std::vector<const Lowered*> members;
+    List members;
     int cost = 0;
-    uint32_t record = 0;
+    uint32_t record = 0, gates = 0;
   };
   std::vector<const Lowered*> out;
   out.reserve(seg.size());
-  std::vector<std::vector<size_t>> waiting(kMaxQubits);  // out indices of one-qubit gates waiting per qubit
-  std::vector<int> open(kMaxQubits, -1);
+  List waiting[kMaxQubits];  // one-qubit gates waiting per qubit
+  int open[kMaxQubits];
+  std::fill(open, open + kMaxQubits, -1);
   std::vector<Block> blocks;
+  blocks.reserve(seg.size() / 3 + 1);
+  auto member = [&](Block& B, const Lowered* L, size_t at) {
+    fold_into_4x4(*L, B.a, B.b, B.m);
+    append(B.members, at);
+    B.cost += gate_cost(*L);
+    B.gates += gates_of(*L);
+  };
+  std::vector<size_t> source;  // per op of out: its index in seg
+  source.reserve(seg.size());
+  auto emit = [&](const Lowered* L, size_t at) {
+    out.push_back(L);
+    source.push_back(at);
+  };
   auto close = [&](uint32_t q) {
     const int k = open[q];
     if (k < 0) return;
     Block& B = blocks[(size_t)k];
     open[B.a] = open[B.b] = -1;
+    waiting[B.a] = waiting[B.b] = List();
     if (B.cost >= min_cost) {
       store.emplace_back();
       Lowered& F = store.back();
@@ -995,91 +1104,75 @@ std::vector<const Lowered*> fuse_pairs(const std::vector<const Lowered*>& seg, s
       F.nondiag = (1ull << B.a) | (1ull << B.b);
       F.diag = 0;
       F.record = B.record;
-      F.gates = 0;
-      for (const Lowered* L : B.members) F.gates += gates_of(*L);
-      out.push_back(&F);
-      waiting[B.a].clear();
-      waiting[B.b].clear();
+      F.gates = B.gates;
+      emit(&F, 0);
       return;
     }
     // not worth a 4x4: the gates go out as they came; the one-qubit gates
     // after the block's last two-qubit gate wait again on their qubits
-    size_t last2 = 0;
-    for (size_t i = 0; i < B.members.size(); ++i)
-      if (__builtin_popcountll(B.members[i]->nondiag | B.members[i]->diag) == 2) last2 = i;
-    waiting[B.a].clear();
-    waiting[B.b].clear();
-    for (size_t i = 0; i < B.members.size(); ++i) {
-      out.push_back(B.members[i]);
-      if (i > last2) {
-        const uint64_t t = B.members[i]->nondiag | B.members[i]->diag;
-        waiting[(uint32_t)__builtin_ctzll(t)].push_back(out.size() - 1);
-      }
+    int last2 = -1;
+    for (int i = B.members.head; i >= 0; i = links[(size_t)i].next) {
+      const Lowered* L = seg[links[(size_t)i].at];
+      if (__builtin_popcountll(L->nondiag | L->diag) == 2) last2 = i;
+    }
+    bool behind = false;
+    for (int i = B.members.head; i >= 0; i = links[(size_t)i].next) {
+      const size_t at = links[(size_t)i].at;
+      emit(seg[at], at);
+      if (behind) append(waiting[__builtin_ctzll(seg[at]->nondiag | seg[at]->diag)], out.size() - 1);
+      behind = behind || i == last2;
     }
   };
-  for (const Lowered* L : seg) {
+  for (size_t at = 0; at < seg.size(); ++at) {
+    const Lowered* L = seg[at];
     const uint64_t touched = L->nondiag | L->diag;
     const int width = __builtin_popcountll(touched);
     if (fusable_type(*L) && width == 1) {
       const uint32_t q = (uint32_t)__builtin_ctzll(touched);
-      const int k = open[q];
-      if (k >= 0) {
-        Block& B = blocks[(size_t)k];
-        fold_into_4x4(*L, B.a, B.b, B.m);
-        B.members.push_back(L);
-        B.cost += gate_cost(*L);
+      if (open[q] >= 0) {
+        member(blocks[(size_t)open[q]], L, at);
       } else {
-        out.push_back(L);
-        waiting[q].push_back(out.size() - 1);
+        emit(L, at);
+        append(waiting[q], out.size() - 1);
       }
       continue;
     }
     if (fusable_type(*L) && width == 2) {
       const uint32_t lo = (uint32_t)__builtin_ctzll(touched), hi = 63u - (uint32_t)__builtin_clzll(touched);
       if (open[lo] >= 0 && open[lo] == open[hi]) {  // another gate on the same pair
-        Block& B = blocks[(size_t)open[lo]];
-        fold_into_4x4(*L, B.a, B.b, B.m);
-        B.members.push_back(L);
-        B.cost += gate_cost(*L);
+        member(blocks[(size_t)open[lo]], L, at);
         continue;
       }
       close(lo);
       close(hi);
-      Block B;
+      blocks.emplace_back();
+      Block& B = blocks.back();
       B.a = hi;
       B.b = lo;
       for (int i = 0; i < 16; ++i) B.m[i] = Cx{(i % 5) == 0 ? 1.0 : 0.0, 0.0};
       B.record = L->record;
       for (uint32_t q : {hi, lo}) {
-        for (size_t idx : waiting[q]) {
-          const Lowered* W = out[idx];
-          fold_into_4x4(*W, B.a, B.b, B.m);
-          B.members.push_back(W);
-          B.cost += gate_cost(*W);
-          out[idx] = nullptr;
+        for (int i = waiting[q].head; i >= 0; i = links[(size_t)i].next) {
+          const size_t o = links[(size_t)i].at;
+          member(B, out[o], source[o]);
+          out[o] = nullptr;
         }
-        waiting[q].clear();
+        waiting[q] = List();
       }
-      fold_into_4x4(*L, B.a, B.b, B.m);
-      B.members.push_back(L);
-      B.cost += gate_cost(*L);
-      blocks.push_back(std::move(B));
+      member(B, L, at);
       open[hi] = open[lo] = (int)blocks.size() - 1;
       continue;
     }
-    for (uint32_t q = 0; q < kMaxQubits; ++q)
-      if ((touched >> q) & 1) {
-        close(q);
-        waiting[q].clear();
-      }
-    out.push_back(L);
+    for (uint64_t t = touched; t; t &= t - 1) {
+      const uint32_t q = (uint32_t)__builtin_ctzll(t);
+      close(q);
+      waiting[q] = List();
+    }
+    emit(L, at);
   }
   for (uint32_t q = 0; q < kMaxQubits; ++q) close(q);
-  std::vector<const Lowered*> compact;
-  compact.reserve(out.size());
-  for (const Lowered* L : out)
-    if (L) compact.push_back(L);
-  return compact;
+  out.erase(std::remove(out.begin(), out.end(), nullptr), out.end());
+  return out;
 }
 
 // Shared-memory passes: after pair fusion, two dense one-qubit gates in a row
@@ -1261,49 +1354,79 @@ int plan_segment_tiles(const std::vector<const Lowered*>& seg, uint32_t n, uint3
 struct WideTake {
   uint64_t set = 0;
   std::vector<const Lowered*> take, rest;
-  double score = 0.0;  // arithmetic taken, older ops counting more (see BlockTake)
 };
 
 double wide_weight(const Lowered& L) {  // arithmetic, and a little for every op's own overhead
   return 2.0 + tile_cost(L);
 }
 
-void wide_take(const std::vector<const Lowered*>& pending, uint64_t have, uint32_t room, uint32_t base, WideTake* out) {
+// What the choice of a set needs of an op.
+struct WideOp {
+  uint64_t nondiag, diag;
+  double score;  // arithmetic, older ops counting more (see BlockTake); 0 for diagonal ops
+  bool joins;    // not a k-qubit unitary, which has a pass of its own
+};
+
+// The score and the set of one choice. `all`: the qubits of the ops; once every one
+// of them is blocked no further op can score.
+double wide_score(const std::vector<WideOp>& ops, uint64_t have, uint32_t room, uint64_t all, uint64_t* out) {
   uint64_t set = have, blocked_full = 0, blocked_diag = 0;
-  for (const Lowered* L : pending) {
-    bool ok = L->op.type != OP_KQ && !(L->nondiag & (blocked_full | blocked_diag)) && !(L->diag & blocked_full);
-    const uint64_t need = L->nondiag & ~set;
-    const uint32_t count = (uint32_t)__builtin_popcountll(need);
-    if (ok && count > room) ok = false;
-    if (ok) {
+  double score = 0.0;
+  for (const WideOp& o : ops) {
+    const uint64_t need = o.nondiag & ~set;
+    if (o.joins && !(o.nondiag & (blocked_full | blocked_diag)) && !(o.diag & blocked_full) &&
+        (!need || (uint32_t)__builtin_popcountll(need) <= room)) {
       set |= need;
-      room -= count;
-      out->take.push_back(L);
-      if (L->nondiag) out->score += wide_weight(*L) / (1.0 + (L->record > base ? (double)(L->record - base) / 256.0 : 0.0));
+      room -= (uint32_t)__builtin_popcountll(need);
+      score += o.score;
     } else {
-      blocked_full |= L->nondiag;
-      blocked_diag |= L->diag;
-      out->rest.push_back(L);
+      blocked_full |= o.nondiag;
+      blocked_diag |= o.diag;
+      if (blocked_full == all) break;
     }
   }
-  out->set = set;
+  *out = set;
+  return score;
 }
 
 // The best of the first-come set and of every window of consecutive qubits
 // (on a brickwall the windows follow the light cone).
 WideTake wide_best(const std::vector<const Lowered*>& pending, uint64_t have, uint32_t room, const uint8_t* qubits,
-                   uint32_t nq) {
+                   uint32_t nq, std::vector<WideOp>& ops) {
   const uint32_t base = pending.front()->record;
-  WideTake best;
-  wide_take(pending, have, room, base, &best);
-  for (uint32_t a = 0; a + room <= nq; ++a) {
-    uint64_t window = have;
-    for (uint32_t k = 0; k < room; ++k) window |= 1ull << qubits[a + k];
-    WideTake c;
-    wide_take(pending, window, 0, base, &c);
-    if (c.score > best.score) best = std::move(c);
+  uint64_t all = 0;
+  ops.clear();
+  for (const Lowered* L : pending) {
+    const double age = L->record > base ? (double)(L->record - base) : 0.0;
+    ops.push_back(WideOp{L->nondiag, L->diag, L->nondiag ? wide_weight(*L) / (1.0 + age / 256.0) : 0.0,
+                         L->op.type != OP_KQ});
+    all |= L->nondiag | L->diag;
   }
-  return best;
+  uint64_t set = 0;
+  double best = wide_score(ops, have, room, all, &set);
+  for (uint32_t a = 0; a + room <= nq; ++a) {
+    uint64_t window = have, s;
+    for (uint32_t k = 0; k < room; ++k) window |= 1ull << qubits[a + k];
+    const double score = wide_score(ops, window, 0, all, &s);
+    if (score > best) {
+      best = score;
+      set = s;
+    }
+  }
+  WideTake T;
+  T.set = set;
+  uint64_t blocked_full = 0, blocked_diag = 0;
+  for (const Lowered* L : pending) {
+    if (L->op.type != OP_KQ && !(L->nondiag & (blocked_full | blocked_diag)) && !(L->diag & blocked_full) &&
+        !(L->nondiag & ~set)) {
+      T.take.push_back(L);
+    } else {
+      blocked_full |= L->nondiag;
+      blocked_diag |= L->diag;
+      T.rest.push_back(L);
+    }
+  }
+  return T;
 }
 
 // Appends the ops of one phase, `reg_of[q]` the register bit of qubit q (255:
@@ -1328,14 +1451,13 @@ void emit_wide_phase(const std::vector<const Lowered*>& ops, const uint8_t* reg_
   std::vector<Group> groups;
   std::vector<Item> items;
   uint64_t after = 0;  // qubits acted on non-diagonally after the last group
+  uint64_t in_regs = 0;
+  for (uint32_t q = 0; q < n; ++q)
+    if (reg_of[q] != 255) in_regs |= 1ull << q;
   auto split = [&](uint64_t m, uint64_t* rest, uint32_t* regs) {
-    *rest = m;
+    *rest = m & ~in_regs;
     *regs = 0;
-    for (uint32_t q = 0; q < n; ++q)
-      if (((m >> q) & 1) && reg_of[q] != 255) {
-        *regs |= 1u << reg_of[q];
-        *rest &= ~(1ull << q);
-      }
+    for (uint64_t t = m & in_regs; t; t &= t - 1) *regs |= 1u << reg_of[__builtin_ctzll(t)];
   };
   for (const Lowered* L : ops) {
     uint64_t rest = 0;
@@ -1446,6 +1568,7 @@ void emit_wide_phase(const std::vector<const Lowered*>& ops, const uint8_t* reg_
 // R: register qubits of a phase, 4 or 5.
 int plan_segment_wide(const std::vector<const Lowered*>& seg, uint32_t n, bool f64, uint32_t tile_r, uint32_t R, Plan* P) {
   std::vector<const Lowered*> pending = seg;
+  std::vector<WideOp> scored;  // wide_best's, kept between its calls
   uint8_t all[kMaxQubits];
   for (uint32_t q = 0; q < n; ++q) all[q] = (uint8_t)q;
   while (!pending.empty()) {
@@ -1455,7 +1578,7 @@ int plan_segment_wide(const std::vector<const Lowered*>& seg, uint32_t n, bool f
       pending.erase(pending.begin());
       continue;
     }
-    WideTake T = wide_best(pending, 0xFull, kWideBits - 4, all + 4, n - 4);
+    WideTake T = wide_best(pending, 0xFull, kWideBits - 4, all + 4, n - 4, scored);
     if (T.take.empty()) return ALEPH_B200_OPTIMIZATION;
     // the tile: the chosen qubits, padded with the lowest unused ones
     uint64_t set = T.set;
@@ -1505,7 +1628,7 @@ int plan_segment_wide(const std::vector<const Lowered*>& seg, uint32_t n, bool f
     const uint32_t kIoRegs = ((1u << W.R) - 1) << (kWideBits - W.R);  // the top tile bits: lanes take bits 0..4
     bool first = true;
     while (!left.empty()) {
-      WideTake F = wide_best(left, 0, W.R, tile, kWideBits);
+      WideTake F = wide_best(left, 0, W.R, tile, kWideBits, scored);
       if (F.take.empty()) return ALEPH_B200_OPTIMIZATION;
       uint32_t regs = 0;
       for (uint32_t b = 0; b < kWideBits; ++b)
@@ -1551,8 +1674,7 @@ void apply_local(const Lowered& L, const uint32_t* bq, Cx* s) {
   };
   auto lmask = [&](uint64_t m) -> uint32_t {
     uint32_t r = 0;
-    for (uint32_t q = 0; q < 64; ++q)
-      if ((m >> q) & 1) r |= 1u << lbit(q);
+    for (; m; m &= m - 1) r |= 1u << lbit((uint32_t)__builtin_ctzll(m));
     return r;
   };
   auto gidx = [&](uint32_t x) -> uint64_t {
