@@ -1,0 +1,51 @@
+"""The routes of sampling against the oracle's sequential builds, exactly: states of
+one CTA, states whose chain runs step by step (half of the basis at one
+probability: every sum lies on a binade's edge), and tables of many groups."""
+import numpy as np
+import pytest
+
+from aleph_b200.backend import B200SvBackend
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def state(kind, n, rng):
+    size = 1 << n
+    psi = np.zeros(size, dtype=np.complex128)
+    if kind == "half":
+        psi[rng.permutation(size)[: max(1, size // 2)]] = 1.0
+    elif kind == "one":
+        psi[int(rng.integers(0, size))] = 1j
+    elif kind == "uniform":
+        psi += 1.0
+    elif kind == "scrambled":
+        psi = rng.standard_normal(size) + 1j * rng.standard_normal(size)
+    elif kind == "product":
+        psi = np.ones(1, dtype=np.complex128)
+        for th in rng.uniform(0.2, np.pi - 0.2, n):
+            psi = np.kron(np.array([np.cos(th / 2), 1j * np.sin(th / 2)]), psi)
+    return psi / np.linalg.norm(psi)
+
+
+def on_device(kind, n, precision, seed):
+    be = B200SvBackend(seed=0, precision=precision)
+    st = be.allocate(n)
+    be.set_statevector(st, state(kind, n, np.random.default_rng(seed)))
+    return be, st, be.statevector(st)  # the state as the device holds it
+
+
+def check_alias(be, st, psi):
+    prob, alias = oracle.alias_table(psi.real * psi.real + psi.imag * psi.imag)
+    edge = np.clip(np.floor(prob * 2.0 ** 32), 0, 2 ** 32 - 1).astype(np.uint64)
+    idx = np.arange(psi.size, dtype=np.uint64) << np.uint64(32)
+    words = np.concatenate([idx | np.uint64(0xFFFFFFFF), idx | edge, idx | (edge - (edge > 0).astype(np.uint64))])
+    got = be.sample(st, words.size, variates=words, mode="alias")
+    i, v = (words >> np.uint64(32)).astype(np.int64), (words & np.uint64(0xFFFFFFFF)).astype(np.float64) / 2.0 ** 32
+    assert np.array_equal(got, np.where(v < prob[i], i, alias[i].astype(np.int64)).astype(np.uint64))
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("kind,n", [("half", 11), ("half", 13), ("half", 17), ("scrambled", 20), ("product", 20)])
+def test_alias_tables_of_long_chains(kind, n, precision):
+    check_alias(*on_device(kind, n, precision, n))
