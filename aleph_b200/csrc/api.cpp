@@ -1568,9 +1568,11 @@ int aleph_b200_sample(aleph_b200_handle* h, aleph_b200_state* st, uint32_t shots
   CK(cudaMemsetAsync(dstatus, 0, 64, h->stream), "status clear");
   CK(cudaMemsetAsync(base, 0, sb, h->stream), "scratch clear");
   CK(copy_async(h, dvar, variates, vb, cudaMemcpyHostToDevice, h->stream), "variates upload");
-  CK(launch_sample(st->amps, st->precision, st->n, shots, mode, dvar, dout, base, sb, dstatus, h->sm_count, h->stream),
+  uint32_t launches = 0;
+  CK(launch_sample(st->amps, st->precision, st->n, shots, mode, dvar, dout, base, sb, dstatus, h->sm_count, &launches,
+                   h->stream),
      "sample");
-  h->stats.kernel_launches += mode == ALEPH_B200_SAMPLE_ALIAS ? 12 : 11;
+  h->stats.kernel_launches += launches;
   int32_t status[4];
   CK(copy_async(h, status, dstatus, 16, cudaMemcpyDeviceToHost, h->stream), "status readback");
   CK(copy_async(h, out, dout, vb, cudaMemcpyDeviceToHost, h->stream), "sample readback");
@@ -1647,10 +1649,11 @@ int aleph_b200_sample_cumulative_noalloc(aleph_b200_handle* h, aleph_b200_state*
   CK(cudaMemsetAsync(dstatus, 0, 64, h->stream), "status clear");
   CK(cudaMemsetAsync(base, 0, sb, h->stream), "scratch clear");
   if (shots) CK(copy_async(h, dvar, variates, vb, cudaMemcpyHostToDevice, h->stream), "variates upload");
+  uint32_t launches = 0;
   CK(launch_sample(st->amps, st->precision, st->n, shots, ALEPH_B200_SAMPLE_CUMULATIVE, dvar, dout, base, sb, dstatus,
-                   h->sm_count, h->stream),
+                   h->sm_count, &launches, h->stream),
      "sample");
-  h->stats.kernel_launches += shots ? 11 : 5;
+  h->stats.kernel_launches += launches;
   int32_t status[4];
   CK(copy_async(h, status, dstatus, 16, cudaMemcpyDeviceToHost, h->stream), "status readback");
   if (shots) CK(copy_async(h, out, dout, vb, cudaMemcpyDeviceToHost, h->stream), "sample readback");

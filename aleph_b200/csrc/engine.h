@@ -374,9 +374,10 @@ double dfma_per_launch(uint32_t blocks, uint32_t iters);
 // exact sequential prefix sum up to this n; the count goes to status[2].
 constexpr uint32_t kExactCumulativeMaxN = 28;
 size_t sample_scratch_bytes(uint32_t n, int mode, uint32_t shots);
+// *launches: the kernels launched.
 cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t shots, int mode, const void* variates_dev,
                           uint64_t* out_dev, void* scratch, size_t scratch_bytes, int32_t* status, int sm_count,
-                          cudaStream_t s);
+                          uint32_t* launches, cudaStream_t s);
 // Fixed device buffer of aleph_b200_sample_cumulative_noalloc: a file-scope
 // __device__ array of this many bytes; its address is looked up with
 // cudaGetSymbolAddress, with the target device current.

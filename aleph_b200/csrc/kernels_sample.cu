@@ -153,6 +153,11 @@ __device__ __forceinline__ uint32_t block_scan_u32(uint32_t v, uint32_t* tot) {
   return block_scan_1024<uint32_t>(v, tot, [](uint32_t x, int o) { return __shfl_up_sync(0xffffffffu, x, o); });
 }
 
+// Norm check of validate_state (sampling.rs:36-57): sets status on failure.
+__device__ __forceinline__ void check_norm(double total, double bad, double tol, int32_t* status) {
+  if (bad > 0.0 || !isfinite(total) || fabs(total - 1.0) > tol) status[0] = ALEPH_B200_INVALID_STATE;
+}
+
 // Thread t of block b takes element b * PART_B + (PART_B - 1 - t): ascending
 // threads are the pop order (stacks are filled in ascending index order).
 __device__ __forceinline__ uint64_t part_element() { return (uint64_t)blockIdx.x * PART_B + (PART_B - 1 - threadIdx.x); }
@@ -217,11 +222,11 @@ __global__ void __launch_bounds__(PART_B) alias_scale_kernel(const V2<Real>* __r
 }
 
 // What pops before each block (blocks pop from the last to the first): counts
-// of smalls, deficits and surpluses; the totals and the norm. One CTA; a
-// thread takes a contiguous range of blocks. (One thread for all of them was
+// of smalls, deficits and surpluses; the totals and the norm with its check. One
+// CTA; a thread takes a contiguous range of blocks. (One thread for all of them was
 // 0.7 ms at n = 22.)
 __global__ void __launch_bounds__(1024) alias_offsets_kernel(AliasScratch s, uint64_t len, uint32_t nblocks,
-                                                             double* norm_out) {
+                                                             double tol, int32_t* status) {
   __shared__ u128 tot[32];
   __shared__ uint32_t tot32[32];
   __shared__ double red[2][32];
@@ -276,8 +281,7 @@ __global__ void __launch_bounds__(1024) alias_offsets_kernel(AliasScratch s, uin
       a += red[0][w];
       b += red[1][w];
     }
-    norm_out[0] = a;
-    norm_out[1] = b;
+    check_norm(a, b, tol, status);
   }
 }
 
@@ -723,12 +727,100 @@ __global__ void alias_draw_kernel(AliasScratch s, uint64_t mask, const uint64_t*
   }
 }
 
-// Norm check of validate_state (sampling.rs:36-57): sets status on failure.
-__global__ void check_norm_kernel(const double* norm2, double tol, int32_t* status) {
-  if (threadIdx.x != 0) return;
-  const double total = norm2[0];
-  if (norm2[1] > 0.0 || !isfinite(total) || fabs(total - 1.0) > tol)
-    status[0] = ALEPH_B200_INVALID_STATE;
+// States of at most PART_B amplitudes: the whole build and the draws in one kernel, the
+// table in shared memory. The chain is short (some 40 ns a step), and the launches
+// of the parallel build alone cost more. Each CTA builds the table for its share of the shots.
+template <typename Real>
+__global__ void __launch_bounds__(PART_B) alias_small_kernel(const V2<Real>* __restrict__ amps, uint32_t len,
+                                                             const uint64_t* __restrict__ words, uint32_t shots,
+                                                             uint64_t* __restrict__ out, double tol, int32_t* status) {
+  __shared__ double prob[PART_B], sv[PART_B + 2], lv[PART_B + 2];
+  __shared__ uint16_t alias[PART_B], si[PART_B + 2], li[PART_B + 2];
+  __shared__ uint32_t smalls[32];
+  __shared__ double red[2][32];
+  __shared__ uint32_t m_sh, ok_sh;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5, warps = blockDim.x >> 5;
+  const bool valid = tid < len;
+  const uint32_t i0 = valid ? len - 1 - tid : 0;  // pop order: descending basis states
+  double sc = 0.0, psum = 0.0, bad = 0.0;
+  if (valid) {
+    const double p = prob_exact<Real>(amps, i0);
+    if (isfinite(p)) psum = p;
+    else bad = 1.0;
+    sc = __dmul_rn((double)len, p);
+    prob[i0] = 1.0;  // what is never popped keeps itself
+    alias[i0] = (uint16_t)i0;
+  }
+  const unsigned bs = __ballot_sync(0xffffffffu, valid && sc < 1.0);
+  for (int o = 16; o; o >>= 1) {
+    psum += __shfl_down_sync(0xffffffffu, psum, o);
+    bad += __shfl_down_sync(0xffffffffu, bad, o);
+  }
+  if (lane == 0) {
+    smalls[w] = __popc(bs);
+    red[0][w] = psum;
+    red[1][w] = bad;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    uint32_t m = 0;
+    double a = 0.0, b = 0.0;
+    for (uint32_t x = 0; x < warps; ++x) {
+      const uint32_t c = smalls[x];
+      smalls[x] = m;
+      m += c;
+      a += red[0][x];
+      b += red[1][x];
+    }
+    m_sh = m;
+    ok_sh = !(b > 0.0) && isfinite(a) && fabs(a - 1.0) <= tol;
+    check_norm(a, b, tol, status);
+  }
+  __syncthreads();
+  if (!ok_sh) return;
+  if (valid) {
+    const uint32_t before = smalls[w] + __popc(bs & ((1u << lane) - 1u));  // smalls popped before this element
+    if (sc < 1.0) {
+      sv[before] = sc;
+      si[before] = (uint16_t)i0;
+    } else {
+      lv[tid - before] = sc;
+      li[tid - before] = (uint16_t)i0;
+    }
+  }
+  __syncthreads();
+  const uint32_t m = m_sh, k = len - m;
+  if (tid == 0 && m && k) {  // see raw_steps
+    uint32_t i = 0, j = 0, cs = si[0], cs1 = si[1], cl = li[0], cl1 = li[1], cl2 = li[2];
+    double V = lv[0], va = sv[0], va1 = sv[1], vb = lv[1], vb1 = lv[2];
+    for (;;) {
+      const bool t = V >= 1.0;
+      if (t ? i >= m : j + 1 >= k) break;
+      const double Sa = __dadd_rn(V, va), Sb = __dadd_rn(V, vb);
+      const uint32_t at = t ? cs : cl;
+      prob[at] = t ? va : V;
+      alias[at] = (uint16_t)(t ? cl : cl1);
+      i += t ? 1u : 0u;
+      j += t ? 0u : 1u;
+      va = t ? va1 : va;
+      cs = t ? cs1 : cs;
+      vb = t ? vb : vb1;
+      cl = t ? cl : cl1;
+      cl1 = t ? cl1 : cl2;
+      va1 = sv[i + 1];  // i <= m, j < k: inside the arrays
+      cs1 = si[i + 1];
+      vb1 = lv[j + 2];
+      cl2 = li[j + 2];
+      V = __dsub_rn(t ? Sa : Sb, 1.0);
+    }
+  }
+  __syncthreads();
+  for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + tid; x < shots; x += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t bits = words[x];
+    const uint32_t i = (uint32_t)(bits >> 32) & (len - 1);
+    const double u = (double)(uint32_t)bits * (1.0 / 4294967296.0);
+    out[x] = u < prob[i] ? i : alias[i];
+  }
 }
 
 // ------------------------------------------------------------- CUMULATIVE ----
@@ -767,7 +859,7 @@ constexpr double kSeqMin = 0x1p-500;  // smaller sums (zero among them) are adde
 
 struct CumScratch {
   double* bsum;      // nb + 1: block sums, then exclusive block prefix (bsum[nb] = total)
-  double* norm;      // 2: [total, non-finite count]
+  double* norm;      // 2: [unused, non-finite count]
   uint32_t* namb;    // ambiguous shot count
   uint32_t* amb;     // shots: ambiguous shot ids
   double* ck;        // exact mode: sequential sum at the end of every SEQ_CH chunk
@@ -832,21 +924,25 @@ __global__ void __launch_bounds__(RANGE_T) cum_range_kernel(CumScratch c, uint32
   for (uint32_t b = b0; b < b1; ++b) s += c.bsum[b];
   c.part[t] = s;
 }
-__global__ void __launch_bounds__(PREFIX_T) cum_prefix_kernel(CumScratch c, uint32_t nb) {
+// ONE: up to PREFIX_T blocks, a block per range: this kernel alone does it (three
+// kernels took 8 us more from small states).
+template <bool ONE>
+__global__ void __launch_bounds__(PREFIX_T) cum_prefix_kernel(CumScratch c, uint32_t nb, double tol, int32_t* status) {
   __shared__ double part[PREFIX_T];
   const uint32_t t = threadIdx.x;
-  part[t] = c.part[t];
+  part[t] = !ONE ? c.part[t] : t < nb ? c.bsum[t] : 0.0;
   __syncthreads();
-  for (uint32_t off = 1; off < PREFIX_T; off <<= 1) {  // inclusive Hillis-Steele scan
+  for (uint32_t off = 1; off < blockDim.x; off <<= 1) {  // inclusive Hillis-Steele scan
     const double v = t >= off ? part[t - off] : 0.0;
     __syncthreads();
     part[t] += v;
     __syncthreads();
   }
-  c.part[t] = part[t];
-  if (t == PREFIX_T - 1) {
-    c.bsum[nb] = part[PREFIX_T - 1];
-    c.norm[0] = part[PREFIX_T - 1];
+  if (!ONE) c.part[t] = part[t];
+  else if (t < nb) c.bsum[t] = t ? part[t - 1] : 0.0;
+  if (t == blockDim.x - 1) {
+    c.bsum[nb] = part[t];
+    check_norm(part[t], c.norm[1], tol, status);
   }
 }
 __global__ void __launch_bounds__(RANGE_T) cum_spread_kernel(CumScratch c, uint32_t nb) {
@@ -1123,8 +1219,21 @@ __global__ void __launch_bounds__(WALK_T) cum_walk_kernel(const V2<Real>* __rest
   if (*c.namb == 0) return;
   const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
   const uint32_t per = (nch + WALK_T - 1) / WALK_T;
-  sfn[t] = c.sfn[t];
-  se[t] = c.sfe[t];
+  if (nch == 1) {  // one chunk, scanned by the whole CTA: no functions were formed
+    if (t == 0) c.fe[0] = kNoBinade;
+    const uint64_t i = 2 * t;
+    const bool p0 = i < len && prob_exact<Real>(amps, i) > 0.0, p1 = i + 1 < len && prob_exact<Real>(amps, i + 1) > 0.0;
+    if (p0 || p1) atomicMax((unsigned long long*)&c.seq[1], (unsigned long long)(i + (p1 ? 2 : 1)));  // 1 + index
+    se[t] = kNoBinade;
+  } else if (per == 1) {  // a chunk per segment: nothing was composed
+    if (t < nch) {
+      sfn[t] = c.fn[t];
+      se[t] = c.fe[t];
+    }
+  } else {
+    sfn[t] = c.sfn[t];
+    se[t] = c.sfe[t];
+  }
   if (t == 0) {
     S_sh = 0.0;
     seg_sh = 0;
@@ -1138,7 +1247,8 @@ __global__ void __launch_bounds__(WALK_T) cum_walk_kernel(const V2<Real>* __rest
       for (; g < nseg; ++g) {
         const SeqSum at = S;
         if (!seq_step(&S, se[g], sfn[g])) break;
-        c.sstart[g] = S_sh > 0.0 ? seq_value(at) : 0.0;
+        if (per == 1) c.ck[g] = S_sh > 0.0 ? seq_value(S) : 0.0;
+        else c.sstart[g] = S_sh > 0.0 ? seq_value(at) : 0.0;
       }
       if (S_sh > 0.0) S_sh = seq_value(S);
       seg_sh = g;
@@ -1317,9 +1427,8 @@ struct Carver {
   }
 };
 
-// The alias table's scratch (40 bytes per amplitude and 1.3 more for the
-// chunks); *norm2 receives the norm's two words.
-AliasScratch alias_scratch(Carver& c, uint32_t n, double** norm2) {
+// The alias table's scratch (40 bytes per amplitude and 1.3 more for the chunks).
+AliasScratch alias_scratch(Carver& c, uint32_t n) {
   const uint64_t len = 1ull << n;
   const uint64_t nb = (len + PART_B - 1) / PART_B;
   const uint64_t nc = alias_chunks(len), ng = (nc + CGROUP - 1) / CGROUP;
@@ -1334,7 +1443,6 @@ AliasScratch alias_scratch(Carver& c, uint32_t n, double** norm2) {
   s.bsur = c.take<u128>(nb);
   s.normsum = c.take<double>(2 * nb);
   s.totals = c.take<uint32_t>(4);
-  *norm2 = c.take<double>(2);
   s.ci = c.take<uint32_t>(nc + 1);
   s.cj = c.take<uint32_t>(nc + 1);
   s.cbase = c.take<double>(nc + 1);
@@ -1355,9 +1463,9 @@ AliasScratch alias_scratch(Carver& c, uint32_t n, double** norm2) {
 size_t sample_scratch_bytes(uint32_t n, int mode, uint32_t shots) {
   const uint64_t len = 1ull << n;
   if (mode == ALEPH_B200_SAMPLE_ALIAS) {
+    if (len <= PART_B) return 256;
     Carver c{nullptr};
-    double* norm2;
-    alias_scratch(c, n, &norm2);
+    alias_scratch(c, n);
     return c.off + 256;
   }
   const uint64_t nb = (len + CUM_BLOCK - 1) / CUM_BLOCK;
@@ -1371,20 +1479,30 @@ static inline char* align_up(char* p, size_t a) {
 
 cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t shots, int mode, const void* variates,
                           uint64_t* out, void* scratch, size_t scratch_bytes, int32_t* status, int sm_count,
-                          cudaStream_t st) {
+                          uint32_t* launches, cudaStream_t st) {
   const uint64_t len = 1ull << n;
   const bool f64 = precision == ALEPH_B200_F64;
+  const double tol = norm_tolerance(len, precision);
+  if (mode == ALEPH_B200_SAMPLE_ALIAS && len <= PART_B) {
+    const unsigned threads = len < 32 ? 32u : (unsigned)len;
+    const unsigned want = shots / 4096 + 1, grid = want < (unsigned)sm_count ? want : (unsigned)sm_count;
+    const uint64_t* words = (const uint64_t*)variates;
+    if (f64)
+      alias_small_kernel<double><<<grid, threads, 0, st>>>((const double2*)amps, (uint32_t)len, words, shots, out, tol, status);
+    else
+      alias_small_kernel<float><<<grid, threads, 0, st>>>((const float2*)amps, (uint32_t)len, words, shots, out, tol, status);
+    *launches = 1;
+    return cudaGetLastError();
+  }
   if (mode == ALEPH_B200_SAMPLE_ALIAS) {
     const uint32_t nb = (uint32_t)((len + PART_B - 1) / PART_B);
     const uint32_t nc = alias_chunks(len), ng = (nc + CGROUP - 1) / CGROUP;
     Carver c{(char*)scratch};
-    double* norm2;
-    const AliasScratch s = alias_scratch(c, n, &norm2);
+    const AliasScratch s = alias_scratch(c, n);
     if (c.off > scratch_bytes) return cudaErrorInvalidValue;
     if (f64) alias_scale_kernel<double><<<nb, PART_B, 0, st>>>((const double2*)amps, len, s);
     else alias_scale_kernel<float><<<nb, PART_B, 0, st>>>((const float2*)amps, len, s);
-    alias_offsets_kernel<<<1, 1024, 0, st>>>(s, len, nb, norm2);
-    check_norm_kernel<<<1, 32, 0, st>>>(norm2, norm_tolerance(len, precision), status);
+    alias_offsets_kernel<<<1, 1024, 0, st>>>(s, len, nb, tol, status);
     alias_partition_kernel<<<nb, PART_B, 0, st>>>(len, s, status);
     if (nc) {
       alias_cuts_kernel<<<nc / 4 + 1, 128, 0, st>>>(s, nc, status);
@@ -1399,6 +1517,7 @@ cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t 
     alias_drain_kernel<<<(unsigned)sm_count * 4, 256, 0, st>>>(s, status);
     if (shots)
       alias_draw_kernel<<<(shots + 255) / 256, 256, 0, st>>>(s, len - 1, (const uint64_t*)variates, shots, out, status);
+    *launches = (nc ? 10 : 5) + (shots ? 1 : 0);
     return cudaGetLastError();
   }
   char* p = (char*)scratch;
@@ -1423,10 +1542,17 @@ cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t 
   cudaMemsetAsync(c.norm, 0, 48, st);  // norm, namb, seq
   if (f64) cum_blocks_kernel<double><<<nb, 256, 0, st>>>((const double2*)amps, len, c);
   else cum_blocks_kernel<float><<<nb, 256, 0, st>>>((const float2*)amps, len, c);
-  cum_range_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nb);
-  cum_prefix_kernel<<<1, PREFIX_T, 0, st>>>(c, nb);
-  cum_spread_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nb);
-  check_norm_kernel<<<1, 32, 0, st>>>(c.norm, norm_tolerance(len, precision), status);
+  if (nb <= PREFIX_T) {
+    uint32_t threads = 32;
+    while (threads < nb) threads *= 2;
+    cum_prefix_kernel<true><<<1, threads, 0, st>>>(c, nb, tol, status);
+    *launches = 2;
+  } else {
+    cum_range_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nb);
+    cum_prefix_kernel<false><<<1, PREFIX_T, 0, st>>>(c, nb, tol, status);
+    cum_spread_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nb);
+    *launches = 4;
+  }
   if (shots) {
     const unsigned wb = (shots + 3) / 4;  // a warp per shot
     const double* u = (const double*)variates;
@@ -1434,20 +1560,19 @@ cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t 
     else cum_draw_kernel<float><<<wb, 128, 0, st>>>((const float2*)amps, len, nb, c, u, shots, out);
     // status[2]: the shots inside the guard band (re-resolved below when n <= EXACT_MAX_N)
     cudaMemcpyAsync(status + 2, c.namb, 4, cudaMemcpyDeviceToDevice, st);
+    *launches += 1;
     if (n <= EXACT_MAX_N) {
-      if (f64) {
-        cum_fn_kernel<double><<<nch, 256, 0, st>>>((const double2*)amps, len, c);
-        cum_compose_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nch);
-        cum_walk_kernel<double><<<1, WALK_T, 0, st>>>((const double2*)amps, len, nch, c);
-        cum_expand_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nch);
-        cum_exact_kernel<double><<<wb, 128, 0, st>>>((const double2*)amps, len, c, u, out, status);
-      } else {
-        cum_fn_kernel<float><<<nch, 256, 0, st>>>((const float2*)amps, len, c);
-        cum_compose_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nch);
-        cum_walk_kernel<float><<<1, WALK_T, 0, st>>>((const float2*)amps, len, nch, c);
-        cum_expand_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nch);
-        cum_exact_kernel<float><<<wb, 128, 0, st>>>((const float2*)amps, len, c, u, out, status);
-      }
+      // one chunk needs no function, and up to a segment each need no composition
+      const bool fn = nch > 1, compose = nch > PREFIX_T;
+      if (fn && f64) cum_fn_kernel<double><<<nch, 256, 0, st>>>((const double2*)amps, len, c);
+      else if (fn) cum_fn_kernel<float><<<nch, 256, 0, st>>>((const float2*)amps, len, c);
+      if (compose) cum_compose_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nch);
+      if (f64) cum_walk_kernel<double><<<1, WALK_T, 0, st>>>((const double2*)amps, len, nch, c);
+      else cum_walk_kernel<float><<<1, WALK_T, 0, st>>>((const float2*)amps, len, nch, c);
+      if (compose) cum_expand_kernel<<<PREFIX_T / RANGE_T, RANGE_T, 0, st>>>(c, nch);
+      if (f64) cum_exact_kernel<double><<<wb, 128, 0, st>>>((const double2*)amps, len, c, u, out, status);
+      else cum_exact_kernel<float><<<wb, 128, 0, st>>>((const float2*)amps, len, c, u, out, status);
+      *launches += 2 + (fn ? 1 : 0) + (compose ? 2 : 0);
     }
   }
   return cudaGetLastError();
