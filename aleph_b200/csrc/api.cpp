@@ -1558,9 +1558,17 @@ int aleph_b200_sample(aleph_b200_handle* h, aleph_b200_state* st, uint32_t shots
     return set_error(h, ALEPH_B200_INVALID_ARGUMENT, "alias sampling supports n <= 28; use CUMULATIVE");
   if (int r = bind(h)) return r;
   if (shots == 0) return check_norm_host(h, st, nullptr);
-  const size_t sb = sample_scratch_bytes(st->n, mode, shots);
+  size_t sb = sample_scratch_bytes(st->n, mode, shots);
   const size_t vb = (size_t)shots * 8;
-  if (int r = ensure(h, h->sample, al(sb) + 2 * al(vb) + 256)) return r;
+  int r = ensure(h, h->sample, al(sb) + 2 * al(vb) + 256);
+  if (r && mode == ALEPH_B200_SAMPLE_ALIAS) {
+    // beside resident states that leave no room for the parallel build: the
+    // table step by step, in 16 bytes per amplitude instead of 41
+    cudaGetLastError();
+    sb = sample_scratch_bytes(st->n, mode, shots, true);
+    r = ensure(h, h->sample, al(sb) + 2 * al(vb) + 256);
+  }
+  if (r) return r;
   char* base = (char*)h->sample.ptr;
   void* dvar = base + al(sb);
   uint64_t* dout = (uint64_t*)(base + al(sb) + al(vb));

@@ -373,7 +373,8 @@ double dfma_per_launch(uint32_t blocks, uint32_t iters);
 // CUMULATIVE: shots in the rounding guard band are re-resolved against the
 // exact sequential prefix sum up to this n; the count goes to status[2].
 constexpr uint32_t kExactCumulativeMaxN = 28;
-size_t sample_scratch_bytes(uint32_t n, int mode, uint32_t shots);
+// least: the fewest bytes that will do (an alias table built step by step).
+size_t sample_scratch_bytes(uint32_t n, int mode, uint32_t shots, bool least = false);
 // *launches: the kernels launched.
 cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t shots, int mode, const void* variates_dev,
                           uint64_t* out_dev, void* scratch, size_t scratch_bytes, int32_t* status, int sm_count,

@@ -76,8 +76,8 @@ using u128 = unsigned __int128;
 struct AliasScratch {
   double* prob;       // N: scaled probabilities, then the table thresholds
   uint32_t* alias;    // N
-  double* val;        // N: scaled values in pop order, the m smalls, then the k larges
-  uint32_t* idx;      // N: their basis states
+  uint32_t* idx;      // N: basis states in pop order, the m smalls, then the k larges
+  double* val;        // N: their scaled values (null: step by step only, see sample_scratch_bytes)
   u128* pre;          // N: D_i of small i (deficits before it), E_j of large j (surpluses up to it)
   // per partition block: smalls, deficits, surpluses (then what pops before the block), norm partials
   uint32_t* bcount;
@@ -308,8 +308,9 @@ __global__ void __launch_bounds__(PART_B) alias_partition_kernel(uint64_t len, A
   uint64_t at;
   if (small) at = sb + rank - 1;
   else at = m + (popped - sb) + (threadIdx.x - pad - rank);
-  s.val[at] = sc;
   s.idx[at] = (uint32_t)i;
+  if (!s.val) return;
+  s.val[at] = sc;
   s.pre[at] = small ? s.bdef[blockIdx.x] + di - d : s.bsur[blockIdx.x] + ei;
 }
 
@@ -508,8 +509,13 @@ __device__ bool raw_steps(const AliasScratch& s, uint32_t m, uint32_t k, RawShar
     if (V >= 1.0 ? i >= m : j + 1 >= k) return false;
     if (steps == 0) return true;
     const uint32_t ns = min(RAW, m - i), nl = min(RAW, k - 1 - j);
-    for (uint32_t x = lane; x < ns; x += 32) sh.a[x] = s.val[i + x];
-    for (uint32_t x = lane; x < nl; x += 32) sh.b[x] = s.val[(uint64_t)m + j + 1 + x];
+    if (s.val) {
+      for (uint32_t x = lane; x < ns; x += 32) sh.a[x] = s.val[i + x];
+      for (uint32_t x = lane; x < nl; x += 32) sh.b[x] = s.val[(uint64_t)m + j + 1 + x];
+    } else {  // no values in pop order: what has not been popped still has its value in the table
+      for (uint32_t x = lane; x < ns; x += 32) sh.a[x] = s.prob[s.idx[i + x]];
+      for (uint32_t x = lane; x < nl; x += 32) sh.b[x] = s.prob[s.idx[(uint64_t)m + j + 1 + x]];
+    }
     __syncwarp();
     uint32_t is = 0, n = 0;
     if (lane == 0) {
@@ -576,7 +582,7 @@ __global__ void __launch_bounds__(32) alias_walk_kernel(AliasScratch s, uint32_t
   const int lane = threadIdx.x;
   const uint32_t m = s.totals[0], k = s.totals[1];
   if (status[0] != 0 || m == 0 || k == 0) return;
-  double V = s.val[m];
+  double V = s.val ? s.val[m] : s.prob[s.idx[m]];
   uint32_t i = 0, j = 0;
   bool more = true;
   // records [r0, r1) of chunks (per = 1) or groups (per = CGROUP): staged in shared memory
@@ -1427,22 +1433,24 @@ struct Carver {
   }
 };
 
-// The alias table's scratch (40 bytes per amplitude and 1.3 more for the chunks).
-AliasScratch alias_scratch(Carver& c, uint32_t n) {
+// The alias table's scratch: 41.3 bytes per amplitude, or 16 without the values,
+// prefixes and chunks of the parallel build (the chain then runs step by step).
+AliasScratch alias_scratch(Carver& c, uint32_t n, bool parallel) {
   const uint64_t len = 1ull << n;
   const uint64_t nb = (len + PART_B - 1) / PART_B;
   const uint64_t nc = alias_chunks(len), ng = (nc + CGROUP - 1) / CGROUP;
-  AliasScratch s;
+  AliasScratch s{};
   s.prob = c.take<double>(len);
   s.alias = c.take<uint32_t>(len);
-  s.val = c.take<double>(len);
   s.idx = c.take<uint32_t>(len);
-  s.pre = c.take<u128>(len);
   s.bcount = c.take<uint32_t>(nb);
   s.bdef = c.take<u128>(nb);
   s.bsur = c.take<u128>(nb);
   s.normsum = c.take<double>(2 * nb);
   s.totals = c.take<uint32_t>(4);
+  if (!parallel) return s;
+  s.val = c.take<double>(len);
+  s.pre = c.take<u128>(len);
   s.ci = c.take<uint32_t>(nc + 1);
   s.cj = c.take<uint32_t>(nc + 1);
   s.cbase = c.take<double>(nc + 1);
@@ -1460,12 +1468,12 @@ AliasScratch alias_scratch(Carver& c, uint32_t n) {
 }
 }  // namespace
 
-size_t sample_scratch_bytes(uint32_t n, int mode, uint32_t shots) {
+size_t sample_scratch_bytes(uint32_t n, int mode, uint32_t shots, bool least) {
   const uint64_t len = 1ull << n;
   if (mode == ALEPH_B200_SAMPLE_ALIAS) {
     if (len <= PART_B) return 256;
     Carver c{nullptr};
-    alias_scratch(c, n);
+    alias_scratch(c, n, !least);
     return c.off + 256;
   }
   const uint64_t nb = (len + CUM_BLOCK - 1) / CUM_BLOCK;
@@ -1496,9 +1504,10 @@ cudaError_t launch_sample(const void* amps, int precision, uint32_t n, uint32_t 
   }
   if (mode == ALEPH_B200_SAMPLE_ALIAS) {
     const uint32_t nb = (uint32_t)((len + PART_B - 1) / PART_B);
-    const uint32_t nc = alias_chunks(len), ng = (nc + CGROUP - 1) / CGROUP;
+    const bool parallel = scratch_bytes >= sample_scratch_bytes(n, mode, shots, false);
+    const uint32_t nc = parallel ? alias_chunks(len) : 0, ng = (nc + CGROUP - 1) / CGROUP;
     Carver c{(char*)scratch};
-    const AliasScratch s = alias_scratch(c, n);
+    const AliasScratch s = alias_scratch(c, n, parallel);
     if (c.off > scratch_bytes) return cudaErrorInvalidValue;
     if (f64) alias_scale_kernel<double><<<nb, PART_B, 0, st>>>((const double2*)amps, len, s);
     else alias_scale_kernel<float><<<nb, PART_B, 0, st>>>((const float2*)amps, len, s);
