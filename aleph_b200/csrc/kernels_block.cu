@@ -327,8 +327,7 @@ __global__ void __launch_bounds__(blk::THREADS, 1) block_kernel(const __grid_con
   __shared__ uint64_t fold_cmask[MAX_POST];
   __shared__ int8_t fold_rbit[MAX_POST], fold_col[MAX_POST];
   __shared__ float2 fold_c0[MAX_POST], fold_c1[MAX_POST];
-  __shared__ Op post_ops[MAX_POST];
-  __shared__ int8_t other_ops[MAX_POST];  // indices in post_ops
+  __shared__ Op post_ops[MAX_POST];  // all of them, then those of neither class, moved to the front
   __shared__ int n_neg_sh, n_other_sh, n_fold_sh;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -413,9 +412,9 @@ __global__ void __launch_bounds__(blk::THREADS, 1) block_kernel(const __grid_con
           fold_col[k] = corner ? (int8_t)-1 : (int8_t)op.q[0];
           fold_c0[k] = a.coef[op.coef];
           fold_c1[k] = a.coef[op.coef + (corner ? 0 : 1)];
-        } else if (other) {
-          other_ops[no + __popc(bo & below)] = (int8_t)o;
         }
+        __syncwarp();  // every lane holds its op; the slots up to this group's are free
+        if (other) post_ops[no + __popc(bo & below)] = op;
         nn += __popc(bn);
         nf += __popc(bf);
         no += __popc(bo);
@@ -641,7 +640,7 @@ __global__ void __launch_bounds__(blk::THREADS, 1) block_kernel(const __grid_con
                 for (int r = 0; r < 8; ++r) {
                   float2 y = eo[r * 32 + lane];
                   const uint64_t g = a.grow[j0 + r];
-                  for (int o = 0; o < n_other; ++o) y = apply_diag_op<float>(post_ops[other_ops[o]], y, gc | g, a.coef, a.poly);
+                  for (int o = 0; o < n_other; ++o) y = apply_diag_op<float>(post_ops[o], y, gc | g, a.coef, a.poly);
                   __stcs(pc + g, y);
                 }
               }
