@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import ctypes as ct
 from dataclasses import dataclass
-from itertools import chain
+from itertools import accumulate, chain
 from operator import index
 
 import numpy as np
@@ -352,23 +352,11 @@ class B200SvBackend:
         if gam.shape != bet.shape:
             raise ValueError("gammas and betas must have the same shape")
         p = gam.shape[1]
-        # whole columns at once: a 384-graph batch holds some 12,000 edges
-        lens = [len(edges) for _, edges in graphs]
-        sets = np.zeros(max(1, count), dtype=np.dtype(abi.QaoaSet))
-        sets["num_qubits"][:count] = [index(nq) & 0xFFFFFFFF for nq, _ in graphs]
-        sets["num_edges"][:count] = lens
-        sets["edge_offset"][:count] = np.cumsum([0] + lens[:-1]) if count else 0
-        pairs = list(chain.from_iterable(edges for _, edges in graphs))
-        if set(map(len, pairs)) - {2}:
-            raise ValueError("an edge is a pair of qubits")
-        ends = np.fromiter(chain.from_iterable(pairs), dtype=np.int64, count=2 * len(pairs))
-        if ends.size and (ends.min() < 0 or ends.max() > 0xFFFFFFFF):
-            raise OverflowError("an edge's qubit is out of range")
-        edges_arr = ends.astype(np.uint32)
+        sets_ptr, edges_arr = _stage_graphs(graphs)
         ang = np.ascontiguousarray(np.concatenate([gam, bet], axis=1))
         out = np.zeros(max(1, count), dtype=np.float64)
         self._check(self.lib.aleph_b200_qaoa_sweep(
-            self.handle, p, sets.ctypes.data_as(ct.POINTER(abi.QaoaSet)), count,
+            self.handle, p, sets_ptr, count,
             edges_arr.ctypes.data_as(ct.POINTER(ct.c_uint32)) if edges_arr.size else None,
             edges_arr.size // 2, ang.ctypes.data_as(ct.POINTER(ct.c_double)), out.ctypes.data_as(ct.POINTER(ct.c_double))))
         return out[:count]
@@ -387,6 +375,35 @@ def _record_dict(r) -> dict:
     return {"kind": abi.PASS_KINDS.get(r.kind, r.kind), "gates": r.gates, "n": r.n, "qubits": list(r.qubits[: r.nq]),
             "post_ops": r.post_ops, "lane_ops": r.lane_ops, "dense_ops": r.dense_ops, "diag_ops": r.diag_ops,
             "variant": r.variant, "fma_per_amp": r.fma_per_amp, "ms": r.ms, "bytes": r.bytes}
+
+
+def _stage_graphs(graphs):
+    """A sweep's graphs as the C ABI takes them: the sets, and all edges' qubits in a row."""
+    count = len(graphs)
+    if count <= 4:  # a few graphs: the array calls below take longer than a loop
+        few = (abi.QaoaSet * max(1, count))()
+        pool = []
+        for k, (nq, edges) in enumerate(graphs):
+            few[k].num_qubits, few[k].num_edges, few[k].edge_offset = nq, len(edges), len(pool) // 2
+            for (i, j) in edges:
+                pool += [int(i), int(j)]
+        return few, np.asarray(pool, dtype=np.uint32)
+    # whole columns at once: a 384-graph batch holds some 12,000 edges
+    lens = [len(edges) for _, edges in graphs]
+    sets = np.zeros(count, dtype=_QAOA_SET)
+    sets["num_qubits"] = [index(nq) & 0xFFFFFFFF for nq, _ in graphs]
+    sets["num_edges"] = lens
+    sets["edge_offset"] = [0, *accumulate(lens[:-1])]
+    pairs = list(chain.from_iterable(edges for _, edges in graphs))
+    if set(map(len, pairs)) - {2}:
+        raise ValueError("an edge is a pair of qubits")
+    ends = np.fromiter(chain.from_iterable(pairs), dtype=np.int64, count=2 * len(pairs))
+    if ends.size and (ends.min() < 0 or ends.max() > 0xFFFFFFFF):
+        raise OverflowError("an edge's qubit is out of range")
+    return sets.ctypes.data_as(ct.POINTER(abi.QaoaSet)), ends.astype(np.uint32)
+
+
+_QAOA_SET = np.dtype(abi.QaoaSet)
 
 
 class CompiledPlan:
