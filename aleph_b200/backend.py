@@ -395,7 +395,12 @@ def _stage_graphs(graphs):
     sets["num_edges"] = lens
     sets["edge_offset"] = [0, *accumulate(lens[:-1])]
     pairs = list(chain.from_iterable(edges for _, edges in graphs))
-    if set(map(len, pairs)) - {2}:
+    try:
+        widths = set(map(len, pairs))
+    except TypeError:  # pairs that can only be iterated
+        pairs = [tuple(e) for e in pairs]
+        widths = set(map(len, pairs))
+    if widths - {2}:
         raise ValueError("an edge is a pair of qubits")
     ends = np.fromiter(chain.from_iterable(pairs), dtype=np.int64, count=2 * len(pairs))
     if ends.size and (ends.min() < 0 or ends.max() > 0xFFFFFFFF):

@@ -44,3 +44,9 @@ def test_staged_graphs_are_a_plain_loops(count):
 def test_edges_that_are_no_pairs_of_qubits_are_refused(edge, error, count):
     with pytest.raises(error):
         _stage_graphs([(4, [(0, 1), edge])] * count)
+
+
+@pytest.mark.parametrize("count", [1, 6])
+def test_edges_may_be_any_iterables_of_two(count):
+    sets, edges = _stage_graphs([(4, [iter((0, 1)), map(int, "23")]) for _ in range(count)])
+    assert edges.tolist() == [0, 1, 2, 3] * count
