@@ -1884,20 +1884,22 @@ int aleph_b200_probabilities(aleph_b200_handle* h, aleph_b200_state* st, const u
   const size_t dim = (size_t)1 << k;
   if (int r = ensure_reduce(h, probabilities_scratch_bytes(st->n, qubits, k, h->sm_count) + 256)) return r;
   if (int r = ensure(h, h->sample, dim * 8 + 256)) return r;
-  double* dnorm = (double*)h->sample.ptr;  // the norm's two sums, then the marginal
-  double* dout = dnorm + 2;
+  double* dout = (double*)h->sample.ptr;  // the marginal, then the norm's two sums
+  double* dnorm = dout + dim;
   CK(launch_probabilities(st->amps, st->precision, st->n, qubits, k, reduce_area(h), dout, dnorm, h->sm_count,
                           h->stream),
      "probabilities");
   h->stats.kernel_launches += 2;
-  // a small marginal comes back with the norm in one copy
-  const size_t head = dim <= 4096 ? dim + 2 : 2;
-  std::vector<double> host(head);
-  CK(copy_async(h, host.data(), dnorm, head * 8, cudaMemcpyDeviceToHost, h->stream), "probabilities readback");
+  // a small marginal comes back with the norm in one copy; a large one by itself, from
+  // the buffer's start (copied from 16 bytes on it took 1.1 ms longer at 2^22 outcomes)
+  const bool together = dim <= 4096;
+  std::vector<double> host(together ? dim + 2 : 2);
+  CK(copy_async(h, host.data(), together ? dout : dnorm, host.size() * 8, cudaMemcpyDeviceToHost, h->stream),
+     "probabilities readback");
   CK(cudaStreamSynchronize(h->stream), "stream synchronize");
-  if (int r = check_norm(h, st, host.data())) return r;
-  if (head > 2) {
-    std::memcpy(out, host.data() + 2, dim * 8);
+  if (int r = check_norm(h, st, host.data() + (together ? dim : 0))) return r;
+  if (together) {
+    std::memcpy(out, host.data(), dim * 8);
     return ALEPH_B200_OK;
   }
   CK(copy_async(h, out, dout, dim * 8, cudaMemcpyDeviceToHost, h->stream), "probabilities readback");

@@ -420,8 +420,33 @@ struct Marginal {
   uint32_t k, lane_sel;  // selected count; mask of the selected lane qubits
   uint32_t lanes;        // active lanes (32, or 2^n below 5 qubits)
   uint32_t pat_bits, split_bits;
-  uint64_t pat_mask, split_mask, loop_mask;  // qubits above 4: selected / split / added in the loop
+  uint64_t split_mask, loop_mask;  // qubits above 4: split / added in the loop
   uint64_t loops;
+  // Index bits move in runs of consecutive ones (bit by bit, the moves of a marginal
+  // over all qubits took longer than its loads): pattern -> selected qubits above 4, and
+  // those qubits -> the outcome's bits.
+  struct Runs {
+    uint32_t count;
+    uint8_t from[40], to[40];
+    uint64_t mask[40];
+    __device__ __forceinline__ uint64_t operator()(uint64_t x) const {
+      uint64_t r = 0;
+      for (uint32_t k = 0; k < count; ++k) r |= ((x >> from[k]) & mask[k]) << to[k];
+      return r;
+    }
+    void add(uint32_t a, uint32_t b) {  // bit a goes to bit b; extends the last run where it can
+      if (count) {
+        const uint32_t len = (uint32_t)__builtin_popcountll(mask[count - 1]);
+        if (from[count - 1] + len == a && to[count - 1] + len == b) {
+          mask[count - 1] = mask[count - 1] << 1 | 1;
+          return;
+        }
+      }
+      from[count] = (uint8_t)a;
+      to[count] = (uint8_t)b;
+      mask[count++] = 1;
+    }
+  } place, outcome;
   uint8_t qubits[64];
 };
 
@@ -453,7 +478,7 @@ __global__ void __launch_bounds__(RB) marginal_kernel(const V2<Real>* __restrict
     const uint64_t id = item * (RB / 32) + w;
     double s = 0.0;
     const uint64_t pat = id >> m.split_bits, split = id & ((1ull << m.split_bits) - 1);
-    const uint64_t fixed = deposit(pat, m.pat_mask);
+    const uint64_t fixed = m.place(pat);
     if (id < warps && on) {
       const V2<Real>* base = amps + (fixed | deposit(split, m.split_mask) | lane);
       uint64_t x = 0;
@@ -499,10 +524,7 @@ __global__ void __launch_bounds__(RB) marginal_kernel(const V2<Real>* __restrict
       table = split >> 3;
     }
     if (writes) {
-      uint64_t o = o_lane;
-      for (uint32_t t = 0; t < m.k; ++t)
-        if (m.qubits[t] >= 5) o |= ((fixed >> m.qubits[t]) & 1) << t;
-      tables[(table << m.k) + o] = s;
+      tables[(table << m.k) + (o_lane | m.outcome(fixed))] = s;
     }
   }
   __syncthreads();
@@ -539,8 +561,10 @@ MarginalPlan plan_marginal(uint32_t n, const uint32_t* qubits, uint32_t k, int s
   }
   m.lane_sel = (uint32_t)(sel & 31u) | (n < 5 ? 31u & ~((1u << n) - 1) : 0u);  // absent lane qubits: nothing to add
   const uint64_t high = n > 5 ? ((1ull << n) - 1) & ~31ull : 0ull;
-  m.pat_mask = sel & high;
-  m.pat_bits = (uint32_t)__builtin_popcountll(m.pat_mask);
+  for (uint32_t q = 5; q < n; ++q)
+    if ((sel >> q) & 1) m.place.add(m.pat_bits++, q);
+  for (uint32_t t = 0; t < k; ++t)
+    if (qubits[t] >= 5) m.outcome.add(qubits[t], t);
   uint64_t rest = high & ~sel;
   const uint32_t rest_bits = (uint32_t)__builtin_popcountll(rest);
   // about 2^13 warps: 55 per SM, a little under what an SM holds
