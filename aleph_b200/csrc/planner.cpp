@@ -1662,6 +1662,73 @@ int plan_segment_wide(const std::vector<const Lowered*>& seg, uint32_t n, bool f
   return ALEPH_B200_OK;
 }
 
+// ---- warp or wide tiles for a short list ----------------------------------------------
+// A list of a few gates often fits one pass of either kind, and then a wide tile
+// has nothing to save: it pays an exchange for every further set of register
+// qubits (two for one gate on a low qubit), a warp tile pays shuffles on the lane
+// qubits only. Both are planned and the cheaper one by this table is taken.
+// The table: milliseconds per 2^27 amplitudes, least squares over 1700 measured
+// passes (single families of 1 to 40 gates, n = 16..27; 5 to 10% rms). Up to
+// n = 21 a pass is one wave or less and its latency counts, above that its
+// throughput. Measured with the choice against wide tiles alone: FP64 n = 24, one H
+// on qubit 0 161 -> 118 us, 4 U3 163 -> 121 us; n = 27, 4 H 1.13 -> 0.85 ms; FP32
+// n = 24, 4 controlled rotations and Toffolis 0.78 of the time.
+// Gates: in FP32 longer lists save passes with wide tiles; in FP64 lists of one-qubit gates
+// alone may not (n = 27, 120 U3: 0.93 of the speed), and beyond its limit planning
+// twice costs more than the choice gives.
+constexpr size_t kShortList[2] = {64, 512};
+constexpr double kWideLead = 1.06;  // wide tiles are taken where the table has them ahead by its error
+struct TileCosts {
+  double pass, x, x_lane, one, one_real, one_lane, two, two_real, two_lane, two_lanes, controlled, sign, phase, group,
+      member, table, exchange;
+};
+double tiles_ms(const Plan& P, size_t pass0, bool f64, uint32_t n) {
+  static const TileCosts costs[2][2][2] = {
+      // FP32: n < 22 (warp, wide), n >= 22
+      {{{1.05, .060, .100, .115, .115, .135, .335, .335, .380, .470, .070, .040, .200, .0, .0, .400, .0},
+        {1.05, .050, .0, .086, .071, .0, .152, .100, .0, .0, .055, .040, .200, .250, .05, .390, .140}},
+       {{.310, .026, .044, .047, .047, .068, .140, .140, .190, .200, .010, .020, .080, .0, .0, .212, .0},
+        {.285, .026, .0, .034, .023, .0, .098, .050, .0, .0, .027, .020, .080, .095, .015, .196, .076}}},
+      // FP64
+      {{{1.30, .070, .110, .130, .130, .170, .290, .290, .460, .780, .150, .050, .265, .0, .0, .400, .0},
+        {1.30, .068, .0, .146, .086, .0, .218, .120, .0, .0, .030, .050, .265, .280, .05, .405, .150}},
+       {{.600, .044, .071, .070, .070, .150, .140, .140, .320, .530, .030, .030, .115, .0, .0, .310, .0},
+        {.600, .044, .0, .088, .073, .0, .155, .090, .0, .0, .017, .030, .115, .190, .02, .312, .136}}}};
+  double ms = 0.0;
+  // a wide pass's launch takes the host some 2 us longer
+  if (pass0 < P.passes.size() && P.passes[pass0].kind == PASS_WIDE) ms += .002 * (double)(1u << (27 - std::min(27u, std::max(n, 20u))));
+  for (size_t k = pass0; k < P.passes.size(); ++k) {
+    const Pass& ps = P.passes[k];
+    if (ps.kind != PASS_TILE && ps.kind != PASS_WIDE) continue;  // k-qubit unitaries: the same in both
+    const bool wide = ps.kind == PASS_WIDE;
+    const TileCosts& c = costs[f64][n >= 22][wide];
+    ms += c.pass + (wide ? (ps.wide.phase_count - 1) * c.exchange : 0.0);
+    const uint32_t begin = wide ? ps.wide.op_begin : ps.tile.op_begin, count = wide ? ps.wide.op_count : ps.tile.op_count;
+    for (uint32_t i = begin; i < begin + count; ++i) {
+      const Op& op = P.ops[i];
+      const int lanes = wide ? 0 : (op.a < 5) + (op.type == OP_2Q && op.b < 5);
+      const bool real = wide && op.dsrc == WIDE_REAL;
+      switch (op.type) {
+        case OP_X: ms += lanes ? c.x_lane : c.x; break;
+        case OP_1Q: ms += (lanes ? c.one_lane : real ? c.one_real : c.one) + (op.ctrl || op.creg ? c.controlled : 0.0); break;
+        case OP_2Q: ms += lanes == 2 ? c.two_lanes : lanes ? c.two_lane : real ? c.two_real : c.two; break;
+        case OP_NEG: ms += c.sign; break;
+        case OP_SIGNS:
+          ms += c.sign;
+          i += op.aux;
+          break;
+        case OP_CPHASE: ms += c.phase; break;
+        case OP_PHASES:
+          ms += c.group + op.aux * c.member;
+          i += op.aux;
+          break;
+        default: ms += c.table; break;
+      }
+    }
+  }
+  return ms;
+}
+
 // ---- tensor-core dense blocks ------------------------------------------------
 // Apply a lowered op to a vector over the block qubits bq[0..6) (index bit b
 // <-> qubit bq[b]); the op's qubits must all be block qubits, except for the
@@ -1964,7 +2031,7 @@ int build_plan(const std::vector<Lowered>& ops, uint32_t n, bool f64, const Plan
       ps.tile.n = n;
       ps.tile.op_begin = (uint32_t)P->ops.size();
       std::deque<Lowered> fused;
-      const std::vector<const Lowered*> list = o.pair_fusion ? fuse_for_smem(diagonal_cores(seg, fused, true), fused) : seg;
+      const std::vector<const Lowered*> list = o.pair_fusion && seg.size() > 1 ? fuse_for_smem(diagonal_cores(seg, fused, true), fused) : seg;
       for (const Lowered* L : list) {
         Op op = L->op;
         if ((op.type == OP_1Q || op.type == OP_2Q) && real_matrix(*L)) op.dsrc = WIDE_REAL;
@@ -1991,8 +2058,26 @@ int build_plan(const std::vector<Lowered>& ops, uint32_t n, bool f64, const Plan
         // relabel_swaps off) compare the parts of the warp-tile planner, and a state
         // smaller than one wide tile has no choice.
         const bool wide = n >= kWideBits && o.relabel_swaps && ((o.tile_r == 5 && o.tile_occupancy == 0) || o.tile_r == 4);
-        status = wide ? plan_segment_wide(fuse_pairs(cancel_phases(diagonal_cores(seg, fused), fused), fused), n, f64, R, o.tile_r == 4 ? 4 : 5, P)
-                      : plan_segment_tiles(fuse_pairs(seg, fused), n, R, P);
+        auto plan_wide = [&](Plan* to) {
+          return plan_segment_wide(fuse_pairs(cancel_phases(diagonal_cores(seg, fused), fused), fused), n, f64, R,
+                                   o.tile_r == 4 ? 4 : 5, to);
+        };
+        auto plan_warp = [&](Plan* to) { return plan_segment_tiles(fuse_pairs(seg, fused), n, R, to); };
+        if (wide && o.tile_r == 5 && seg.size() == 1 && seg[0]->op.type != OP_2Q) {
+          status = plan_warp(P);  // the table's answer, without the second plan
+        } else if (wide && o.tile_r == 5 && seg.size() <= kShortList[f64]) {
+          Plan W, T;
+          W.renormalize = T.renormalize = P->renormalize;
+          status = plan_wide(&W);
+          if (!status) status = plan_warp(&T);
+          if (!status) {
+            const bool warp = tiles_ms(T, 0, f64, n) <= kWideLead * tiles_ms(W, 0, f64, n);
+            if (P->passes.empty()) *P = std::move(warp ? T : W);
+            else status = warp ? plan_warp(P) : plan_wide(P);
+          }
+        } else {
+          status = wide ? plan_wide(P) : plan_warp(P);
+        }
       } else {
         status = plan_segment_tiles(seg, n, R, P);
       }
