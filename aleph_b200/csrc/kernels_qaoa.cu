@@ -23,10 +23,11 @@
 // A tile is a contiguous chunk; a B tile spans the high qubits and the lowest
 // c = 26 - n ones.
 //
-// In a tile, bits 8..12 are mixed in registers and bits 0..4 by lane shuffles
-// (layout 1), one trip through shared memory brings bits 5..7 into registers
-// (layout 2), where the cost phase is applied and the next layer's part starts,
-// and a second trip brings bits 8..12 back.
+// In a tile, the top bits are mixed in registers and bits 0..4 by lane shuffles
+// (layout 1), one trip through shared memory brings the bits between (5..7 in FP32,
+// 5..8 in FP64) into registers (layout 2), where the cost phase is applied and the
+// next layer's part starts, and a second trip brings the top bits back. The first
+// pass goes the same way from a constant tile with nothing to finish.
 //
 // cut(z) of a tile amplitude i: T[i] (edges inside the tile's qubits, a table per
 // set and tile kind, built once by prep_kernel) + edges among the tile's fixed
@@ -41,9 +42,14 @@
 // those are held by CTAs that already run, so the queue cannot lock up; every
 // wait is bounded all the same.
 //
-// Measured (384 FP32 sets, n = 12..22, p = 4): one CTA per set with 2p passes took
-// 39 ms, most of it the last n = 22 sets on one CTA each; the queue with p + 1
-// passes takes 10.1 ms, host staging included.
+// Measured (n = 12..22, p = 4): one CTA per set with 2p passes took 39 ms for 384
+// FP32 sets, most of it the last n = 22 sets on one CTA each; the queue with p + 1
+// passes takes 10.9 ms, host staging included. FP64: 35.6 and 19.4 ms. 1024 FP64 sets
+// of n = 12..24, which kept the former kernel busy to the end: 177 ms; 207 with the
+// queue on 8 warps, 195 with 16, 189 with the next tile fetched ahead, 160 with the
+// first pass on the common way (its own form held both results of every register and
+// spilled; a third of the shared-memory pipe's work was spills). That pipe is what
+// bounds FP64 then: shuffles of 16-byte amplitudes and two trips per tile.
 
 #include "common.cuh"
 
@@ -51,7 +57,7 @@ namespace ab {
 
 namespace qaoa {
 
-constexpr int THREADS = 256;
+constexpr int PREP_THREADS = 256;
 constexpr int TILE_BITS = 13;
 constexpr uint32_t TILE = 1u << TILE_BITS;
 constexpr int MAX_EDGES = 128;
@@ -61,6 +67,9 @@ struct Cfg {
   // FP32 tiles (64 KiB) leave room for two CTAs per SM, which overlap one
   // CTA's tile loads with the other's arithmetic
   static constexpr int CTAS_PER_SM = sizeof(Real) == 4 ? 2 : 1;
+  // FP64: 16 warps on the one 128 KiB tile, 16 amplitudes a thread
+  static constexpr int WARP_BITS = sizeof(Real) == 4 ? 3 : 4;
+  static constexpr int THREADS = 32 << WARP_BITS;
 };
 
 // Per streamed set and tile kind (0: A, 1: B): the neighbour masks in bit planes.
@@ -91,7 +100,7 @@ struct Args {
 // Rx(2 beta) on tile-local bit k of every pair in S[0..len): (a, b) -> (c a - i s b, c b - i s a).
 template <typename Real>
 __device__ __forceinline__ void mixer_bit(V2<Real>* S, uint32_t len, uint32_t k, Real c, Real s) {
-  for (uint32_t i = threadIdx.x; i < len / 2; i += THREADS) {
+  for (uint32_t i = threadIdx.x; i < len / 2; i += Cfg<Real>::THREADS) {
     const uint32_t j0 = (uint32_t)insert_zero(i, k), j1 = j0 | (1u << k);
     const V2<Real> a = S[j0], b = S[j1];
     S[j0] = mk<Real>(c * a.x + s * b.y, c * a.y - s * b.x);
@@ -108,7 +117,7 @@ __device__ __forceinline__ void mixer_bits2(V2<Real>* S, uint32_t len, uint32_t 
     a = mk<Real>(c * x.x + s * y.y, c * x.y - s * y.x);
     b = mk<Real>(c * y.x + s * x.y, c * y.y - s * x.x);
   };
-  for (uint32_t i = threadIdx.x; i < len / 4; i += THREADS) {
+  for (uint32_t i = threadIdx.x; i < len / 4; i += Cfg<Real>::THREADS) {
     const uint32_t e00 = (uint32_t)insert_zero(insert_zero(i, k0), k1);
     const uint32_t e01 = e00 | (1u << k0), e10 = e00 | (1u << k1), e11 = e01 | (1u << k1);
     V2<Real> a00 = S[e00], a01 = S[e01], a10 = S[e10], a11 = S[e11];
@@ -139,10 +148,8 @@ __device__ __forceinline__ void mixer_range(V2<Real>* S, uint32_t len, uint32_t 
 }
 
 // Streamed tiles are swept in registers. Register layout: tile index
-// i = tid | r << 8 (lane = tile bits 0..4, warp = bits 5..7, register r =
-// bits 8..12), so one thread issues all REGS of its loads before it uses one.
-constexpr int REGS = TILE / THREADS;
-static_assert(THREADS == 256 && REGS == 32, "the sweep layouts assume 8 warps and 32 registers");
+// i = tid | r << (5 + w) for 2^w warps (lane = tile bits 0..4, warp = the next w,
+// register r = the rest), so one thread issues all of its loads before it uses one.
 
 template <typename Real>
 __device__ __forceinline__ void rx_pair(V2<Real>& a, V2<Real>& b, Real c, Real s) {
@@ -168,10 +175,10 @@ __device__ __forceinline__ void rx_regs(V2<Real> (&v)[NR], uint32_t mask, Real c
 // take the same form x' = c x - i s y.
 template <typename Real, int NR>
 __device__ __forceinline__ void rx_lanes(V2<Real> (&v)[NR], uint32_t mask, Real c, Real s) {
-  // FP32: the lane bit is a runtime shuffle mask, so a rolled loop keeps one
-  // copy of the body (unrolled, the FP32 sweeps stall on instruction fetch;
-  // rolled they ran 4% faster). FP64 keeps it unrolled (2% faster so).
-#pragma unroll(sizeof(Real) == 4 ? 1 : 5)
+  // The lane bit is a runtime shuffle mask, so a rolled loop keeps one copy of the
+  // body (unrolled, the FP32 sweeps stall on instruction fetch, and ran 4% slower;
+  // the FP64 ones spill 2.4 KiB a thread).
+#pragma unroll 1
   for (int k = 0; k < 5; ++k) {
     if (!((mask >> k) & 1u)) continue;
 #pragma unroll
@@ -183,16 +190,23 @@ __device__ __forceinline__ void rx_lanes(V2<Real> (&v)[NR], uint32_t mask, Real 
   }
 }
 
+template <int WARPS>
 __device__ __forceinline__ double block_sum(double v, double* red) {
   for (int o = 16; o; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
   __syncthreads();
   double s = 0.0;
   if (threadIdx.x == 0)
-    for (int w = 0; w < THREADS / 32; ++w) s += red[w];
+    for (int w = 0; w < WARPS; ++w) s += red[w];
   __syncthreads();
   return s;
 }
+
+// 16 bytes global -> shared, asynchronously (L2 only).
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Tile bit of qubit q for tile kind B (c lowest qubits, then 13..n-1), or 16 + its fixed index.
 __device__ __forceinline__ uint32_t place(uint32_t kind, uint32_t n, uint32_t q) {
@@ -203,17 +217,17 @@ __device__ __forceinline__ uint32_t place(uint32_t kind, uint32_t n, uint32_t q)
 
 // One CTA per streamed set and tile kind: masks, the table T, and (kind 0) the layers' phases.
 template <typename Real>
-__global__ void __launch_bounds__(THREADS) prep_kernel(Args a, const uint32_t* __restrict__ streamed) {
+__global__ void __launch_bounds__(PREP_THREADS) prep_kernel(Args a, const uint32_t* __restrict__ streamed) {
   __shared__ uint32_t mult[2 * TILE_BITS][2 * TILE_BITS];  // edge multiplicities: tile bits, then fixed qubits
   __shared__ uint16_t tt[TILE_BITS][PLANES];
   __shared__ uint32_t used;
   const uint32_t slot = blockIdx.x >> 1, kind = blockIdx.x & 1, tid = threadIdx.x;
   const aleph_b200_qaoa_set cs = a.sets[streamed[slot]];
   const uint32_t n = cs.num_qubits, m = cs.num_edges;
-  for (uint32_t i = tid; i < 4 * TILE_BITS * TILE_BITS; i += THREADS) (&mult[0][0])[i] = 0;
+  for (uint32_t i = tid; i < 4 * TILE_BITS * TILE_BITS; i += PREP_THREADS) (&mult[0][0])[i] = 0;
   if (tid == 0) used = 1;
   __syncthreads();
-  for (uint32_t e = tid; e < m; e += THREADS) {
+  for (uint32_t e = tid; e < m; e += PREP_THREADS) {
     uint32_t u = place(kind, n, a.edges[2 * (cs.edge_offset + e)]), v = place(kind, n, a.edges[2 * (cs.edge_offset + e) + 1]);
     u = u < 16 ? u : u - 16 + TILE_BITS;
     v = v < 16 ? v : v - 16 + TILE_BITS;
@@ -222,7 +236,7 @@ __global__ void __launch_bounds__(THREADS) prep_kernel(Args a, const uint32_t* _
   }
   __syncthreads();
   Masks& M = a.masks[2 * slot + kind];
-  for (uint32_t i = tid; i < TILE_BITS * PLANES; i += THREADS) {
+  for (uint32_t i = tid; i < TILE_BITS * PLANES; i += PREP_THREADS) {
     const uint32_t q = i / PLANES, b = i % PLANES;
     uint32_t x = 0, y = 0, z = 0;
     for (uint32_t f = 0; f < TILE_BITS; ++f) {
@@ -239,7 +253,7 @@ __global__ void __launch_bounds__(THREADS) prep_kernel(Args a, const uint32_t* _
   const uint32_t np = used;
   if (tid == 0) M.planes = np;
   uint8_t* T = a.tables + (2 * (size_t)slot + kind) * TILE;
-  for (uint32_t z = tid; z < TILE; z += THREADS) {
+  for (uint32_t z = tid; z < TILE; z += PREP_THREADS) {
     uint32_t c = 0;
     for (uint32_t b = 0; b < np; ++b)
 #pragma unroll
@@ -250,7 +264,7 @@ __global__ void __launch_bounds__(THREADS) prep_kernel(Args a, const uint32_t* _
   if (kind == 0) {
     const double* gam = a.angles + (size_t)streamed[slot] * 2 * a.p;
     V2<Real>* ph = (V2<Real>*)a.phases + (size_t)slot * a.p * (MAX_EDGES + 1);
-    for (uint32_t i = tid; i < a.p * (m + 1); i += THREADS) {
+    for (uint32_t i = tid; i < a.p * (m + 1); i += PREP_THREADS) {
       const uint32_t l = i / (m + 1), k = i % (m + 1);
       double sn, cn;
       sincos(-gam[l] * ((double)m - 2.0 * (double)k), &sn, &cn);
@@ -274,7 +288,8 @@ template <typename Real>
 struct Shared {
   V2<Real> S[TILE];
   V2<Real> ph[MAX_EDGES + 1];  // cost-layer phase by cut value
-  double red[THREADS / 32];
+  double red[Cfg<Real>::THREADS / 32];
+  Real rot[4];
   alignas(16) uint8_t cutT[TILE];  // filled by 16-byte copies
   uint8_t X0[2][128], X1[2][64];
   uint32_t ch[2];
@@ -285,7 +300,11 @@ struct Shared {
 };
 
 template <typename Real>
-__global__ void __launch_bounds__(THREADS, Cfg<Real>::CTAS_PER_SM) sweep_kernel(Args a) {
+__global__ void __launch_bounds__(Cfg<Real>::THREADS, Cfg<Real>::CTAS_PER_SM) sweep_kernel(Args a) {
+  constexpr int THREADS = Cfg<Real>::THREADS, WB = Cfg<Real>::WARP_BITS;
+  constexpr bool AHEAD = sizeof(Real) == 8;
+  constexpr int R1 = 5 + WB, REGS = TILE / THREADS;           // layout 1: registers from bit R1
+  constexpr int G2 = 1 << WB, LOOPS = TILE / (32 * G2) >> WB;  // layout 2: registers from bit 5, LOOPS groups a warp
   extern __shared__ __align__(16) uint8_t qsm[];
   Shared<Real>& sh = *(Shared<Real>*)qsm;
   V2<Real>* S = sh.S;
@@ -356,7 +375,7 @@ __global__ void __launch_bounds__(THREADS, Cfg<Real>::CTAS_PER_SM) sweep_kernel(
         const double x = (double)S[i].x, y = (double)S[i].y;
         acc += (x * x + y * y) * (double)sh.cutT[i];
       }
-      const double tot = block_sum(acc, sh.red);
+      const double tot = block_sum<THREADS / 32>(acc, sh.red);
       if (tid == 0) a.out[g.set] = tot;
       continue;
     }
@@ -368,23 +387,37 @@ __global__ void __launch_bounds__(THREADS, Cfg<Real>::CTAS_PER_SM) sweep_kernel(
     const bool pre = k > 0, last = k == a.p;
     const uint32_t c = 2 * TILE_BITS - n, lowm = (1u << c) - 1;
     const uint32_t mix = kind == 0 ? TILE - 1 : (TILE - 1) & ~lowm;  // tile bits mixed by this pass
+    const uint32_t ends = pre ? mix : 0;                             // ... for the layer that ends in it
     V2<Real>* X = (V2<Real>*)a.scratch + g.state_off;
     // state offset of tile amplitude i (offsets fit in 32 bits: n <= 26)
     auto at_tile = [&](uint32_t t, uint32_t i) -> uint32_t {
       return kind == 0 ? (t << TILE_BITS) | i : (i & lowm) | t << c | (i >> c) << TILE_BITS;
     };
-    Real pc = 1, ps = 0, nc = 1, ns = 0;  // Rx of the finishing and of the starting layer
-    {
+    // offset of register bit j of layout 1; the offsets of a thread's registers are
+    // walked in Gray-code order (16 or 32 of them kept were spilled)
+    static_assert(REGS == 1 << (8 - WB), "layout 1 has the bits from R1 up in registers");
+    uint32_t step[8 - WB];
+#pragma unroll
+    for (int j = 0; j < 8 - WB; ++j) step[j] = at_tile(0, 1u << (R1 + j));
+    auto each_register = [&](uint32_t t, auto&& f) {  // f(r, its state offset)
+      uint32_t off = at_tile(t, tid);
+#pragma unroll
+      for (int q = 0; q < REGS; ++q) {
+        if (q) off ^= step[(q & 1) ? 0 : (q & 2) ? 1 : (q & 4) ? 2 : (q & 8) ? 3 : 7 - WB];
+        f(q ^ (q >> 1), off);
+      }
+    };
+    if (tid == 0) {  // Rx of the finishing and of the starting layer (in shared memory: registers are short)
       double sn, cn;
       if (pre) {
         sincos(bet[k - 1], &sn, &cn);
-        pc = (Real)cn;
-        ps = (Real)sn;
+        sh.rot[0] = (Real)cn;
+        sh.rot[1] = (Real)sn;
       }
       if (!last) {
         sincos(bet[k], &sn, &cn);
-        nc = (Real)cn;
-        ns = (Real)sn;
+        sh.rot[2] = (Real)cn;
+        sh.rot[3] = (Real)sn;
       }
     }
     {
@@ -443,66 +476,82 @@ __global__ void __launch_bounds__(THREADS, Cfg<Real>::CTAS_PER_SM) sweep_kernel(
       }
     };
     V2<Real> v[REGS];
+    // AHEAD (FP64, one CTA per SM: nothing else hides the loads): the next tile's
+    // amplitudes come straight into shared memory. In layout 1 a thread has slots of its
+    // own there, free as soon as it has read them.
+    auto fetch_tile = [&](uint32_t t) {
+      each_register(t, [&](int r, uint32_t off) { copy16_async(S + (tid | (uint32_t)r << R1), X + off); });
+    };
+    if (AHEAD && pre) fetch_tile(t0);
     for (uint32_t t = t0; t < t1; ++t) {
       const int b = t & 1;
       tile_tables(t, b);
-      if (pre) {
+      if (!pre) {
 #pragma unroll
-        for (int r = 0; r < REGS; ++r) v[r] = ld_amp<Real>(X + at_tile(t, tid | (uint32_t)r << 8));
-        rx_regs<Real, REGS>(v, mix >> 8, pc, ps);
-        rx_lanes<Real, REGS>(v, mix & 0x1fu, pc, ps);
-        __syncthreads();  // the previous tile's layout-1 reads are done
+        for (int r = 0; r < REGS; ++r) v[r] = mk<Real>(amp0, (Real)0);
+      } else if constexpr (AHEAD) {
+        copies_wait();
 #pragma unroll
-        for (int r = 0; r < REGS; ++r) S[tid | (uint32_t)r << 8] = v[r];
+        for (int r = 0; r < REGS; ++r) v[r] = S[tid | (uint32_t)r << R1];
+      } else {
+        each_register(t, [&](int r, uint32_t off) { v[r] = ld_amp<Real>(X + off); });
       }
+      rx_regs<Real, REGS>(v, ends >> R1, sh.rot[0], sh.rot[1]);
+      rx_lanes<Real, REGS>(v, ends & 0x1fu, sh.rot[0], sh.rot[1]);
+      if (!AHEAD) __syncthreads();  // the previous tile's reads are done
+#pragma unroll
+      for (int r = 0; r < REGS; ++r) S[tid | (uint32_t)r << R1] = v[r];
       __syncthreads();  // the tile and its tables are visible
-      // layout 2: lane = tile bits 0..4, register = bits 5..7, warp and loop = bits 8..12
+      // layout 2: lane = tile bits 0..4, register = the next WB, warp and loop = the rest
       const uint32_t ch = sh.ch[b];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t hi = (w | (uint32_t)j << 3) << 8;
-        V2<Real> u[8];
-        if (pre) {
+      for (int j = 0; j < LOOPS; ++j) {
+        const uint32_t hi = (w | (uint32_t)j << WB) << R1;
+        V2<Real> u[G2];
 #pragma unroll
-          for (int r = 0; r < 8; ++r) u[r] = S[hi | (uint32_t)r << 5 | lane];
-          rx_regs<Real, 8>(u, (mix >> 5) & 0x7u, pc, ps);
+        for (int r = 0; r < G2; ++r) u[r] = S[hi | (uint32_t)r << 5 | lane];
+        static_assert(!AHEAD || LOOPS == 1, "a tile read ahead takes the place of one that is in registers");
+        if (AHEAD && last) {
+          __syncthreads();
+          if (t + 1 < t1) fetch_tile(t + 1);
         }
-        uint32_t cut[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) {
+        rx_regs<Real, G2>(u, (ends >> 5) & (G2 - 1), sh.rot[0], sh.rot[1]);
+        auto cut = [&](int r) -> uint32_t {
           const uint32_t i = hi | (uint32_t)r << 5 | lane;
-          cut[r] = sh.cutT[i] + ch + sh.X0[b][i & 127] + sh.X1[b][i >> 7];
-        }
+          return sh.cutT[i] + ch + sh.X0[b][i & 127] + sh.X1[b][i >> 7];
+        };
         if (last) {
 #pragma unroll
-          for (int r = 0; r < 8; ++r) {
+          for (int r = 0; r < G2; ++r) {
             const double x = (double)u[r].x, y = (double)u[r].y;
-            acc += (x * x + y * y) * (double)cut[r];
+            acc += (x * x + y * y) * (double)cut(r);
           }
         } else {
 #pragma unroll
-          for (int r = 0; r < 8; ++r) {
-            const V2<Real> f = sh.ph[cut[r]];
-            u[r] = pre ? cmul<Real>(f, u[r]) : mk<Real>(f.x * amp0, f.y * amp0);
+          for (int r = 0; r < G2; ++r) {
+            const V2<Real> f = sh.ph[cut(r)];
+            u[r] = cmul<Real>(f, u[r]);
           }
-          rx_regs<Real, 8>(u, (mix >> 5) & 0x7u, nc, ns);
-          rx_lanes<Real, 8>(u, mix & 0x1fu, nc, ns);
+          rx_regs<Real, G2>(u, (mix >> 5) & (G2 - 1), sh.rot[2], sh.rot[3]);
+          rx_lanes<Real, G2>(u, mix & 0x1fu, sh.rot[2], sh.rot[3]);
 #pragma unroll
-          for (int r = 0; r < 8; ++r) S[hi | (uint32_t)r << 5 | lane] = u[r];
+          for (int r = 0; r < G2; ++r) S[hi | (uint32_t)r << 5 | lane] = u[r];
         }
       }
       if (!last) {
         __syncthreads();
 #pragma unroll
-        for (int r = 0; r < REGS; ++r) v[r] = S[tid | (uint32_t)r << 8];
-        rx_regs<Real, REGS>(v, mix >> 8, nc, ns);
-#pragma unroll
-        for (int r = 0; r < REGS; ++r) st_amp<Real>(X + at_tile(t, tid | (uint32_t)r << 8), v[r]);
-        if (!pre) __syncthreads();  // the next tile writes shared memory at once
+        for (int r = 0; r < REGS; ++r) v[r] = S[tid | (uint32_t)r << R1];
+        if (AHEAD && pre && t + 1 < t1) {
+          __syncwarp();  // the reads above come first
+          fetch_tile(t + 1);
+        }
+        rx_regs<Real, REGS>(v, mix >> R1, sh.rot[2], sh.rot[3]);
+        each_register(t, [&](int r, uint32_t off) { st_amp<Real>(X + off, v[r]); });
       }
     }
     if (last) {
-      const double tot = block_sum(acc, sh.red);
+      const double tot = block_sum<THREADS / 32>(acc, sh.red);
       if (tid == 0) a.partials[g.part0 + chunk] = tot;
     }
     __syncthreads();
@@ -546,8 +595,8 @@ static cudaError_t launch_qaoa_t(const qaoa::Args& a, const uint32_t* streamed, 
     if (e != cudaSuccess) return e;
     if (dev < 64) attr_devices |= 1ull << dev;
   }
-  if (n_streamed) qaoa::prep_kernel<Real><<<2 * n_streamed, qaoa::THREADS, 0, s>>>(a, streamed);
-  qaoa::sweep_kernel<Real><<<grid, qaoa::THREADS, bytes, s>>>(a);
+  if (n_streamed) qaoa::prep_kernel<Real><<<2 * n_streamed, qaoa::PREP_THREADS, 0, s>>>(a, streamed);
+  qaoa::sweep_kernel<Real><<<grid, qaoa::Cfg<Real>::THREADS, bytes, s>>>(a);
   if (n_streamed) qaoa::total_kernel<<<a.n_groups, 32, 0, s>>>(a);
   return cudaGetLastError();
 }
