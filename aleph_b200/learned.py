@@ -183,7 +183,8 @@ def candidates(precision: str) -> list[PlanChoice]:
     """The configurations the learned planner chooses among (greedy first)."""
     tile_prec = "f32" if precision == "tc32" else precision
     occs = [0] + [o for o in (2, 3, 4) if o != default_occupancy(tile_prec)]  # 0 is the default variant
-    tiles = [PlanChoice(tile_r=r, tile_occupancy=o) for r in (3, 4, 5) for o in occs]
+    # four register qubits always run wide tiles, whatever the occupancy: one candidate, not one per occupancy
+    tiles = [PlanChoice(tile_r=r, tile_occupancy=o) for r in (3, 4, 5) for o in (occs if r != 4 else [0])]
     if precision == "tc32":
         blocks = [PlanChoice(block_window_search=w) for w in (True, False)]
         return blocks + [PlanChoice(tile_r=c.tile_r, tile_occupancy=c.tile_occupancy, tensor_blocks=False)
@@ -321,9 +322,17 @@ class AutotuneResult:
     rejected: list = field(default_factory=list)
 
 
+def plan_key(n: int, flat: Flat, choice: PlanChoice, precision: str) -> tuple:
+    """What a configuration's plan is made of: equal for configurations that plan the same passes."""
+    recs = describe_plan(n, flat, choice.describe_precision(precision), tile_r=choice.tile_r,
+                         block_window_search=choice.block_window_search, tile_occupancy=choice.tile_occupancy)
+    return tuple(tuple(tuple(v) if isinstance(v, list) else v for v in r.values()) for r in recs)
+
+
 def autotune(backend: B200SvBackend, n: int, instructions, planner: LearnedPlanner | None = None, top_k: int = 2):
-    """Measure the greedy plan and the planner's top-k; keep the fastest whose
-    state matches the greedy plan's within tolerance (the greedy plan otherwise)."""
+    """Measure the greedy plan and the planner's first top_k other plans; keep the fastest
+    whose state matches the greedy plan's within tolerance (the greedy plan otherwise).
+    A configuration that plans the same passes as one already measured is not measured again."""
     flat = instructions if isinstance(instructions, Flat) else flatten(instructions)
     g_ms, _, g_psi = measure(backend, n, flat, GREEDY)
     res = AutotuneResult(GREEDY, g_ms, g_ms, {GREEDY: g_ms})
@@ -331,7 +340,14 @@ def autotune(backend: B200SvBackend, n: int, instructions, planner: LearnedPlann
         GREEDY.apply(backend)
         return res
     tol = TOLERANCE[backend.precision]
-    for s in [s for s in planner.score(n, flat, backend.precision) if s.choice != GREEDY][:top_k]:
+    plans = {plan_key(n, flat, GREEDY, backend.precision)}
+    for s in planner.score(n, flat, backend.precision):
+        key = plan_key(n, flat, s.choice, backend.precision)
+        if key in plans:
+            continue
+        if len(plans) > top_k:
+            break
+        plans.add(key)
         try:
             ms, _, psi = measure(backend, n, flat, s.choice)
         except BackendError as e:
@@ -389,9 +405,8 @@ def large_training_circuits(precision: str, seed: int = 7):
 
 
 def large_choices(precision: str) -> list[PlanChoice]:
-    """The candidates sampled at the largest sizes: the greedy configuration
-    and its nearest neighbours (4 and 3 register qubits, the other occupancy
-    variants at 4)."""
+    """The candidates sampled at the largest sizes: the greedy configuration and
+    its nearest neighbours (four register qubits; FP32: the occupancy variants)."""
     c = candidates(precision)
     if precision == "tc32":
         return c[:2] + [x for x in c[2:] if x.tile_r == 5][:2]
