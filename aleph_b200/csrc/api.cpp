@@ -1548,6 +1548,17 @@ static void count_guard_band(aleph_b200_handle* h, uint32_t n, const int32_t* st
   if (n > kExactCumulativeMaxN) h->stats.guard_band_inexact += (uint32_t)status[2];
 }
 
+// status[0] of a sampling call: the norm check, or a chunk outside its group's margin
+// (which the groups' own checks rule out).
+static int sample_failed(aleph_b200_handle* h, int32_t status) {
+  if (status != ALEPH_B200_INVALID_STATE)
+    return set_error(h, status, "device operation failed: alias table chunk outside its group");
+  aleph_b200_error_info e{};
+  e.status = status;
+  std::snprintf(e.kind, sizeof(e.kind), "state norm2 deviates from 1");
+  return report(h, e);
+}
+
 int aleph_b200_sample(aleph_b200_handle* h, aleph_b200_state* st, uint32_t shots, int mode, const void* variates,
                       uint64_t* out) {
   if (!h || !st || (shots && (!variates || !out))) return ALEPH_B200_INVALID_ARGUMENT;
@@ -1587,10 +1598,7 @@ int aleph_b200_sample(aleph_b200_handle* h, aleph_b200_state* st, uint32_t shots
   CK(cudaStreamSynchronize(h->stream), "stream synchronize");
   if (mode == ALEPH_B200_SAMPLE_CUMULATIVE) count_guard_band(h, st->n, status);
   if (status[0]) {
-    aleph_b200_error_info e{};
-    e.status = status[0];
-    std::snprintf(e.kind, sizeof(e.kind), "state norm2 deviates from 1");
-    return report(h, e);
+    return sample_failed(h, status[0]);
   }
   return ALEPH_B200_OK;
 }
@@ -1668,10 +1676,7 @@ int aleph_b200_sample_cumulative_noalloc(aleph_b200_handle* h, aleph_b200_state*
   CK(cudaStreamSynchronize(h->stream), "stream synchronize");
   count_guard_band(h, st->n, status);
   if (status[0]) {
-    aleph_b200_error_info e{};
-    e.status = status[0];
-    std::snprintf(e.kind, sizeof(e.kind), "state norm2 deviates from 1");
-    return report(h, e);
+    return sample_failed(h, status[0]);
   }
   return ALEPH_B200_OK;
 }
