@@ -7,14 +7,21 @@
 // (Gate::matrix, crates/aleph-core/src/gate/kinds.rs:213-400) and the
 // unitarity check (validation.rs:25-51, AMPLITUDE_TOL = 1e-10).
 //
-// Planning: the gate list is cut into HBM passes. A warp-tile pass owns
-// qubits 0..4 plus R "register" qubits; the planner walks the pending gates
-// in order and takes every gate that (a) commutes past all gates it defers
-// and (b) acts non-diagonally only on tile qubits — diagonal gates (CZ,
-// phases, DiagonalPhase) and controls may sit on any qubit. This is the
+// Planning: the gate list is cut into HBM passes. First it is rewritten: gate
+// sequences on a few qubits that multiply out to a diagonal become corner phases
+// (diagonal_cores), phases on the same qubits join and cancel (cancel_phases), and the
+// gates on a pair of qubits become one 4x4 (fuse_pairs). Then passes take gates:
+// * wide-tile passes (the default from n = 12): qubits 0..3 and eight more, in phases
+//   of five register qubits;
+// * warp-tile passes (short lists that they run faster, changed tuning keys, smaller
+//   states): qubits 0..4 plus R register qubits;
+// * tensor-core blocks (TC32): six qubits, one dense 64x64 matrix.
+// Each walks the pending gates in order and takes every gate that (a) commutes past
+// all gates it defers and (b) acts non-diagonally only on its qubits; diagonal
+// gates (CZ, phases, DiagonalPhase) and controls may sit on any qubit. This is the
 // greedy open-block idea of FuseKq (crates/aleph-ir/src/passes/fuse_kq.rs:144-400)
-// applied to cache tiles instead of matrices: no matrix is ever formed, the
-// gates run in registers one after the other.
+// applied to tiles instead of matrices. A state of at most 12 qubits is one
+// shared-memory pass.
 
 #include <algorithm>
 #include <deque>
