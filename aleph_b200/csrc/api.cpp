@@ -304,7 +304,7 @@ int execute(aleph_b200_handle* h, aleph_b200_state* st, const Plan& P, const dou
         const size_t next = (size_t)ps.tile.op_begin + ps.tile.op_count;
         const uint32_t coef_end = next < P.ops.size() ? P.ops[next].coef : (uint32_t)(P.coef.size() / 2);
         e = launch_smem_pass(st->amps, st->precision, st->n, d.ops + ps.tile.op_begin, ps.tile.op_count, d.coef,
-                             coef_end, d.poly, h->stream);
+                             coef_end, ps.has_poly, d.poly, h->stream);
         h->stats.passes++;
         h->stats.algorithmic_bytes += 2 * len * bpa;
         break;

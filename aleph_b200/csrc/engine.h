@@ -130,6 +130,7 @@ struct Pass {
   WidePass wide;       // PASS_WIDE
   BlockPass block;     // PASS_BLOCK
   uint32_t qubit;      // PASS_MEASURE
+  bool has_poly = false;  // PASS_SMEM: the list has DiagonalPhase ops
   // PASS_PERMUTE: an involution of the qubit positions; the pass maps
   // psi(j) -> psi(sigma(j)), sigma(j) moving bit q of j to position sigma[q]
   uint8_t sigma[kMaxQubits];
@@ -265,7 +266,7 @@ cudaError_t launch_wide_pass(void* amps, int precision, const WidePass& p, const
 // Fills a phase's layout (ts, rs, tq, rq) for the tile bits `regs` in registers.
 void wide_layout(const uint8_t* tile_qubits, uint32_t R, uint32_t regs, bool io, bool f64, WidePhase* P);
 cudaError_t launch_smem_pass(void* amps, int precision, uint32_t n, const Op* ops, uint32_t op_count,
-                             const void* coef, uint32_t coef_end, PolyTables poly, cudaStream_t s);
+                             const void* coef, uint32_t coef_end, bool has_poly, PolyTables poly, cudaStream_t s);
 cudaError_t launch_kq_pass(void* amps, int precision, uint32_t n, const Op* op_dev, const Op& op_host,
                            const void* coef, cudaStream_t s);
 cudaError_t launch_block_pass(void* amps, const BlockPass& p, const uint8_t* images, const Op* ops,

@@ -133,7 +133,8 @@ __device__ __forceinline__ void smem_diag_run(V2<Real>* sm, uint32_t len, const 
         }
       } else {
 #pragma unroll
-        for (int k = 0; k < PER; ++k) a[k] = apply_diag_op<Real>(ops[x], a[k], at[k], coef, poly);
+        for (int k = 0; k < PER; ++k)
+          if (at[k] < len) a[k] = apply_diag_op<Real>(ops[x], a[k], at[k], coef, poly);
       }
     }
 #pragma unroll
@@ -186,7 +187,7 @@ __global__ void __launch_bounds__(512) smem_kernel(V2<Real>* __restrict__ amps, 
 
 template <typename Real>
 static cudaError_t launch_smem_t(V2<Real>* amps, uint32_t n, const Op* ops, uint32_t op_count, const V2<Real>* coef,
-                                 uint32_t coef_end, PolyTables poly, cudaStream_t s) {
+                                 uint32_t coef_end, bool has_poly, PolyTables poly, cudaStream_t s) {
   const size_t bytes = (((size_t)1 << n) + SMEM_COEFS) * sizeof(V2<Real>);
   static uint64_t ready = 0;  // devices with the shared-memory opt-in
   int dev = 0;
@@ -199,18 +200,20 @@ static cudaError_t launch_smem_t(V2<Real>* amps, uint32_t n, const Op* ops, uint
     if (dev < 64) ready |= 1ull << dev;
   }
   // a quartet per thread: fewer warps than that idle the SM, more only slow the barriers
-  const uint32_t quartets = n > 2 ? 1u << (n - 2) : 1u;
+  // (a DiagonalPhase's terms and sine are long enough to want a thread per amplitude:
+  // 20 terms twice at n = 10 take 96 us on 256 threads and 78 on 512)
+  const uint32_t quartets = has_poly ? 1u << n : n > 2 ? 1u << (n - 2) : 1u;
   const uint32_t threads = quartets < 64 ? 64 : quartets > 512 ? 512 : quartets;
   smem_kernel<Real><<<1, threads, bytes, s>>>(amps, n, ops, op_count, coef, coef_end, poly);
   return cudaGetLastError();
 }
 
 cudaError_t launch_smem_pass(void* amps, int precision, uint32_t n, const Op* ops, uint32_t op_count,
-                             const void* coef, uint32_t coef_end, PolyTables poly, cudaStream_t s) {
+                             const void* coef, uint32_t coef_end, bool has_poly, PolyTables poly, cudaStream_t s) {
   if (n > 12) return cudaErrorInvalidValue;
   if (precision == ALEPH_B200_F64)
-    return launch_smem_t<double>((double2*)amps, n, ops, op_count, (const double2*)coef, coef_end, poly, s);
-  return launch_smem_t<float>((float2*)amps, n, ops, op_count, (const float2*)coef, coef_end, poly, s);
+    return launch_smem_t<double>((double2*)amps, n, ops, op_count, (const double2*)coef, coef_end, has_poly, poly, s);
+  return launch_smem_t<float>((float2*)amps, n, ops, op_count, (const float2*)coef, coef_end, has_poly, poly, s);
 }
 
 // ---- dense k-qubit op on arbitrary qubits (UnitaryKq, k = 3..5) --------------

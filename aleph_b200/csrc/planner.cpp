@@ -2042,6 +2042,7 @@ int build_plan(const std::vector<Lowered>& ops, uint32_t n, bool f64, const Plan
       for (const Lowered* L : list) {
         Op op = L->op;
         if ((op.type == OP_1Q || op.type == OP_2Q) && real_matrix(*L)) op.dsrc = WIDE_REAL;
+        ps.has_poly = ps.has_poly || op.type == OP_POLY;
         append_op(P, *L, op);
       }
       ps.tile.op_count = (uint32_t)P->ops.size() - ps.tile.op_begin;

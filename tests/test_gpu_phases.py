@@ -71,3 +71,19 @@ def test_long_runs_of_small_rotations_add_up(angle, count, n):
                   C.GateInstance(C.Phase(angle), [2])]
     insts += [C.GateInstance(C.H(), [q]) for q in range(3)]
     check(n, insts, "f64")
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32"])
+@pytest.mark.parametrize("n", [1, 2, 5, 6, 9, 10, 12, 14])
+def test_phase_polynomials_between_gates(n, precision):
+    # a thread per amplitude in shared-memory passes, more threads than amplitudes below six qubits
+    rng = np.random.default_rng(n)
+
+    def poly():
+        masks = [tuple(int(m) for m in rng.integers(1, 1 << n, int(rng.integers(1, 3)))) for _ in range(12)]
+        return C.DiagonalPhase(n, [C.PhaseTerm(m, float(rng.uniform(-3, 3))) for m in masks])
+
+    insts = [C.GateInstance(C.H(), [q]) for q in range(n)]
+    insts += [poly(), C.GateInstance(C.T(), [0]), poly()]
+    insts += [C.GateInstance(C.U3(0.3, 0.4 + q, -1.1), [q]) for q in range(n)] + [poly()]
+    check(n, insts, precision)
