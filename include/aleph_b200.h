@@ -213,7 +213,9 @@ int aleph_b200_apply_gate_stream(aleph_b200_handle* h, aleph_b200_state* st, con
  * uploaded to device memory at the first execute and stay resident.
  * aleph_b200_execute then applies the plan to `st` (same qubit count) with
  * the semantics of aleph_b200_apply_gate_stream. A plan belongs to the handle
- * that compiled it; calls on one handle are stream-ordered. */
+ * that compiled it; calls on one handle are stream-ordered. The state may be of
+ * either precision: a plan for the other one than the handle's is made when such
+ * a state first comes. */
 typedef struct aleph_b200_plan aleph_b200_plan;
 int aleph_b200_compile(aleph_b200_handle* h, uint32_t num_qubits, const aleph_b200_instr* instrs, uint64_t count,
                        const aleph_b200_pools* pools, aleph_b200_plan** out);
@@ -356,7 +358,8 @@ int aleph_b200_last_error_info(const aleph_b200_handle* h, aleph_b200_error_info
 
 /* ---- planner tuning (the autotuner's knobs) ----
  * keys: "tile_r" (register qubits per thread, 1..5; 5 and 4 choose wide tile
- * passes for n >= 12 where the keys below leave them on, else warp tiles),
+ * passes for n >= 12 where the keys below leave them on, else warp tiles; with 5,
+ * short gate lists take warp tiles where those are the faster),
  * "smem_max_n" (states with n <= this run as one shared-memory pass, 0..12),
  * "record_passes" (0/1: time every pass of later gate streams with CUDA events),
  * "relabel_swaps" (0/1, default 1: an uncontrolled SWAP of a state larger

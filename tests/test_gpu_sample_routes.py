@@ -89,3 +89,16 @@ def test_many_shots_of_a_small_state():
     be, st, psi = on_device("scrambled", 7, "f64", 5)
     words = np.random.default_rng(1).integers(0, 1 << 64, 100_003, dtype=np.uint64)
     assert np.array_equal(be.sample(st, words.size, variates=words, mode="alias"), oracle.sample_alias(psi, words))
+
+
+@pytest.mark.parametrize("n", [19, 21, 22])
+def test_cumulative_draws_up_to_and_above_a_segment_per_chunk(n):
+    # n = 21: 1024 blocks and chunks, one kernel scans them and nothing is composed
+    be, st, psi = on_device("scrambled", n, "f64", n)
+    sums = np.add.accumulate(psi.real * psi.real + psi.imag * psi.imag)
+    rng = np.random.default_rng(n)
+    edge = sums[rng.integers(0, psi.size, 60)] / sums[-1]
+    u = np.concatenate([edge, np.nextafter(edge, 0), np.nextafter(edge, 2), [0.0, 1 - 2.0 ** -53]]).clip(0, 1 - 2.0 ** -53)
+    want = np.searchsorted(sums, u * sums[-1], side="right")
+    want = np.where(want < psi.size, want, np.flatnonzero(psi)[-1]).astype(np.uint64)
+    assert np.array_equal(be.sample(st, u.size, variates=u, mode="cumulative"), want)
