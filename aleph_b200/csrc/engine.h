@@ -158,6 +158,7 @@ struct Lowered {
   std::vector<uint8_t> sigma;
   uint32_t gates = 0;
   bool absorbed = false;  // its gates are counted by another op
+  bool given = false;     // entries that are the caller's own, not a named gate's
   // OP_POLY terms (DiagonalPhase): angle, condition count, condition masks
   std::vector<double> poly_angle;
   std::vector<uint32_t> poly_cnt;
