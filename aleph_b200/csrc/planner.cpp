@@ -382,6 +382,7 @@ int lower_gate(const aleph_b200_instr& g, uint32_t n, const double* pool, uint64
     set_kind(e, gate_name(g.kind));
     return fail(e, ALEPH_B200_UNSUPPORTED_GATE);
   }
+  L->given = g.kind >= ALEPH_GATE_UNITARY1Q && g.kind <= ALEPH_GATE_UNITARY2QDIAG;
   if (g.kind == ALEPH_GATE_UNITARYKQ) {
     // validate_unitary_kq, crates/aleph-sv/src/validation.rs:113-155
     const uint32_t k = g.aux;
@@ -435,7 +436,6 @@ int lower_gate(const aleph_b200_instr& g, uint32_t n, const double* pool, uint64
   Cx flat[64];
   for (int i = 0; i < dim; ++i)
     for (int j = 0; j < dim; ++j) flat[i * dim + j] = m[i][j];
-  L->given = g.kind >= ALEPH_GATE_UNITARY1Q && g.kind <= ALEPH_GATE_UNITARY2QDIAG;
   if (tiled) {
     // TiledBlock gates: the tile kernels take 2x2 and 4x4 matrices; an 8x8
     // is UnsupportedGate, and no unitarity check is made (backend.rs:265-299)

@@ -37,6 +37,23 @@ def test_products_of_named_gates_are_no_worse_than_their_gates(n):
 
 
 @pytest.mark.parametrize("n", [6, 10, 14])
+def test_a_given_two_qubit_matrix_keeps_its_rows(n):
+    # as a Unitary2q and as a UnitaryKq on two qubits, beside named gates
+    m = np.eye(4, dtype=complex)[[0, 1, 3, 2]] * (1 + 2.0 ** -51)
+    for gate in (C.Unitary2q(m), C.UnitaryKq(m)):
+        insts = []
+        for layer in range(LAYERS):
+            insts += [C.GateInstance(gate, [q, q + 1]) for q in range(0, n, 2)]
+            insts += [C.GateInstance(C.S(), [q]) for q in range(0, n, 2)]
+        be = B200SvBackend(seed=0, precision="f64")
+        st = be.allocate(n)
+        be.apply_stream(st, insts)
+        gates = LAYERS * n // 2
+        want = gates * (float(np.longdouble(1 + 2.0 ** -51) ** 2 - 1))
+        assert abs(np.linalg.norm(be.statevector(st)) ** 2 - 1 - want) <= gates * 2.0 ** -52
+
+
+@pytest.mark.parametrize("n", [6, 10, 14])
 def test_products_of_given_matrices_keep_their_rows(n):
     # rows too long by 4 ulp; a product's entries and the arithmetic round by 2^-53 each
     r = np.sqrt(0.5) * (1 + 2.0 ** -50)
